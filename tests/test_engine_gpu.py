@@ -156,3 +156,22 @@ def test_native_layer_entry_same_logits_as_per_op_path():
     assert all(eq for *_, eq in seen), seen
     assert all(n >= 8 * cfg.num_layers for _, _, n, _ in seen)       # the launches are counted
     assert ops.read_status() == 0
+
+
+def test_async_chunks_of_a_long_prompt_behind_a_busy_gpu():
+    """Chunks that sample nothing are not waited for, so the host runs ahead of the GPU: the inputs of a step must still
+    be in its staging buffer when the copy of them runs."""
+    cfg = _cfg()
+    prompt = _prompts(cfg, (600,))[0]
+    got = []
+    for mode in (False, True):
+        llm = LLM(EngineArgs(model_config=cfg, device="cuda", block_size=16, num_blocks=200, max_model_len=640, max_num_seqs=2,
+                             max_num_batched_tokens=64, async_scheduling=mode, enable_prefix_caching=False, max_score_rows=2))
+        llm.score_positions("a", [len(prompt) - 1])
+        torch.cuda._sleep(200_000_000)                    # about 0.1 s of work ahead of the first copy
+        llm.add_request(prompt, SamplingParams(temperature=0.0, max_tokens=2, ignore_eos=True), request_id="a")
+        while llm.has_unfinished_requests():
+            llm.step()
+        got.append(llm.take_scores()["a"][0][1])
+    assert ops.read_status() == 0
+    assert torch.equal(got[0], got[1])

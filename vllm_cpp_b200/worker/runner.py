@@ -102,6 +102,9 @@ class ModelRunner(E.ModelRunnerBase):
         self.host_bufs = [torch.zeros(nbytes, dtype=torch.uint8, pin_memory=self.is_cuda)
                           for _ in range(2 if async_mode else 1)]
         self.host_buf = self.host_bufs[0]
+        # recorded behind the copy out of each staging buffer: nothing else says that the copy has run (a
+        # step that samples nothing, such as a chunk of a long prompt, is not waited for)
+        self._staged = [torch.cuda.Event() for _ in self.host_bufs] if self.is_cuda else []
         self._step_no = 0
         self.dev_buf = torch.zeros(nbytes, dtype=torch.uint8, device=self.device)
         self.batch = E.InputBatch(max_num_seqs, max_model_len, self.max_tokens,
@@ -312,6 +315,14 @@ class ModelRunner(E.ModelRunnerBase):
     # ------------------------------------------------------------------ step
     offload = None   # KVOffloadWorker when KV offloading is configured
 
+    def _next_staging(self) -> None:
+        """Turns to the next staging buffer, once the copy of the step that filled it last has run."""
+        self._step_no += 1
+        k = self._step_no % len(self.host_bufs)
+        if self.is_cuda:
+            self._staged[k].synchronize()
+        self.host_buf, self.host_views = self.host_bufs[k], self.host_views_all[k]
+
     def execute_model(self, so) -> None:
         self.batch.update_states(so)
         if self.offload is not None:
@@ -319,9 +330,7 @@ class ModelRunner(E.ModelRunnerBase):
         if so.total_num_scheduled_tokens == 0:
             self._info = None
             return
-        self._step_no += 1
-        k = self._step_no % len(self.host_bufs)
-        self.host_buf, self.host_views = self.host_bufs[k], self.host_views_all[k]
+        self._next_staging()
         info = self.batch.prepare(so, self.layout, self.host_buf.data_ptr(), self.async_mode)
         self._info = info
         self._scheduled_spec = dict(so.scheduled_spec_decode_tokens) if self.spec else {}
@@ -367,6 +376,7 @@ class ModelRunner(E.ModelRunnerBase):
             self._capture(pad)                 # before this step's inputs reach the device buffer
         if self.is_cuda:
             self.dev_buf.copy_(self.host_buf, non_blocking=True)
+            self._staged[self._step_no % len(self.host_bufs)].record()
         else:
             self.dev_buf.copy_(self.host_buf)
         self.h2d_bytes += nbytes
@@ -524,9 +534,7 @@ class ModelRunner(E.ModelRunnerBase):
                 if msg["kind"] != "step":
                     raise RuntimeError(f"worker rank: unexpected message {msg['kind']!r}")
                 info = types.SimpleNamespace(**msg["info"])
-                self._step_no += 1
-                k = self._step_no % len(self.host_bufs)
-                self.host_buf, self.host_views = self.host_bufs[k], self.host_views_all[k]
+                self._next_staging()
                 self.host_buf.numpy()[:] = np.frombuffer(msg["buf"], dtype=np.uint8)
                 self._info = info
                 self._launch_step(info, msg["pad"], msg["plain"])
