@@ -245,89 +245,212 @@ __device__ __forceinline__ float fkey_inv(uint32_t k) {
   uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
   return __uint_as_float(u);
 }
-// One block per row. top-k: bitwise radix select of the k-th largest key (count based).
-// top-p: bisection on the key for the largest threshold whose kept mass is >= p, mass summed
-// with a fixed-order block reduction. Ties at the threshold are all kept (same as the
-// sort-based rule for distinct logits).
-__global__ void __launch_bounds__(kSB)
+// A row belongs to a cluster of kRowCtas CTAs: one SM alone reads a vocabulary of 150000 logits at the pace of its own
+// loads. Each CTA keeps its slice in shared memory (rows too long for that are read from memory again), sums are taken
+// within the CTA in a fixed order and then over the cluster in the order of its CTAs.
+static constexpr int kRowCtas = 8, kRowThreads = 512;
+static constexpr int kMostStaged = 200 * 1024;      // bytes of a slice in shared memory
+
+struct RowSlice {
+  float* x;         // the slice in memory
+  const float* v;   // where to read it (shared memory, or x)
+  int lo, n;        // first column, columns
+};
+__device__ __forceinline__ int row_slice_cols(int V) { return ((V + kRowCtas - 1) / kRowCtas + 3) & ~3; }
+// Loads this CTA's slice of its row (blockIdx.x / kRowCtas); out-of-place callers pass x as const.
+__device__ __forceinline__ RowSlice load_row_slice(float* row, int V, float* stage) {
+  const int per = row_slice_cols(V), rank = (int)cluster_ctarank();
+  RowSlice s;
+  s.lo = min(V, rank * per);
+  s.n = min(V, s.lo + per) - s.lo;
+  s.x = row + s.lo;
+  s.v = s.x;
+  if (per * 4 <= kMostStaged) {
+    if (!(reinterpret_cast<uintptr_t>(s.x) & 15)) {
+      const int n4 = s.n & ~3;
+#pragma unroll 4
+      for (int i = threadIdx.x * 4; i < n4; i += kRowThreads * 4)
+        *reinterpret_cast<float4*>(stage + i) = *reinterpret_cast<const float4*>(s.x + i);
+      for (int i = n4 + threadIdx.x; i < s.n; i += kRowThreads) stage[i] = s.x[i];
+    } else {
+#pragma unroll 4
+      for (int i = threadIdx.x; i < s.n; i += kRowThreads) stage[i] = s.x[i];
+    }
+    s.v = stage;
+    __syncthreads();
+  }
+  return s;
+}
+// Exchange of one value of W words per CTA; two buffers in turn, so that one cluster barrier a call is enough.
+template <int W>
+struct RowExchange {
+  float slot[2][W];
+};
+template <int W>
+__device__ __forceinline__ void row_gather(RowExchange<W>& ex, int turn, const float (&mine)[W], float (&all)[kRowCtas][W]) {
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int w = 0; w < W; ++w) ex.slot[turn & 1][w] = mine[w];
+  cluster_sync_all();
+  const uint32_t a = smem_u32(&ex.slot[turn & 1][0]);
+#pragma unroll
+  for (int r = 0; r < kRowCtas; ++r)
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(all[r][w]) : "r"(mapa_u32(a, r) + 4 * w) : "memory");
+}
+// Sums of W numbers a thread over the whole row (counts stay exact up to 2^24).
+template <int W>
+__device__ __forceinline__ void row_sum(RowExchange<W>& ex, int turn, float (&v)[W], float (&sh)[kRowThreads / 32][W]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int w = 0; w < W; ++w)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[w] += __shfl_xor_sync(0xffffffffu, v[w], o);
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int w = 0; w < W; ++w) sh[warp][w] = v[w];
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    float r = lane < kRowThreads / 32 ? sh[lane][w] : 0.f;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    v[w] = __shfl_sync(0xffffffffu, r, 0);
+  }
+  float all[kRowCtas][W];
+  row_gather<W>(ex, turn, v, all);
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    v[w] = all[0][w];
+#pragma unroll
+    for (int r = 1; r < kRowCtas; ++r) v[w] += all[r][w];
+  }
+}
+__device__ __forceinline__ float row_max(RowExchange<1>& ex, int turn, float v, float* sh) {
+  const float mine[1] = {block_reduce_max(v, sh)};
+  float all[kRowCtas][1];
+  row_gather<1>(ex, turn, mine, all);
+  v = all[0][0];
+#pragma unroll
+  for (int r = 1; r < kRowCtas; ++r) v = fmaxf(v, all[r][0]);
+  return v;
+}
+
+// One cluster per row. top-k: radix select of the k-th largest key, two bits a pass (count based). top-p: the same search
+// for the largest threshold whose kept mass is >= p. Ties at the threshold are all kept (same as the sort-based rule for
+// distinct logits). Bound by the passes' barriers and shared-memory reads, about 2 us a pass, at most 32 passes: 40 rows of
+// 151936 with k = 50, p = 0.95 took 7717 us with a block of 256 threads per row that read the row from L2 for every bit.
+__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
     top_k_top_p_kernel(float* logits, int ld, int V, const int* __restrict__ top_k,
                        const float* __restrict__ top_p) {
-  __shared__ float shf[32];
-  __shared__ int shi[32];
-  const int row = blockIdx.x;
-  float* x = logits + (size_t)row * ld;
+  extern __shared__ float4 stage_raw[];
+  __shared__ RowExchange<1> ex1;
+  __shared__ RowExchange<3> ex3;
+  __shared__ float sh1[kRowThreads / 32][1], sh3[kRowThreads / 32][3], shm[32];
+  const int row = blockIdx.x / kRowCtas;
   const int k = top_k ? top_k[row] : 0;
   const float pth = top_p ? top_p[row] : 1.f;
   const bool do_k = (k > 0 && k < V);
   const bool do_p = (pth < 1.f);
-  if (!do_k && !do_p) return;
+  if (!do_k && !do_p) return;                          // (the whole cluster)
+  const RowSlice s = load_row_slice(logits + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
   uint32_t thr_key = 0;
+  int turn = 0;
   if (do_k) {
     // find the largest key T such that count(key >= T) >= k
     uint32_t prefix = 0;
-    for (int bit = 31; bit >= 0; --bit) {
-      const uint32_t cand = prefix | (1u << bit);
-      int c = 0;
-      for (int i = threadIdx.x; i < V; i += blockDim.x) c += (fkey(x[i]) >= cand);
-      c = block_reduce_sum_int(c, shi);
-      if (c >= k) prefix = cand;
+    for (int bit = 30; bit >= 0; bit -= 2, ++turn) {
+      const uint32_t c1 = prefix | (1u << bit), c2 = prefix | (2u << bit), c3 = prefix | (3u << bit);
+      int n1 = 0, n2 = 0, n3 = 0;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+        const uint32_t kk = fkey(s.v[i]);
+        n1 += kk >= c1; n2 += kk >= c2; n3 += kk >= c3;
+      }
+      float c[3] = {(float)n1, (float)n2, (float)n3};
+      row_sum<3>(ex3, turn, c, sh3);
+      if (c[2] >= (float)k) prefix = c3;
+      else if (c[1] >= (float)k) prefix = c2;
+      else if (c[0] >= (float)k) prefix = c1;
     }
     thr_key = prefix;
   }
   if (do_p) {
     float mx = -FLT_MAX;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float v = x[i];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+      const float v = s.v[i];
       if (fkey(v) >= thr_key) mx = fmaxf(mx, v);
     }
-    mx = block_reduce_max(mx, shf);
-    float tot = 0.f;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float v = x[i];
-      if (fkey(v) >= thr_key) tot += __expf(v - mx);
+    mx = row_max(ex1, 0, mx, shm);
+    float tot[1] = {0.f};
+#pragma unroll 4
+    for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+      const float v = s.v[i];
+      if (fkey(v) >= thr_key) tot[0] += __expf(v - mx);
     }
-    tot = block_reduce_sum(tot, shf);
-    const float need = pth * tot;
+    row_sum<1>(ex1, 1, tot, sh1);
+    const float need = pth * tot[0];
     // largest key T (>= thr_key) with mass(key >= T) >= need
     uint32_t prefix = 0;
-    for (int bit = 31; bit >= 0; --bit) {
-      const uint32_t cand = prefix | (1u << bit);
-      float s = 0.f;
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float v = x[i];
+    for (int bit = 30; bit >= 0; bit -= 2, ++turn) {
+      const uint32_t c1 = prefix | (1u << bit), c2 = prefix | (2u << bit), c3 = prefix | (3u << bit);
+      const uint32_t least = c1 > thr_key ? c1 : thr_key;
+      float m[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+        const float v = s.v[i];
         const uint32_t kk = fkey(v);
-        if (kk >= cand && kk >= thr_key) s += __expf(v - mx);
+        if (kk >= least) {
+          const float e = __expf(v - mx);
+          m[0] += e;
+          m[1] += kk >= c2 ? e : 0.f;
+          m[2] += kk >= c3 ? e : 0.f;
+        }
       }
-      s = block_reduce_sum(s, shf);
-      if (s >= need) prefix = cand;
+      row_sum<3>(ex3, turn, m, sh3);
+      if (m[2] >= need) prefix = c3;
+      else if (m[1] >= need) prefix = c2;
+      else if (m[0] >= need) prefix = c1;
     }
     if (prefix > thr_key) thr_key = prefix;
   }
-  for (int i = threadIdx.x; i < V; i += blockDim.x)
-    if (fkey(x[i]) < thr_key) x[i] = -INFINITY;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < s.n; i += kRowThreads)
+    if (fkey(s.v[i]) < thr_key) s.x[i] = -INFINITY;
+  cluster_sync_all();                                  // nobody reads this CTA's sums any more
 }
 
 // ---- softmax / log-softmax (out may alias in) ----
-__global__ void __launch_bounds__(kSB)
-    softmax_kernel(const float* __restrict__ logits, int ld, float* out, int ldo, int V,
-                   int log_mode) {
-  __shared__ float sh[32];
-  const int row = blockIdx.x;
-  const float* x = logits + (size_t)row * ld;
-  float* o = out + (size_t)row * ldo;
+// One cluster per row (331 us for 40 rows of 151936 with a block of 256 threads per row).
+__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
+    softmax_kernel(const float* logits, int ld, float* out, int ldo, int V, int log_mode) {
+  extern __shared__ float4 stage_raw[];
+  __shared__ RowExchange<1> ex;
+  __shared__ float sh[kRowThreads / 32][1], shm[32];
+  const int row = blockIdx.x / kRowCtas;
+  const RowSlice s = load_row_slice(const_cast<float*>(logits) + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
+  float* o = out + (size_t)row * ldo + s.lo;
   float mx = -FLT_MAX;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, x[i]);
-  mx = block_reduce_max(mx, sh);
-  float s = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) s += __expf(x[i] - mx);
-  s = block_reduce_sum(s, sh);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < s.n; i += kRowThreads) mx = fmaxf(mx, s.v[i]);
+  mx = row_max(ex, 0, mx, shm);
+  float sum[1] = {0.f};
+#pragma unroll 4
+  for (int i = threadIdx.x; i < s.n; i += kRowThreads) sum[0] += __expf(s.v[i] - mx);
+  row_sum<1>(ex, 1, sum, sh);
   if (log_mode) {
-    const float lz = mx + logf(s);
-    for (int i = threadIdx.x; i < V; i += blockDim.x) o[i] = x[i] - lz;
+    const float lz = mx + logf(sum[0]);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < s.n; i += kRowThreads) o[i] = s.v[i] - lz;
   } else {
-    const float inv = 1.f / s;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) o[i] = __expf(x[i] - mx) * inv;
+    const float inv = 1.f / sum[0];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < s.n; i += kRowThreads) o[i] = __expf(s.v[i] - mx) * inv;
   }
+  cluster_sync_all();
 }
 
 // ---- seeded exponential-race sample: argmax_i p_i / (-log u_i) ----
@@ -343,21 +466,32 @@ __device__ __forceinline__ float race_key(float prob, uint64_t seed, uint64_t st
   const float e = (float)(-log(u));
   return prob / e;
 }
-__global__ void __launch_bounds__(kSB)
+// One cluster per row (117 us for 40 rows of 151936 with a block of 256 threads per row).
+__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
     random_sample_kernel(const float* __restrict__ probs, int ld, int V,
                          const uint64_t* __restrict__ seeds, const uint64_t* __restrict__ steps,
                          int64_t* out) {
   __shared__ ArgPair sh[32];
-  const int row = blockIdx.x;
+  __shared__ RowExchange<2> ex;
+  const int row = blockIdx.x / kRowCtas, per = row_slice_cols(V), lo = min(V, (int)cluster_ctarank() * per), hi = min(V, lo + per);
   const float* x = probs + (size_t)row * ld;
   const uint64_t seed = seeds[row], step = steps[row];
   ArgPair a{-FLT_MAX, 0x7fffffff};
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
+#pragma unroll 4
+  for (int i = lo + threadIdx.x; i < hi; i += kRowThreads) {
     const float pr = x[i];
     if (pr > 0.f) a = arg_better(a, ArgPair{race_key(pr, seed, step, i), i});
   }
   a = block_argmax(a, sh);
-  if (threadIdx.x == 0) out[row] = (a.i >= V || a.i < 0) ? 0 : a.i;
+  const float mine[2] = {a.v, __int_as_float(a.i)};
+  float all[kRowCtas][2];
+  row_gather<2>(ex, 0, mine, all);
+  if (cluster_ctarank() == 0 && threadIdx.x == 0) {
+    a = ArgPair{all[0][0], __float_as_int(all[0][1])};
+    for (int r = 1; r < kRowCtas; ++r) a = arg_better(a, ArgPair{all[r][0], __float_as_int(all[r][1])});
+    out[row] = (a.i >= V || a.i < 0) ? 0 : a.i;
+  }
+  cluster_sync_all();
 }
 
 // out[row] = is_greedy ? greedy[row] : random[row]
@@ -420,6 +554,11 @@ __global__ void scatter_sampled_kernel(int64_t* last_sampled, const int* __restr
                                        const int64_t* __restrict__ sampled, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && row_of[i] >= 0) last_sampled[row_of[i]] = sampled[i];
+}
+
+static size_t row_stage_bytes(int V) {
+  const size_t bytes = (size_t)((((V + kRowCtas - 1) / kRowCtas) + 3) & ~3) * 4;
+  return bytes <= kMostStaged ? bytes : 0;
 }
 
 }  // namespace b200
@@ -525,22 +664,28 @@ int b200_apply_min_p(void* logits, int ld, int n, int V, const void* min_p, cuda
 int b200_apply_top_k_top_p(void* logits, int ld, int n, int V, const void* top_k,
                            const void* top_p, cudaStream_t stream) {
   if (n <= 0) return 0;
-  top_k_top_p_kernel<<<n, kSB, 0, stream>>>((float*)logits, ld, V, (const int*)top_k,
-                                            (const float*)top_p);
+  static PerDeviceOnce attr_once;
+  if (attr_once.first())
+    cudaFuncSetAttribute(top_k_top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostStaged);
+  top_k_top_p_kernel<<<n * kRowCtas, kRowThreads, row_stage_bytes(V), stream>>>((float*)logits, ld, V, (const int*)top_k,
+                                                                               (const float*)top_p);
   RET_LAUNCH;
 }
 
 int b200_softmax(const void* logits, int ld, void* out, int ldo, int n, int V, int log_mode,
                  cudaStream_t stream) {
   if (n <= 0) return 0;
-  softmax_kernel<<<n, kSB, 0, stream>>>((const float*)logits, ld, (float*)out, ldo, V, log_mode);
+  static PerDeviceOnce attr_once;
+  if (attr_once.first()) cudaFuncSetAttribute(softmax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostStaged);
+  softmax_kernel<<<n * kRowCtas, kRowThreads, row_stage_bytes(V), stream>>>((const float*)logits, ld, (float*)out, ldo, V,
+                                                                           log_mode);
   RET_LAUNCH;
 }
 
 int b200_random_sample(const void* probs, int ld, int n, int V, const void* seeds,
                        const void* steps, void* out_i64, cudaStream_t stream) {
   if (n <= 0) return 0;
-  random_sample_kernel<<<n, kSB, 0, stream>>>((const float*)probs, ld, V, (const uint64_t*)seeds,
+  random_sample_kernel<<<n * kRowCtas, kRowThreads, 0, stream>>>((const float*)probs, ld, V, (const uint64_t*)seeds,
                                               (const uint64_t*)steps, (int64_t*)out_i64);
   RET_LAUNCH;
 }

@@ -529,3 +529,43 @@ def test_gemm_gated_activation(M, I, K, kind):
         assert _rel_err(ops.gemm_gated(a, w_il, kind, force_path=9), exp) < 2e-2
     else:
         assert torch.equal(out, ops.act_and_mul(ops.gemm(a, merged_w), kind))
+
+
+@pytest.mark.parametrize("V,ld", [(5, 8), (37, 37), (1003, 1003), (32000, 32000), (151936, 151936), (420001, 420004)])
+def test_row_kernels_over_a_cluster(V, ld):
+    """Rows shared by the CTAs of a cluster: slices of no, few and many columns, unaligned rows, rows too long for shared
+    memory. The threshold of top-p may move by one logit where the mass is within 1e-5 of p (order of the sums)."""
+    torch.manual_seed(V)
+    n = 6
+    x = torch.randn(n, ld, device=DEV)[:, :V] * 2
+    x[1, V // 2:] = -float("inf")
+    k = torch.tensor([0, min(3, V), min(50, V), 1, V, min(7, V)], dtype=torch.int32, device=DEV)
+    p = torch.tensor([0.9, 1.0, 0.95, 0.5, 0.3, 1.0], device=DEV)
+    got = torch.empty(n, ld, device=DEV)[:, :V]
+    got.copy_(x)
+    ops.apply_top_k_top_p(got, k, p)
+    for r in range(n):
+        srt = x[r].double().sort(descending=True).values
+        keep = V if k[r] <= 0 or k[r] >= V else int(k[r])
+        if p[r] < 1:
+            mass = torch.softmax(srt[:keep], 0).cumsum(0)
+            least, most = (min(int((mass < float(p[r]) + d).sum()), keep - 1) + 1 for d in (-1e-5, 1e-5))
+        else:
+            least = most = keep
+        kept = torch.isfinite(got[r])
+        n_kept = int(kept.sum())
+        assert least <= n_kept <= most or n_kept == int(torch.isfinite(x[r]).sum()) < least
+        assert not n_kept or bool((x[r][kept].min() > x[r][~kept]).all())      # the largest ones
+        assert torch.equal(got[r][kept], x[r][kept])
+    soft = ops.softmax(x)
+    exact = torch.softmax(x.double(), -1)
+    assert ((soft.double() - exact).norm() / exact.norm()).item() < 2e-6 + 4e-7 * float(x[torch.isfinite(x)].abs().max())
+    logp = ops.softmax(x, log=True)
+    fin = torch.isfinite(x)
+    assert (logp.double() - torch.log_softmax(x.double(), -1))[fin].abs().max().item() < 2e-5
+    seeds = torch.arange(n, dtype=torch.int64, device=DEV) + 11
+    steps = torch.full((n,), 3, dtype=torch.int64, device=DEV)
+    tok = ops.random_sample(torch.softmax(got, -1).contiguous(), seeds, steps)
+    again = ops.random_sample(torch.softmax(got, -1).contiguous(), seeds, steps)
+    assert torch.equal(tok, again) and all(torch.isfinite(got[r, tok[r]]) for r in range(n))
+    assert ops.read_status() == 0
