@@ -65,15 +65,6 @@ struct alignas(8) DecodeTcBars {
   float red_sum[4][kNQ];
 };
 
-__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-      "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-      "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 // Sync of the 4 softmax warps through an mbarrier (count 4) so that, like every other wait
 // in this kernel, it is bounded: a hardware named barrier would wait forever if one warp had
 // left the loop after a timeout.

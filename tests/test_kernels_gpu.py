@@ -240,6 +240,46 @@ def test_attn_prefill(D, Hq, Hkv, bs):
     assert torch.allclose(lse, exp_lse, atol=2e-2, rtol=1e-3)
 
 
+@pytest.mark.parametrize("Hq,Hkv,bs,window,causal,peak", [(4, 2, 8, 0, True, 1.0), (8, 1, 256, 0, True, 8.0), (12, 2, 32, 150, True, 1.0),
+                                                          (8, 4, 64, -200, True, 1.0), (4, 2, 16, 0, False, 8.0)])
+def test_attn_prefill_head_pairs(Hq, Hkv, bs, window, causal, peak):
+    """128-dim heads in even groups: edges of the 128-row and 128-key tiles, cached prefixes, windows and chunks, keys that
+    raise a row's maximum late (``peak``: the later half of the keys is that much longer). P and the output are rounded to
+    bf16 once each (2 x 2^-8)."""
+    torch.manual_seed(Hq + bs)
+    D, q_lens, ctx = 128, [1, 127, 128, 129, 300], [400, 0, 128, 1, 513]
+    seq_lens = [a + b for a, b in zip(q_lens, ctx)]
+    cache, bt = _make_paged(seq_lens, Hkv, D, bs)
+    for r, n in enumerate(seq_lens):
+        cache[bt[r, (n + bs - 1) // bs // 2: (n + bs - 1) // bs].long(), 0] *= peak
+    T = sum(q_lens)
+    q = _rand(T, Hq * D + 64)[:, :Hq * D]
+    qs = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    sl = torch.tensor(seq_lens, dtype=torch.int32, device=DEV)
+    treq, tq0 = ref.build_prefill_tiles(q_lens)
+    lse = torch.empty(T, Hq, dtype=torch.float32, device=DEV)
+    out = ops.attn_prefill(q, cache, block_table=bt, seq_lens=sl, q_start=qs, tile_req=torch.tensor(treq, dtype=torch.int32, device=DEV),
+                           tile_q0=torch.tensor(tq0, dtype=torch.int32, device=DEV), num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D,
+                           block_size=bs, scale=D ** -0.5, window=window, causal=causal, lse=lse)
+    G = Hq // Hkv
+    for r, (n, c) in enumerate(zip(q_lens, ctx)):
+        rows = slice(int(qs[r]), int(qs[r]) + n)
+        k, v = (cache[bt[r].long(), i].reshape(-1, Hkv, D)[: n + c].double().repeat_interleave(G, 1) for i in (0, 1))
+        score = torch.einsum("qhd,khd->hqk", q[rows].reshape(n, Hq, D).double(), k) * D ** -0.5
+        i, j = torch.arange(c, c + n, device=DEV)[:, None], torch.arange(n + c, device=DEV)[None]
+        see = (j <= i) if causal else torch.ones_like(j <= i)
+        if window > 0:
+            see &= j > i - window
+        elif window < 0:
+            see &= j >= i // -window * -window
+        score = score.masked_fill(~see, -float("inf"))
+        exp = torch.einsum("hqk,khd->qhd", torch.softmax(score, -1), v)
+        got = out[rows].view(n, Hq, D).double()
+        assert ((got - exp).norm() / exp.norm()).item() < 2 * 2.0 ** -8
+        assert (lse[rows].double().t() - torch.logsumexp(score, -1)).abs().max().item() < 1e-3
+    assert ops.read_status() == 0
+
+
 def test_attn_prefill_window_softcap():
     torch.manual_seed(10)
     D, Hq, Hkv, bs = 128, 4, 2, 16
