@@ -4,10 +4,11 @@
 //   gemm_bf16_tn_kernel   persistent, 128 x BN output tiles (BN = 128 | 256), TMA-fed
 //                         smem ring, accumulators double-buffered in TMEM so the epilogue
 //                         of tile i overlaps the main loop of tile i+1. For M > 256.
-//   gemm_bf16_swap_kernel small-M ("decode") form: the weight tile is the 128-row MMA
-//                         operand and the activations are the N operand (UMMA N = M padded
-//                         to 16), so the weight stream is read exactly once; split-K over
-//                         blockIdx.y with fp32 partials reduced in fixed order.
+//   gemm_bf16_swap_kernel small-M form of the tensor-parallel and the allocation-free entries:
+//                         the weight tile is the 128-row MMA operand and the activations are the
+//                         N operand (UMMA N = M padded to 16), so the weight stream is read exactly
+//                         once; split-K over blockIdx.y with fp32 partials reduced in fixed order.
+//                         Plain products of up to 128 rows run in gemm_cluster.cu instead.
 //
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
 // warps 2..5 = epilogue (each owns the TMEM lane quarter warp_id % 4).
@@ -1132,7 +1133,7 @@ struct TmapKeyHash {
   }
 };
 
-static bool get_tmap_bf16(CUtensorMap* out, const void* p, uint64_t rows, uint64_t cols,
+bool get_tmap_bf16(CUtensorMap* out, const void* p, uint64_t rows, uint64_t cols,
                           uint64_t ld, uint32_t br, uint32_t bc) {
   static std::mutex mu;
   static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
@@ -1349,8 +1350,8 @@ extern "C" int b200_gemm_bf16(const void* A, int lda, const void* W, int ldw, vo
 
 // Gated-MLP first half in one kernel: out[M, N / 2] = act(A W_gate^T) * (A W_up^T), where W holds
 // the gate and up rows interleaved in blocks of 128 ([128 gate | 128 up] per 256 rows) so that
-// every 256-column accumulator tile contains both halves of 128 outputs. M > 256 (the CTA-pair
-// kernel); smaller batches run the plain GEMM and the interleave-aware activation kernel.
+// every 256-column accumulator tile contains both halves of 128 outputs (CTA-pair kernel); up to 128 rows a
+// cluster holds the gate and the up tile.
 // kind: 0 SiLU, 1 GELU-tanh, 2 GELU-erf. Replaces MatmulBT + SiluAndMul / GeluAndMul of the
 // reference (src/vt/cuda/cuda_matmul.cu, cuda_ops.cu) on the prefill-sized path.
 extern "C" int b200_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* out,
@@ -1427,12 +1428,27 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   const int w_early = (force_path >> 8) & 1, act = (force_path >> 9) & 7;
   force_path &= 0xff;
   if (act > 4 || (act && (tp || act_fuse))) return -1;
-  if (act_fuse && ((tp && tp->scatter) || M <= 128 || (N & 255) || bias || residual || out_f32)) return -1;
-  if (act_fuse && force_path == 0) force_path = 9;      // the gated epilogue lives in the pair kernel
+  if (act_fuse && ((tp && tp->scatter) || (tp && M <= 128) || (N & 255) || bias || residual || out_f32)) return -1;
+  // Up to 128 rows: K split over a cluster, two CTAs per SM. On the widest matrices (no split to gain from) the tiled
+  // kernel, which reads 256 weight rows with one copy of the batch, is the faster one from some rows on
+  // (128256 x 4096: 172.6 against 169.9 us at 40 rows, 178 against 172 at 64; at 32 rows 167 against 170, at 1 158 against 185).
+  const bool cluster = !tp && M <= 128 && !((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(residual)) & 7) &&
+                       (force_path == 0 ? act_fuse || M <= 32 || N < 16384 : force_path >= 32 && force_path <= 40);
+  if (act_fuse && !cluster && force_path == 0) force_path = 9;      // the gated epilogue lives in the pair kernel
   if ((K & 7) || (lda & 7) || (ldw & 7) || (N & 7) || (ldo & 7) || (residual && (ldr & 7))) return -1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) |
        reinterpret_cast<uintptr_t>(out)) & 15)
     return -1;
+  if (cluster) {       // (force_path 32 + s: with K in s parts)
+    GemmCluster g{};
+    g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.out = out; g.ldo = ldo; g.out_f32 = out_f32;
+    g.bias = bias; g.residual = residual; g.ldr = ldr;
+    g.M = M; g.N = N; g.K = K;
+    g.act = act; g.gated = act_fuse; g.w_early = w_early;
+    g.splits = force_path ? force_path - 32 : 0;
+    g.batch = 1;
+    return launch_gemm_cluster(g, stream);
+  }
   if (tp && tp->scatter && !out) out = const_cast<void*>(A);  // unused by the scatter epilogue
   GemmParams p{};
   p.w_early = (w_early && !tp) ? 1 : 0;
@@ -1465,16 +1481,10 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   const int kblocks = (K + kBK - 1) / kBK;
 
   bool use_swap = (M <= 256);
-  // Small batches. An MMA instruction takes about the same time whatever its N, so swap-AB (the
-  // batch as the narrow N operand) spends one instruction per 128 weight rows x 16 k and becomes
-  // issue-bound on wide weight matrices; there the batch goes on the (padded) M side and 256
-  // weight rows share an instruction, with stream-K filling the SMs. Measured on B200:
-  // N >= 16384: 1-CTA 128 x 256 tiles + stream-K up to 128 rows, CTA pairs above;
-  // narrower matrices: swap-AB up to 128 rows, 128 x 128 tiles + stream-K above.
-  if (force_path == 0 && !tp && M <= 256) {
-    if (N >= 16384) force_path = M <= 128 ? 5 : 9;
-    else if (M > 128) force_path = 6;
-  }
+  // Batches that the cluster kernel does not take. On wide matrices the batch goes on the (padded) M side
+  // and 256 weight rows share an instruction, with stream-K filling the SMs: 1-CTA 128 x 256 tiles up to 128
+  // rows, CTA pairs above; narrower matrices: 128 x 128 tiles + stream-K.
+  if (force_path == 0 && !tp && M <= 256) force_path = N < 16384 ? (M <= 128 ? 2 : 6) : M <= 128 ? 5 : 9;
   if (force_path == 1 || force_path >= 3) use_swap = false;     // an explicit tiling was asked for
   if (force_path == 2 && M <= 256) use_swap = true;
 
@@ -1618,6 +1628,13 @@ extern "C" int b200_gemm_bf16_batched(const void* A, int lda, int a_batch_cols, 
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
   if (M > 256 || (K & 63) || (lda & 7) || (ldw & 7) || (a_batch_cols & 7)) return -1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return -1;
+  if (M <= 128 && !((N | ldo | out_batch_stride) & 7) && !(reinterpret_cast<uintptr_t>(out) & 15) && N % kBM == 0) {
+    GemmCluster g{};          // (its stores are vectors, and a tile stays within one product's weight rows)
+    g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.out = out; g.ldo = ldo;
+    g.M = M; g.N = N; g.K = K;
+    g.batch = batch; g.batch_a_cols = a_batch_cols; g.batch_out = out_batch_stride;
+    return launch_gemm_cluster(g, stream);
+  }
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.out = out; p.ldo = ldo; p.out_f32 = 0;

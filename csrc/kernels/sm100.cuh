@@ -270,6 +270,21 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t smem_addr, uint32_t rank) 
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// Sum of four columns over S CTAs of the cluster from rank `first` on, in their order.
+template <int S>
+__device__ __forceinline__ float4 sum_of(uint32_t addr, int first) {
+  float4 v[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) v[s] = ld_cluster_f4(mapa_u32(addr, first + s));
+#pragma unroll
+  for (int s = 1; s < S; ++s) { v[0].x += v[s].x; v[0].y += v[s].y; v[0].z += v[s].z; v[0].w += v[s].w; }
+  return v[0];
+}
 // Arrive on an mbarrier of another CTA of the cluster (address from mapa_u32).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -470,6 +485,48 @@ bool encode_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType dtyp
                     size_t elem_bytes, uint64_t d0, uint64_t d1, uint64_t d2,
                     uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1,
                     uint32_t b2, CUtensorMapSwizzle swizzle);
+// bf16 matrix with 128-byte swizzled boxes; the maps of a process are kept (gemm_bf16.cu).
+bool get_tmap_bf16(CUtensorMap* out, const void* p, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t br, uint32_t bc);
+
+// Product of at most 128 rows with K split over a cluster (gemm_cluster.cu).
+struct GemmCluster {
+  const void *A, *W;
+  void* out;
+  const void *bias, *residual;
+  int lda, ldw, ldr, M, N, K;
+  long long ldo;
+  int out_f32, act;          // act: act_epilogue
+  int gated;                 // 1 + kind: W in blocks of [128 gate | 128 up] rows, out[M, N / 2] = act(gate) * up
+  int w_early;               // W is constant: fetched before the predecessor kernel has finished
+  int splits;                // CTAs that share a row tile (0: chosen)
+  int batch;                 // products side by side (gridDim.z)
+  int batch_a_cols;
+  long long batch_out;
+  // e4m3 A and W (set a_scale): the sums times a_scale (per tensor or row) and w_scale (per tensor or column)
+  const float *a_scale, *w_scale;
+  int a_per_row, w_per_col;
+};
+int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream);
+
+// One or two rows, on the CUDA cores; optionally with the residual addition and RMSNorm of the rows in front (gemv.cu).
+struct GemvNorm {
+  const void *weight, *res_in;      // res_in: [M, K] or null
+  void* res_out;                    // [M, K], another buffer than res_in
+  float eps;
+  int gemma;
+};
+bool gemv_takes(int M, int N, int K);
+int launch_gemv(const GemmCluster& g, const GemvNorm* norm, cudaStream_t stream);
+
+// The same for the rows of a sorted batch, each chunk of them with its expert's weights (gemm_cluster.cu).
+struct ExpertsCluster {
+  const void *xs, *W;        // [max_rows + 256, K], [E, N, K]
+  void* out;
+  const int32_t *chunk_expert, *chunk_row0, *chunk_n, *num_chunks;
+  int max_rows, max_chunks, E, N, K, gated, act;
+};
+int launch_experts_cluster(const ExpertsCluster& g, cudaStream_t stream);
+
 // Process-wide device status word (lazily allocated per device).
 int* device_status_word();
 long long peer_wait_cycles();   // current limit of waits on other GPUs (b200_set_peer_wait_cycles)
@@ -481,7 +538,8 @@ long long peer_wait_cycles();   // current limit of waits on other GPUs (b200_se
 // pdl_wait() returns only when the predecessor grid has completed and its writes are visible.
 // Rule for kernels launched this way: no global read of produced data and no global write before
 // pdl_wait(). pdl_launch_dependents() only affects when the successor may become resident; both
-// instructions are no-ops in a kernel launched the ordinary way.
+// instructions are no-ops in a kernel launched the ordinary way. It is called right after pdl_wait(): ahead of it the
+// successors' successors come in as well, and a step of one row of the 8B shape took 4.3 instead of 3.7 ms.
 // B200_PDL=0 in the environment makes launch_pdl() an ordinary launch.
 // ------------------------------------------------------------------------------------
 bool pdl_enabled();
@@ -518,7 +576,32 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(static_cast<Args&&>(args))...);
 }
+// The same for a grid of clusters of `ranks` CTAs (1: none).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_cluster_pdl(void (*kernel)(KArgs...), dim3 grid, int ranks, int threads, size_t smem, cudaStream_t stream,
+                                      Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  if (ranks > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)ranks;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (pdl_enabled()) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(static_cast<Args&&>(args))...);
+}
 #endif
+// CTAs of two to an SM that share the K of each of `tiles` row tiles: as many as one wave holds, `most` at most (gemm_cluster.cu).
+int cluster_splits(int tiles, int most);
 // Activations in the epilogue of a product: 0 none, 1 SiLU, 2 GELU-tanh, 3 GELU-erf, 4 squared ReLU. FAST (results that are
 // rounded to bf16): 0.5 (1 + tanh u) = 1 / (1 + e^(-2 u)) with the approximate exponential and quotient.
 template <bool FAST>

@@ -111,6 +111,40 @@ def test_gemm_epilogues():
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 16, 17, 48, 127, 128])
+@pytest.mark.parametrize("N,K", [(8, 64), (136, 72), (128, 512), (1032, 1000), (6144, 1024)])
+def test_gemm_over_a_cluster(M, N, K):
+    """Up to 128 rows, K in 1 to 8 parts over a cluster: edges of row tiles and of k-blocks, every number of parts, what
+    follows the product. A value is off by its rounding to bf16 at most (8 significant bits: 2^-8), in 32 bits by the sums' order."""
+    torch.manual_seed(M * 7 + N + K)
+    a, w = _rand(M, K + 8)[:, :K], _rand(N, K, scale=0.05)
+    bias, res = _rand(N), _rand(M, N + 8)[:, :N]
+    exact = a.double() @ w.double().t()
+    for parts in (0, 1, 2, 3, 5, 8):
+        path = 32 + parts if parts else 0
+        o32 = ops.gemm(a, w, out_dtype=torch.float32, force_path=path)
+        assert _rel_err(o32.double(), exact) < 5e-5
+        assert _rel_err(ops.gemm(a, w, force_path=path).double(), exact) < 2.0 ** -8
+        both = ops.gemm(a, w, bias=bias, residual=res, force_path=path)
+        assert _rel_err(both.double(), exact + bias.double() + res.double()) < 2.0 ** -8
+    act = ops.gemm(a, w, act=4)
+    assert _rel_err(act.double(), exact.clamp_min(0).square()) < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("M", [1, 33, 128])
+@pytest.mark.parametrize("I,K", [(128, 64), (384, 200), (3072, 1024)])
+def test_gemm_gated_over_a_cluster(M, I, K):
+    torch.manual_seed(M + I)
+    a, g, u = _rand(M, K), _rand(I, K, scale=0.05), _rand(I, K, scale=0.05)
+    for kind in (0, 1, 2):
+        out = ops.gemm_gated(a, ops.interleave_gate_up(g, u), kind)
+        merged = ops.gemm(a, torch.cat([g, u], 0), force_path=1)           # rounded before the activation, as here
+        exp = ref.act_and_mul(merged, kind)
+        assert _rel_err(out, exp) < 2.0 ** -6      # gate, up and their product are rounded once each (3 x 2^-8)
+    assert ops.read_status() == 0
+
+
 def test_gemm_deterministic():
     torch.manual_seed(3)
     a, w = _rand(48, 4096), _rand(4096, 4096, scale=0.05)

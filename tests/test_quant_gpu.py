@@ -75,6 +75,31 @@ def test_nvfp4_weights(M, N, K):
     assert _rel(out, exp) < 1e-2
 
 
+def _within_sum_error(out, a64, w64, exp64, extra=0.0):
+    """The products are exact in fp32, so what is left is one rounding per addition (K of 2^-24 of the sum of magnitudes,
+    doubled for the tensor cores' truncation) and the bf16 rounding of the result (2^-8)."""
+    K = a64.shape[1]
+    bound = exp64.abs() * 2**-8 + K * 2.0**-23 * (a64.abs() @ w64.abs().t()) + extra
+    return ((out.double() - exp64).abs() <= bound + 1e-30).all().item()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 16), (17, 520, 144), (65, 136, 4112), (128, 4104, 8192)])
+@pytest.mark.parametrize("per_token,per_channel", [(False, False), (True, True)])
+def test_gemm_fp8_over_a_cluster(M, N, K, per_token, per_channel):
+    """Up to 128 rows: ragged rows, columns and last k block, K in one part and in many."""
+    torch.manual_seed(12)
+    a8 = (torch.randn(M, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    w8 = (torch.randn(N, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    sa = torch.rand(M if per_token else 1, device=DEV) + 0.5
+    sw = torch.rand(N if per_channel else 1, device=DEV) * 0.1 + 0.01
+    a64, w64 = a8.double() * sa.double()[:, None], w8.double() * sw.double()[:, None]
+    for bias in (None, torch.randn(N, device=DEV).to(torch.bfloat16)):
+        exp = a64 @ w64.t() + (0 if bias is None else bias.double())
+        out = Q.gemm_fp8(a8, w8, sa, sw, bias=bias)
+        assert ops.read_status() == 0
+        assert _within_sum_error(out, a64, w64, exp)
+
+
 def test_quant_fp8_static_and_rmsnorm():
     torch.manual_seed(2)
     x = (torch.randn(37, 512, device=DEV) * 3).to(torch.bfloat16)

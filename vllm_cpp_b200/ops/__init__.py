@@ -134,24 +134,17 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 def gemm_gated(a: torch.Tensor, w_il: torch.Tensor, kind: int = ACT_SILU, *,
                out: torch.Tensor | None = None, scratch: torch.Tensor | None = None,
                force_path: int = 0) -> torch.Tensor:
-    """``act(a @ w_gate^T) * (a @ w_up^T)`` with ``w_il`` from :func:`interleave_gate_up`.
-    Above 128 rows the activation runs in the GEMM epilogue (one kernel, the merged
-    projection never reaches memory); below, the small-M GEMM writes the interleaved
-    projection to ``scratch`` and the activation kernel reads it."""
+    """``act(a @ w_gate^T) * (a @ w_up^T)`` with ``w_il`` (a model weight) from :func:`interleave_gate_up`; the
+    activation runs in the GEMM epilogue, the merged projection never reaches memory. ``scratch`` is not used."""
     M, K = a.shape
     N = w_il.shape[0]
     assert a.dtype == torch.bfloat16 and w_il.dtype == torch.bfloat16 and N % 256 == 0
     if out is None:
         out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=a.device)
-    if M > 128:
-        check(lib().b200_gemm_bf16_gated(ptr(a), a.stride(0), ptr(w_il), w_il.stride(0), ptr(out),
-                                         out.stride(0), M, N, K, kind, force_path, stream_ptr()),
-              f"gemm_gated M={M} N={N} K={K}")
-        return out
-    if scratch is None:
-        scratch = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    gemm(a, w_il, out=scratch, const_w=True)      # w_il is a model weight by construction
-    return act_and_mul(scratch, kind, out, interleaved=True)
+    check(lib().b200_gemm_bf16_gated(ptr(a), a.stride(0), ptr(w_il), w_il.stride(0), ptr(out),
+                                     out.stride(0), M, N, K, kind, force_path | 0x100, stream_ptr()),
+          f"gemm_gated M={M} N={N} K={K}")
+    return out
 
 
 def silu_and_mul(x, out=None):
