@@ -129,6 +129,84 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The same for ungrouped routers of up to 256 experts: one warp per token, E / 32 scores a lane, no barrier (a block
+// needed two to three a choice: 9.7 us for 3 tokens, 128 experts, k = 8).
+template <int PER>
+__global__ void __launch_bounds__(128)
+    moe_router_warp_kernel(const float* __restrict__ logits, int ld, int T, int E, int k, int renorm, int scoring,
+                           const float* __restrict__ e_bias, float routed_scale, int32_t* topk_ids, float* topk_w) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const float* x = logits + (size_t)t * ld;
+  float v[PER], score[PER], sel[PER];
+  float mx = -FLT_MAX;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    v[i] = lane + 32 * i < E ? x[lane + 32 * i] : -INFINITY;
+    mx = fmaxf(mx, v[i]);
+  }
+  if (scoring == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      score[i] = lane + 32 * i < E ? expf(v[i] - mx) : 0.f;
+      s += score[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const float inv = 1.f / s;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) score[i] *= inv;
+  } else {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) score[i] = 1.f / (1.f + expf(-v[i]));
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane + 32 * i;
+    // plain sigmoid scores are ranked by their logits: no ties of fp32 scores near 1
+    sel[i] = e >= E ? -FLT_MAX : scoring == 1 && !e_bias ? v[i] : score[i] + (e_bias ? e_bias[e] : 0.f);
+  }
+  float wsum = 0.f, my_w = 0.f;
+  int my_id = 0;
+  for (int j = 0; j < k; ++j) {
+    float bv = -FLT_MAX, bs = 0.f;
+    int bi = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (sel[i] > bv || (sel[i] == bv && lane + 32 * i < bi)) { bv = sel[i]; bi = lane + 32 * i; bs = score[i]; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o), os = __shfl_xor_sync(0xffffffffu, bs, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; bs = os; }
+    }
+    if (bi >= E) {                    // nothing comparable is left (NaN logits): expert 0, as in the block kernel
+      bi = 0;
+      bs = __shfl_sync(0xffffffffu, score[0], 0);
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (lane + 32 * i == bi) sel[i] = -FLT_MAX;
+    wsum += bs;
+    if (lane == (j & 31)) { my_id = bi; my_w = bs; }
+    if ((j & 31) == 31 || j == k - 1) {
+      const int j0 = j & ~31;
+      if (j0 + lane <= j) {
+        topk_ids[(size_t)t * k + j0 + lane] = my_id;
+        topk_w[(size_t)t * k + j0 + lane] = my_w;
+      }
+    }
+  }
+  const float denom = (renorm && wsum > 0.f) ? wsum : 1.f;
+  __syncwarp();
+  for (int j = lane; j < k; j += 32) topk_w[(size_t)t * k + j] = topk_w[(size_t)t * k + j] / denom * routed_scale;
+}
+
 // ------------------------------------------------------------------------------ expert sort
 // meta layout (int32): [0, E) counts | [E, 2E] offsets | [2E+1, 3E+1) cursors | 3E+1 num_chunks
 __global__ void moe_hist_kernel(const int32_t* __restrict__ topk_ids, int P, int e0, int e1,
@@ -167,6 +245,8 @@ __global__ void __launch_bounds__(1024)
                           int max_chunks, int32_t* sorted_token, int32_t* pair_pos) {
   __shared__ int cnt[256], off[256], cbase[256], cursor[256];
   __shared__ int wsum[8], wcsum[8];
+  pdl_wait();
+  pdl_launch_dependents();
   const int E = e1 - e0, tid = threadIdx.x;
   if (tid < 256) cnt[tid] = 0;
   __syncthreads();
@@ -244,6 +324,8 @@ __global__ void moe_scatter_kernel(const int32_t* __restrict__ topk_ids, int P, 
 __global__ void __launch_bounds__(128)
     moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* sorted_token,
                       const int32_t* meta, int E, __nv_bfloat16* xs, int H) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int pos = blockIdx.x;
   if (pos >= meta[2 * E]) return;
   const uint4* s = reinterpret_cast<const uint4*>(x + (size_t)sorted_token[pos] * ldx);
@@ -269,9 +351,10 @@ struct GroupedParams {
   const int32_t* meta;
   int E;
   int stages;
+  int sub_rows;             // sorted rows of a CTA: 256, gated 128 (blockIdx.y = chunk * (256 / sub_rows) + part of it)
   // Gated mode (act_fuse = activation kind + 1): W_e is [gate rows (N/2) | up rows (N/2)]; a CTA
   // takes 128 gate rows and the 128 up rows of the same outputs, keeps one accumulator for each in
-  // TMEM (columns [0, np) and [256, 256 + np)) and writes act(gate) * up to out[rows, N / 2], so the
+  // TMEM (columns [0, np) and [128, 128 + np)) and writes act(gate) * up to out[rows, N / 2], so the
   // merged projection never reaches memory. Both values are rounded to bf16 first, as the separate
   // activation kernel would see them.
   int act_fuse;
@@ -285,19 +368,22 @@ struct alignas(8) GroupedBars {
   float row_w[256];        // clamped pair: routing weights of the chunk's rows
 };
 
-// grid: (N / 128, max_chunks). A CTA whose chunk index is past the device-side count exits.
-__global__ void __launch_bounds__(192, 1)
+// grid: (N / 128, max_chunks). A CTA whose chunk index is past the device-side count exits. Two CTAs share an SM (96 KB of
+// stages and 256 TMEM columns each), so that one stores its outputs while the other multiplies; a CTA alone, with twice
+// the stages and both halves of the gated accumulators for 256 rows, left the tensor pipe idle during its epilogue (us at
+// 8192 tokens, gated / down: 128 experts of 768, top 8, 608 / 525 -> 492 / 349; 64 of 1408, top 6, 799 / 511 -> 637 / 349).
+__global__ void __launch_bounds__(192, 2)
     moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW,
                             const __grid_constant__ CUtensorMap tmX, GroupedParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
-  const int chunk = blockIdx.y;
-  if (chunk >= p.meta[3 * p.E + 1]) return;
-  const int e = p.chunk_expert[chunk], row0 = p.chunk_row0[chunk], rows = p.chunk_n[chunk];
+  const int subs = 256 / p.sub_rows, chunk = blockIdx.y / subs, first = blockIdx.y % subs * p.sub_rows;
+  if (chunk >= p.meta[3 * p.E + 1] || first >= p.chunk_n[chunk]) return;
+  const int e = p.chunk_expert[chunk], row0 = p.chunk_row0[chunk] + first, rows = min(p.sub_rows, p.chunk_n[chunk] - first);
   const int np = (rows + 15) & ~15;                 // UMMA N
   constexpr int kWBytes = kGBM * kGBK * 2;
-  constexpr int kXBytes = 256 * kGBK * 2;           // TMA box is always 256 rows
+  const int kXBytes = p.sub_rows * kGBK * 2;        // TMA box: always sub_rows rows
   const bool gated = p.act_fuse != 0;
   const int half_n = p.N >> 1;                      // gated: outputs per expert
   const int kStage = kWBytes * (gated ? 2 : 1) + kXBytes;
@@ -311,7 +397,7 @@ __global__ void __launch_bounds__(192, 1)
     mbar_init(&bars->acc_full, 1);
     mbar_fence_init();
   }
-  const uint32_t tmem_cols = gated ? 512 : 256;
+  constexpr uint32_t tmem_cols = 256;
   if (warp == 1) { tmem_alloc(&bars->tmem_base, tmem_cols); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
@@ -346,7 +432,7 @@ __global__ void __launch_bounds__(192, 1)
           umma_bf16_ss(tmem_base, umma_desc_k_sw128(wa + kk * 32, 1024),
                        umma_desc_k_sw128(xa + kk * 32, 1024), idesc, (i | kk) != 0);
           if (gated)
-            umma_bf16_ss(tmem_base + 256, umma_desc_k_sw128(wa + kWBytes + kk * 32, 1024),
+            umma_bf16_ss(tmem_base + 128, umma_desc_k_sw128(wa + kWBytes + kk * 32, 1024),
                          umma_desc_k_sw128(xa + kk * 32, 1024), idesc, (i | kk) != 0);
         }
         umma_commit(&bars->empty[s]);
@@ -369,7 +455,7 @@ __global__ void __launch_bounds__(192, 1)
       for (int c = 0; c < np / 16; ++c) {
         uint32_t g[16], u[16];
         tmem_ld_32x32b_x16(ta + c * 16, g);
-        tmem_ld_32x32b_x16(ta + 256 + c * 16, u);
+        tmem_ld_32x32b_x16(ta + 128 + c * 16, u);
         tmem_ld_wait();
         if (n < half_n) {
 #pragma unroll
@@ -389,7 +475,7 @@ __global__ void __launch_bounds__(192, 1)
       for (int c = 0; c < np / 16; ++c) {
         uint32_t g[16], u[16];
         tmem_ld_32x32b_x16(ta + c * 16, g);
-        tmem_ld_32x32b_x16(ta + 256 + c * 16, u);
+        tmem_ld_32x32b_x16(ta + 128 + c * 16, u);
         tmem_ld_wait();
         if (n < half_n) {
 #pragma unroll
@@ -460,7 +546,9 @@ struct CombineParams {
   int rs_flag_parity_stride;
   const uint32_t* op_counter;
 };
-__global__ void __launch_bounds__(128) moe_combine_kernel(CombineParams p) {
+__global__ void __launch_bounds__(256) moe_combine_kernel(CombineParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x;
   const int nv = p.H >> 3;
   __nv_bfloat16* dst;
@@ -478,16 +566,27 @@ __global__ void __launch_bounds__(128) moe_combine_kernel(CombineParams p) {
     float acc[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-    for (int j = 0; j < p.k; ++j) {
-      const int pos = p.pair_pos[(size_t)t * p.k + j];
-      if (pos < 0) continue;
-      const float w = p.topk_w[(size_t)t * p.k + j];
-      const uint4 v = *reinterpret_cast<const uint4*>(p.y + (size_t)pos * p.H + i * 8);
-      float2 f;
-      f = unpack_bf16x2(v.x); acc[0] += w * f.x; acc[1] += w * f.y;
-      f = unpack_bf16x2(v.y); acc[2] += w * f.x; acc[3] += w * f.y;
-      f = unpack_bf16x2(v.z); acc[4] += w * f.x; acc[5] += w * f.y;
-      f = unpack_bf16x2(v.w); acc[6] += w * f.x; acc[7] += w * f.y;
+    for (int j0 = 0; j0 < p.k; j0 += 4) {          // four expert rows on the way at a time
+      int pos[4];
+      float w[4];
+      uint4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        pos[j] = j0 + j < p.k ? p.pair_pos[(size_t)t * p.k + j0 + j] : -1;
+        w[j] = j0 + j < p.k ? p.topk_w[(size_t)t * p.k + j0 + j] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (pos[j] >= 0) v[j] = *reinterpret_cast<const uint4*>(p.y + (size_t)pos[j] * p.H + i * 8);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (pos[j] < 0) continue;
+        float2 f;
+        f = unpack_bf16x2(v[j].x); acc[0] += w[j] * f.x; acc[1] += w[j] * f.y;
+        f = unpack_bf16x2(v[j].y); acc[2] += w[j] * f.x; acc[3] += w[j] * f.y;
+        f = unpack_bf16x2(v[j].z); acc[4] += w[j] * f.x; acc[5] += w[j] * f.y;
+        f = unpack_bf16x2(v[j].w); acc[6] += w[j] * f.x; acc[7] += w[j] * f.y;
+      }
     }
     uint4 o;
     o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
@@ -552,6 +651,11 @@ int b200_moe_router_topk(const void* logits_f32, int ld, int T, int E, int k, in
                          float routed_scale, void* topk_ids, void* topk_w, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (k > E || n_group > 64 || (n_group > 1 && E % n_group)) return -1;
+  if (n_group <= 1 && E <= 256) {
+    auto kernel = E <= 64 ? moe_router_warp_kernel<2> : E <= 128 ? moe_router_warp_kernel<4> : moe_router_warp_kernel<8>;
+    return launch_pdl(kernel, dim3((T + 3) / 4), dim3(128), 0, stream, (const float*)logits_f32, ld, T, E, k, renorm, scoring,
+                      (const float*)e_bias, routed_scale, (int32_t*)topk_ids, (float*)topk_w) == cudaSuccess ? 0 : -2;
+  }
   moe_router_topk_kernel<<<T, 256, (size_t)2 * E * sizeof(float), stream>>>(
       (const float*)logits_f32, ld, E, k, renorm, scoring, (const float*)e_bias, n_group,
       topk_group, group_best, routed_scale, (int32_t*)topk_ids, (float*)topk_w);
@@ -566,10 +670,9 @@ int b200_moe_sort(const void* topk_ids, int T, int k, int e0, int e1, void* meta
   const int P = T * k, E = e1 - e0;
   if (P <= 0) return 0;
   if (E <= 256 && P <= 16384) {
-    moe_sort_small_kernel<<<1, 1024, 0, stream>>>((const int32_t*)topk_ids, P, k, e0, e1, (int32_t*)meta, 256,
-                                                  (int32_t*)chunk_expert, (int32_t*)chunk_row0, (int32_t*)chunk_n,
-                                                  max_chunks, (int32_t*)sorted_token, (int32_t*)pair_pos);
-    RETL;
+    return launch_pdl(moe_sort_small_kernel, dim3(1), dim3(1024), 0, stream, (const int32_t*)topk_ids, P, k, e0, e1,
+                      (int32_t*)meta, 256, (int32_t*)chunk_expert, (int32_t*)chunk_row0, (int32_t*)chunk_n, max_chunks,
+                      (int32_t*)sorted_token, (int32_t*)pair_pos) == cudaSuccess ? 0 : -2;
   }
   cudaMemsetAsync(meta, 0, (size_t)(3 * E + 2) * sizeof(int32_t), stream);
   moe_hist_kernel<<<(P + 255) / 256, 256, 0, stream>>>((const int32_t*)topk_ids, P, e0, e1,
@@ -585,9 +688,8 @@ int b200_moe_sort(const void* topk_ids, int T, int k, int e0, int e1, void* meta
 int b200_moe_gather(const void* x, int ldx, const void* sorted_token, const void* meta, int E,
                     void* xs, int H, int max_rows, cudaStream_t stream) {
   if (max_rows <= 0) return 0;
-  moe_gather_kernel<<<max_rows, 128, 0, stream>>>((const bf16*)x, ldx, (const int32_t*)sorted_token,
-                                                  (const int32_t*)meta, E, (bf16*)xs, H);
-  RETL;
+  return launch_pdl(moe_gather_kernel, dim3(max_rows), dim3(128), 0, stream, (const bf16*)x, ldx, (const int32_t*)sorted_token,
+                    (const int32_t*)meta, E, (bf16*)xs, H) == cudaSuccess ? 0 : -2;
 }
 
 // out[P, N] = grouped(xs[P, K], W[E, N, K]); xs must have at least max_rows + 256 rows allocated.
@@ -599,21 +701,33 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
   if ((K & 7) || (N & 7) || act < 0 || act > 4) return -1;
   if (act_fuse && ((N & 1) || ((N / 2) & 7) || act_fuse < 1 || act_fuse > 4 || (act_fuse == 4) != (clamp != nullptr)))
     return -1;
-  static std::mutex mu;
+  // up to 64 rows an expert on average: weight-bound, see gemm_cluster.cu (us, gated + down, against the kernel above:
+  // 3 tokens of 128 experts of 768, top 8, 28 + 31 -> 29 + 19; 64 tokens 150 + 132 -> 132 + 71; 1024 tokens 194 + 158 ->
+  // 166 + 94; from there on the wider tiles win: 2048 tokens 250 + 130 against 240 + 188, less with two CTAs per SM)
+  if (act_fuse != 4 && max_rows <= 64 * E && !(reinterpret_cast<uintptr_t>(out) & 15)) {
+    ExpertsCluster g{};
+    g.xs = xs; g.W = W; g.out = out;
+    g.chunk_expert = (const int32_t*)chunk_expert; g.chunk_row0 = (const int32_t*)chunk_row0;
+    g.chunk_n = (const int32_t*)chunk_n; g.num_chunks = (const int32_t*)meta + 3 * E + 1;
+    g.max_rows = max_rows; g.max_chunks = max_chunks; g.E = E; g.N = N; g.K = K; g.gated = act_fuse; g.act = act;
+    return launch_experts_cluster(g, stream);
+  }
+  const int sub_rows = act_fuse ? 128 : 256;
   CUtensorMap tmW, tmX;
   if (!encode_tmap_3d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)N,
                       (uint64_t)E, (uint64_t)K * 2, (uint64_t)N * K * 2, kGBK, kGBM, 1,
                       CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
   if (!encode_tmap_2d(&tmX, xs, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)max_rows + 256,
-                      (uint64_t)K, (uint64_t)K, 256, kGBK, CU_TENSOR_MAP_SWIZZLE_128B))
+                      (uint64_t)K, (uint64_t)K, sub_rows, kGBK, CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
   GroupedParams p;
+  p.sub_rows = sub_rows;
   p.N = N; p.K = K; p.out = (bf16*)out;
   p.chunk_expert = (const int32_t*)chunk_expert; p.chunk_row0 = (const int32_t*)chunk_row0;
   p.chunk_n = (const int32_t*)chunk_n; p.meta = (const int32_t*)meta; p.E = E;
-  const int stage = kGBM * kGBK * 2 * (act_fuse ? 2 : 1) + 256 * kGBK * 2;
-  int stages = (200 * 1024) / stage;
+  const int stage = kGBM * kGBK * 2 * (act_fuse ? 2 : 1) + sub_rows * kGBK * 2;
+  int stages = (96 * 1024) / stage;
   if (stages > kGMaxStages) stages = kGMaxStages;
   const int nkb = (K + kGBK - 1) / kGBK;
   if (stages > nkb) stages = nkb < 2 ? 2 : nkb;
@@ -623,9 +737,9 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
     cudaFuncSetAttribute(moe_grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         220 * 1024);
+                         110 * 1024);
   }
-  dim3 grid(((act_fuse ? N / 2 : N) + kGBM - 1) / kGBM, max_chunks);
+  dim3 grid(((act_fuse ? N / 2 : N) + kGBM - 1) / kGBM, max_chunks * (256 / sub_rows));
   moe_grouped_gemm_kernel<<<grid, 192, smem, stream>>>(tmW, tmX, p);
   RETL;
 }
@@ -691,8 +805,11 @@ int b200_moe_combine(const void* y, const void* pair_pos, const void* topk_w, in
     p.rs_flag_parity_stride = sc->rs_flag_parity_stride;
     p.op_counter = (const uint32_t*)sc->op_counter;
   }
-  moe_combine_kernel<<<T, 128, 0, stream>>>(p);
-  RETL;
+  if (sc && sc->world > 1) {
+    moe_combine_kernel<<<T, 128, 0, stream>>>(p);
+    RETL;
+  }
+  return launch_pdl(moe_combine_kernel, dim3(T), dim3(H >= 2048 ? 256 : 128), 0, stream, p) == cudaSuccess ? 0 : -2;
 }
 
 int b200_shared_gate(const void* x, int ldx, const void* w, int T, int H, void* out,

@@ -28,6 +28,21 @@ def test_router_topk_softmax_renorm(T, E, k):
     assert ids[0, 0].item() == 3 and ids[0, 1].item() == 5
 
 
+@pytest.mark.parametrize("T,E,k", [(1, 1, 1), (5, 33, 33), (3, 64, 40), (9, 256, 8), (4, 257, 8)])
+@pytest.mark.parametrize("scoring,biased", [("softmax", False), ("sigmoid", True), ("sigmoid", False)])
+def test_router_of_a_warp_and_of_a_block(T, E, k, scoring, biased):
+    """A warp per token up to 256 experts, a block beyond; more choices than lanes, expert counts around 32, and rows of
+    equal logits (the lower index first)."""
+    torch.manual_seed(E)
+    logits = torch.randn(T, E, device=DEV)
+    logits[-1] = logits[-1].round()
+    bias = torch.randn(E, device=DEV) * 0.1 if biased else None
+    ids, w = M.router_topk(logits, k, renorm=True, scoring=scoring, e_bias=bias, routed_scale=1.5)
+    eids, ew = M.ref_router_topk(logits, k, renorm=True, scoring=scoring, e_bias=bias, routed_scale=1.5)
+    assert torch.equal(ids, eids)
+    assert torch.allclose(w, ew, atol=1e-6, rtol=1e-5)
+
+
 def test_router_grouped_sigmoid_bias():
     torch.manual_seed(1)
     T, E, k = 40, 64, 6
@@ -77,6 +92,39 @@ def test_moe_block_matches_reference(T, E, k, H, I, e0, el):
     local = ((ids >= e0) & (ids < e0 + el)).sum().item()
     assert ws.meta[2 * el].item() == local
     assert (ws.pair_pos.view(T, k)[(ids >= e0) & (ids < e0 + el)] >= 0).all()
+
+
+@pytest.mark.parametrize("T,E,H,I,skew", [(1, 64, 72, 136, False), (3, 128, 256, 128, False), (17, 16, 200, 1408, False),
+                                          (129, 64, 128, 192, True), (300, 64, 256, 64, True)])
+def test_grouped_gemm_of_few_rows_an_expert(T, E, H, I, skew):
+    """Weight-bound chunks over a cluster: ragged row tiles and k-blocks, boxes of 16 to 128 rows, more rows than one pass
+    takes (``skew``: every token goes to expert 1 too). Each of the two products rounds its values to bf16 (2^-8), the gated
+    one three times."""
+    torch.manual_seed(T + I)
+    x = (torch.randn(T, H, device=DEV)).to(torch.bfloat16)
+    wgu = (torch.randn(E, 2 * I, H, device=DEV) * H ** -0.5).to(torch.bfloat16)
+    wd = (torch.randn(E, H, I, device=DEV) * I ** -0.5).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E - 2, device=DEV)[:2] + 2 for _ in range(T)]).int()
+    if skew:
+        ids[:, 1] = 1
+    ws = M.MoeWorkspace(torch.device(DEV), T, 2, E, H, I)
+    M.moe_sort(ids, 0, E, ws)
+    P = 2 * T
+    M.moe_gather(x, ws, E, P)
+    ws.act.fill_(7.0)
+    M.grouped_gemm_gated(ws.xs, wgu, ws.act, ws, P, kind=1)
+    M.grouped_gemm(ws.act, wd, ws.y, ws, P)
+    pos, tok = ws.pair_pos.view(T, 2).long(), torch.arange(T, device=DEV)
+    for j in range(2):
+        e = ids[:, j].long()
+        g, u = (torch.einsum("th,tih->ti", x.float(), wgu[e][:, h * I:(h + 1) * I].float()) for h in range(2))
+        act = torch.nn.functional.gelu(g, approximate="tanh") * u
+        got = ws.act[pos[:, j]].float()
+        assert ((got - act).norm() / act.norm()).item() < 3 * 2.0 ** -8
+        y = torch.einsum("ti,thi->th", got, wd[e].float())
+        assert ((ws.y[pos[:, j]].float() - y).norm() / y.norm()).item() < 2.0 ** -8
+    assert bool((ws.act[P:] == 7.0).all())                      # nothing beyond the sorted rows
+    assert ops.read_status() == 0
 
 
 def test_moe_engine_gpu_vs_cpu():

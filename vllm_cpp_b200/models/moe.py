@@ -220,11 +220,11 @@ class MoeModel(DenseModel):
 
     # ------------------------------------------------------------------ MoE block
     def _moe_block(self, x: torch.Tensor, L: dict, T: int, scatter=None, shared=None,
-                   shared_gate=None) -> torch.Tensor:
+                   shared_gate=None, out=None) -> torch.Tensor:
         """Routed experts over ``x`` [T, H]. Returns this rank's (partial, if EP) output, or
         stores it into the owners' receive slots when ``scatter`` is given. ``shared`` [T, H]
         (this rank's part of the shared experts' output), scaled per row by ``shared_gate`` [T]
-        when given, is added in the combine kernel."""
+        when given, is added in the combine kernel. ``out``: where the sum goes (not ``x``)."""
         c = self.cfg
         if self.device.type != "cuda":
             return self._moe_block_cpu(x, L)
@@ -246,7 +246,8 @@ class MoeModel(DenseModel):
             M.grouped_gemm(ws.xs, L["w_gate_up"], ws.gu, ws, P, chunks)
             self.be.act_and_mul(ws.gu[:P], ACT_KIND.get(c.hidden_act, 0), out=ws.act[:P])
         M.grouped_gemm(ws.act, L["w_down"], ws.y, ws, P, chunks)
-        out = None if scatter is not None else self.bufs.get("moe_out", T, c.hidden_size)
+        if scatter is None and out is None:
+            out = self.bufs.get("moe_out", T, c.hidden_size)
         M.combine(ws.y, ws, w, out, shared=shared, shared_gate=shared_gate, scatter=scatter)
         return out
 
@@ -309,9 +310,10 @@ class MoeModel(DenseModel):
             if self.tp > 1:
                 self.comm.all_reduce(hidden)
             x = be.rmsnorm(hidden, L["ln2"], eps, residual=resid, out=normed)
-            m = self._moe_block(x, L, T)
             hidden = self.bufs.get("hidden", T, H)
-            hidden.copy_(m)
+            m = self._moe_block(x, L, T, out=hidden)
+            if m is not hidden:
+                hidden.copy_(m)
             if self.ep > 1:
                 self.comm.all_reduce(hidden)
         full = be.rmsnorm(hidden, self.w["final_norm"], eps, residual=resid, out=normed)
