@@ -1447,6 +1447,7 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
     g.act = act; g.gated = act_fuse; g.w_early = w_early;
     g.splits = force_path ? force_path - 32 : 0;
     g.batch = 1;
+    if (force_path == 0 && gemv_takes(M, N, K)) return launch_gemv(g, nullptr, stream);
     return launch_gemm_cluster(g, stream);
   }
   if (tp && tp->scatter && !out) out = const_cast<void*>(A);  // unused by the scatter epilogue

@@ -158,6 +158,33 @@ def test_native_layer_entry_same_logits_as_per_op_path():
     assert ops.read_status() == 0
 
 
+def test_dense_layer_of_one_and_two_rows():
+    """The block that takes its norms into the products against the per-op path: the same bits."""
+    cfg = synthetic_config("tiny-qwen3")
+    cfg.head_dim, cfg.hidden_size, cfg.intermediate_size, cfg.num_layers = 128, 1024, 1536, 3
+    llm = LLM(EngineArgs(model_config=cfg, device="cuda", block_size=16, num_blocks=64, max_model_len=256, max_num_seqs=2,
+                         max_num_batched_tokens=64, enable_cuda_graphs=False))
+    m, seen = llm.runner.model, []
+    orig = type(m).forward
+
+    def both(self, ctx):
+        self.native_layers = False
+        a = orig(self, ctx).clone()
+        self.native_layers = True
+        b = orig(self, ctx)
+        seen.append((ctx.num_tokens, torch.equal(a, b)))
+        return b
+
+    type(m).forward = both
+    try:
+        llm.generate([[5, 6, 7, 8], [9, 10, 11]], SamplingParams(temperature=0.0, max_tokens=4, ignore_eos=True))
+        llm.generate([[1]], SamplingParams(temperature=0.0, max_tokens=4, ignore_eos=True))
+    finally:
+        type(m).forward = orig
+    assert {t for t, _ in seen} >= {1, 2} and all(eq for _, eq in seen), seen
+    assert ops.read_status() == 0
+
+
 def test_async_chunks_of_a_long_prompt_behind_a_busy_gpu():
     """Chunks that sample nothing are not waited for, so the host runs ahead of the GPU: the inputs of a step must still
     be in its staging buffer when the copy of them runs."""

@@ -145,6 +145,22 @@ def test_gemm_gated_over_a_cluster(M, I, K):
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("N,K", [(8, 8), (264, 72), (1032, 1000), (6144, 1024), (4096, 14336), (40000, 512)])
+def test_gemm_of_one_or_two_rows(M, N, K):
+    """Warp-wide products: ragged chunks of K, one to eight warps a pair of rows, several turns of a block. Off by the
+    rounding to bf16 at most (2^-8)."""
+    torch.manual_seed(M + N)
+    a, w = _rand(M, K + 8)[:, :K], _rand(N, K, scale=0.05)
+    bias, res = _rand(N), _rand(M, N + 8)[:, :N]
+    exact = a.double() @ w.double().t()
+    assert _rel_err(ops.gemm(a, w, out_dtype=torch.float32).double(), exact) < 5e-6 * K ** 0.5
+    assert _rel_err(ops.gemm(a, w, const_w=True).double(), exact) < 2.0 ** -8
+    assert _rel_err(ops.gemm(a, w, bias=bias, residual=res).double(), exact + bias.double() + res.double()) < 2.0 ** -8
+    assert _rel_err(ops.gemm(a, w, act=4).double(), exact.clamp_min(0).square()) < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
 def test_gemm_deterministic():
     torch.manual_seed(3)
     a, w = _rand(48, 4096), _rand(4096, 4096, scale=0.05)
