@@ -205,25 +205,34 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Fixed-order merge of split partials: out = sum_s w_s * o_s, w_s = 2^(lse_s - lse_max) / sum.
+// Fixed-order merge of split partials: out = sum_s w_s * o_s, w_s = 2^(lse_s - lse_max) / sum. The weights are taken once a
+// block (splits floats of shared memory); the partial rows are on the way four at a time.
 __global__ void __launch_bounds__(128)
     attn_decode_merge_kernel(const float* __restrict__ tmp_o, const float* __restrict__ tmp_lse,
                              __nv_bfloat16* out, int ldo, int Hq, int D, int splits) {
+  extern __shared__ float wgt[];
+  pdl_wait();
+  pdl_launch_dependents();
   const int b = blockIdx.x, h = blockIdx.y;
   const size_t row0 = ((size_t)b * Hq + h) * splits;
+  for (int s = threadIdx.x; s < splits; s += blockDim.x) wgt[s] = tmp_lse[row0 + s];
+  __syncthreads();
   float mx = -INFINITY;
-  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, tmp_lse[row0 + s]);
+  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, wgt[s]);
+  __syncthreads();
+  for (int s = threadIdx.x; s < splits; s += blockDim.x) wgt[s] = wgt[s] == -INFINITY ? 0.f : exp2f(wgt[s] - mx);
+  __syncthreads();
   float den = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float v = tmp_lse[row0 + s];
-    den += (v == -INFINITY) ? 0.f : exp2f(v - mx);
-  }
+  for (int s = 0; s < splits; ++s) den += wgt[s];
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float acc = 0.f;
-    for (int s = 0; s < splits; ++s) {
-      const float v = tmp_lse[row0 + s];
-      const float w = (v == -INFINITY) ? 0.f : exp2f(v - mx);
-      acc += w * tmp_o[(row0 + s) * D + d];
+    for (int s = 0; s < splits; s += 4) {
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = s + e < splits ? tmp_o[(row0 + s + e) * D + d] : 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (s + e < splits) acc += wgt[s + e] * o[e];
     }
     out[(size_t)b * ldo + (size_t)h * D + d] = __float2bfloat16(den > 0.f ? acc / den : 0.f);
   }
@@ -308,21 +317,13 @@ int b200_attn_decode(const void* q, int ldq, void* out, int ldo, const void* kv_
   else if (D == 128) rc = launch_decode<128>(p, B, stream);
   else rc = launch_decode<256>(p, B, stream);
   if (rc) return rc;
-  if (splits > 1) {
-    dim3 grid(B, Hq);
-    attn_decode_merge_kernel<<<grid, 128, 0, stream>>>(p.tmp_o, p.tmp_lse, p.out, ldo, Hq, D,
-                                                       splits);
-    if (cudaGetLastError() != cudaSuccess) return -2;
-  }
-  return 0;
+  return splits > 1 ? b200_attn_decode_merge(p.tmp_o, p.tmp_lse, p.out, ldo, B, Hq, D, splits, stream) : 0;
 }
 
 int b200_attn_decode_merge(const void* tmp_o, const void* tmp_lse, void* out, int ldo, int B,
                            int Hq, int D, int splits, cudaStream_t stream) {
-  dim3 grid(B, Hq);
-  attn_decode_merge_kernel<<<grid, 128, 0, stream>>>((const float*)tmp_o, (const float*)tmp_lse,
-                                                     (__nv_bfloat16*)out, ldo, Hq, D, splits);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(attn_decode_merge_kernel, dim3(B, Hq), dim3(128), (size_t)splits * sizeof(float), stream, (const float*)tmp_o, (const float*)tmp_lse,
+                    (__nv_bfloat16*)out, ldo, Hq, D, splits) == cudaSuccess ? 0 : -2;
 }
 
 int b200_merge_attn_states(const void* a, const void* lse_a, const void* b, const void* lse_b,

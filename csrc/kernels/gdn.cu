@@ -111,6 +111,8 @@ __global__ void __launch_bounds__(128)
     gdn_conv1d_update_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ w,
                              bf16* __restrict__ state, const int* __restrict__ slots,
                              bf16* __restrict__ out, long ldo, int C) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int c = blockIdx.x * 128 + threadIdx.x;
   const int b = blockIdx.y;
   if (c >= C) return;
@@ -176,6 +178,8 @@ __global__ void __launch_bounds__(128)
                              const float* __restrict__ dt_bias, float* __restrict__ state,
                              const int* __restrict__ slots, bf16* __restrict__ out, int Hk, int Hv,
                              float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int D = 128;
   __shared__ float qs[D], ks[D];
   __shared__ float red[8];
@@ -253,6 +257,8 @@ __global__ void __launch_bounds__(128)
     rmsnorm_gated_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ z, long ldz,
                          const bf16* __restrict__ w, bf16* __restrict__ out, long ldo, long R, int D,
                          float eps, int gate_kind, int heads) {
+  pdl_wait();
+  pdl_launch_dependents();
   const long r = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= R) return;
@@ -312,9 +318,8 @@ int b200_gdn_conv1d_update(const void* x, long ldx, const void* w, void* conv_st
   if (B <= 0) return 0;
   if (C & 3) return -1;
   dim3 grid((C + 127) / 128, B);
-  gdn_conv1d_update_kernel<<<grid, 128, 0, stream>>>((const bf16*)x, ldx, (const bf16*)w,
-                                                     (bf16*)conv_state, slots, (bf16*)out, ldo, C);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(gdn_conv1d_update_kernel, grid, dim3(128), 0, stream, (const bf16*)x, ldx, (const bf16*)w, (bf16*)conv_state,
+                    slots, (bf16*)out, ldo, C) == cudaSuccess ? 0 : -2;
 }
 
 int b200_gdn_post_conv(const void* xc, long ld, int T, int Hk, int Hv, int Dk, const void* a,
@@ -336,10 +341,8 @@ int b200_gdn_packed_decode(const void* xc, long ld, const void* a, const void* b
   if (B <= 0) return 0;
   if (Dk != 128 || Dv != 128 || Hk <= 0 || Hv % Hk) return -1;
   dim3 grid(Dv / 32, B * Hv);
-  gdn_packed_decode_kernel<<<grid, 128, 0, stream>>>((const bf16*)xc, ld, (const bf16*)a,
-                                                     (const bf16*)b, ldab, A_log, dt_bias, state,
-                                                     slots, (bf16*)out, Hk, Hv, eps);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(gdn_packed_decode_kernel, grid, dim3(128), 0, stream, (const bf16*)xc, ld, (const bf16*)a, (const bf16*)b,
+                    ldab, A_log, dt_bias, state, slots, (bf16*)out, Hk, Hv, eps) == cudaSuccess ? 0 : -2;
 }
 
 int b200_rmsnorm_gated(const void* x, long ldx, const void* z, long ldz, const void* w, void* out,
@@ -348,9 +351,8 @@ int b200_rmsnorm_gated(const void* x, long ldx, const void* z, long ldz, const v
   if (R <= 0) return 0;
   if (heads < 1) heads = 1;
   if ((D & 3) || (ldx & 3) || (ldz & 3) || (ldo & 3)) return -1;
-  rmsnorm_gated_kernel<<<(unsigned)((R + 3) / 4), 128, 0, stream>>>(
-      (const bf16*)x, ldx, (const bf16*)z, ldz, (const bf16*)w, (bf16*)out, ldo, R, D, eps, gate_kind, heads);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(rmsnorm_gated_kernel, dim3((unsigned)((R + 3) / 4)), dim3(128), 0, stream, (const bf16*)x, ldx, (const bf16*)z,
+                    ldz, (const bf16*)w, (bf16*)out, ldo, R, D, eps, gate_kind, heads) == cudaSuccess ? 0 : -2;
 }
 
 }  // extern "C"

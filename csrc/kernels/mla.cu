@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(192, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.x, split = blockIdx.y;
   const int head0 = blockIdx.z * kNQ, G = min(p.Hq - head0, kNQ);
+  pdl_wait();
   const int seq_len = p.seq_lens[b];
   const int first_tok = p.window > 0 ? max(seq_len - p.window, 0) : 0, first_tile = first_tok / kTok;
   const int tiles_total = (seq_len + kTok - 1) / kTok - first_tile;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(192, 1)
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_s = tmem_base;         // 2 x 16 columns
   const uint32_t tmem_o = tmem_base + 32;    // 4 x 16 columns
+  pdl_launch_dependents();
 
   if (ntiles > 0) {
     if (warp == 0) {
@@ -469,6 +471,8 @@ __global__ void __launch_bounds__(128)
 // q_pe (64 values at column 128 of each 192-wide head) -> column 512 of each 576-wide row.
 __global__ void __launch_bounds__(128)
     mla_copy_qpe_kernel(const bf16* __restrict__ q, long ldq, bf16* __restrict__ qabs, int H) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t t = blockIdx.x;
   for (int i = threadIdx.x; i < H * 8; i += blockDim.x) {
     const int h = i >> 3, c = i & 7;
@@ -553,7 +557,7 @@ int b200_latent_decode(const void* qabs, void* out, int ldo, const void* cache, 
   auto launch = [&](auto kernel, PerDeviceOnce& attr_once, int pieces) {
     const size_t smem = (size_t)kRingBytes + (2 * pieces + 1) * 2048 + 8192 + 1024 + sizeof(MlaBars);
     if (attr_once.first()) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kernel<<<dim3(B, splits, hgroups), 192, smem, stream>>>(tmQ, tmC, p);
+    launch_pdl(kernel, dim3(B, splits, hgroups), dim3(192), smem, stream, tmQ, tmC, p);
   };
   static PerDeviceOnce once[4];
   switch (rank / 128) {
@@ -604,8 +608,7 @@ int b200_mla_pad_q(const void* q, long ldq, void* out, int T, int H, cudaStream_
 
 int b200_mla_copy_qpe(const void* q, long ldq, void* qabs, int T, int H, cudaStream_t stream) {
   if (T <= 0) return 0;
-  mla_copy_qpe_kernel<<<T, 128, 0, stream>>>((const bf16*)q, ldq, (bf16*)qabs, H);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(mla_copy_qpe_kernel, dim3(T), dim3(128), 0, stream, (const bf16*)q, ldq, (bf16*)qabs, H) == cudaSuccess ? 0 : -2;
 }
 
 }  // extern "C"

@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(256)
                         uint8_t* __restrict__ out, long ldo, float* __restrict__ scales, int K) {
   __shared__ float red[32];
   extern __shared__ uint4 row_cache[];  // K/8 vectors
+  pdl_wait();
+  pdl_launch_dependents();
   const long t = blockIdx.x;
   const int nv = K >> 3;
   float amax = 0.f;
@@ -387,10 +389,9 @@ int b200_quant_fp8_rowwise(const void* x, long ldx, void* residual, const void* 
   static PerDeviceOnce attr_once;
   if (attr_once.first())
     cudaFuncSetAttribute(rowquant_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 2);
-  rowquant_fp8_kernel<<<T, threads, (size_t)K * 2, stream>>>((const bf16*)x, ldx, (bf16*)residual, (const bf16*)norm_w,
-                                                           eps, gemma, mode, kind_flags, (uint8_t*)out, ldo,
-                                                           (float*)scales, K);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(rowquant_fp8_kernel, dim3(T), dim3(threads), (size_t)K * 2, stream, (const bf16*)x, ldx, (bf16*)residual,
+                    (const bf16*)norm_w, eps, gemma, mode, kind_flags, (uint8_t*)out, ldo, (float*)scales, K) == cudaSuccess
+             ? 0 : -2;
 }
 
 int b200_layernorm(const void* x, const void* w, const void* b, void* out, int T, int H, float eps,

@@ -127,18 +127,19 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(RopeKvParams p, int T) {
 // consecutive heads of one token. Lane l holds dims 4l..4l+3 of a head (one 8-byte load), its
 // rotation partner (dim +-64) sits in lane l ^ 16; the token's cos / sin row and cache slot are
 // fetched once per warp and the kHG head loads are issued together, so the dependent global
-// round trips are paid once per eight heads instead of once per head.
-static constexpr int kHG = 8;
+// round trips are paid once per eight heads instead of once per head. A few tokens do not fill the chip with that: there
+// every head has its own warp (kHG = 1).
+template <int kHG>
 __global__ void __launch_bounds__(128) rope_kv_vec4_kernel(RopeKvParams p, int T) {
   pdl_wait();                 // predecessor grid complete, its writes visible
   pdl_launch_dependents();    // the successor may become resident (it waits the same way)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nheads = p.Hq + 2 * p.Hkv;
   const int groups = (nheads + kHG - 1) / kHG;
-  const long long gw = (long long)blockIdx.x * 4 + warp;
-  if (gw >= (long long)T * groups) return;
-  const int t = (int)(gw / groups);
-  const int h0 = (int)(gw % groups) * kHG;
+  const uint32_t gw = blockIdx.x * 4 + warp;               // (T * groups < 2^31)
+  if (gw >= (uint32_t)(T * groups)) return;
+  const int t = (int)(gw / (uint32_t)groups);
+  const int h0 = ((int)gw - t * groups) * kHG;
   const int nh = min(kHG, nheads - h0);
   __nv_bfloat16* row = p.qkv + (size_t)t * p.ld;
   const int kv0 = p.Hq;              // first k head
@@ -159,7 +160,9 @@ __global__ void __launch_bounds__(128) rope_kv_vec4_kernel(RopeKvParams p, int T
   if (p.slot_mapping && h0 + nh > kv0) {
     const int64_t slot = p.slot_mapping[t];
     if (slot >= 0) {
-      const int64_t blk = slot / p.block_size, off = slot % p.block_size;
+      const bool small = (slot >> 31) == 0;               // (64-bit division takes longer than the loads)
+      const int64_t blk = small ? (int64_t)((uint32_t)slot / (uint32_t)p.block_size) : slot / p.block_size;
+      const int64_t off = slot - blk * p.block_size;
       kdst = p.kv_cache + ((blk * 2 + 0) * p.block_size + off) * (int64_t)p.Hkv * 128;
       vdst = p.kv_cache + ((blk * 2 + 1) * p.block_size + off) * (int64_t)p.Hkv * 128;
     }
@@ -246,6 +249,8 @@ __global__ void __launch_bounds__(128)
                                 const __nv_bfloat16* __restrict__ k_pe, int ldr,
                                 const int64_t* __restrict__ slots, __nv_bfloat16* cache, int Lc,
                                 int Lr) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int t = blockIdx.x;
   const int64_t slot = slots[t];
   if (slot < 0) return;
@@ -294,11 +299,11 @@ int b200_rope_kv(void* qkv, int ld, int q_off, int k_off, int v_off, int q_head_
             !(ptr_bits & 7) && !(reinterpret_cast<uintptr_t>(cos_sin) & 15)) ? 1 : 0;
   long long warps = (long long)T * (Hq + 2 * Hkv);
   int blocks = (int)((warps + 3) / 4);
-  if (p.vec4) {
-    const int groups = (Hq + 2 * Hkv + kHG - 1) / kHG;
+  if (p.vec4 && warps < (1ll << 31)) {
+    const int hg = warps <= 4096 ? 1 : 8, groups = (Hq + 2 * Hkv + hg - 1) / hg;
     const long long w4 = (long long)T * groups;
-    return launch_pdl(rope_kv_vec4_kernel, dim3((unsigned)((w4 + 3) / 4)), dim3(128), 0, stream, p, T) == cudaSuccess
-               ? 0 : -2;
+    return launch_pdl(hg == 1 ? rope_kv_vec4_kernel<1> : rope_kv_vec4_kernel<8>, dim3((unsigned)((w4 + 3) / 4)), dim3(128), 0,
+                      stream, p, T) == cudaSuccess ? 0 : -2;
   }
   return launch_pdl(rope_kv_kernel, dim3(blocks), dim3(128), 0, stream, p, T) == cudaSuccess ? 0 : -2;
 }
@@ -318,10 +323,8 @@ int b200_concat_and_cache_mla(const void* kv_c, int ldc, const void* k_pe, int l
                               const void* slots, void* cache, int Lc, int Lr, int T,
                               cudaStream_t stream) {
   if (T <= 0) return 0;
-  concat_and_cache_mla_kernel<<<T, 128, 0, stream>>>((const bf16*)kv_c, ldc, (const bf16*)k_pe,
-                                                     ldr, (const int64_t*)slots, (bf16*)cache, Lc,
-                                                     Lr);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(concat_and_cache_mla_kernel, dim3(T), dim3(128), 0, stream, (const bf16*)kv_c, ldc, (const bf16*)k_pe, ldr,
+                    (const int64_t*)slots, (bf16*)cache, Lc, Lr) == cudaSuccess ? 0 : -2;
 }
 
 int b200_rope_table(const void* inv_freq_f64, void* out_f32, int max_pos, int half, float mscale,
