@@ -283,6 +283,207 @@ __global__ void __launch_bounds__(kWThreads, 1)
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
+// ---------------------------------------------------------------------------------------
+// Up to 64 rows: 128 weight rows as the MMA's M, the batch (padded to 16) as its N, K split over a cluster, two CTAs per
+// SM that fill each other's waits; the parts of K are summed from shared memory to shared memory instead of through a
+// workspace and a second kernel. Bound by the chain expansion - MMA - release of a 64-k tile, about 0.5 us each, of which
+// four MMAs and their barriers are 0.36 (measured with conversions, scale loads and split of the warps varied). us at
+// 9 / 64 rows, the reducing kernel included, against the form above:
+//   16480 x 5120 33.0 / 41.8 -> 31.8 / 33.8    5120 x 6144 18.6 / 26.4 -> 16.8 / 19.6
+//   34816 x 5120 76.1 / 56.4 -> 55.2 / 57.9    5120 x 17408 34.6 / 42.3 -> 36.4 / 39.2
+// ---------------------------------------------------------------------------------------
+static constexpr int kCRows = 128, kCRaw = kCRows * 128, kCExp = kCRows * 128;
+static constexpr int kCRS = 2, kCES = 3, kCAS = 12, kCConv = 8, kCThreads = (3 + kCConv) * 32, kCRowsMax = 64;
+
+struct W4CParams {
+  int M, N, K, mp, splits, act_stages;
+  bf16* out;
+  int ldo;
+  const uint8_t* sf;
+  const float* gscale;
+  const bf16* bias;
+  int* status;
+};
+struct alignas(8) W4CBars {
+  uint64_t raw_full[kCRS], raw_empty[kCRS], exp_full[kCES], exp_empty[kCES], act_full[kCAS], act_empty[kCAS], acc;
+  uint32_t tmem_base;
+};
+
+template <int S>
+__device__ __forceinline__ void w4_reduce(const W4CParams& p, uint32_t partial, int rank, int tile, int warp, int lane) {
+  const float g = *p.gscale * 128.f;
+  const int col = tile * kCRows + lane * 4;
+  for (int m = rank + warp * S; m < p.M; m += (3 + kCConv) * S) {
+    float4 a = sum_of<S>(partial + (uint32_t)m * (kCRows * 4) + lane * 16, 0);
+    if (col >= p.N) continue;                        // N is a multiple of 8
+    a.x *= g; a.y *= g; a.z *= g; a.w *= g;
+    if (p.bias) {
+      a.x += __bfloat162float(p.bias[col]); a.y += __bfloat162float(p.bias[col + 1]);
+      a.z += __bfloat162float(p.bias[col + 2]); a.w += __bfloat162float(p.bias[col + 3]);
+    }
+    *reinterpret_cast<uint2*>(p.out + (size_t)m * p.ldo + col) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+  }
+}
+
+// K is a multiple of 256.
+__global__ void __launch_bounds__(kCThreads, 2)
+    gemm_w4a16_cluster_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA,
+                              W4CParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ W4CBars bars;
+  uint8_t* sExp = smem;
+  uint8_t* sRaw = sExp + kCES * kCExp;
+  uint8_t* sAct = sRaw + kCRS * kCRaw;
+  const int act_bytes = p.mp * 128;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, tile = blockIdx.x / p.splits, n0 = tile * kCRows;
+  const int blocks = p.K / 256, b0 = blocks * rank / p.splits, nr = blocks * (rank + 1) / p.splits - b0, ne = 4 * nr;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kCRS; ++s) { mbar_init(&bars.raw_full[s], 1); mbar_init(&bars.raw_empty[s], kCConv); }
+    for (int s = 0; s < kCES; ++s) {
+      mbar_init(&bars.exp_full[s], kCConv / 2);
+      mbar_init(&bars.exp_empty[s], 1);
+    }
+    for (int s = 0; s < p.act_stages; ++s) { mbar_init(&bars.act_full[s], 1); mbar_init(&bars.act_empty[s], 1); }
+    mbar_init(&bars.acc, 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) { tmem_alloc(&bars.tmem_base, 64); tmem_relinquish(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = bars.tmem_base;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmW);
+      for (int i = 0; i < nr; ++i) {
+        const int rs = i % kCRS;
+        if (!mbar_wait(&bars.raw_empty[rs], ((i / kCRS) & 1) ^ 1, p.status)) break;
+        mbar_expect_tx(&bars.raw_full[rs], kCRaw);
+        tma_load_2d(sRaw + rs * kCRaw, &tmW, &bars.raw_full[rs], (b0 + i) * 128, n0);
+      }
+    }
+  } else if (warp == 2 + kCConv) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmA);
+      for (int e = 0; e < ne; ++e) {
+        const int as = e % p.act_stages;
+        if (!mbar_wait(&bars.act_empty[as], ((e / p.act_stages) & 1) ^ 1, p.status)) break;
+        mbar_expect_tx(&bars.act_full[as], act_bytes);
+        tma_load_2d(sAct + as * act_bytes, &tmA, &bars.act_full[as], b0 * 256 + e * 64, 0);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_f16(kCRows, p.mp);
+      bool ok = true;
+      for (int e = 0; e < ne; ++e) {
+        const int es = e % kCES, as = e % p.act_stages;
+        ok = mbar_wait(&bars.act_full[as], (e / p.act_stages) & 1, p.status) && mbar_wait(&bars.exp_full[es], (e / kCES) & 1, p.status);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint64_t wd = umma_desc_k_sw128(smem_u32(sExp + es * kCExp), 1024);
+        const uint64_t ad = umma_desc_k_sw128(smem_u32(sAct + as * act_bytes), 1024);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_f16_ss(tmem, wd + 2 * k, ad + 2 * k, idesc, (e | k) != 0);
+        umma_commit(&bars.exp_empty[es]);
+        umma_commit(&bars.act_empty[as]);
+      }
+      if (ok) umma_commit(&bars.acc);
+    }
+  } else {
+    // A nibble's three magnitude bits in bits 9 to 11 of an f16 are its value times 2^-14 (subnormals included), nibbles k and
+    // k + 4 of a word lie 16 bits apart: four shifts and masks expand two weights (in the order 0 4 1 5 2 6 3 7, which the
+    // cast of the batch follows). Times the block scale x 2^7 they are exact in f16 (5 significant bits, multiples of
+    // 2^-17 up to 21); the 2^7 that is missing joins the global scale.
+    constexpr uint32_t kMag = 0x0e000e00u, kSign = 0x80008000u;
+    // Four warps expand the even tiles of 64 k, four the odd ones, a thread a row: a warp's expansion ends in a fence, and
+    // the other half's work covers it.
+    // The row's 16 block scales of 256 k come as one load, two blocks ahead.
+    const int ct = threadIdx.x - 64, r = ct & 127, half = ct >> 7;
+    const uint4* sf_row = reinterpret_cast<const uint4*>(p.sf + (size_t)min(n0 + r, p.N - 1) * (p.K / 16)) + b0;
+    uint4 sf_next = __ldg(sf_row), sf_after = __ldg(sf_row + min(1, nr - 1));
+    bool ok = true;
+    for (int i = 0; i < nr && ok; ++i) {
+      const int rs = i % kCRS;
+      const uint4 sf = sf_next;
+      sf_next = sf_after;
+      sf_after = __ldg(sf_row + min(i + 2, nr - 1));
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.raw_full[rs], (i / kCRS) & 1, p.status));
+      if (!ok) break;
+      const uint8_t* raw = sRaw + rs * kCRaw + r * 128;
+      const uint32_t sfw[4] = {sf.x, sf.y, sf.z, sf.w};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int sub = 2 * q + half, e = 4 * i + sub, es = e % kCES;
+        const uint4 ra[2] = {*reinterpret_cast<const uint4*>(raw + (((2 * sub) ^ (r & 7)) << 4)),        // (swizzled)
+                             *reinterpret_cast<const uint4*>(raw + (((2 * sub + 1) ^ (r & 7)) << 4))};
+        const uint32_t sfq = half ? sfw[2 * q + 1] : sfw[2 * q];
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars.exp_empty[es], ((e / kCES) & 1) ^ 1, p.status));
+        if (!ok) break;
+        uint8_t* dst = sExp + es * kCExp + r * 128;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t s2 = hmul2_bits(cvt_e4m3x2((uint16_t)(sfq >> (16 * h))), 0x58005800u);             // scales x 2^7
+          const uint32_t sc[2] = {__byte_perm(s2, 0, 0x1010), __byte_perm(s2, 0, 0x3232)};
+          const uint32_t words[4] = {ra[h].x, ra[h].y, ra[h].z, ra[h].w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const uint32_t w = words[c], s = sc[c >> 1];
+            *reinterpret_cast<uint4*>(dst + (((h * 4 + c) ^ (r & 7)) << 4)) =
+                make_uint4(hmul2_bits(((w << 9) & kMag) | ((w << 12) & kSign), s), hmul2_bits(((w << 5) & kMag) | ((w << 8) & kSign), s),
+                           hmul2_bits(((w << 1) & kMag) | ((w << 4) & kSign), s), hmul2_bits(((w >> 3) & kMag) | (w & kSign), s));
+          }
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.exp_full[es]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars.raw_empty[rs]);
+    }
+    // accumulator (lane = weight row, column = batch row) -> partial tile [M][128] over the rings
+    if (ok && warp < 6) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.acc, 0, p.status));
+      tc_fence_after_sync();
+      if (ok) {
+        const int quarter = warp & 3;
+        float* dst = reinterpret_cast<float*>(smem) + quarter * 32 + lane;
+        for (int c = 0; c < p.mp; c += 16) {
+          uint32_t rr[16];
+          tmem_ld_32x32b_x16(tmem + ((uint32_t)(quarter * 32) << 16) + c, rr);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) dst[(c + j) * kCRows] = __uint_as_float(rr[j]);
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (p.splits > 1) cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t partial = smem_u32(smem);
+  switch (p.splits) {
+    case 1: w4_reduce<1>(p, partial, rank, tile, warp, lane); break;
+    case 2: w4_reduce<2>(p, partial, rank, tile, warp, lane); break;
+    case 3: w4_reduce<3>(p, partial, rank, tile, warp, lane); break;
+    case 4: w4_reduce<4>(p, partial, rank, tile, warp, lane); break;
+    case 5: w4_reduce<5>(p, partial, rank, tile, warp, lane); break;
+    case 6: w4_reduce<6>(p, partial, rank, tile, warp, lane); break;
+    case 7: w4_reduce<7>(p, partial, rank, tile, warp, lane); break;
+    default: w4_reduce<8>(p, partial, rank, tile, warp, lane); break;
+  }
+  if (p.splits > 1) cluster_sync_all();
+  else __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, 64);
+}
+
 __global__ void w4s_splitk_reduce_kernel(const float* __restrict__ ws, int splits, int M, int N, bf16* out,
                                          int ldo, const bf16* __restrict__ bias) {
   const size_t total = (size_t)M * N;
@@ -297,7 +498,9 @@ __global__ void w4s_splitk_reduce_kernel(const float* __restrict__ ws, int split
 
 // bf16 -> f16 with saturation (the MMA runs in f16; activations beyond the f16 range clamp).
 __global__ void __launch_bounds__(256)
-    cast_bf16_f16_kernel(const bf16* __restrict__ a, int lda, __half* __restrict__ out, int M, int K) {
+    cast_bf16_f16_kernel(const bf16* __restrict__ a, int lda, __half* __restrict__ out, int M, int K, int nibble_order) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t total = (size_t)M * (K / 8);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int m = (int)(i / (K / 8)), c = (int)(i % (K / 8));
@@ -312,7 +515,11 @@ __global__ void __launch_bounds__(256)
       __half2 h = __floats2half2_rn(f.x, f.y);
       o[j] = *reinterpret_cast<uint32_t*>(&h);
     }
-    *reinterpret_cast<uint4*>(out + (size_t)m * K + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    if (nibble_order)      // 0 4 1 5 2 6 3 7: as the cluster kernel expands the weights
+      *reinterpret_cast<uint4*>(out + (size_t)m * K + c * 8) = make_uint4(__byte_perm(o[0], o[2], 0x5410), __byte_perm(o[0], o[2], 0x7632),
+                                                                          __byte_perm(o[1], o[3], 0x5410), __byte_perm(o[1], o[3], 0x7632));
+    else
+      *reinterpret_cast<uint4*>(out + (size_t)m * K + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -355,15 +562,34 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
   p.splits = splits; p.ne_per_split = ne_per;
   p.workspace = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + a16_bytes);
 
+  const bool cluster = M <= kCRowsMax && (K & 255) == 0 && !(reinterpret_cast<uintptr_t>(sf) & 15) && !(N & 7) &&
+                       !(reinterpret_cast<uintptr_t>(out) & 7);
   __half* a16 = reinterpret_cast<__half*>(workspace);
   {
     const size_t total = (size_t)M * (K / 8);
     int blocks = (int)((total + 255) / 256);
     if (blocks > sms * 4) blocks = sms * 4;
-    cast_bf16_f16_kernel<<<blocks, 256, 0, stream>>>((const bf16*)A, lda, a16, M, K);
-    if (cudaGetLastError() != cudaSuccess) return -2;
+    if (launch_pdl(cast_bf16_f16_kernel, dim3(blocks), dim3(256), 0, stream, (const bf16*)A, lda, a16, M, K,
+                   cluster ? 1 : 0) != cudaSuccess)
+      return -2;
   }
   CUtensorMap tmW, tmA, tmS;
+  if (cluster) {
+    W4CParams c{};
+    c.M = M; c.N = N; c.K = K; c.mp = (M + 15) & ~15;
+    c.out = (bf16*)out; c.ldo = ldo; c.sf = (const uint8_t*)sf; c.gscale = gscale; c.bias = (const bf16*)bias; c.status = device_status_word();
+    const int tiles = (N + kCRows - 1) / kCRows, blocks = K / 256;
+    c.splits = cluster_splits(tiles, blocks / 2);
+    if (!encode_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, K / 2, kCRows, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_tmap_2d(&tmA, a16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, M, K, K, c.mp, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+      return -3;
+    c.act_stages = 24576 / (c.mp * 128) < kCAS ? 24576 / (c.mp * 128) : kCAS;
+    const size_t smem = (size_t)kCES * kCExp + (size_t)c.act_stages * c.mp * 128 + (size_t)kCRS * kCRaw + 1024;
+    static PerDeviceOnce once;
+    if (once.first()) cudaFuncSetAttribute(gemm_w4a16_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+    return launch_cluster_pdl(gemm_w4a16_cluster_kernel, tiles * c.splits, c.splits, kCThreads, smem, stream, tmW, tmA, c) ==
+                   cudaSuccess ? 0 : -2;
+  }
   p.sf_tma = ((K & 255) == 0 && (reinterpret_cast<uintptr_t>(sf) & 15) == 0) ? 1 : 0;
   if (!encode_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, K / 2, kWN, 128,
                       CU_TENSOR_MAP_SWIZZLE_128B))

@@ -83,6 +83,23 @@ def _within_sum_error(out, a64, w64, exp64, extra=0.0):
     return ((out.double() - exp64).abs() <= bound + 1e-30).all().item()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (16, 264, 512), (17, 520, 4096), (64, 4096, 1024), (48, 1032, 14336)])
+def test_w4a16_over_a_cluster(M, N, K):
+    """Up to 64 rows: K split over a cluster of CTAs; row counts at the edges of the 16-row padding, ragged column tiles,
+    one 256-k block and many."""
+    torch.manual_seed(11)
+    packed, sf, g = Q.ref_quant_nvfp4_weights(torch.randn(N, K, device=DEV) * 0.05)
+    a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
+    w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
+    # a small activation is rounded to the 2^-24 grid of f16's subnormals
+    extra = 2**-25 * w64.abs().sum(1)
+    for bias in (None, torch.randn(N, device=DEV).to(torch.bfloat16)):
+        exp = a64 @ w64.t() + (0 if bias is None else bias.double())
+        out = Q.gemm_w4a16(a, packed, sf, g, bias=bias)
+        assert ops.read_status() == 0
+        assert _within_sum_error(out, a64, w64, exp, extra)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 16), (17, 520, 144), (65, 136, 4112), (128, 4104, 8192)])
 @pytest.mark.parametrize("per_token,per_channel", [(False, False), (True, True)])
 def test_gemm_fp8_over_a_cluster(M, N, K, per_token, per_channel):
