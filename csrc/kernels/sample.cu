@@ -257,8 +257,9 @@ struct RowSlice {
   int lo, n;        // first column, columns
 };
 __device__ __forceinline__ int row_slice_cols(int V) { return ((V + kRowCtas - 1) / kRowCtas + 3) & ~3; }
-// Loads this CTA's slice of its row (blockIdx.x / kRowCtas); out-of-place callers pass x as const.
+// Loads this CTA's slice of its row (blockIdx.x / kRowCtas). Every CTA of the cluster runs when it returns.
 __device__ __forceinline__ RowSlice load_row_slice(float* row, int V, float* stage) {
+  cluster_sync_all();
   const int per = row_slice_cols(V), rank = (int)cluster_ctarank();
   RowSlice s;
   s.lo = min(V, rank * per);
@@ -281,23 +282,24 @@ __device__ __forceinline__ RowSlice load_row_slice(float* row, int V, float* sta
   }
   return s;
 }
-// Exchange of one value of W words per CTA; two buffers in turn, so that one cluster barrier a call is enough.
+// Exchange of W words per CTA: each CTA stores its own into every CTA of the cluster, and after one cluster barrier all
+// threads read them at home. Two buffers in turn, so that one barrier a call is enough.
 template <int W>
 struct RowExchange {
-  float slot[2][W];
+  float slot[2][kRowCtas][W];
 };
 template <int W>
 __device__ __forceinline__ void row_gather(RowExchange<W>& ex, int turn, const float (&mine)[W], float (&all)[kRowCtas][W]) {
-  if (threadIdx.x == 0)
+  if (threadIdx.x < kRowCtas) {
+    const uint32_t to = mapa_u32(smem_u32(&ex.slot[turn & 1][cluster_ctarank()][0]), threadIdx.x);
 #pragma unroll
-    for (int w = 0; w < W; ++w) ex.slot[turn & 1][w] = mine[w];
+    for (int w = 0; w < W; ++w) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * w), "f"(mine[w]) : "memory");
+  }
   cluster_sync_all();
-  const uint32_t a = smem_u32(&ex.slot[turn & 1][0]);
 #pragma unroll
   for (int r = 0; r < kRowCtas; ++r)
 #pragma unroll
-    for (int w = 0; w < W; ++w)
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(all[r][w]) : "r"(mapa_u32(a, r) + 4 * w) : "memory");
+    for (int w = 0; w < W; ++w) all[r][w] = ex.slot[turn & 1][r][w];
 }
 // Sums of W numbers a thread over the whole row (counts stay exact up to 2^24).
 template <int W>
@@ -420,7 +422,6 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
 #pragma unroll 4
   for (int i = threadIdx.x; i < s.n; i += kRowThreads)
     if (fkey(s.v[i]) < thr_key) s.x[i] = -INFINITY;
-  cluster_sync_all();                                  // nobody reads this CTA's sums any more
 }
 
 // ---- softmax / log-softmax (out may alias in) ----
@@ -450,7 +451,6 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
 #pragma unroll 4
     for (int i = threadIdx.x; i < s.n; i += kRowThreads) o[i] = __expf(s.v[i] - mx) * inv;
   }
-  cluster_sync_all();
 }
 
 // ---- seeded exponential-race sample: argmax_i p_i / (-log u_i) ----
@@ -474,6 +474,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
   __shared__ ArgPair sh[32];
   __shared__ RowExchange<2> ex;
   const int row = blockIdx.x / kRowCtas, per = row_slice_cols(V), lo = min(V, (int)cluster_ctarank() * per), hi = min(V, lo + per);
+  cluster_sync_all();                                  // (before the first store into another CTA)
   const float* x = probs + (size_t)row * ld;
   const uint64_t seed = seeds[row], step = steps[row];
   ArgPair a{-FLT_MAX, 0x7fffffff};
@@ -491,7 +492,6 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
     for (int r = 1; r < kRowCtas; ++r) a = arg_better(a, ArgPair{all[r][0], __float_as_int(all[r][1])});
     out[row] = (a.i >= V || a.i < 0) ? 0 : a.i;
   }
-  cluster_sync_all();
 }
 
 // out[row] = is_greedy ? greedy[row] : random[row]
