@@ -150,10 +150,13 @@ __global__ void __launch_bounds__(256)
 //   mode 1  v = RMSNorm(x (+ residual, written back)) -- the arithmetic of rmsnorm_kernel, so the
 //           normalised row has the bytes the bf16 path would hand to its GEMM
 //   mode 2  v = act(gate) * up from [gate | up] rows (kind_flags as act_and_mul_kernel takes them)
-// The row (bf16) stays in shared memory between the producer and the quantisation.
-__global__ void __launch_bounds__(256)
+// The row (bf16) stays in shared memory between the producer and the quantisation. One kernel per mode and activation,
+// packed maxima and conversions: bound by instructions, then by memory (8192 rows, us: plain 4096 31.0 -> 21.9, 4.6 TB/s;
+// act 14336 152 -> 146, its exponential and division).
+template <int MODE, int KIND>
+__global__ void __launch_bounds__(MODE == 1 ? 256 : 1024)
     rowquant_fp8_kernel(const __nv_bfloat16* __restrict__ x, long ldx, __nv_bfloat16* residual,
-                        const __nv_bfloat16* __restrict__ w, float eps, int gemma, int mode, int kind_flags,
+                        const __nv_bfloat16* __restrict__ w, float eps, int gemma, int interleaved,
                         uint8_t* __restrict__ out, long ldo, float* __restrict__ scales, int K) {
   __shared__ float red[32];
   extern __shared__ uint4 row_cache[];  // K/8 vectors
@@ -161,15 +164,14 @@ __global__ void __launch_bounds__(256)
   pdl_launch_dependents();
   const long t = blockIdx.x;
   const int nv = K >> 3;
-  float amax = 0.f;
+  // (maximum of magnitudes in packed bf16: exact, NaNs drop out as with fmaxf)
+  __nv_bfloat162 amax2 = __floats2bfloat162_rn(0.f, 0.f);
   auto vec_amax = [&](const uint4& v) {
-    float2 f;
-    f = unpack_bf16x2(v.x); amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    f = unpack_bf16x2(v.y); amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    f = unpack_bf16x2(v.z); amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    f = unpack_bf16x2(v.w); amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) amax2 = __hmax2(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w4[j])));
   };
-  if (mode == 1) {
+  if constexpr (MODE == 1) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + t * ldx);
     uint4* rr = residual ? reinterpret_cast<uint4*>(residual + t * (long)K) : nullptr;
     float ss = 0.f;
@@ -207,31 +209,33 @@ __global__ void __launch_bounds__(256)
       row_cache[i] = o;
       vec_amax(o);
     }
-  } else if (mode == 2) {
-    const int kind = kind_flags & 0xff;
-    const bool il = (kind_flags & 0x100) != 0;
+  } else if constexpr (MODE == 2) {
+    const bool il = interleaved != 0;
+#pragma unroll 2
     for (int i = threadIdx.x; i < nv; i += blockDim.x) {
       const int goff = il ? ((i * 8) >> 7) * 256 + ((i * 8) & 127) : i * 8;
       const int uoff = il ? goff + 128 : K + i * 8;
-      const uint4 gt = *reinterpret_cast<const uint4*>(x + t * ldx + goff);
-      const uint4 u = *reinterpret_cast<const uint4*>(x + t * ldx + uoff);
+      const uint4 gt = __ldg(reinterpret_cast<const uint4*>(x + t * ldx + goff));
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + t * ldx + uoff));
       uint4 o;
       float2 a, b;
-      a = unpack_bf16x2(gt.x); b = unpack_bf16x2(u.x); o.x = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
-      a = unpack_bf16x2(gt.y); b = unpack_bf16x2(u.y); o.y = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
-      a = unpack_bf16x2(gt.z); b = unpack_bf16x2(u.z); o.z = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
-      a = unpack_bf16x2(gt.w); b = unpack_bf16x2(u.w); o.w = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
+      a = unpack_bf16x2(gt.x); b = unpack_bf16x2(u.x); o.x = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.y); b = unpack_bf16x2(u.y); o.y = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.z); b = unpack_bf16x2(u.z); o.z = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.w); b = unpack_bf16x2(u.w); o.w = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
       row_cache[i] = o;
       vec_amax(o);
     }
   } else {
     const uint4* xr = reinterpret_cast<const uint4*>(x + t * ldx);
+#pragma unroll 2
     for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      const uint4 v = xr[i];
+      const uint4 v = __ldg(xr + i);
       row_cache[i] = v;
       vec_amax(v);
     }
   }
+  float amax = fmaxf(__low2float(amax2), __high2float(amax2));
   // block maximum (every thread re-reads only the vectors it wrote, so no barrier is needed for
   // row_cache itself)
 #pragma unroll
@@ -252,7 +256,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 f = unpack_bf16x2(wds[j]);
-      const uint32_t two = (uint32_t)float_to_e4m3(f.x * is) | ((uint32_t)float_to_e4m3(f.y * is) << 8);
+      const uint32_t two = __nv_cvt_float2_to_fp8x2(make_float2(f.x * is, f.y * is), __NV_SATFINITE, __NV_E4M3);
       if (j < 2) lo |= two << (16 * j); else hi |= two << (16 * (j - 2));
     }
     *reinterpret_cast<uint2*>(out + t * ldo + (long)i * 8) = make_uint2(lo, hi);
@@ -384,13 +388,20 @@ int b200_quant_fp8_rowwise(const void* x, long ldx, void* residual, const void* 
   if ((K & 7) || (ldx & 7) || (ldo & 7) || K > 32768 || mode < 0 || mode > 2) return -1;
   if (((uintptr_t)x & 15) || ((uintptr_t)out & 7) || (mode == 1 && !norm_w)) return -1;
   if (mode == 2 && (kind_flags & 0x100) && (K & 127)) return -1;
-  int threads = K / 8 >= 256 ? 256 : ((K / 8 + 31) / 32) * 32;
+  // Few rows leave SMs idle and are bound by the latency of a thread's loads: up to 1024 threads a row (32 rows, act
+  // 14336: 7.8 -> 4.5 us); beyond two rows an SM the other rows cover it. Mode 1 adds in rmsnorm_kernel's order: 256.
+  const int most = mode == 1 || T > 2 * b200_num_sms() ? 256 : 1024;
+  int threads = K / 8 >= most ? most : ((K / 8 + 31) / 32) * 32;
   if (threads < 32) threads = 32;
-  static PerDeviceOnce attr_once;
-  if (attr_once.first())
-    cudaFuncSetAttribute(rowquant_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 2);
-  return launch_pdl(rowquant_fp8_kernel, dim3(T), dim3(threads), (size_t)K * 2, stream, (const bf16*)x, ldx, (bf16*)residual,
-                    (const bf16*)norm_w, eps, gemma, mode, kind_flags, (uint8_t*)out, ldo, (float*)scales, K) == cudaSuccess
+  const int kind = kind_flags & 0xff;
+  auto kernel = mode == 0 ? rowquant_fp8_kernel<0, 0> : mode == 1 ? rowquant_fp8_kernel<1, 0>
+              : kind == kSilu ? rowquant_fp8_kernel<2, kSilu> : kind == kGeluTanh ? rowquant_fp8_kernel<2, kGeluTanh>
+                                                                                  : rowquant_fp8_kernel<2, kGeluTanh + 1>;
+  static PerDeviceOnce attr_once[5];
+  if (attr_once[mode < 2 ? mode : kind == kSilu ? 2 : kind == kGeluTanh ? 3 : 4].first())
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 2);
+  return launch_pdl(kernel, dim3(T), dim3(threads), (size_t)K * 2, stream, (const bf16*)x, ldx, (bf16*)residual,
+                    (const bf16*)norm_w, eps, gemma, (kind_flags >> 8) & 1, (uint8_t*)out, ldo, (float*)scales, K) == cudaSuccess
              ? 0 : -2;
 }
 

@@ -117,6 +117,26 @@ def test_gemm_fp8_over_a_cluster(M, N, K, per_token, per_channel):
         assert _within_sum_error(out, a64, w64, exp)
 
 
+@pytest.mark.parametrize("T", [1, 296, 297])
+@pytest.mark.parametrize("K", [8, 264, 2056, 14336, 32768])
+def test_rowwise_fp8_of_few_and_many_rows(T, K):
+    """Up to 1024 threads a row for few rows, 256 for many; the bytes are those of the rounded row's quotients."""
+    torch.manual_seed(T + K)
+    x = torch.randn(T, K + 8, device=DEV).to(torch.bfloat16)[:, :K]
+    q, sc = Q.quant_fp8_rowwise(x)
+    top = x.float().abs().amax(1).clamp_min(1e-12)
+    exp_sc = top / torch.full_like(top, 448)           # (a scalar divisor would become a product with its reciprocal)
+    assert torch.equal(sc.reshape(-1), exp_sc)
+    assert torch.equal(q.view(torch.uint8), (x.float() * (torch.ones_like(top) / exp_sc)[:, None]).to(torch.float8_e4m3fn).view(torch.uint8))
+    if K > 16384:
+        return
+    gu = torch.randn(T, 2 * K, device=DEV).to(torch.bfloat16)
+    for kind in (0, 1, 2):
+        a8, a_sc = Q.quant_fp8_rowwise(gu, act_kind=kind)
+        b8, b_sc = Q.quant_fp8_rowwise(ops.act_and_mul(gu, kind))
+        assert torch.equal(a_sc, b_sc) and torch.equal(a8.view(torch.uint8), b8.view(torch.uint8))
+
+
 def test_quant_fp8_static_and_rmsnorm():
     torch.manual_seed(2)
     x = (torch.randn(37, 512, device=DEV) * 3).to(torch.bfloat16)
