@@ -32,7 +32,7 @@ NativeRunner::NativeRunner(std::unique_ptr<DenseModel> model, int block_size, in
       max_num_seqs_(max_num_seqs), max_tokens_(std::max(max_num_batched_tokens, max_num_seqs)),
       max_model_len_(max_model_len), max_blocks_((max_model_len + block_size - 1) / block_size + 1),
       layout_(StepLayout::make(max_tokens_, max_num_seqs, max_blocks_, 1, 0)),
-      batch_(max_num_seqs, max_model_len, max_tokens_, std::vector<int>{block_size}) {
+      batch_(max_num_seqs, max_model_len, max_tokens_, std::vector<int>{block_size}), staged_(dev_) {
   set_device(dev_);
   if (dev_.cuda && b200_init_device() != 0) throw std::runtime_error("kernel library: device set-up failed");
   model_->alloc_kv_cache(num_blocks, block_size);
@@ -74,10 +74,13 @@ void NativeRunner::execute_model(const SchedulerOutput& so) {
     return;
   }
   set_device(dev_);
+  // a step that samples nothing (a chunk of a long prompt) is not waited for: its copy may still have to read the buffer
+  staged_.synchronize();
   info_ = batch_.prepare(so, layout_, host_buf_.as<uint8_t>(), /*async_mode=*/false);
   const StepInfo& info = *info_;
   if (dev_.cuda) {
     copy(dev_buf_.data(), dev_, host_buf_.data(), Device{}, layout_.total_bytes);
+    staged_.record();
     h2d_bytes += (int64_t)layout_.total_bytes;
   }
   StepInputs in;

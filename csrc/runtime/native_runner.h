@@ -39,6 +39,7 @@ class NativeRunner : public ModelRunnerBase {
   StepLayout layout_;
   InputBatch batch_;
   Buffer host_buf_, dev_buf_, sampled_dev_, sampled_host_, scratch_dev_, probs_dev_, status_host_;
+  Event staged_;                    // behind the copy out of host_buf_
   uint8_t* dev_base_ = nullptr;
   std::optional<StepInfo> info_;
   float* logits_ = nullptr;

@@ -96,20 +96,25 @@ void free_and_total_memory(Device d, size_t* f, size_t* t) {
 }
 
 Event::Event(Device d) {
-  if (d.cuda) {
-    cudaEvent_t e;
-    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) ev_ = e;
-    stream_dev_ = d.index;
-  }
+  if (!d.cuda) return;
+  set_device(d);                    // an event belongs to the device that is current when it is created
+  cudaEvent_t e;
+  if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+    throw std::runtime_error(std::string("cudaEventCreate failed: ") + cudaGetErrorString(cudaGetLastError()));
+  ev_ = e;
+  stream_dev_ = d.index;
 }
 Event::~Event() {
   if (ev_) cudaEventDestroy((cudaEvent_t)ev_);
 }
 void Event::record() {
-  if (ev_) cudaEventRecord((cudaEvent_t)ev_, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)stream_dev_).stream());
+  if (!ev_) return;
+  if (cudaEventRecord((cudaEvent_t)ev_, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)stream_dev_).stream()) != cudaSuccess)
+    throw std::runtime_error(std::string("cudaEventRecord failed: ") + cudaGetErrorString(cudaGetLastError()));
 }
 void Event::synchronize() {
-  if (ev_) cudaEventSynchronize((cudaEvent_t)ev_);
+  if (ev_ && cudaEventSynchronize((cudaEvent_t)ev_) != cudaSuccess)
+    throw std::runtime_error(std::string("cudaEventSynchronize failed: ") + cudaGetErrorString(cudaGetLastError()));
 }
 
 }  // namespace b200::rt

@@ -48,10 +48,12 @@ void memset_zero(void* p, Device d, size_t n);
 void synchronize(Device d);                    // waits for the current stream
 void free_and_total_memory(Device d, size_t* free_bytes, size_t* total_bytes);
 
-// CUDA events for the asynchronous device->host copy of sampled ids.
+// A CUDA event (nothing on CPU): says when the work ahead of it on the stream has run.
 class Event {
  public:
   explicit Event(Device d);
+  Event(const Event&) = delete;
+  Event& operator=(const Event&) = delete;
   ~Event();
   void record();          // on the device's current stream
   void synchronize();

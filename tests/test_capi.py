@@ -384,3 +384,45 @@ def test_native_library_on_the_gpu_matches_the_python_engine(lib, ckpt_gpu):
         lib.vllm_completion_free(ctypes.byref(out))
     assert got[0] == got[1]
     lib.vllm_engine_free(eng)
+
+
+@pytest.mark.gpu
+def test_native_runner_chunks_of_a_long_prompt_behind_a_busy_gpu(lib, tmp_path):
+    """Chunks that sample nothing are not waited for: the inputs of a chunk must still be in the pinned buffer when the copy
+    of them runs, also with the GPU far behind the host. Five chunks of up to 2048 tokens, of which four sample nothing."""
+    import random
+
+    import torch
+
+    from vllm_cpp_b200 import loader
+    from vllm_cpp_b200.config import EngineArgs, synthetic_config
+    from vllm_cpp_b200.engine import LLM, SamplingParams as SP
+    cfg = synthetic_config("tiny-qwen3")
+    cfg.head_dim, cfg.tie_word_embeddings = 128, False
+    path = loader.write_synthetic_checkpoint(str(tmp_path / "ck"), cfg, seed=6, std=0.05)
+    r = random.Random(1)
+    prompt = " ".join("".join(r.choice("abcdefghij") for _ in range(r.randint(2, 7))) for _ in range(2000))
+    llm = LLM(EngineArgs(model=path, device="cuda", block_size=16, num_blocks=800, max_model_len=12288, max_num_seqs=2,
+                         max_num_batched_tokens=2048, enable_cuda_graphs=False))
+    tokens = llm.tokenizer.encode(prompt)
+    assert 4 * 2048 < len(tokens) < 12000
+    llm.add_request(tokens, SP(temperature=0.0, max_tokens=24, ignore_eos=True))
+    want = ""
+    while llm.has_unfinished_requests():
+        for out in llm.step():
+            want = out.outputs[0].text if out.finished else want
+        torch.cuda.synchronize()
+    del llm
+    mp = lib.vllm_model_params_default()
+    mp.model_path, mp.max_model_len, mp.block_size, mp.num_blocks = path.encode(), 12288, 16, 800
+    eng = ctypes.c_void_p()
+    opt = EngineOptions(ctypes.sizeof(EngineOptions), 1, 0, b"cuda")
+    assert lib.vllm_engine_load_ex(ctypes.byref(mp), ctypes.byref(opt), ctypes.byref(eng)) == 0, lib.vllm_last_error()
+    sp = lib.vllm_sampling_params_default()
+    sp.temperature, sp.max_tokens, sp.ignore_eos = 0.0, 24, 1
+    out = Completion()
+    torch.cuda._sleep(400_000_000)                        # about 0.2 s of work ahead of the first copy
+    assert lib.vllm_complete(eng, prompt.encode(), ctypes.byref(sp), ctypes.byref(out)) == 0, lib.vllm_last_error()
+    assert out.prompt_tokens == len(tokens) and ctypes.string_at(out.text).decode() == want
+    lib.vllm_completion_free(ctypes.byref(out))
+    lib.vllm_engine_free(eng)
