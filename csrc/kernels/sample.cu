@@ -43,18 +43,6 @@ __device__ __forceinline__ ArgPair block_argmax(ArgPair a, ArgPair* sh) {
   __syncthreads();
   return r;
 }
-__device__ __forceinline__ float block_reduce_sum(float v, float* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  float r = (lane < nw) ? sh[lane] : 0.f;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-  __syncthreads();
-  return r;
-}
 __device__ __forceinline__ float block_reduce_max(float v, float* sh) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -245,10 +233,10 @@ __device__ __forceinline__ float fkey_inv(uint32_t k) {
   uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
   return __uint_as_float(u);
 }
-// A row belongs to a cluster of kRowCtas CTAs: one SM alone reads a vocabulary of 150000 logits at the pace of its own
-// loads. Each CTA keeps its slice in shared memory (rows too long for that are read from memory again), sums are taken
-// within the CTA in a fixed order and then over the cluster in the order of its CTAs.
-static constexpr int kRowCtas = 8, kRowThreads = 512;
+// A row belongs to a cluster of CTAS CTAs: eight for a long row, as one SM alone reads a vocabulary of 150000 logits at the
+// pace of its own loads; one for a short row, whose passes are all barrier (row_ctas). Each CTA keeps its slice in shared
+// memory (rows too long for that are read from memory again), sums are taken within the CTA in a fixed order and then over
+// the cluster in the order of its CTAs.
 static constexpr int kMostStaged = 200 * 1024;      // bytes of a slice in shared memory
 
 struct RowSlice {
@@ -256,11 +244,21 @@ struct RowSlice {
   const float* v;   // where to read it (shared memory, or x)
   int lo, n;        // first column, columns
 };
-__device__ __forceinline__ int row_slice_cols(int V) { return ((V + kRowCtas - 1) / kRowCtas + 3) & ~3; }
-// Loads this CTA's slice of its row (blockIdx.x / kRowCtas). Every CTA of the cluster runs when it returns.
+__host__ __device__ __forceinline__ int row_slice_cols(int V, int ctas) { return ((V + ctas - 1) / ctas + 3) & ~3; }
+template <int CTAS>
+__device__ __forceinline__ int row_rank() {
+  if constexpr (CTAS > 1) return (int)cluster_ctarank();
+  return 0;
+}
+template <int CTAS>
+__device__ __forceinline__ void row_sync() {
+  if constexpr (CTAS > 1) cluster_sync_all();
+}
+// Loads this CTA's slice of its row (blockIdx.x / CTAS). Every CTA of the cluster runs when it returns.
+template <int CTAS, int T>
 __device__ __forceinline__ RowSlice load_row_slice(float* row, int V, float* stage) {
-  cluster_sync_all();
-  const int per = row_slice_cols(V), rank = (int)cluster_ctarank();
+  row_sync<CTAS>();
+  const int per = row_slice_cols(V, CTAS), rank = row_rank<CTAS>();
   RowSlice s;
   s.lo = min(V, rank * per);
   s.n = min(V, s.lo + per) - s.lo;
@@ -270,12 +268,12 @@ __device__ __forceinline__ RowSlice load_row_slice(float* row, int V, float* sta
     if (!(reinterpret_cast<uintptr_t>(s.x) & 15)) {
       const int n4 = s.n & ~3;
 #pragma unroll 4
-      for (int i = threadIdx.x * 4; i < n4; i += kRowThreads * 4)
+      for (int i = threadIdx.x * 4; i < n4; i += T * 4)
         *reinterpret_cast<float4*>(stage + i) = *reinterpret_cast<const float4*>(s.x + i);
-      for (int i = n4 + threadIdx.x; i < s.n; i += kRowThreads) stage[i] = s.x[i];
+      for (int i = n4 + threadIdx.x; i < s.n; i += T) stage[i] = s.x[i];
     } else {
 #pragma unroll 4
-      for (int i = threadIdx.x; i < s.n; i += kRowThreads) stage[i] = s.x[i];
+      for (int i = threadIdx.x; i < s.n; i += T) stage[i] = s.x[i];
     }
     s.v = stage;
     __syncthreads();
@@ -284,26 +282,31 @@ __device__ __forceinline__ RowSlice load_row_slice(float* row, int V, float* sta
 }
 // Exchange of W words per CTA: each CTA stores its own into every CTA of the cluster, and after one cluster barrier all
 // threads read them at home. Two buffers in turn, so that one barrier a call is enough.
-template <int W>
+template <int CTAS, int W>
 struct RowExchange {
-  float slot[2][kRowCtas][W];
+  float slot[2][CTAS][W];
 };
-template <int W>
-__device__ __forceinline__ void row_gather(RowExchange<W>& ex, int turn, const float (&mine)[W], float (&all)[kRowCtas][W]) {
-  if (threadIdx.x < kRowCtas) {
+template <int CTAS, int W>
+__device__ __forceinline__ void row_gather(RowExchange<CTAS, W>& ex, int turn, const float (&mine)[W], float (&all)[CTAS][W]) {
+  if constexpr (CTAS == 1) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) all[0][w] = mine[w];
+    return;
+  }
+  if (threadIdx.x < CTAS) {
     const uint32_t to = mapa_u32(smem_u32(&ex.slot[turn & 1][cluster_ctarank()][0]), threadIdx.x);
 #pragma unroll
     for (int w = 0; w < W; ++w) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * w), "f"(mine[w]) : "memory");
   }
   cluster_sync_all();
 #pragma unroll
-  for (int r = 0; r < kRowCtas; ++r)
+  for (int r = 0; r < CTAS; ++r)
 #pragma unroll
     for (int w = 0; w < W; ++w) all[r][w] = ex.slot[turn & 1][r][w];
 }
 // Sums of W numbers a thread over the whole row (counts stay exact up to 2^24).
-template <int W>
-__device__ __forceinline__ void row_sum(RowExchange<W>& ex, int turn, float (&v)[W], float (&sh)[kRowThreads / 32][W]) {
+template <int CTAS, int T, int W>
+__device__ __forceinline__ void row_sum(RowExchange<CTAS, W>& ex, int turn, float (&v)[W], float (&sh)[T / 32][W]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int w = 0; w < W; ++w)
@@ -316,48 +319,50 @@ __device__ __forceinline__ void row_sum(RowExchange<W>& ex, int turn, float (&v)
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < W; ++w) {
-    float r = lane < kRowThreads / 32 ? sh[lane][w] : 0.f;
+    float r = lane < T / 32 ? sh[lane][w] : 0.f;
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    for (int o = T / 64; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
     v[w] = __shfl_sync(0xffffffffu, r, 0);
   }
-  float all[kRowCtas][W];
-  row_gather<W>(ex, turn, v, all);
+  float all[CTAS][W];
+  row_gather<CTAS, W>(ex, turn, v, all);
 #pragma unroll
   for (int w = 0; w < W; ++w) {
     v[w] = all[0][w];
 #pragma unroll
-    for (int r = 1; r < kRowCtas; ++r) v[w] += all[r][w];
+    for (int r = 1; r < CTAS; ++r) v[w] += all[r][w];
   }
 }
-__device__ __forceinline__ float row_max(RowExchange<1>& ex, int turn, float v, float* sh) {
+template <int CTAS>
+__device__ __forceinline__ float row_max(RowExchange<CTAS, 1>& ex, int turn, float v, float* sh) {
   const float mine[1] = {block_reduce_max(v, sh)};
-  float all[kRowCtas][1];
-  row_gather<1>(ex, turn, mine, all);
+  float all[CTAS][1];
+  row_gather<CTAS, 1>(ex, turn, mine, all);
   v = all[0][0];
 #pragma unroll
-  for (int r = 1; r < kRowCtas; ++r) v = fmaxf(v, all[r][0]);
+  for (int r = 1; r < CTAS; ++r) v = fmaxf(v, all[r][0]);
   return v;
 }
 
-// One cluster per row. top-k: radix select of the k-th largest key, two bits a pass (count based). top-p: the same search
+// top-k: radix select of the k-th largest key, two bits a pass (count based). top-p: the same search
 // for the largest threshold whose kept mass is >= p. Ties at the threshold are all kept (same as the sort-based rule for
 // distinct logits). Bound by the passes' barriers and shared-memory reads, about 2 us a pass, at most 32 passes: 40 rows of
 // 151936 with k = 50, p = 0.95 took 7717 us with a block of 256 threads per row that read the row from L2 for every bit.
-__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
+template <int CTAS, int T>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(T)
     top_k_top_p_kernel(float* logits, int ld, int V, const int* __restrict__ top_k,
                        const float* __restrict__ top_p) {
   extern __shared__ float4 stage_raw[];
-  __shared__ RowExchange<1> ex1;
-  __shared__ RowExchange<3> ex3;
-  __shared__ float sh1[kRowThreads / 32][1], sh3[kRowThreads / 32][3], shm[32];
-  const int row = blockIdx.x / kRowCtas;
+  __shared__ RowExchange<CTAS, 1> ex1;
+  __shared__ RowExchange<CTAS, 3> ex3;
+  __shared__ float sh1[T / 32][1], sh3[T / 32][3], shm[32];
+  const int row = blockIdx.x / CTAS;
   const int k = top_k ? top_k[row] : 0;
   const float pth = top_p ? top_p[row] : 1.f;
   const bool do_k = (k > 0 && k < V);
   const bool do_p = (pth < 1.f);
   if (!do_k && !do_p) return;                          // (the whole cluster)
-  const RowSlice s = load_row_slice(logits + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
+  const RowSlice s = load_row_slice<CTAS, T>(logits + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
   uint32_t thr_key = 0;
   int turn = 0;
   if (do_k) {
@@ -367,12 +372,12 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
       const uint32_t c1 = prefix | (1u << bit), c2 = prefix | (2u << bit), c3 = prefix | (3u << bit);
       int n1 = 0, n2 = 0, n3 = 0;
 #pragma unroll 4
-      for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+      for (int i = threadIdx.x; i < s.n; i += T) {
         const uint32_t kk = fkey(s.v[i]);
         n1 += kk >= c1; n2 += kk >= c2; n3 += kk >= c3;
       }
       float c[3] = {(float)n1, (float)n2, (float)n3};
-      row_sum<3>(ex3, turn, c, sh3);
+      row_sum<CTAS, T, 3>(ex3, turn, c, sh3);
       if (c[2] >= (float)k) prefix = c3;
       else if (c[1] >= (float)k) prefix = c2;
       else if (c[0] >= (float)k) prefix = c1;
@@ -382,18 +387,18 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
   if (do_p) {
     float mx = -FLT_MAX;
 #pragma unroll 4
-    for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+    for (int i = threadIdx.x; i < s.n; i += T) {
       const float v = s.v[i];
       if (fkey(v) >= thr_key) mx = fmaxf(mx, v);
     }
-    mx = row_max(ex1, 0, mx, shm);
+    mx = row_max<CTAS>(ex1, 0, mx, shm);
     float tot[1] = {0.f};
 #pragma unroll 4
-    for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+    for (int i = threadIdx.x; i < s.n; i += T) {
       const float v = s.v[i];
       if (fkey(v) >= thr_key) tot[0] += __expf(v - mx);
     }
-    row_sum<1>(ex1, 1, tot, sh1);
+    row_sum<CTAS, T, 1>(ex1, 1, tot, sh1);
     const float need = pth * tot[0];
     // largest key T (>= thr_key) with mass(key >= T) >= need
     uint32_t prefix = 0;
@@ -402,7 +407,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
       const uint32_t least = c1 > thr_key ? c1 : thr_key;
       float m[3] = {0.f, 0.f, 0.f};
 #pragma unroll 4
-      for (int i = threadIdx.x; i < s.n; i += kRowThreads) {
+      for (int i = threadIdx.x; i < s.n; i += T) {
         const float v = s.v[i];
         const uint32_t kk = fkey(v);
         if (kk >= least) {
@@ -412,7 +417,7 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
           m[2] += kk >= c3 ? e : 0.f;
         }
       }
-      row_sum<3>(ex3, turn, m, sh3);
+      row_sum<CTAS, T, 3>(ex3, turn, m, sh3);
       if (m[2] >= need) prefix = c3;
       else if (m[1] >= need) prefix = c2;
       else if (m[0] >= need) prefix = c1;
@@ -420,36 +425,37 @@ __global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
     if (prefix > thr_key) thr_key = prefix;
   }
 #pragma unroll 4
-  for (int i = threadIdx.x; i < s.n; i += kRowThreads)
+  for (int i = threadIdx.x; i < s.n; i += T)
     if (fkey(s.v[i]) < thr_key) s.x[i] = -INFINITY;
 }
 
 // ---- softmax / log-softmax (out may alias in) ----
-// One cluster per row (331 us for 40 rows of 151936 with a block of 256 threads per row).
-__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
+// (40 rows of 151936: 331 us with a block of 256 threads per row, 15 with a cluster.)
+template <int CTAS, int T>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(T)
     softmax_kernel(const float* logits, int ld, float* out, int ldo, int V, int log_mode) {
   extern __shared__ float4 stage_raw[];
-  __shared__ RowExchange<1> ex;
-  __shared__ float sh[kRowThreads / 32][1], shm[32];
-  const int row = blockIdx.x / kRowCtas;
-  const RowSlice s = load_row_slice(const_cast<float*>(logits) + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
+  __shared__ RowExchange<CTAS, 1> ex;
+  __shared__ float sh[T / 32][1], shm[32];
+  const int row = blockIdx.x / CTAS;
+  const RowSlice s = load_row_slice<CTAS, T>(const_cast<float*>(logits) + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
   float* o = out + (size_t)row * ldo + s.lo;
   float mx = -FLT_MAX;
 #pragma unroll 4
-  for (int i = threadIdx.x; i < s.n; i += kRowThreads) mx = fmaxf(mx, s.v[i]);
-  mx = row_max(ex, 0, mx, shm);
+  for (int i = threadIdx.x; i < s.n; i += T) mx = fmaxf(mx, s.v[i]);
+  mx = row_max<CTAS>(ex, 0, mx, shm);
   float sum[1] = {0.f};
 #pragma unroll 4
-  for (int i = threadIdx.x; i < s.n; i += kRowThreads) sum[0] += __expf(s.v[i] - mx);
-  row_sum<1>(ex, 1, sum, sh);
+  for (int i = threadIdx.x; i < s.n; i += T) sum[0] += __expf(s.v[i] - mx);
+  row_sum<CTAS, T, 1>(ex, 1, sum, sh);
   if (log_mode) {
     const float lz = mx + logf(sum[0]);
 #pragma unroll 4
-    for (int i = threadIdx.x; i < s.n; i += kRowThreads) o[i] = s.v[i] - lz;
+    for (int i = threadIdx.x; i < s.n; i += T) o[i] = s.v[i] - lz;
   } else {
     const float inv = 1.f / sum[0];
 #pragma unroll 4
-    for (int i = threadIdx.x; i < s.n; i += kRowThreads) o[i] = __expf(s.v[i] - mx) * inv;
+    for (int i = threadIdx.x; i < s.n; i += T) o[i] = __expf(s.v[i] - mx) * inv;
   }
 }
 
@@ -466,30 +472,31 @@ __device__ __forceinline__ float race_key(float prob, uint64_t seed, uint64_t st
   const float e = (float)(-log(u));
   return prob / e;
 }
-// One cluster per row (117 us for 40 rows of 151936 with a block of 256 threads per row).
-__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
+// (40 rows of 151936 dense probabilities: 314 us with a block of 256 threads per row, 52 with a cluster.)
+template <int CTAS, int T>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(T)
     random_sample_kernel(const float* __restrict__ probs, int ld, int V,
                          const uint64_t* __restrict__ seeds, const uint64_t* __restrict__ steps,
                          int64_t* out) {
   __shared__ ArgPair sh[32];
-  __shared__ RowExchange<2> ex;
-  const int row = blockIdx.x / kRowCtas, per = row_slice_cols(V), lo = min(V, (int)cluster_ctarank() * per), hi = min(V, lo + per);
-  cluster_sync_all();                                  // (before the first store into another CTA)
+  __shared__ RowExchange<CTAS, 2> ex;
+  const int row = blockIdx.x / CTAS, per = row_slice_cols(V, CTAS), lo = min(V, row_rank<CTAS>() * per), hi = min(V, lo + per);
+  row_sync<CTAS>();                                    // (before the first store into another CTA)
   const float* x = probs + (size_t)row * ld;
   const uint64_t seed = seeds[row], step = steps[row];
   ArgPair a{-FLT_MAX, 0x7fffffff};
 #pragma unroll 4
-  for (int i = lo + threadIdx.x; i < hi; i += kRowThreads) {
+  for (int i = lo + threadIdx.x; i < hi; i += T) {
     const float pr = x[i];
     if (pr > 0.f) a = arg_better(a, ArgPair{race_key(pr, seed, step, i), i});
   }
   a = block_argmax(a, sh);
   const float mine[2] = {a.v, __int_as_float(a.i)};
-  float all[kRowCtas][2];
-  row_gather<2>(ex, 0, mine, all);
-  if (cluster_ctarank() == 0 && threadIdx.x == 0) {
+  float all[CTAS][2];
+  row_gather<CTAS, 2>(ex, 0, mine, all);
+  if (row_rank<CTAS>() == 0 && threadIdx.x == 0) {
     a = ArgPair{all[0][0], __float_as_int(all[0][1])};
-    for (int r = 1; r < kRowCtas; ++r) a = arg_better(a, ArgPair{all[r][0], __float_as_int(all[r][1])});
+    for (int r = 1; r < CTAS; ++r) a = arg_better(a, ArgPair{all[r][0], __float_as_int(all[r][1])});
     out[row] = (a.i >= V || a.i < 0) ? 0 : a.i;
   }
 }
@@ -556,9 +563,27 @@ __global__ void scatter_sampled_kernel(int64_t* last_sampled, const int* __restr
   if (i < n && row_of[i] >= 0) last_sampled[row_of[i]] = sampled[i];
 }
 
-static size_t row_stage_bytes(int V) {
-  const size_t bytes = (size_t)((((V + kRowCtas - 1) / kRowCtas) + 3) & ~3) * 4;
+// CTAs of a row. A pass of eight CTAs ends in a cluster barrier, which takes the longer the more clusters there are, one of
+// a single CTA reads the whole row: us with one / eight CTAs, and with a block of 256 threads that reads the row from L2
+// for every bit. top-k with top-p, 4000 columns: 1 row 32 / 41 (84), 120 rows 34 / 200 (86); 16000: 1 row 69 / 48 (278), 40 rows
+// 70 / 111 (282), 120 rows 71 / 236 (283); 32000: 40 rows 119 / 121, 120 rows 122 / 265. Softmax, 1000: 40 rows 3.3 / 5.1
+// (3.8); 32000: 40 rows 9.5 / 6.5, 120 rows 10 / 14. The draw's logarithms are a CTA's whole time: 1000: 120 rows 3.9 / 9.5 (4.9);
+// 2000: 1 row 6.0 / 3.4, 40 rows 6.4 / 4.5, 80 rows 6.3 / 7.4 (6.4). More rows than SMs need no second CTA each.
+static constexpr int kMostOneCta = kMostStaged / 4;       // columns
+static int row_ctas(int n, int V, int base, int per_row) {
+  return V <= kMostOneCta && (n > b200_num_sms() || V <= base + per_row * n) ? 1 : 8;
+}
+static size_t row_stage_bytes(int V, int ctas) {
+  const size_t bytes = (size_t)row_slice_cols(V, ctas) * 4;
   return bytes <= kMostStaged ? bytes : 0;
+}
+template <typename... KArgs, typename... Args>
+static int launch_rows(void (*kernel)(KArgs...), int n, int ctas, int threads, size_t smem, cudaStream_t stream, PerDeviceOnce& once,
+                       Args... args) {
+  if (smem > 32 * 1024 && once.first())             // (48 KB with the static part go without)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostStaged);
+  kernel<<<n * ctas, threads, smem, stream>>>(args...);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 }  // namespace b200
@@ -664,30 +689,30 @@ int b200_apply_min_p(void* logits, int ld, int n, int V, const void* min_p, cuda
 int b200_apply_top_k_top_p(void* logits, int ld, int n, int V, const void* top_k,
                            const void* top_p, cudaStream_t stream) {
   if (n <= 0) return 0;
-  static PerDeviceOnce attr_once;
-  if (attr_once.first())
-    cudaFuncSetAttribute(top_k_top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostStaged);
-  top_k_top_p_kernel<<<n * kRowCtas, kRowThreads, row_stage_bytes(V), stream>>>((float*)logits, ld, V, (const int*)top_k,
-                                                                               (const float*)top_p);
-  RET_LAUNCH;
+  // (up to 1024 columns, a few a thread, 256 threads pass the search's barriers sooner: 256 rows of 256 columns 31 -> 23 us)
+  static PerDeviceOnce once[3];
+  const int ctas = row_ctas(n, V, 6500, 420), form = ctas == 8 ? 2 : V > 1024 ? 1 : 0;
+  return launch_rows(form == 2 ? top_k_top_p_kernel<8, 512> : form ? top_k_top_p_kernel<1, 512> : top_k_top_p_kernel<1, 256>, n,
+                     ctas, form ? 512 : 256, row_stage_bytes(V, ctas), stream, once[form], (float*)logits, ld, V,
+                     (const int*)top_k, (const float*)top_p);
 }
 
 int b200_softmax(const void* logits, int ld, void* out, int ldo, int n, int V, int log_mode,
                  cudaStream_t stream) {
   if (n <= 0) return 0;
-  static PerDeviceOnce attr_once;
-  if (attr_once.first()) cudaFuncSetAttribute(softmax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostStaged);
-  softmax_kernel<<<n * kRowCtas, kRowThreads, row_stage_bytes(V), stream>>>((const float*)logits, ld, (float*)out, ldo, V,
-                                                                           log_mode);
-  RET_LAUNCH;
+  static PerDeviceOnce once[2];
+  const int ctas = row_ctas(n, V, 6500, 420);
+  return launch_rows(ctas == 8 ? softmax_kernel<8, 512> : softmax_kernel<1, 512>, n, ctas, 512, row_stage_bytes(V, ctas), stream,
+                     once[ctas == 8], (const float*)logits, ld, (float*)out, ldo, V, log_mode);
 }
 
 int b200_random_sample(const void* probs, int ld, int n, int V, const void* seeds,
                        const void* steps, void* out_i64, cudaStream_t stream) {
   if (n <= 0) return 0;
-  random_sample_kernel<<<n * kRowCtas, kRowThreads, 0, stream>>>((const float*)probs, ld, V, (const uint64_t*)seeds,
-                                              (const uint64_t*)steps, (int64_t*)out_i64);
-  RET_LAUNCH;
+  static PerDeviceOnce once;
+  const int ctas = row_ctas(n, V, 600, 30);
+  return launch_rows(ctas == 8 ? random_sample_kernel<8, 512> : random_sample_kernel<1, 512>, n, ctas, 512, 0, stream, once,
+                     (const float*)probs, ld, V, (const uint64_t*)seeds, (const uint64_t*)steps, (int64_t*)out_i64);
 }
 
 int b200_merge_greedy_random(const void* g, const void* r, const void* temp, void* out, int n,

@@ -659,3 +659,41 @@ def test_row_kernels_over_a_cluster(V, ld):
     again = ops.random_sample(torch.softmax(got, -1).contiguous(), seeds, steps)
     assert torch.equal(tok, again) and all(torch.isfinite(got[r, tok[r]]) for r in range(n))
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("V", [9021, 20000])
+def test_rows_of_one_and_of_eight_ctas(V):
+    """Six rows of V columns take a cluster of eight CTAs each, 160 copies of them (more rows than SMs) one CTA each. Top-k,
+    top-p away from a tie of the mass, ties and infinities at the threshold, and the draw from the same probabilities: the
+    same bits; softmax: sums in another order."""
+    torch.manual_seed(V)
+    inf = float("inf")
+    x = torch.randn(6, V, device=DEV) * 2
+    x[1, 4:] = -inf                                       # fewer finite logits than k: the threshold is -inf
+    x[2] = x[2].round()                                   # many ties at the threshold: all are kept
+    x[3, 17] = inf                                        # its mass is not a number: top-k alone decides
+    x[4] = -inf
+    x[4, V - 1] = 3.0
+    k = torch.tensor([50, 10, 20, 8, 5, 0], dtype=torch.int32, device=DEV)
+    p = torch.tensor([1.0, 1.0, 1.0, 0.9, 0.9, 0.8], device=DEV)
+    many = [t.repeat(27, *([1] * (t.dim() - 1)))[:160].contiguous() for t in (x, k, p)]
+    few, lots = x.clone(), many[0].clone()
+    ops.apply_top_k_top_p(few, k, p)
+    ops.apply_top_k_top_p(lots, many[1], many[2])
+    rows = torch.arange(160, device=DEV) % 6
+    assert torch.equal(few[rows], lots)
+    kept = (few == x) & (x > -inf)
+    assert int(kept[0].sum()) == 50 and torch.equal(few[1], x[1]) and torch.equal(few[4], x[4])
+    kth = x[2].sort(descending=True).values[19]
+    assert torch.equal(kept[2], x[2] >= kth)
+    assert int(kept[3].sum()) == 8 and bool(kept[3, 17])
+    mass = torch.softmax(x[5].double(), 0).sort(descending=True).values.cumsum(0)
+    assert abs(int(kept[5].sum()) - int((mass < 0.8).sum()) - 1) <= 1
+    soft = [ops.softmax(t[[0, 2, 5]] if t.shape[0] == 6 else t) for t in (few, lots)]
+    assert (soft[0] - soft[1][[0, 2, 5]]).abs().max().item() < 1e-6
+    probs = torch.softmax(few[[0, 2, 5]], -1)
+    seeds = torch.arange(3, dtype=torch.int64, device=DEV) + 5
+    big = [t.repeat(54, *([1] * (t.dim() - 1)))[:160].contiguous() for t in (probs, seeds)]
+    steps = torch.full((160,), 9, dtype=torch.int64, device=DEV)
+    assert torch.equal(ops.random_sample(probs, seeds, steps[:3])[torch.arange(160, device=DEV) % 3], ops.random_sample(*big, steps))
+    assert ops.read_status() == 0
