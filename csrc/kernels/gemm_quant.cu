@@ -518,6 +518,24 @@ using namespace b200;
 
 extern "C" {
 
+// Where 128 x 128 tiles beat the cluster form up to 128 rows. What a CTA of the cluster form does behind its last product
+// grows with the rows (its partial tile goes through shared memory), and it is in the open where a CTA has few k-blocks or the
+// grid needs a second wave; the tiled kernel is persistent and has a second accumulator, but idles where its last wave is
+// thin. With t row tiles in waves filled to a share f, us, tiles / cluster:
+//   one wave    16384 x 512 (f = 0.86) at 64 / 96 / 128 rows 7.8 / 8.1, 7.9 / 10.0, 8.1 / 12.2; 16384 x 2048 at 128 12.8 / 14.4;
+//               12288 x 2048 (0.65) at 96 / 128 12.7 / 12.1, 13.0 / 13.6; 8192 x 512 (0.43) at 96 7.3 / 8.2, x 2048 12.3 / 9.7
+//   two waves   28672 x 1024 (0.76) at 96 / 128 13.1 / 12.8, 13.5 / 14.9; x 4096 at 128 33.4 / 30.4
+//   more        57344 x 1024 at 64 / 128 19.9 / 21.9, 22.3 / 29.4; x 4096 56.4 / 50.2, 58.4 / 60.7
+// (The tiles read the channel scales and write the result in 16-byte pieces, the cluster form does not.)
+// The lines below are within 5 % of the better one at all but two of 540 measured shapes (45056 x 512 at 48 rows and 128256 x
+// 4096 at 64 and 80: 11 %).
+static bool fp8_tiles_win(int M, int N, int K) {
+  const long long t = (N + kQN - 1) / kQN, sms = b200_num_sms(), slots = (t + sms - 1) / sms * sms;       // f = t / slots
+  if (t <= sms) return M > 64 && (K <= 512 || K * slots * slots <= 80 * t * t * (M - 48));
+  if (t <= 2 * sms) return M > 96 && K * slots * slots <= 40 * t * t * (M - 48);
+  return M > 48 && K <= 64 * (M - 32);
+}
+
 int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo,
                        const float* a_scale, const float* w_scale, int w_scale_per_channel, const void* bias,
                        int M, int N, int K, cudaStream_t stream);
@@ -534,7 +552,8 @@ int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int
                               stream);
   // up to 128 rows: weight-bound, K split over a cluster (gemm_cluster.cu); 32 requests of the fp8 8B shape 166 -> 148 ms
   // against 128 x 128 tiles with split-K partials in memory
-  if (M <= 128 && !(reinterpret_cast<uintptr_t>(bias) & 7)) {
+  if (M <= 128 && !(reinterpret_cast<uintptr_t>(bias) & 7) &&
+      (!fp8_tiles_win(M, N, K) || ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w_scale)) & 15))) {
     GemmCluster g{};
     g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.out = out; g.ldo = ldo; g.bias = bias;
     g.M = M; g.N = N; g.K = K;

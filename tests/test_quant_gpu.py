@@ -117,6 +117,23 @@ def test_gemm_fp8_over_a_cluster(M, N, K, per_token, per_channel):
         assert _within_sum_error(out, a64, w64, exp)
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 4104, 512), (65, 4104, 512), (128, 136, 16), (128, 19000, 1040), (97, 20480, 400), (96, 20480, 400),
+                                   (49, 38016, 1088), (48, 38016, 1088), (128, 38016, 6160)])
+def test_gemm_fp8_tiles_and_clusters(M, N, K):
+    """Both sides of the lines between the tiled kernel and the cluster form up to 128 rows, with the scales at an address that
+    the tiled kernel cannot read and at one that it can. Equal sums of k up to their order."""
+    torch.manual_seed(13)
+    a8 = (torch.randn(M, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    w8 = (torch.randn(N, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    sa, sw = torch.rand(M, device=DEV) + 0.5, torch.rand(N + 4, device=DEV) * 0.1 + 0.01
+    a64 = a8.double() * sa.double()[:, None]
+    for off in (0, 1):
+        w64 = w8.double() * sw[off: off + N].double()[:, None]
+        out = Q.gemm_fp8(a8, w8, sa, sw[off: off + N])
+        assert ops.read_status() == 0
+        assert _within_sum_error(out, a64, w64, a64 @ w64.t())
+
+
 @pytest.mark.parametrize("T", [1, 296, 297])
 @pytest.mark.parametrize("K", [8, 264, 2056, 14336, 32768])
 def test_rowwise_fp8_of_few_and_many_rows(T, K):
