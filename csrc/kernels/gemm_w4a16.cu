@@ -8,7 +8,7 @@
 // elements) straight into 128-byte-swizzled K-major tiles; one thread issues f16 tcgen05 MMAs
 // with the (pre-cast f16, zero-padded) batch as the 128-row operand and 256 weight rows as the N
 // operand - an MMA instruction costs about the same whatever its N, so the wide side is where the
-// weights go. value x block scale is exact in f16 (at most 5 significant bits, magnitude <= 2688);
+// weights go. value x block scale is exact in f16 (at most 6 significant bits, magnitude <= 2688);
 // the fp32 global scale is applied to the accumulators in the epilogue. Each converter thread
 // reads its four block scales of a stage as one word, one stage ahead. Split-K over blockIdx.y
 // with fp32 partials.
@@ -288,9 +288,9 @@ __global__ void __launch_bounds__(kWThreads, 1)
 // SM that fill each other's waits; the parts of K are summed from shared memory to shared memory instead of through a
 // workspace and a second kernel. Bound by the chain expansion - MMA - release of a 64-k tile, about 0.5 us each, of which
 // four MMAs and their barriers are 0.36 (measured with conversions, scale loads and split of the warps varied). us at
-// 9 / 64 rows, the reducing kernel included, against the form above:
-//   16480 x 5120 33.0 / 41.8 -> 31.8 / 33.8    5120 x 6144 18.6 / 26.4 -> 16.8 / 19.6
-//   34816 x 5120 76.1 / 56.4 -> 55.2 / 57.9    5120 x 17408 34.6 / 42.3 -> 36.4 / 39.2
+// 9 / 64 rows, the reducing kernel included, against the form above (b200_gemm_w4a16 chooses):
+//   16480 x 5120 33.2 / 43.4 -> 31.8 / 33.9    5120 x 6144 19.9 / 26.5 -> 16.8 / 19.5
+//   34816 x 5120 72.0 / 57.4 -> 55.7 / 58.6    5120 x 17408 34.9 / 42.7 -> 36.6 / 39.5
 // ---------------------------------------------------------------------------------------
 static constexpr int kCRows = 128, kCRaw = kCRows * 128, kCExp = kCRows * 128;
 static constexpr int kCRS = 2, kCES = 3, kCAS = 12, kCConv = 8, kCThreads = (3 + kCConv) * 32, kCRowsMax = 64;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
   } else {
     // A nibble's three magnitude bits in bits 9 to 11 of an f16 are its value times 2^-14 (subnormals included), nibbles k and
     // k + 4 of a word lie 16 bits apart: four shifts and masks expand two weights (in the order 0 4 1 5 2 6 3 7, which the
-    // cast of the batch follows). Times the block scale x 2^7 they are exact in f16 (5 significant bits, multiples of
+    // cast of the batch follows). Times the block scale x 2^7 they are exact in f16 (6 significant bits, multiples of
     // 2^-17 up to 21); the 2^7 that is missing joins the global scale.
     constexpr uint32_t kMag = 0x0e000e00u, kSign = 0x80008000u;
     // Four warps expand the even tiles of 64 k, four the odd ones, a thread a row: a warp's expansion ends in a fence, and
@@ -562,8 +562,22 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
   p.splits = splits; p.ne_per_split = ne_per;
   p.workspace = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + a16_bytes);
 
-  const bool cluster = M <= kCRowsMax && (K & 255) == 0 && !(reinterpret_cast<uintptr_t>(sf) & 15) && !(N & 7) &&
-                       !(reinterpret_cast<uintptr_t>(out) & 7);
+  bool cluster = M <= kCRowsMax && (K & 255) == 0 && !(reinterpret_cast<uintptr_t>(sf) & 15) && !(N & 7) &&
+                 !(reinterpret_cast<uintptr_t>(out) & 7);
+  int csplits = 1;
+  if (cluster) {
+    // Both forms walk their part of K in steps of 64, in 0.62 (cluster) and 0.64 us a step; start, exchange and end take 6.0 and
+    // 8.9 us, and a row of the batch 0.05 and 0.12 us (the stream form's partials go through memory). So the cluster form
+    // may have a few steps more, but not where a cluster that fits beside its neighbours splits K too coarsely: us, stream /
+    // cluster form, 4096 x 14336 (28 against 40 steps) 26.8 / 31.6 at 9 rows and 30.7 / 34.4 at 64, 12288 x 4096 (24 against
+    // 32) 25.0 / 26.2 and 32.9 / 28.1, 2560 x 9728 (12 against 20) 17.5 / 18.7 and 23.3 / 21.6, 5120 x 6144 (16 and 16)
+    // 19.9 / 16.8 and 26.5 / 19.5. Grids beyond one wave have no partials to save: from 33 rows on the wider tiles win
+    // (34816 x 5120 at 64 rows 57.4 / 58.6).
+    const int tiles = (N + kCRows - 1) / kCRows, blocks = K / 256;
+    csplits = cluster_splits(tiles, blocks / 2);
+    const int more = 4 * ((blocks + csplits - 1) / csplits) - ne_per;
+    if (100 * more > 460 + 11 * M || (M > 32 && tiles > sms)) cluster = false;
+  }
   __half* a16 = reinterpret_cast<__half*>(workspace);
   {
     const size_t total = (size_t)M * (K / 8);
@@ -578,8 +592,8 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
     W4CParams c{};
     c.M = M; c.N = N; c.K = K; c.mp = (M + 15) & ~15;
     c.out = (bf16*)out; c.ldo = ldo; c.sf = (const uint8_t*)sf; c.gscale = gscale; c.bias = (const bf16*)bias; c.status = device_status_word();
-    const int tiles = (N + kCRows - 1) / kCRows, blocks = K / 256;
-    c.splits = cluster_splits(tiles, blocks / 2);
+    const int tiles = (N + kCRows - 1) / kCRows;
+    c.splits = csplits;
     if (!encode_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, K / 2, kCRows, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&tmA, a16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, M, K, K, c.mp, 64, CU_TENSOR_MAP_SWIZZLE_128B))
       return -3;

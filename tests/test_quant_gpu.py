@@ -100,6 +100,21 @@ def test_w4a16_over_a_cluster(M, N, K):
         assert _within_sum_error(out, a64, w64, exp, extra)
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 2560, 9728), (34, 2560, 9728), (64, 4096, 14336), (32, 38016, 256), (33, 38016, 256)])
+def test_w4a16_stream_and_cluster(M, N, K):
+    """Both sides of the lines between the two forms up to 64 rows: parts of K that are too coarse over a cluster, more rows
+    that make up for it, grids beyond one wave."""
+    torch.manual_seed(14)
+    packed = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device=DEV)
+    sf = torch.randint(0x20, 0x60, (N, K // 16), dtype=torch.uint8, device=DEV)
+    g = torch.full((1,), 0.01, device=DEV)
+    a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
+    w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
+    out = Q.gemm_w4a16(a, packed, sf, g)
+    assert ops.read_status() == 0
+    assert _within_sum_error(out, a64, w64, a64 @ w64.t(), 2**-25 * w64.abs().sum(1))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 16), (17, 520, 144), (65, 136, 4112), (128, 4104, 8192)])
 @pytest.mark.parametrize("per_token,per_channel", [(False, False), (True, True)])
 def test_gemm_fp8_over_a_cluster(M, N, K, per_token, per_channel):
