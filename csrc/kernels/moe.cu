@@ -351,10 +351,10 @@ struct GroupedParams {
   const int32_t* meta;
   int E;
   int stages;
-  int sub_rows;             // sorted rows of a CTA: 256, gated 128 (blockIdx.y = chunk * (256 / sub_rows) + part of it)
+  int sub_rows;             // sorted rows of a CTA: 256, or 128 (gated): blockIdx.x = part of the chunk * column tiles + column tile
   // Gated mode (act_fuse = activation kind + 1): W_e is [gate rows (N/2) | up rows (N/2)]; a CTA
   // takes 128 gate rows and the 128 up rows of the same outputs, keeps one accumulator for each in
-  // TMEM (columns [0, np) and [128, 128 + np)) and writes act(gate) * up to out[rows, N / 2], so the
+  // TMEM (columns [0, np) and [sub_rows, sub_rows + np)) and writes act(gate) * up to out[rows, N / 2], so the
   // merged projection never reaches memory. Both values are rounded to bf16 first, as the separate
   // activation kernel would see them.
   int act_fuse;
@@ -368,17 +368,18 @@ struct alignas(8) GroupedBars {
   float row_w[256];        // clamped pair: routing weights of the chunk's rows
 };
 
-// grid: (N / 128, max_chunks). A CTA whose chunk index is past the device-side count exits. Two CTAs share an SM (96 KB of
-// stages and 256 TMEM columns each), so that one stores its outputs while the other multiplies; a CTA alone, with twice
-// the stages and both halves of the gated accumulators for 256 rows, left the tensor pipe idle during its epilogue (us at
-// 8192 tokens, gated / down: 128 experts of 768, top 8, 608 / 525 -> 492 / 349; 64 of 1408, top 6, 799 / 511 -> 637 / 349).
+// grid: (column tiles x parts of a chunk, max_chunks). A CTA whose chunk index is past the device-side count exits. Two CTAs
+// share an SM (96 KB of stages and 256 TMEM columns each), so that one stores its outputs while the other multiplies; a CTA
+// alone, with twice the stages and both halves of the gated accumulators for 256 rows, left the tensor pipe idle during
+// its epilogue (us at 8192 tokens, gated / down: 128 experts of 768, top 8, 608 / 525 -> 492 / 349; 64 of 1408, top 6,
+// 799 / 511 -> 637 / 349).
 __global__ void __launch_bounds__(192, 2)
     moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW,
                             const __grid_constant__ CUtensorMap tmX, GroupedParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
-  const int subs = 256 / p.sub_rows, chunk = blockIdx.y / subs, first = blockIdx.y % subs * p.sub_rows;
+  const int tiles = (int)gridDim.x * p.sub_rows >> 8, chunk = blockIdx.y, first = (int)blockIdx.x / tiles * p.sub_rows;
   if (chunk >= p.meta[3 * p.E + 1] || first >= p.chunk_n[chunk]) return;
   const int e = p.chunk_expert[chunk], row0 = p.chunk_row0[chunk] + first, rows = min(p.sub_rows, p.chunk_n[chunk] - first);
   const int np = (rows + 15) & ~15;                 // UMMA N
@@ -390,14 +391,14 @@ __global__ void __launch_bounds__(192, 2)
   const int stages = p.stages;
   GroupedBars* bars = reinterpret_cast<GroupedBars*>(smem + (size_t)stages * kStage);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tn = blockIdx.x;
+  const int tn = (int)blockIdx.x % tiles;
   const int nkb = (p.K + kGBK - 1) / kGBK;
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
     mbar_init(&bars->acc_full, 1);
     mbar_fence_init();
   }
-  constexpr uint32_t tmem_cols = 256;
+  const uint32_t tmem_cols = gated ? 2 * p.sub_rows : 256;
   if (warp == 1) { tmem_alloc(&bars->tmem_base, tmem_cols); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(192, 2)
           umma_bf16_ss(tmem_base, umma_desc_k_sw128(wa + kk * 32, 1024),
                        umma_desc_k_sw128(xa + kk * 32, 1024), idesc, (i | kk) != 0);
           if (gated)
-            umma_bf16_ss(tmem_base + 128, umma_desc_k_sw128(wa + kWBytes + kk * 32, 1024),
+            umma_bf16_ss(tmem_base + p.sub_rows, umma_desc_k_sw128(wa + kWBytes + kk * 32, 1024),
                          umma_desc_k_sw128(xa + kk * 32, 1024), idesc, (i | kk) != 0);
         }
         umma_commit(&bars->empty[s]);
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(192, 2)
       for (int c = 0; c < np / 16; ++c) {
         uint32_t g[16], u[16];
         tmem_ld_32x32b_x16(ta + c * 16, g);
-        tmem_ld_32x32b_x16(ta + 128 + c * 16, u);
+        tmem_ld_32x32b_x16(ta + p.sub_rows + c * 16, u);
         tmem_ld_wait();
         if (n < half_n) {
 #pragma unroll
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(192, 2)
       for (int c = 0; c < np / 16; ++c) {
         uint32_t g[16], u[16];
         tmem_ld_32x32b_x16(ta + c * 16, g);
-        tmem_ld_32x32b_x16(ta + 128 + c * 16, u);
+        tmem_ld_32x32b_x16(ta + p.sub_rows + c * 16, u);
         tmem_ld_wait();
         if (n < half_n) {
 #pragma unroll
@@ -712,6 +713,7 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
     g.max_rows = max_rows; g.max_chunks = max_chunks; g.E = E; g.N = N; g.K = K; g.gated = act_fuse; g.act = act;
     return launch_experts_cluster(g, stream);
   }
+  const int tiles = ((act_fuse ? N / 2 : N) + kGBM - 1) / kGBM;
   const int sub_rows = act_fuse ? 128 : 256;
   CUtensorMap tmW, tmX;
   if (!encode_tmap_3d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)N,
@@ -739,7 +741,7 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
     cudaFuncSetAttribute(moe_grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          110 * 1024);
   }
-  dim3 grid(((act_fuse ? N / 2 : N) + kGBM - 1) / kGBM, max_chunks * (256 / sub_rows));
+  dim3 grid((unsigned)(tiles * (256 / sub_rows)), (unsigned)max_chunks);
   moe_grouped_gemm_kernel<<<grid, 192, smem, stream>>>(tmW, tmX, p);
   RETL;
 }

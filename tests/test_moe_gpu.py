@@ -146,3 +146,21 @@ def test_moe_engine_gpu_vs_cpu():
     assert [a[0] for a in gpu] == [a[0] for a in cpu]
     hit = sum(sum(1 for p, q in zip(a, b) if p == q) for a, b in zip(gpu, cpu))
     assert hit / sum(len(a) for a in gpu) > 0.7
+
+
+@pytest.mark.parametrize("chunks", [3, 40000, 65535])
+def test_grouped_gemm_gated_with_a_long_chunk_list(chunks):
+    """As many chunks as a grid's second dimension holds, whatever the parts that a chunk is taken in; those past the count on
+    the device are nothing."""
+    torch.manual_seed(1)
+    T, H, I = 300, 64, 136
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    wgu = (torch.randn(1, 2 * I, H, device=DEV) * H ** -0.5).to(torch.bfloat16)
+    ws = M.MoeWorkspace(torch.device(DEV), T, 1, 1, H, I)
+    M.moe_sort(torch.zeros(T, 1, dtype=torch.int32, device=DEV), 0, 1, ws)
+    M.moe_gather(x, ws, 1, T)
+    M.grouped_gemm_gated(ws.xs, wgu, ws.act, ws, T, max_chunks=chunks)
+    assert ops.read_status() == 0
+    g, u = (x.float() @ wgu[0, h * I:(h + 1) * I].float().t() for h in range(2))
+    got = ws.act[ws.pair_pos.long()].float()
+    assert _rel(got, torch.nn.functional.silu(g) * u) < 3 * 2.0 ** -8
