@@ -370,9 +370,9 @@ struct alignas(8) GroupedBars {
 
 // grid: (column tiles x parts of a chunk, max_chunks). A CTA whose chunk index is past the device-side count exits. Two CTAs
 // share an SM (96 KB of stages and 256 TMEM columns each), so that one stores its outputs while the other multiplies; a CTA
-// alone, with twice the stages and both halves of the gated accumulators for 256 rows, left the tensor pipe idle during
+// alone, with twice the stages and both halves of the gated accumulators for 256 rows, leaves the tensor pipe idle during
 // its epilogue (us at 8192 tokens, gated / down: 128 experts of 768, top 8, 608 / 525 -> 492 / 349; 64 of 1408, top 6,
-// 799 / 511 -> 637 / 349).
+// 799 / 511 -> 637 / 349). The gated product keeps that form where there are too few CTAs to pair up (moe_grouped_gemm_impl).
 __global__ void __launch_bounds__(192, 2)
     moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW,
                             const __grid_constant__ CUtensorMap tmX, GroupedParams p) {
@@ -713,8 +713,20 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
     g.max_rows = max_rows; g.max_chunks = max_chunks; g.E = E; g.N = N; g.K = K; g.gated = act_fuse; g.act = act;
     return launch_experts_cluster(g, stream);
   }
+  // Gated: 128 rows a CTA and two CTAs an SM, or 256 rows, a CTA with three stages of 64 KB alone on its SM. The smaller CTA
+  // hides its epilogue behind its neighbour, but reads the weights once for every 128 rows and has two stages of 48 KB.
+  //  - Few CTAs (about 1.35 an SM; an expert's last 128 rows are half full on average) have no neighbour. us, 256 / 128 rows:
+  //    8 experts of 1792, width 4096, 70 and 190 rows each 55 / 81, 73 / 91; 16 of 1024, width 2048, 70 rows 39 / 51. With
+  //    more than 192 rows an expert the second CTA halves the time all the same: 4 of 2048, width 2048, 256 rows 53 / 44.
+  //  - Long products (K of 4096 on) have little epilogue: 8 of 14336, width 4096, 150 rows 459 / 551, 400 rows 902 / 1056;
+  //    16 of 8192, width 5120, 150 rows 560 / 699, 1024 rows 2740 / 3024. Up to 128 rows there is no second reading: 70 rows
+  //    386 / 344 and 479 / 442.
+  //  - Shorter ones: 128 of 768, width 2048, 70 rows 202 / 162, 1024 rows 1128 / 917; 32 of 2880, width 2880, 512 rows 670 / 595.
   const int tiles = ((act_fuse ? N / 2 : N) + kGBM - 1) / kGBM;
-  const int sub_rows = act_fuse ? 128 : 256;
+  const long long sms = b200_num_sms(), per128 = (long long)tiles * E * ((max_rows + 128 * E - 1) / (128 * E));
+  const bool few = max_rows <= 192 * E ? 20LL * tiles * (max_rows / 128 + E / 2) < 27 * sms : per128 <= 2 * sms;
+  const bool pairs = act_fuse && (max_rows <= 192 * E ? !few && (K < 4096 || max_rows <= 128 * E) : few || K < 4096);
+  const int sub_rows = pairs ? 128 : 256;
   CUtensorMap tmW, tmX;
   if (!encode_tmap_3d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)N,
                       (uint64_t)E, (uint64_t)K * 2, (uint64_t)N * K * 2, kGBK, kGBM, 1,
@@ -729,7 +741,7 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
   p.chunk_expert = (const int32_t*)chunk_expert; p.chunk_row0 = (const int32_t*)chunk_row0;
   p.chunk_n = (const int32_t*)chunk_n; p.meta = (const int32_t*)meta; p.E = E;
   const int stage = kGBM * kGBK * 2 * (act_fuse ? 2 : 1) + sub_rows * kGBK * 2;
-  int stages = (96 * 1024) / stage;
+  int stages = (act_fuse && !pairs ? 200 : 96) * 1024 / stage;
   if (stages > kGMaxStages) stages = kGMaxStages;
   const int nkb = (K + kGBK - 1) / kGBK;
   if (stages > nkb) stages = nkb < 2 ? 2 : nkb;
@@ -739,7 +751,7 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
     cudaFuncSetAttribute(moe_grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         110 * 1024);
+                         220 * 1024);
   }
   dim3 grid((unsigned)(tiles * (256 / sub_rows)), (unsigned)max_chunks);
   moe_grouped_gemm_kernel<<<grid, 192, smem, stream>>>(tmW, tmX, p);

@@ -164,3 +164,30 @@ def test_grouped_gemm_gated_with_a_long_chunk_list(chunks):
     g, u = (x.float() @ wgu[0, h * I:(h + 1) * I].float().t() for h in range(2))
     got = ws.act[ws.pair_pos.long()].float()
     assert _rel(got, torch.nn.functional.silu(g) * u) < 3 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(512, 8, 2, 256, 1792), (700, 8, 2, 256, 1792), (1024, 8, 2, 256, 1792), (1100, 2, 2, 72, 136)])
+def test_grouped_gemm_gated_of_128_and_256_rows(T, E, k, H, I):
+    """More than 64 rows an expert: 256 rows a CTA where the CTAs are few, 128 and two CTAs an SM otherwise, chunks of less, of
+    exactly and of more than that; the bits of the product and the activation as two kernels."""
+    torch.manual_seed(T)
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    wgu = (torch.randn(E, 2 * I, H, device=DEV) * H ** -0.5).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E, device=DEV)[:k] for _ in range(T)]).int()
+    ids[:128, 0], ids[:128, 1:] = 0, 1                    # an expert that shares rows with few others
+    ws = M.MoeWorkspace(torch.device(DEV), T, k, E, H, I)
+    M.moe_sort(ids, 0, E, ws)
+    P = T * k
+    M.moe_gather(x, ws, E, P)
+    M.grouped_gemm(ws.xs, wgu, ws.gu, ws, P)
+    ops.act_and_mul(ws.gu[:P], 0, out=ws.act[:P])
+    want = ws.act[:P].clone()
+    ws.act.zero_()
+    M.grouped_gemm_gated(ws.xs, wgu, ws.act, ws, P, kind=0)
+    assert ops.read_status() == 0 and torch.equal(ws.act[:P], want)
+    g, u = (torch.stack([x.float() @ wgu[e, h * I:(h + 1) * I].float().t() for e in range(E)]) for h in range(2))
+    tok = torch.arange(T, device=DEV)
+    for j in range(k):
+        e = ids[:, j].long()
+        got = want[ws.pair_pos.view(T, k)[:, j].long()].float()
+        assert _rel(got, torch.nn.functional.silu(g[e, tok]) * u[e, tok]) < 3 * 2.0 ** -8
