@@ -527,6 +527,7 @@ PYBIND11_MODULE(_engine, m) {
       .def_readonly("num_prefills", &StepInfo::num_prefills)
       .def_readonly("num_prefill_tokens", &StepInfo::num_prefill_tokens)
       .def_readonly("num_tiles", &StepInfo::num_tiles)
+      .def_readonly("prefill_keys", &StepInfo::prefill_keys)
       .def_readonly("max_query_len", &StepInfo::max_query_len)
       .def_readonly("max_seq_len", &StepInfo::max_seq_len)
       .def_readonly("num_logits", &StepInfo::num_logits)

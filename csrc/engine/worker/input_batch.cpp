@@ -260,6 +260,7 @@ StepInfo InputBatch::prepare(const SchedulerOutput& so, const StepLayout& L, uin
         tile_req[info.num_tiles] = pi;
         tile_q0[info.num_tiles] = q0;
         info.num_tiles++;
+        info.prefill_keys += lo + std::min(q0 + 128, n);
       }
       pqs[pi + 1] = pqs[pi] + n;
     }

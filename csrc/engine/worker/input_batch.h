@@ -71,6 +71,7 @@ struct StepInfo {
   int num_decodes = 0, num_decode_tokens = 0;
   int num_prefills = 0, num_prefill_tokens = 0;
   int num_tiles = 0;
+  int64_t prefill_keys = 0;                // sum over the tiles of the positions up to a tile's last row
   int max_query_len = 0, max_seq_len = 0;
   int num_logits = 0;
   int num_splice = 0;

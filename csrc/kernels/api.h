@@ -86,6 +86,7 @@ typedef struct B200DenseStep {
   void* decode_tmp_o;
   void* decode_tmp_lse;
   int num_prefills, num_tiles, num_prefill_tokens;
+  long long prefill_keys;  // sum over the tiles of the positions up to a tile's last row (0: not known)
   const void* prefill_q_start;
   const void* tile_req;
   const void* tile_q0;
@@ -460,6 +461,7 @@ int b200_bias_attn_decode(const B200BiasAttn* a, int any_size, cudaStream_t stre
 int b200_bias_attn_prefill(const B200BiasAttn* a, int any_size, cudaStream_t stream);
 // ---- attn_prefill.cu
 int b200_attn_prefill(const void* q, int ldq, void* out, int ldo, void* lse, const void* kv_cache, int64_t num_blocks, int block_size, int Hq, int Hkv, int D, const void* block_table, int max_blocks, const void* seq_lens, const void* q_start, const void* tile_req, const void* tile_q0, int num_tiles, int total_q, float scale, float softcap, int window, int causal, cudaStream_t stream);
+int b200_attn_prefill_keys(const void* q, int ldq, void* out, int ldo, void* lse, const void* kv_cache, int64_t num_blocks, int block_size, int Hq, int Hkv, int D, const void* block_table, int max_blocks, const void* seq_lens, const void* q_start, const void* tile_req, const void* tile_q0, int num_tiles, int total_q, long long tile_keys, float scale, float softcap, int window, int causal, cudaStream_t stream);
 // ---- common.cu
 long long b200_set_peer_wait_cycles(long long cycles);
 // ---- conv_norm.cu

@@ -381,11 +381,12 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
 // Q and a ring of four K / V tiles.
 //
 // Measured against one head a CTA, 64-key tiles and P in shared memory (32 query / 8 kv heads, TFLOP/s of causal work):
-// 4096 tokens 523 -> 777, 8192 670 -> 961, 7309 after 8192 cached 773 -> 969, 8 x 1024 426 -> 481; prompts of a few
-// hundred tokens take about as long as before (30 x 275: 0.120 -> 0.126 ms, 1000: 0.043 -> 0.040), their time is start and end.
+// 4096 tokens 523 -> 777, 8192 670 -> 961, 7309 after 8192 cached 773 -> 969, 8 x 1024 426 -> 481. Shorter prompts, whose time
+// is a CTA's start and end, stay with one head a CTA (b200_attn_prefill_keys).
 //
-// What bounds it: 128 exponentials a row and tile, 2048 cycles of the special-function units for the two heads of a tile,
-// against 2 x 16 MMAs of about 84 cycles. One issuing thread watches both heads and issues whatever is ready:
+// A tile of two heads takes 4200 to 4900 cycles at 961 TFLOP/s. Its 2 x 16 MMAs of about 84 cycles are 2700 of them, its 128
+// exponentials a row 2050 on the special-function units; either alone would be faster, so what is left is that they
+// alternate no better than this. One issuing thread watches both heads and issues whatever is ready:
 //   P(t, j) written and V(j) there   ->  O(t) += P(t, j) V(j)
 //   P V(t, j) complete and K(j+1)    ->  S(t) = Q(t) K(j+1)^T   (over P(t, j), which has been read)
 //
@@ -684,6 +685,18 @@ extern "C" int b200_attn_prefill(const void* q, int ldq, void* out, int ldo, voi
                                  const void* seq_lens, const void* q_start, const void* tile_req,
                                  const void* tile_q0, int num_tiles, int total_q, float scale,
                                  float softcap, int window, int causal, cudaStream_t stream) {
+  return b200_attn_prefill_keys(q, ldq, out, ldo, lse, kv_cache, num_blocks, block_size, Hq, Hkv, D, block_table, max_blocks,
+                                seq_lens, q_start, tile_req, tile_q0, num_tiles, total_q, 0, scale, softcap, window, causal,
+                                stream);
+}
+
+// The same; tile_keys, the sum over the tiles of the positions up to a tile's last row, only chooses between the kernels.
+extern "C" int b200_attn_prefill_keys(const void* q, int ldq, void* out, int ldo, void* lse,
+                                      const void* kv_cache, int64_t num_blocks, int block_size, int Hq,
+                                      int Hkv, int D, const void* block_table, int max_blocks,
+                                      const void* seq_lens, const void* q_start, const void* tile_req,
+                                      const void* tile_q0, int num_tiles, int total_q, long long tile_keys, float scale,
+                                      float softcap, int window, int causal, cudaStream_t stream) {
   if (num_tiles <= 0) return 0;
   if (D != 64 && D != 128 && D != 256) return -1;
   if (block_size < 8 || (block_size & 7) || (block_size < kKT && kKT % block_size) ||
@@ -696,10 +709,24 @@ extern "C" int b200_attn_prefill(const void* q, int ldq, void* out, int ldo, voi
   if (!encode_tmap_2d(&tmQ, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)total_q,
                       (uint64_t)Hq * D, (uint64_t)ldq, kQT, 64, CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
-  // pairs of heads need an even group, 128-dim heads, no soft-cap (it is applied to the scores one by one) and pages
-  // that divide a tile or are whole tiles
+  // Pairs of heads need an even group, 128-dim heads, no soft-cap (it is applied to the scores one by one) and pages
+  // that divide a tile or are whole tiles.
+  // They pay where a CTA sees keys enough: the start and the end of a CTA that has an SM to itself are in the open, and of 128
+  // keys a tile more are masked. About 250 keys a tile on average are the line, or 96 where the grid is a single wave, and so
+  // is more than half a wave: two heads a CTA leave SMs idle that one head a CTA has work for. A window or chunk shorter than
+  // 1024 ends at both sides within a tile. us, one / two heads a CTA, 32 query heads:
+  //   120 x 64 tokens 84 / 108, 60 x 128 65 / 70, 60 x 275 (220 keys) 210 / 221, 30 x 400 (292) 166 / 168, 30 x 512 180 / 174,
+  //   8 x 1024 150 / 130, 60 x 100 after 2000 355 / 324; one wave: 8 x 40 7.7 / 8.3, 8 x 100 10.5 / 9.1; less than half:
+  //   1 x 512 15.2 / 16.8; 8192 tokens, window 256 106 / 112, 512 144 / 144, 1024 218 / 201
+  if (tile_keys <= 0) {       // not known: half of a request's last tile is empty on average, and nothing came before
+    const long long empty = (long long)num_tiles * kQT - total_q, reqs = empty > kQT / 2 ? empty / (kQT / 2) : 1;
+    tile_keys = num_tiles * (total_q / reqs + kQT) / 2;
+  }
+  const long long ctas = (long long)num_tiles * (Hq / 2), sms = b200_num_sms();
   const bool pair = D == 128 && (Hq / Hkv) % 2 == 0 && softcap == 0.f && scale > 0.f &&
-                    (block_size <= kPT ? kPT % block_size == 0 : block_size % kPT == 0);
+                    (block_size <= kPT ? kPT % block_size == 0 : block_size % kPT == 0) &&
+                    (window == 0 || window >= 1024 || window <= -1024) && 2 * ctas > sms &&
+                    tile_keys >= (ctas <= sms ? 96 : 250) * (long long)num_tiles;
   const int most = pair ? kPT : kKT;
   const int box_rows = block_size < most ? block_size : most;
   const uint64_t rows = (uint64_t)num_blocks * 2 * block_size;

@@ -63,9 +63,9 @@ int dense_attention(const B200DenseLayerWeights* w, const B200DenseStep* s, cuda
     bf16* o = reinterpret_cast<bf16*>(s->attn) + (size_t)nd * Hq * D;
     const int32_t* bt = reinterpret_cast<const int32_t*>(s->block_table) + (size_t)nd * s->max_blocks;
     const int32_t* sl = reinterpret_cast<const int32_t*>(s->seq_lens) + nd;
-    B200_TRY(b200_attn_prefill(q, qkv_w, o, Hq * D, nullptr, w->kv_cache, s->num_blocks, s->block_size, Hq, Hkv, D,
-                               bt, s->max_blocks, sl, s->prefill_q_start, s->tile_req, s->tile_q0, s->num_tiles,
-                               s->num_prefill_tokens, s->scale, s->softcap, s->window, 1, stream));
+    B200_TRY(b200_attn_prefill_keys(q, qkv_w, o, Hq * D, nullptr, w->kv_cache, s->num_blocks, s->block_size, Hq, Hkv, D,
+                                    bt, s->max_blocks, sl, s->prefill_q_start, s->tile_req, s->tile_q0, s->num_tiles,
+                                    s->num_prefill_tokens, s->prefill_keys, s->scale, s->softcap, s->window, 1, stream));
   }
   return launches;
 }
@@ -299,9 +299,9 @@ int b200_dense_layers_tp(const B200DenseLayerWeights* w, int num_layers, const B
       bf16* o = reinterpret_cast<bf16*>(s->attn) + (size_t)nd * Hq * D;
       const int32_t* bt = reinterpret_cast<const int32_t*>(s->block_table) + (size_t)nd * s->max_blocks;
       const int32_t* sl = reinterpret_cast<const int32_t*>(s->seq_lens) + nd;
-      B200_TRY(b200_attn_prefill(q, qkv_w, o, Hq * D, nullptr, L->kv_cache, s->num_blocks, s->block_size, Hq, Hkv,
-                                 D, bt, s->max_blocks, sl, s->prefill_q_start, s->tile_req, s->tile_q0,
-                                 s->num_tiles, s->num_prefill_tokens, s->scale, s->softcap, s->window, 1, stream));
+      B200_TRY(b200_attn_prefill_keys(q, qkv_w, o, Hq * D, nullptr, L->kv_cache, s->num_blocks, s->block_size, Hq, Hkv,
+                                      D, bt, s->max_blocks, sl, s->prefill_q_start, s->tile_req, s->tile_q0, s->num_tiles,
+                                      s->num_prefill_tokens, s->prefill_keys, s->scale, s->softcap, s->window, 1, stream));
     }
     int expected = 0, nsrc = 0;
     B200_TRY(tp.scatter_gemm(s->attn, Hq * D, L->o, &expected, &nsrc));

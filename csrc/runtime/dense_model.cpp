@@ -364,6 +364,7 @@ void DenseModel::forward_cuda(const StepInputs& in) {
   st.num_decodes = nd; st.decode_splits = splits; st.decode_tc = tc ? 1 : 0;
   st.decode_tmp_o = decode_tmp_o_.data(); st.decode_tmp_lse = decode_tmp_lse_.data();
   st.num_prefills = in.num_prefills; st.num_tiles = in.num_tiles; st.num_prefill_tokens = T - nd;
+  st.prefill_keys = in.prefill_keys;
   st.prefill_q_start = in.prefill_q_start; st.tile_req = in.tile_req; st.tile_q0 = in.tile_q0;
   st.hidden = hidden_.data(); st.resid = resid_.data(); st.normed = normed_.data();
   st.qkv_buf = qkv_.data(); st.attn = attn_.data(); st.gate_up_buf = gate_up_.data(); st.act = act_.data();

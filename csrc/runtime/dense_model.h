@@ -46,6 +46,7 @@ struct DenseConfig {
 struct StepInputs {
   int num_tokens = 0, num_reqs = 0, num_decodes = 0, num_prefills = 0, num_prefill_tokens = 0, num_tiles = 0;
   int num_logits = 0;
+  int64_t prefill_keys = 0;
   const int64_t* input_ids = nullptr;
   const int64_t* positions = nullptr;
   const int64_t* slot_mapping = nullptr;

@@ -86,7 +86,7 @@ void NativeRunner::execute_model(const SchedulerOutput& so) {
   StepInputs in;
   in.num_tokens = info.num_tokens; in.num_reqs = info.num_reqs; in.num_decodes = info.num_decodes;
   in.num_prefills = info.num_prefills; in.num_prefill_tokens = info.num_prefill_tokens;
-  in.num_tiles = info.num_tiles; in.num_logits = info.num_logits;
+  in.num_tiles = info.num_tiles; in.prefill_keys = info.prefill_keys; in.num_logits = info.num_logits;
   in.input_ids = dev<int64_t>(layout_.input_ids);
   in.positions = dev<int64_t>(layout_.positions);
   in.slot_mapping = dev<int64_t>(layout_.slot_mapping);

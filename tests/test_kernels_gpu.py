@@ -291,13 +291,16 @@ def test_attn_prefill(D, Hq, Hkv, bs):
 
 
 @pytest.mark.parametrize("Hq,Hkv,bs,window,causal,peak", [(4, 2, 8, 0, True, 1.0), (8, 1, 256, 0, True, 8.0), (12, 2, 32, 150, True, 1.0),
-                                                          (8, 4, 64, -200, True, 1.0), (4, 2, 16, 0, False, 8.0)])
+                                                          (8, 4, 64, -200, True, 1.0), (4, 2, 16, 0, False, 8.0),
+                                                          (12, 2, 32, 1024, True, 1.0), (8, 4, 64, -1100, True, 1.0)])
 def test_attn_prefill_head_pairs(Hq, Hkv, bs, window, causal, peak):
     """128-dim heads in even groups: edges of the 128-row and 128-key tiles, cached prefixes, windows and chunks, keys that
     raise a row's maximum late (``peak``: the later half of the keys is that much longer). P and the output are rounded to
-    bf16 once each (2 x 2^-8)."""
+    bf16 once each (2 x 2^-8). Enough tiles and, as the kernel is told, keys for two heads a CTA, except for the short
+    windows."""
     torch.manual_seed(Hq + bs)
-    D, q_lens, ctx = 128, [1, 127, 128, 129, 300], [400, 0, 128, 1, 513]
+    D, q_lens, ctx = 128, [1, 127, 128, 129, 300, 4200], [400, 0, 128, 1, 513, 0]
+    assert Hq * sum(-(-n // 128) for n in q_lens) > ops.num_sms()
     seq_lens = [a + b for a, b in zip(q_lens, ctx)]
     cache, bt = _make_paged(seq_lens, Hkv, D, bs)
     for r, n in enumerate(seq_lens):
@@ -310,7 +313,7 @@ def test_attn_prefill_head_pairs(Hq, Hkv, bs, window, causal, peak):
     lse = torch.empty(T, Hq, dtype=torch.float32, device=DEV)
     out = ops.attn_prefill(q, cache, block_table=bt, seq_lens=sl, q_start=qs, tile_req=torch.tensor(treq, dtype=torch.int32, device=DEV),
                            tile_q0=torch.tensor(tq0, dtype=torch.int32, device=DEV), num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D,
-                           block_size=bs, scale=D ** -0.5, window=window, causal=causal, lse=lse)
+                           block_size=bs, scale=D ** -0.5, window=window, causal=causal, lse=lse, tile_keys=10 ** 6)
     G = Hq // Hkv
     for r, (n, c) in enumerate(zip(q_lens, ctx)):
         rows = slice(int(qs[r]), int(qs[r]) + n)
@@ -327,6 +330,28 @@ def test_attn_prefill_head_pairs(Hq, Hkv, bs, window, causal, peak):
         got = out[rows].view(n, Hq, D).double()
         assert ((got - exp).norm() / exp.norm()).item() < 2 * 2.0 ** -8
         assert (lse[rows].double().t() - torch.logsumexp(score, -1)).abs().max().item() < 1e-3
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("n,L", [(1, 400), (20, 130), (6, 384), (6, 383)])
+def test_attn_prefill_one_and_two_heads_a_cta(n, L):
+    """Both sides of the rule, told the number of keys or left to guess it: the rounding of P and the output (2 x 2^-8)."""
+    torch.manual_seed(L)
+    D, Hq, Hkv, bs = 128, 16, 4, 32
+    cache, bt = _make_paged([L] * n, Hkv, D, bs)
+    q = _rand(n * L, Hq * D)
+    treq, tq0 = ref.build_prefill_tiles([L] * n)
+    I = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+    kw = dict(block_table=bt, seq_lens=I([L] * n), q_start=I([i * L for i in range(n + 1)]), tile_req=I(treq), tile_q0=I(tq0),
+              num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, block_size=bs, scale=D ** -0.5)
+    keys = n * sum(min(a + 128, L) for a in range(0, L, 128))
+    outs = [ops.attn_prefill(q, cache, tile_keys=r, **kw).double() for r in (keys, 0, 1, 10 ** 6)]
+    k, v = (cache[bt.long(), i].reshape(n, -1, Hkv, D)[:, :L].double().repeat_interleave(Hq // Hkv, 2) for i in (0, 1))
+    score = torch.einsum("nqhd,nkhd->nhqk", q.view(n, L, Hq, D).double(), k) * D ** -0.5
+    score = score.masked_fill(torch.ones(L, L, dtype=torch.bool, device=DEV).triu(1), -float("inf"))
+    exp = torch.einsum("nhqk,nkhd->nqhd", torch.softmax(score, -1), v).reshape(n * L, Hq * D)
+    for got in outs:
+        assert ((got - exp).norm() / exp.norm()).item() < 2 * 2.0 ** -8
     assert ops.read_status() == 0
 
 

@@ -642,7 +642,7 @@ class GpuBackend(FusedLinearMixin):
                                   tile_q0=ctx.tile_q0[:ctx.num_tiles], num_q_heads=num_q_heads,
                                   num_kv_heads=num_kv_heads, head_dim=head_dim,
                                   block_size=block_size, scale=scale, out=out[nd:],
-                                  softcap=softcap, window=window)
+                                  softcap=softcap, window=window, tile_keys=ctx.prefill_keys)
         return out
 
     def stream_norm(self, stream, norm_w, eps, out, **kw):

@@ -36,6 +36,7 @@ class StepContext:
     decode_splits: int = 1
     max_seq_len: int = 0
     max_query_len: int = 0
+    prefill_keys: int = 0       # sum over the tiles of the positions up to a tile's last row (0: not known)
     decode_only_full_logits: bool = False   # decode-only batch: logits for every row
     extra: dict = field(default_factory=dict)
 

@@ -562,6 +562,7 @@ class DenseModel:
         if tmp is not None:
             s.decode_tmp_o, s.decode_tmp_lse = tmp[0].data_ptr(), tmp[1].data_ptr()
         s.num_prefills, s.num_tiles, s.num_prefill_tokens = ctx.num_prefills, ctx.num_tiles, T - nd
+        s.prefill_keys = ctx.prefill_keys
         if ctx.num_prefills > 0:
             s.prefill_q_start, s.tile_req, s.tile_q0 = (ctx.prefill_q_start.data_ptr(), ctx.tile_req.data_ptr(),
                                                         ctx.tile_q0.data_ptr())

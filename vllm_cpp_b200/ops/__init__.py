@@ -272,18 +272,20 @@ def attn_prefill(q: torch.Tensor, kv_cache: torch.Tensor, *, block_table: torch.
                  tile_q0: torch.Tensor, num_q_heads: int, num_kv_heads: int, head_dim: int,
                  block_size: int, scale: float, out: torch.Tensor | None = None,
                  lse: torch.Tensor | None = None, softcap: float = 0.0, window: int = 0,
-                 causal: bool = True):
+                 causal: bool = True, tile_keys: int = 0):
     """Varlen paged prefill attention. ``q``: [T, Hq*D] (row stride free); K/V are read from
-    the paged cache only. ``tile_req/tile_q0`` list the 128-row query tiles (host built)."""
+    the paged cache only. ``tile_req/tile_q0`` list the 128-row query tiles (host built). ``tile_keys``, the
+    sum over the tiles of the positions up to a tile's last row, only chooses between kernels (0: estimated)."""
     T = q.shape[0]
     if out is None:
         out = torch.empty((T, num_q_heads * head_dim), dtype=q.dtype, device=q.device)
     num_blocks = kv_cache.shape[0]
-    check(lib().b200_attn_prefill(
-        ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(lse), ptr(kv_cache), num_blocks,
-        block_size, num_q_heads, num_kv_heads, head_dim, ptr(block_table), block_table.stride(0),
-        ptr(seq_lens), ptr(q_start), ptr(tile_req), ptr(tile_q0), tile_req.numel(), T, scale,
-        softcap, window, int(causal), stream_ptr()), "attn_prefill")
+    args = (ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(lse), ptr(kv_cache), num_blocks,
+            block_size, num_q_heads, num_kv_heads, head_dim, ptr(block_table), block_table.stride(0),
+            ptr(seq_lens), ptr(q_start), ptr(tile_req), ptr(tile_q0), tile_req.numel(), T)
+    tail = (scale, softcap, window, int(causal), stream_ptr())
+    check(lib().b200_attn_prefill_keys(*args, tile_keys, *tail) if tile_keys > 0 else
+          lib().b200_attn_prefill(*args, *tail), "attn_prefill")
     return out
 
 

@@ -72,6 +72,7 @@ _SIGS = {
     "b200_concat_and_cache_mla": ([P, I, P, I, P, P, I, I, I, P], I),
     "b200_rope_table": ([P, P, I, I, F, P], I),
     "b200_attn_prefill": ([P, I, P, I, P, P, L, I, I, I, I, P, I, P, P, P, P, I, I, F, F, I, I, P], I),
+    "b200_attn_prefill_keys": ([P, I, P, I, P, P, L, I, I, I, I, P, I, P, P, P, P, I, I, L, F, F, I, I, P], I),
     "b200_attn_decode_splits": ([I, I, I, I, I], I),
     "b200_attn_decode": ([P, I, P, I, P, I, I, I, I, P, I, P, I, F, F, I, I, P, P, P], I),
     "b200_attn_decode_tc": ([P, I, P, I, P, L, I, I, I, I, P, I, P, I, F, F, I, I, P, P, P], I),

@@ -23,7 +23,7 @@ class DenseStep(C.Structure):
                 ("positions", P), ("cos_sin", P), ("slot_mapping", P), ("block_table", P), ("max_blocks", I),
                 ("seq_lens", P), ("num_decodes", I), ("decode_splits", I), ("decode_tc", I),
                 ("decode_tmp_o", P), ("decode_tmp_lse", P),
-                ("num_prefills", I), ("num_tiles", I), ("num_prefill_tokens", I),
+                ("num_prefills", I), ("num_tiles", I), ("num_prefill_tokens", I), ("prefill_keys", C.c_longlong),
                 ("prefill_q_start", P), ("tile_req", P), ("tile_q0", P),
                 ("hidden", P), ("resid", P), ("normed", P), ("qkv_buf", P), ("attn", P), ("gate_up_buf", P),
                 ("act", P), ("gemm_ws", P), ("gemm_ws_bytes", C.c_ulonglong), ("first_layer", I),

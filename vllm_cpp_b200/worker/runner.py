@@ -34,7 +34,7 @@ _DT = {"input_ids": (torch.int64, 8), "positions": (torch.int64, 8), "slot_mappi
 
 # StepInfo fields a rank needs to run a step it did not prepare itself
 STEP_INFO_FIELDS = ("num_reqs", "num_tokens", "num_decodes", "num_prefills", "num_prefill_tokens",
-                    "num_tiles", "max_query_len", "max_seq_len", "num_logits", "num_splice", "all_greedy",
+                    "num_tiles", "prefill_keys", "max_query_len", "max_seq_len", "num_logits", "num_splice", "all_greedy",
                     "any_penalties", "any_top_k_top_p", "any_min_p", "any_logprobs", "any_logit_edits",
                     "req_ids", "produces_token", "max_logprobs", "num_draft", "logits_row0", "num_score",
                     "score_req_ids", "score_positions")
@@ -233,6 +233,7 @@ class ModelRunner(E.ModelRunnerBase):
             num_decodes=nd, num_prefills=0 if padded is not None else info.num_prefills,
             num_prefill_tokens=0 if padded is not None else info.num_prefill_tokens,
             num_tiles=0 if padded is not None else info.num_tiles,
+            prefill_keys=0 if padded is not None else info.prefill_keys,
             num_logits=T if padded is not None else info.num_logits + info.num_score,
             input_ids=v["input_ids"], positions=v["positions"], slot_mapping=v["slot_mapping"],
             query_start=v["query_start"], seq_lens=v["seq_lens"], block_table=v["block_table"],
