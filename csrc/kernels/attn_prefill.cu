@@ -710,7 +710,7 @@ extern "C" int b200_attn_prefill_keys(const void* q, int ldq, void* out, int ldo
                       (uint64_t)Hq * D, (uint64_t)ldq, kQT, 64, CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
   // Pairs of heads need an even group, 128-dim heads, no soft-cap (it is applied to the scores one by one) and pages
-  // that divide a tile or are whole tiles.
+  // that divide a tile or are whole tiles, and tiles that the grid's second dimension holds.
   // They pay where a CTA sees keys enough: the start and the end of a CTA that has an SM to itself are in the open, and of 128
   // keys a tile more are masked. About 250 keys a tile on average are the line, or 96 where the grid is a single wave, and so
   // is more than half a wave: two heads a CTA leave SMs idle that one head a CTA has work for. A window or chunk shorter than
@@ -725,7 +725,7 @@ extern "C" int b200_attn_prefill_keys(const void* q, int ldq, void* out, int ldo
   const long long ctas = (long long)num_tiles * (Hq / 2), sms = b200_num_sms();
   const bool pair = D == 128 && (Hq / Hkv) % 2 == 0 && softcap == 0.f && scale > 0.f &&
                     (block_size <= kPT ? kPT % block_size == 0 : block_size % kPT == 0) &&
-                    (window == 0 || window >= 1024 || window <= -1024) && 2 * ctas > sms &&
+                    (window == 0 || window >= 1024 || window <= -1024) && num_tiles <= 65535 && 2 * ctas > sms &&
                     tile_keys >= (ctas <= sms ? 96 : 250) * (long long)num_tiles;
   const int most = pair ? kPT : kKT;
   const int box_rows = block_size < most ? block_size : most;

@@ -355,6 +355,26 @@ def test_attn_prefill_one_and_two_heads_a_cta(n, L):
     assert ops.read_status() == 0
 
 
+def test_attn_prefill_of_very_many_tiles():
+    """More tiles than a grid's second dimension holds: 66000 requests of one token, each after up to seven others."""
+    torch.manual_seed(4)
+    D, Hq, Hkv, bs, n = 128, 2, 1, 8, 66000
+    cache = _rand(5, 2, bs, Hkv, D)
+    bt = (torch.arange(n, device=DEV, dtype=torch.int32) % 5)[:, None].contiguous()
+    sl = torch.arange(n, device=DEV, dtype=torch.int32) % bs + 1
+    q = _rand(n, Hq * D)
+    i32 = dict(device=DEV, dtype=torch.int32)
+    out = ops.attn_prefill(q, cache, block_table=bt, seq_lens=sl, q_start=torch.arange(n + 1, **i32), tile_req=torch.arange(n, **i32),
+                           tile_q0=torch.zeros(n, **i32), num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, block_size=bs,
+                           scale=D ** -0.5, tile_keys=10 ** 9)
+    k, v = (cache[bt[:, 0].long(), i, :, 0].double() for i in (0, 1))
+    score = torch.einsum("nhd,nkd->nhk", q.view(n, Hq, D).double(), k) * D ** -0.5
+    score = score.masked_fill(torch.arange(bs, device=DEV)[None, None] >= sl[:, None, None], -float("inf"))
+    exp = torch.einsum("nhk,nkd->nhd", torch.softmax(score, -1), v).reshape(n, Hq * D)
+    assert ((out.double() - exp).norm() / exp.norm()).item() < 2 * 2.0 ** -8
+    assert ops.read_status() == 0
+
+
 def test_attn_prefill_window_softcap():
     torch.manual_seed(10)
     D, Hq, Hkv, bs = 128, 4, 2, 16
