@@ -206,7 +206,10 @@ __global__ void __launch_bounds__(128)
 }
 
 // Fixed-order merge of split partials: out = sum_s w_s * o_s, w_s = 2^(lse_s - lse_max) / sum. The weights are taken once a
-// block (splits floats of shared memory); the partial rows are on the way four at a time.
+// block into shared memory (STAGED: up to kMergeStaged splits; beyond, each thread takes them again); the partial rows are on
+// the way four at a time.
+static constexpr int kMergeStaged = 12288;      // 48 KB
+template <bool STAGED>
 __global__ void __launch_bounds__(128)
     attn_decode_merge_kernel(const float* __restrict__ tmp_o, const float* __restrict__ tmp_lse,
                              __nv_bfloat16* out, int ldo, int Hq, int D, int splits) {
@@ -215,15 +218,21 @@ __global__ void __launch_bounds__(128)
   pdl_launch_dependents();
   const int b = blockIdx.x, h = blockIdx.y;
   const size_t row0 = ((size_t)b * Hq + h) * splits;
-  for (int s = threadIdx.x; s < splits; s += blockDim.x) wgt[s] = tmp_lse[row0 + s];
-  __syncthreads();
+  if constexpr (STAGED) {
+    for (int s = threadIdx.x; s < splits; s += blockDim.x) wgt[s] = tmp_lse[row0 + s];
+    __syncthreads();
+  }
   float mx = -INFINITY;
-  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, wgt[s]);
-  __syncthreads();
-  for (int s = threadIdx.x; s < splits; s += blockDim.x) wgt[s] = wgt[s] == -INFINITY ? 0.f : exp2f(wgt[s] - mx);
-  __syncthreads();
+  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, STAGED ? wgt[s] : tmp_lse[row0 + s]);
+  auto weight_of = [&](float lse) { return lse == -INFINITY ? 0.f : exp2f(lse - mx); };
+  if constexpr (STAGED) {
+    __syncthreads();
+    for (int s = threadIdx.x; s < splits; s += blockDim.x) wgt[s] = weight_of(wgt[s]);
+    __syncthreads();
+  }
+  auto weight = [&](int s) { return STAGED ? wgt[s] : weight_of(tmp_lse[row0 + s]); };
   float den = 0.f;
-  for (int s = 0; s < splits; ++s) den += wgt[s];
+  for (int s = 0; s < splits; ++s) den += weight(s);
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float acc = 0.f;
     for (int s = 0; s < splits; s += 4) {
@@ -232,7 +241,7 @@ __global__ void __launch_bounds__(128)
       for (int e = 0; e < 4; ++e) o[e] = s + e < splits ? tmp_o[(row0 + s + e) * D + d] : 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        if (s + e < splits) acc += wgt[s + e] * o[e];
+        if (s + e < splits) acc += weight(s + e) * o[e];
     }
     out[(size_t)b * ldo + (size_t)h * D + d] = __float2bfloat16(den > 0.f ? acc / den : 0.f);
   }
@@ -322,8 +331,10 @@ int b200_attn_decode(const void* q, int ldq, void* out, int ldo, const void* kv_
 
 int b200_attn_decode_merge(const void* tmp_o, const void* tmp_lse, void* out, int ldo, int B,
                            int Hq, int D, int splits, cudaStream_t stream) {
-  return launch_pdl(attn_decode_merge_kernel, dim3(B, Hq), dim3(128), (size_t)splits * sizeof(float), stream, (const float*)tmp_o, (const float*)tmp_lse,
-                    (__nv_bfloat16*)out, ldo, Hq, D, splits) == cudaSuccess ? 0 : -2;
+  const bool staged = splits <= kMergeStaged;
+  return launch_pdl(staged ? attn_decode_merge_kernel<true> : attn_decode_merge_kernel<false>, dim3(B, Hq), dim3(128),
+                    staged ? (size_t)splits * sizeof(float) : 0, stream, (const float*)tmp_o, (const float*)tmp_lse, (__nv_bfloat16*)out, ldo,
+                    Hq, D, splits) == cudaSuccess ? 0 : -2;
 }
 
 int b200_merge_attn_states(const void* a, const void* lse_a, const void* b, const void* lse_b,

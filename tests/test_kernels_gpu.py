@@ -355,6 +355,25 @@ def test_attn_prefill_one_and_two_heads_a_cta(n, L):
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("splits", [3, 12288, 12289])
+def test_attn_decode_of_very_many_splits(splits):
+    """The merge of split partials with its weights in shared memory and, beyond what that holds, without; most splits are
+    empty. fp32 throughout, one rounding to bf16."""
+    torch.manual_seed(splits)
+    D, Hq, Hkv, bs = 64, 4, 2, 16
+    cache, bt = _make_paged([300, 17], Hkv, D, bs)
+    q = _rand(2, Hq * D)
+    sl = torch.tensor([300, 17], dtype=torch.int32, device=DEV)
+    out = ops.attn_decode(q, cache, block_table=bt, seq_lens=sl, num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, block_size=bs,
+                          scale=D ** -0.5, splits=splits, force_cuda_core=True)
+    for r, n in enumerate((300, 17)):
+        k, v = (cache[bt[r].long(), i].reshape(-1, Hkv, D)[:n].double().repeat_interleave(Hq // Hkv, 1) for i in (0, 1))
+        p = torch.softmax(torch.einsum("hd,khd->hk", q[r].view(Hq, D).double(), k) * D ** -0.5, -1)
+        exp = torch.einsum("hk,khd->hd", p, v)
+        assert ((out[r].view(Hq, D).double() - exp).norm() / exp.norm()).item() < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
 def test_attn_prefill_of_very_many_tiles():
     """More tiles than a grid's second dimension holds: 66000 requests of one token, each after up to seven others."""
     torch.manual_seed(4)
