@@ -88,3 +88,37 @@ def test_nvfp4_plan_file_round_trip(tmp_path, monkeypatch):
     finally:
         Q._NVFP4_PLANS.clear()
         Q._NVFP4_PLANS.update(saved)
+
+
+def test_weights_are_fetched_early_only_where_they_are_said_to_be_constant(monkeypatch):
+    """Bit 8 of the launchers' path flag lets a product read its weights before the previous kernel has finished. A caller
+    that has just written them (and has not said otherwise) must not get it, whatever the number of rows."""
+    from vllm_cpp_b200 import ops
+    from vllm_cpp_b200.models.backend import GpuBackend
+    flags = []
+
+    class Lib:
+        def b200_gemm_bf16_gated(self, *a):
+            flags.append(a[10])
+            return 0
+
+        def b200_gemm_bf16(self, *a):
+            flags.append(a[15])
+            return 0
+
+    monkeypatch.setattr(ops, "lib", lambda: Lib())
+    monkeypatch.setattr(ops, "stream_ptr", lambda: 0)
+    bf = dict(dtype=torch.bfloat16)
+    w = torch.zeros(256, 64, **bf)
+    for M in (1, 128, 129, 700):
+        a = torch.zeros(M, 64, **bf)
+        flags.clear()
+        ops.gemm_gated(a, w)
+        ops.gemm(a, w)
+        assert all(not f & 0x100 for f in flags)
+        flags.clear()
+        ops.gemm_gated(a, w, const_w=True)
+        be = GpuBackend.__new__(GpuBackend)
+        be.ops = ops
+        be.gemm_gated(a, w)
+        assert len(flags) == 2 and all(f & 0x100 for f in flags)

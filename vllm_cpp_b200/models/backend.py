@@ -601,7 +601,7 @@ class GpuBackend(FusedLinearMixin):
         if isinstance(w, (QuantWeight, Fp8Weight)):
             y = self.gemm(a, w, out=scratch)
             return self.ops.act_and_mul(y, kind, out, interleaved=True)
-        return self.ops.gemm_gated(a, w, kind, out=out, scratch=scratch)
+        return self.ops.gemm_gated(a, w, kind, out=out, scratch=scratch, const_w=True)
 
     def embedding(self, ids, table, out=None, vocab_start=0, vocab_total=None, scale=1.0):
         return self.ops.embedding(ids, table, out=out, vocab_start=vocab_start,

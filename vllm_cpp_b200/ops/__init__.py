@@ -133,16 +133,17 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 def gemm_gated(a: torch.Tensor, w_il: torch.Tensor, kind: int = ACT_SILU, *,
                out: torch.Tensor | None = None, scratch: torch.Tensor | None = None,
-               force_path: int = 0) -> torch.Tensor:
-    """``act(a @ w_gate^T) * (a @ w_up^T)`` with ``w_il`` (a model weight) from :func:`interleave_gate_up`; the
-    activation runs in the GEMM epilogue, the merged projection never reaches memory. ``scratch`` is not used."""
+               force_path: int = 0, const_w: bool = False) -> torch.Tensor:
+    """``act(a @ w_gate^T) * (a @ w_up^T)`` with ``w_il`` from :func:`interleave_gate_up`; the activation runs in
+    the GEMM epilogue, the merged projection never reaches memory. ``scratch`` is not used; ``const_w`` as in
+    :func:`gemm`."""
     M, K = a.shape
     N = w_il.shape[0]
     assert a.dtype == torch.bfloat16 and w_il.dtype == torch.bfloat16 and N % 256 == 0
     if out is None:
         out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=a.device)
     check(lib().b200_gemm_bf16_gated(ptr(a), a.stride(0), ptr(w_il), w_il.stride(0), ptr(out),
-                                     out.stride(0), M, N, K, kind, force_path | 0x100, stream_ptr()),
+                                     out.stride(0), M, N, K, kind, force_path | (0x100 if const_w else 0), stream_ptr()),
           f"gemm_gated M={M} N={N} K={K}")
     return out
 
