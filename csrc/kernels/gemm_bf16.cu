@@ -1362,6 +1362,17 @@ extern "C" int b200_gemm_bf16_gated(const void* A, int lda, const void* W, int l
                         force_path, nullptr, stream, kind + 1);
 }
 
+// Whether the gated product of M <= 128 rows is the faster one as a plain product and the activation kernel. The cluster kernel's
+// exchange grows with the rows and is in the open on wide matrices: from 33 rows where the grid needs a second wave (2 N / 256
+// CTAs, two to an SM), from 97 where its one wave is not nearly full; the plain product then runs 128 x 256 tiles with
+// stream-K, and the merged projection costs less than that. us, two kernels / one: 40960 x 5120 at 33 / 128 rows 83.8 / 92.7,
+// 89.2 / 110.2; 57344 x 8192 157 / 152, 166 / 174; 28672 x 4096 at 64 / 112 / 128 50.6 / 48.1, 51.7 / 52.6, 52.2 / 53.3; 22016 x
+// 4096 at 128 45.4 / 47.0; 37888 x 3584 (a full wave) 56.7 / 56.1; 16384 x 2048 28.8 / 20.4.
+extern "C" int b200_gemm_gated_apart(int M, int N) {
+  const int tiles = N / 128, sms = b200_num_sms();
+  return M <= 128 && ((M > 32 && tiles > 2 * sms) || (M > 96 && tiles > sms && 6 * tiles < 10 * sms));
+}
+
 // e4m3 x e4m3 -> bf16 on the CTA-pair kernel (M > 256): out = (A W^T) * a_scale * w_scale (+ bias).
 // Reference: MatmulFp8CublasLt / MatmulFp8Cutlass in src/vt/cuda/cuda_matmul.cu.
 extern "C" int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo,

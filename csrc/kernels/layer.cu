@@ -167,12 +167,13 @@ int b200_dense_layer(const B200DenseLayerWeights* w, const B200DenseStep* s, cud
     return launches;
   }
   B200_TRY(b200_rmsnorm(s->hidden, H, s->resid, w->ln2, s->normed, H, T, H, s->eps, s->gemma, stream));
-  if (s->gate_up_interleaved) {
+  if (s->gate_up_interleaved && !b200_gemm_gated_apart(T, 2 * I)) {
     B200_TRY(b200_gemm_bf16_gated(s->normed, H, w->gate_up, H, s->act, I, T, 2 * I, H, s->act_kind, kConstW, stream));
   } else {
     B200_TRY(b200_gemm_bf16(s->normed, H, w->gate_up, H, s->gate_up_buf, 2 * I, 0, nullptr, nullptr, 0, T, 2 * I,
                             H, s->gemm_ws, (size_t)s->gemm_ws_bytes, kConstW, stream));
-    B200_TRY(b200_act_and_mul(s->gate_up_buf, 2 * I, s->act, T, I, s->act_kind, stream));
+    B200_TRY(b200_act_and_mul(s->gate_up_buf, 2 * I, s->act, T, I, s->act_kind | (s->gate_up_interleaved ? 0x100 : 0),
+                              stream));
   }
   B200_TRY(b200_gemm_bf16(s->act, I, w->down, I, s->hidden, H, 0, nullptr, nullptr, 0, T, H, I, s->gemm_ws,
                           (size_t)s->gemm_ws_bytes, kConstW, stream));

@@ -145,6 +145,23 @@ def test_gemm_gated_over_a_cluster(M, I, K):
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("M,I,apart", [(32, 19200, 0), (33, 19200, 1), (96, 9600, 0), (97, 9600, 1), (128, 16000, 0), (129, 19200, 0)])
+def test_gemm_gated_in_one_and_in_two_kernels(M, I, apart):
+    """Both sides of the lines, against 64 bits: gate, up and their product are rounded once each (3 x 2^-8, and the sums)."""
+    from vllm_cpp_b200.ops import _lib
+    torch.manual_seed(M)
+    K = 264
+    assert bool(_lib.lib().b200_gemm_gated_apart(M, 2 * I)) == bool(apart)
+    a, g, u = _rand(M, K), _rand(I, K, scale=0.05), _rand(I, K, scale=0.05)
+    w = ops.interleave_gate_up(g, u)
+    gd, ud = a.double() @ g.double().t(), a.double() @ u.double().t()
+    exp = gd * torch.sigmoid(gd) * ud
+    forms = [ops.gemm_gated(a, w)] + ([ops.gemm_gated(a, w, force_path=32)] if M <= 128 else [])
+    for out in forms:
+        assert _rel_err(out.double(), exp) < 2.0 ** -6
+    assert ops.read_status() == 0
+
+
 @pytest.mark.parametrize("M", [1, 2])
 @pytest.mark.parametrize("N,K", [(8, 8), (264, 72), (1032, 1000), (6144, 1024), (4096, 14336), (40000, 512)])
 def test_gemm_of_one_or_two_rows(M, N, K):

@@ -102,12 +102,16 @@ def test_weights_are_fetched_early_only_where_they_are_said_to_be_constant(monke
             flags.append(a[10])
             return 0
 
+        def b200_gemm_gated_apart(self, M, N):
+            return M == 128
+
         def b200_gemm_bf16(self, *a):
             flags.append(a[15])
             return 0
 
     monkeypatch.setattr(ops, "lib", lambda: Lib())
     monkeypatch.setattr(ops, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(ops, "act_and_mul", lambda *a, **k: None)
     bf = dict(dtype=torch.bfloat16)
     w = torch.zeros(256, 64, **bf)
     for M in (1, 128, 129, 700):

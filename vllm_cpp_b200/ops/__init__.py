@@ -134,14 +134,17 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 def gemm_gated(a: torch.Tensor, w_il: torch.Tensor, kind: int = ACT_SILU, *,
                out: torch.Tensor | None = None, scratch: torch.Tensor | None = None,
                force_path: int = 0, const_w: bool = False) -> torch.Tensor:
-    """``act(a @ w_gate^T) * (a @ w_up^T)`` with ``w_il`` from :func:`interleave_gate_up`; the activation runs in
-    the GEMM epilogue, the merged projection never reaches memory. ``scratch`` is not used; ``const_w`` as in
-    :func:`gemm`."""
+    """``act(a @ w_gate^T) * (a @ w_up^T)`` with ``w_il`` from :func:`interleave_gate_up`. The activation runs in the
+    GEMM epilogue, except on wide matrices with some tens of rows, where the merged projection (``scratch``) and
+    the activation kernel are the faster way. ``const_w`` as in :func:`gemm`."""
     M, K = a.shape
     N = w_il.shape[0]
     assert a.dtype == torch.bfloat16 and w_il.dtype == torch.bfloat16 and N % 256 == 0
     if out is None:
         out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=a.device)
+    if force_path == 0 and lib().b200_gemm_gated_apart(M, N):
+        scratch = gemm(a, w_il, out=scratch, const_w=const_w)
+        return act_and_mul(scratch, kind, out, interleaved=True)
     check(lib().b200_gemm_bf16_gated(ptr(a), a.stride(0), ptr(w_il), w_il.stride(0), ptr(out),
                                      out.stride(0), M, N, K, kind, force_path | (0x100 if const_w else 0), stream_ptr()),
           f"gemm_gated M={M} N={N} K={K}")
