@@ -250,8 +250,15 @@ __global__ void __launch_bounds__(kVThreads, 3) gemv_kernel(GemvParams p) {
 }
 
 // One row: all but the longest K, where the cluster kernel's deeper ring keeps HBM busier (4096 x 14336: 22.2 against 23.7
-// us). Two rows: small matrices (1024 x 3072 5.3 -> 3.6 us, 5120 x 2048 7.2 -> 5.7; 4096 x 4096 8.5 against 9.5).
-bool gemv_takes(int M, int N, int K) { return M == 1 ? K <= 8192 : M == 2 && K <= 8192 && (long long)N * K <= (12 << 20); }
+// us). Two rows: small matrices (1024 x 3072 5.3 -> 3.6 us, 5120 x 2048 7.2 -> 5.7; 4096 x 4096 8.5 against 9.5). A block that
+// takes several pairs of rows in turn pays for each turn's first loads, which a short K does not cover (us, this kernel / the
+// cluster kernel: 6144 x 256, one turn, 2.4 / 3.5; 8192 x 128 3.8 / 2.8; 14336 x 256 5.3 / 3.6; 16376 x 512, three, 6.2 / 6.3;
+// 24576 x 512, four, 7.9 / 6.6; 57344 x 1024 22.6 / 24.6; two rows: 12288 x 512 5.0 / 5.9, 16376 x 512 6.8 / 6.3).
+bool gemv_takes(int M, int N, int K) {
+  if (M < 1 || M > 2 || K > 8192 || (M == 2 && (long long)N * K > (12 << 20))) return false;
+  const long long warps = 3LL * b200_num_sms() * kVWarps, turns = ((N + 1) / 2 + warps - 1) / warps;
+  return turns == 1 || K >= 1024 || (K >= 512 && turns <= 4 - M);
+}
 
 int launch_gemv(const GemmCluster& g, const GemvNorm* norm, cudaStream_t stream) {
   if (!gemv_takes(g.M, g.N, g.K) || (g.K & 7) || (g.gated && (g.N & 255))) return -1;
