@@ -1442,9 +1442,11 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   if (act_fuse && ((tp && tp->scatter) || (tp && M <= 128) || (N & 255) || bias || residual || out_f32)) return -1;
   // Up to 128 rows: K split over a cluster, two CTAs per SM. On the widest matrices (no split to gain from) the tiled
   // kernel, which reads 256 weight rows with one copy of the batch, is the faster one from some rows on
-  // (128256 x 4096: 172.6 against 169.9 us at 40 rows, 178 against 172 at 64; at 32 rows 167 against 170, at 1 158 against 185).
+  // (128256 x 4096: 172.6 against 169.9 us at 40 rows, 178 against 172 at 64; at 32 rows 167 against 170, at 1 158 against 185;
+  // beyond one wave of CTAs with a short K earlier: 57344 x 512 at 32 rows 16.7 against 15.6, at 16 15.2 against 16.7).
+  const bool tiles_win = N >= 16384 && (M > 32 || (M > 16 && K <= 512 && (N + kBM - 1) / kBM > 2 * b200_num_sms()));
   const bool cluster = !tp && M <= 128 && !((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(residual)) & 7) &&
-                       (force_path == 0 ? act_fuse || M <= 32 || N < 16384 : force_path >= 32 && force_path <= 40);
+                       (force_path == 0 ? act_fuse || !tiles_win : force_path >= 32 && force_path <= 40);
   if (act_fuse && !cluster && force_path == 0) force_path = 9;      // the gated epilogue lives in the pair kernel
   if ((K & 7) || (lda & 7) || (ldw & 7) || (N & 7) || (ldo & 7) || (residual && (ldr & 7))) return -1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) |

@@ -313,7 +313,11 @@ static int clusters_at_once(int ranks) {
 // stages of K each. A grid that needs a second wave loses more than the finer split gains (us at M = 1, splits 4 / 5 / 6 / 8):
 //   6144 x 4096 (48 tiles)   12.6 / 10.7 / 17.7 / 15.2     4096 x 4096 (32)   11.9 / 10.4 / 8.5 / 8.7
 //   5120 x 4096 (40 tiles)   12.2 / 10.3 /  9.4 / 14.8     6144 x 1024 (48)    6.0 /  5.8 / 9.8 / 9.4
+// Up to four stages of K are fetched sooner than they are exchanged, once there are row tiles enough (us at 3 / 64 rows, one
+// part / two: 8192 x 256 3.5 / 4.1, 5.8 / 6.4; 14336 x 256 3.6 / 5.1, 5.8 / 7.7; 4096 x 256 3.6 / 3.6, 5.7 / 5.6). A gated tile
+// is exchanged in any case (12288 x 256 at 64 rows 9.5 / 8.4).
 static int choose_splits(int clusters, int kblocks, int gated) {
+  if (!gated && kblocks <= 4 && clusters >= 64) return 1;
   int s = gated ? 4 : 8;
   while (s > 1 && (s * 2 > kblocks || clusters > clusters_at_once(gated ? 2 * s : s))) --s;
   return s;

@@ -178,6 +178,17 @@ def test_gemm_of_one_or_two_rows(M, N, K):
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(3, 8192, 256), (3, 8064, 264), (1, 7104, 136), (1, 7112, 136), (2, 14208, 520), (2, 14216, 520),
+                                   (1, 21312, 1000), (1, 21320, 1000), (16, 38016, 512), (17, 38016, 512), (17, 38016, 520)])
+def test_gemm_at_the_lines_between_its_forms(M, N, K):
+    """Turns of a block of one- and two-row products, four k-blocks in one part, wide matrices with a short K. Off by the
+    rounding to bf16 at most (2^-8)."""
+    torch.manual_seed(N + K)
+    a, w = _rand(M, K), _rand(N, K, scale=0.05)
+    assert _rel_err(ops.gemm(a, w).double(), a.double() @ w.double().t()) < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
 def test_gemm_deterministic():
     torch.manual_seed(3)
     a, w = _rand(48, 4096), _rand(4096, 4096, scale=0.05)
