@@ -1440,12 +1440,28 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   force_path &= 0xff;
   if (act > 4 || (act && (tp || act_fuse))) return -1;
   if (act_fuse && ((tp && tp->scatter) || (tp && M <= 128) || (N & 255) || bias || residual || out_f32)) return -1;
+  // The epilogues read bias and residual in pieces of 16 bytes (tiles), 8 (cluster, split-K sums) or 2 (gemv, unsplit swap-AB):
+  // an address that a form cannot read goes to one that can, more than 256 rows in slices of as many.
+  const uintptr_t at = reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(residual);
+  if ((at & 15) && force_path != 0 && force_path != 2 && (force_path < 32 || force_path > 40 || (at & 7))) return -1;
+  if ((at & 15) && M > 256) {
+    for (int m = 0; m < M; m += 256) {
+      const auto rows = [&](const void* p, long long ld, int bytes) {
+        return p ? static_cast<const void*>(static_cast<const char*>(p) + m * ld * bytes) : nullptr;
+      };
+      const int rc = gemm_bf16_impl(rows(A, lda, 2), lda, W, ldw, const_cast<void*>(rows(out, ldo, out_f32 ? 4 : 2)), ldo, out_f32,
+                                    bias, rows(residual, ldr, 2), ldr, M - m < 256 ? M - m : 256, N, K, workspace, ws_bytes,
+                                    w_early << 8 | act << 9, tp, stream, act_fuse);
+      if (rc) return rc;
+    }
+    return 0;
+  }
   // Up to 128 rows: K split over a cluster, two CTAs per SM. On the widest matrices (no split to gain from) the tiled
   // kernel, which reads 256 weight rows with one copy of the batch, is the faster one from some rows on
   // (128256 x 4096: 172.6 against 169.9 us at 40 rows, 178 against 172 at 64; at 32 rows 167 against 170, at 1 158 against 185;
   // beyond one wave of CTAs with a short K earlier: 57344 x 512 at 32 rows 16.7 against 15.6, at 16 15.2 against 16.7).
-  const bool tiles_win = N >= 16384 && (M > 32 || (M > 16 && K <= 512 && (N + kBM - 1) / kBM > 2 * b200_num_sms()));
-  const bool cluster = !tp && M <= 128 && !((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(residual)) & 7) &&
+  const bool tiles_win = N >= 16384 && !(at & 15) && (M > 32 || (M > 16 && K <= 512 && (N + kBM - 1) / kBM > 2 * b200_num_sms()));
+  const bool cluster = !tp && M <= 128 && !(at & 7) &&
                        (force_path == 0 ? act_fuse || !tiles_win : force_path >= 32 && force_path <= 40);
   if (act_fuse && !cluster && force_path == 0) force_path = 9;      // the gated epilogue lives in the pair kernel
   if ((K & 7) || (lda & 7) || (ldw & 7) || (N & 7) || (ldo & 7) || (residual && (ldr & 7))) return -1;
@@ -1498,6 +1514,7 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   // Batches that the cluster kernel does not take. On wide matrices the batch goes on the (padded) M side
   // and 256 weight rows share an instruction, with stream-K filling the SMs: 1-CTA 128 x 256 tiles up to 128
   // rows, CTA pairs above; narrower matrices: 128 x 128 tiles + stream-K.
+  if (at & 15) force_path = 2;
   if (force_path == 0 && !tp && M <= 256) force_path = N < 16384 ? (M <= 128 ? 2 : 6) : M <= 128 ? 5 : 9;
   if (force_path == 1 || force_path >= 3) use_swap = false;     // an explicit tiling was asked for
   if (force_path == 2 && M <= 256) use_swap = true;
@@ -1507,7 +1524,7 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
     p.mp = mp;
     p.tiles_n = (N + kBM - 1) / kBM;
     int splits = 1;
-    if (p.tiles_n < sms && !(tp && tp->scatter)) {
+    if (p.tiles_n < sms && !(tp && tp->scatter) && !(at & 7)) {
       splits = sms / p.tiles_n;       // whole CTAs per SM: one wave, never a ragged second one
       int max_by_k = kblocks / 4;
       if (max_by_k < 1) max_by_k = 1;

@@ -545,15 +545,17 @@ int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int
                   cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K & 15) || (lda & 15) || (ldw & 15) || (N & 7) || (ldo & 7)) return -1;
+  const uintptr_t out_at = reinterpret_cast<uintptr_t>(out), bias_at = reinterpret_cast<uintptr_t>(bias);
+  const uintptr_t scale_at = w_scale_per_channel & 1 ? reinterpret_cast<uintptr_t>(w_scale) : 0;
+  if ((out_at & 7) || (M > 128 && ((out_at | scale_at) & 15))) return -1;        // (their vectors)
   // prefill-sized batches: CTA pairs, 256 x 256 tiles, stream-K (the 128 x 128 kernel below keeps
-  // the small batches)
-  if (M > 256 && N >= 256)
+  // the small batches, and biases that are not read in pieces of 16 bytes)
+  if (M > 256 && N >= 256 && !(bias_at & 15))
     return b200_gemm_fp8_pair(A, lda, W, ldw, out, ldo, a_scale, w_scale, w_scale_per_channel, bias, M, N, K,
                               stream);
   // up to 128 rows: weight-bound, K split over a cluster (gemm_cluster.cu); 32 requests of the fp8 8B shape 166 -> 148 ms
   // against 128 x 128 tiles with split-K partials in memory
-  if (M <= 128 && !(reinterpret_cast<uintptr_t>(bias) & 7) &&
-      (!fp8_tiles_win(M, N, K) || ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(w_scale)) & 15))) {
+  if (M <= 128 && !(bias_at & 7) && (!fp8_tiles_win(M, N, K) || ((out_at | scale_at) & 15))) {
     GemmCluster g{};
     g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.out = out; g.ldo = ldo; g.bias = bias;
     g.M = M; g.N = N; g.K = K;
@@ -563,6 +565,7 @@ int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int
     g.batch = 1;
     return launch_gemm_cluster(g, stream);
   }
+  if ((out_at | scale_at) & 15) return -1;
   CUtensorMap tmA, tmB;
   if (!encode_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, lda, kQM, kQKB, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !encode_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, ldw, kQN, kQKB, CU_TENSOR_MAP_SWIZZLE_128B))
@@ -585,7 +588,7 @@ int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int
     int splits = sms / tiles0;
     if (splits > kblocks / 4) splits = kblocks / 4;
     if (splits > 16) splits = 16;
-    if (splits >= 2 && !(N & 3) && !(ldo & 3)) {
+    if (splits >= 2 && !(N & 3) && !(ldo & 3) && !(bias_at & 7)) {
       float* scratch = fp8_splitk_scratch(stream);
       if (scratch) {
         p.kb_per_split = (kblocks + splits - 1) / splits;

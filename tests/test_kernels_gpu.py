@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 
 from vllm_cpp_b200 import ops  # noqa: E402
 from vllm_cpp_b200.ops import reference as ref  # noqa: E402
+from vllm_cpp_b200.ops._lib import KernelError  # noqa: E402
 
 DEV = "cuda"
 
@@ -186,6 +187,25 @@ def test_gemm_at_the_lines_between_its_forms(M, N, K):
     torch.manual_seed(N + K)
     a, w = _rand(M, K), _rand(N, K, scale=0.05)
     assert _rel_err(ops.gemm(a, w).double(), a.double() @ w.double().t()) < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1032, 264), (40, 1032, 2048), (17, 16400, 264), (40, 16400, 264), (200, 1032, 2048), (200, 16400, 264),
+                                   (300, 1032, 264), (600, 16400, 264)])
+def test_gemm_with_bias_and_residual_at_any_address(M, N, K):
+    """Every form reads them in pieces of its own size: addresses that are multiples of 16, 8 and 2 bytes. A tiling that was
+    asked for and cannot read them refuses."""
+    torch.manual_seed(M + N)
+    a, w = _rand(M, K), _rand(N, K, scale=0.05)
+    bias, res = _rand(N + 8), _rand(M * N + 8)
+    exact = a.double() @ w.double().t()
+    for off in (0, 4, 1):
+        b, r = bias[off: off + N], res[off: off + M * N].view(M, N)
+        assert _rel_err(ops.gemm(a, w, bias=b).double(), exact + b.double()) < 2.0 ** -8
+        assert _rel_err(ops.gemm(a, w, bias=bias[:N], residual=r).double(), exact + bias[:N].double() + r.double()) < 2.0 ** -8
+        if off:
+            with pytest.raises(KernelError):
+                ops.gemm(a, w, bias=b, force_path=7)
     assert ops.read_status() == 0
 
 

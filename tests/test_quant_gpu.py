@@ -6,6 +6,7 @@ pytestmark = pytest.mark.gpu
 
 from vllm_cpp_b200 import ops  # noqa: E402
 from vllm_cpp_b200.ops import quant as Q  # noqa: E402
+from vllm_cpp_b200.ops._lib import KernelError  # noqa: E402
 
 DEV = "cuda"
 
@@ -147,6 +148,28 @@ def test_gemm_fp8_tiles_and_clusters(M, N, K):
         out = Q.gemm_fp8(a8, w8, sa, sw[off: off + N])
         assert ops.read_status() == 0
         assert _within_sum_error(out, a64, w64, a64 @ w64.t())
+
+
+@pytest.mark.parametrize("M,N,K", [(40, 1032, 4096), (128, 4104, 512), (200, 1032, 4096), (300, 1032, 4096), (300, 136, 512)])
+def test_gemm_fp8_with_a_bias_at_any_address(M, N, K):
+    """Biases at multiples of 16, 8 and 2 bytes; results and channel scales that the tiles' vectors cannot reach are refused
+    where only tiles are left."""
+    torch.manual_seed(15)
+    a8 = (torch.randn(M, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    w8 = (torch.randn(N, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    sa, sw = torch.rand(M, device=DEV) + 0.5, torch.rand(N + 8, device=DEV) * 0.1 + 0.01
+    bias = torch.randn(N + 8, device=DEV).to(torch.bfloat16)
+    a64, w64 = a8.double() * sa.double()[:, None], w8.double() * sw[:N].double()[:, None]
+    for off in (0, 4, 1):
+        b = bias[off: off + N]
+        out = Q.gemm_fp8(a8, w8, sa, sw[:N], bias=b)
+        assert ops.read_status() == 0
+        assert _within_sum_error(out, a64, w64, a64 @ w64.t() + b.double())
+    if M > 128:
+        room = torch.empty(M * N + 8, dtype=torch.bfloat16, device=DEV)
+        for kw, s in (({"out": room[4: 4 + M * N].view(M, N)}, sw[:N]), ({}, sw[1: 1 + N])):
+            with pytest.raises(KernelError):
+                Q.gemm_fp8(a8, w8, sa, s, **kw)
 
 
 @pytest.mark.parametrize("T", [1, 296, 297])
