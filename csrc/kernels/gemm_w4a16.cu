@@ -576,8 +576,9 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
     const int tiles = (N + kCRows - 1) / kCRows, blocks = K / 256;
     csplits = cluster_splits(tiles, blocks / 2);
     const int more = 4 * ((blocks + csplits - 1) / csplits) - ne_per;
-    if (100 * more > 460 + 11 * M || (M > 32 && tiles > sms)) cluster = false;
+    if (!(reinterpret_cast<uintptr_t>(out) & 15) && (100 * more > 460 + 11 * M || (M > 32 && tiles > sms))) cluster = false;
   }
+  if (!cluster && splits == 1 && (reinterpret_cast<uintptr_t>(out) & 15)) return -1;        // (the stream form's vectors)
   __half* a16 = reinterpret_cast<__half*>(workspace);
   {
     const size_t total = (size_t)M * (K / 8);

@@ -111,9 +111,14 @@ def test_w4a16_stream_and_cluster(M, N, K):
     g = torch.full((1,), 0.01, device=DEV)
     a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
     w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
-    out = Q.gemm_w4a16(a, packed, sf, g)
-    assert ops.read_status() == 0
-    assert _within_sum_error(out, a64, w64, a64 @ w64.t(), 2**-25 * w64.abs().sum(1))
+    room = torch.empty(M * N + 4, dtype=torch.bfloat16, device=DEV)
+    for out in (Q.gemm_w4a16(a, packed, sf, g), Q.gemm_w4a16(a, packed, sf, g, out=room[4:].view(M, N))):    # 8 bytes off: cluster
+        assert ops.read_status() == 0
+        assert _within_sum_error(out, a64, w64, a64 @ w64.t(), 2**-25 * w64.abs().sum(1))
+    if N == 38016:
+        with pytest.raises(KernelError):                   # K not a multiple of 256 and no split: no form can write there
+            Q.gemm_w4a16(a[:, :K - 64].contiguous(), packed[:, :K // 2 - 32].contiguous(), sf[:, :K // 16 - 4].contiguous(), g,
+                         out=room[4:].view(M, N))
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 8, 16), (17, 520, 144), (65, 136, 4112), (128, 4104, 8192)])
