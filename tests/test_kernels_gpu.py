@@ -158,9 +158,11 @@ def test_gemm_gated_in_one_and_in_two_kernels(M, I, apart):
     gd, ud = a.double() @ g.double().t(), a.double() @ u.double().t()
     exp = gd * torch.sigmoid(gd) * ud
     forms = [ops.gemm_gated(a, w)] + ([ops.gemm_gated(a, w, force_path=32)] if M <= 128 else [])
+    room = torch.full((M, I + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    forms.append(ops.gemm_gated(a, w, out=room[:, :I]))                # rows of its own pitch: one kernel
     for out in forms:
         assert _rel_err(out.double(), exp) < 2.0 ** -6
-    assert ops.read_status() == 0
+    assert bool((room[:, I:] == 7.0).all()) and ops.read_status() == 0
 
 
 @pytest.mark.parametrize("M", [1, 2])

@@ -142,7 +142,8 @@ def gemm_gated(a: torch.Tensor, w_il: torch.Tensor, kind: int = ACT_SILU, *,
     assert a.dtype == torch.bfloat16 and w_il.dtype == torch.bfloat16 and N % 256 == 0
     if out is None:
         out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=a.device)
-    if force_path == 0 and lib().b200_gemm_gated_apart(M, N):
+    whole = out.is_contiguous() and out.data_ptr() % 16 == 0           # as the activation kernel writes it
+    if force_path == 0 and whole and lib().b200_gemm_gated_apart(M, N):
         scratch = gemm(a, w_il, out=scratch, const_w=const_w)
         return act_and_mul(scratch, kind, out, interleaved=True)
     check(lib().b200_gemm_bf16_gated(ptr(a), a.stride(0), ptr(w_il), w_il.stride(0), ptr(out),
