@@ -143,8 +143,7 @@ int b200_dense_attn_half(const B200DenseLayerWeights* w, const B200DenseStep* s,
 // Returns the number of launcher calls made (>= 1 kernel each), or a negative error code.
 int b200_dense_layer(const B200DenseLayerWeights* w, const B200DenseStep* s, cudaStream_t stream) {
   if (!w || !s || s->T <= 0) return 0;
-  // (narrow test models keep the launches of the per-op path)
-  if (!w->fp8 && s->gate_up_interleaved && s->H >= 512 && !(s->H & 7) && !(s->inter & 127) &&
+  if (!w->fp8 && s->gate_up_interleaved && !(s->H & 7) && !(s->inter & 127) &&
       b200::gemv_takes(s->T, (s->Hq + 2 * s->Hkv) * s->D, s->H) && b200::gemv_takes(s->T, 2 * s->inter, s->H))
     return dense_layer_rows(w, s, stream);
   int launches = b200_dense_attn_half(w, s, stream);

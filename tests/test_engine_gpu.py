@@ -144,7 +144,9 @@ def test_native_layer_entry_same_logits_as_per_op_path():
         self.native_layers = True
         n0 = _lib.LAUNCHES[0]
         b = orig(self, ctx)
-        seen.append((ctx.num_decodes, ctx.num_prefills, _lib.LAUNCHES[0] - n0, torch.equal(a, b)))
+        # a block of one or two rows takes its norms into the products: six launches, eight otherwise
+        fewest = (6 if ctx.num_tokens <= 2 else 8) * cfg.num_layers
+        seen.append((ctx.num_decodes, ctx.num_prefills, _lib.LAUNCHES[0] - n0 >= fewest, torch.equal(a, b)))
         return b
 
     type(m).forward = both
@@ -154,14 +156,15 @@ def test_native_layer_entry_same_logits_as_per_op_path():
         type(m).forward = orig
     assert any(nd and npf for nd, npf, _, _ in seen) and any(nd and not npf for nd, npf, _, _ in seen)
     assert all(eq for *_, eq in seen), seen
-    assert all(n >= 8 * cfg.num_layers for _, _, n, _ in seen)       # the launches are counted
+    assert all(counted for _, _, counted, _ in seen)                 # the launches are counted
     assert ops.read_status() == 0
 
 
-def test_dense_layer_of_one_and_two_rows():
-    """The block that takes its norms into the products against the per-op path: the same bits."""
+@pytest.mark.parametrize("hidden,inter", [(1024, 1536), (256, 384), (72, 128)])
+def test_dense_layer_of_one_and_two_rows(hidden, inter):
+    """The block that takes its norms into the products against the per-op path: the same bits, of narrow models too."""
     cfg = synthetic_config("tiny-qwen3")
-    cfg.head_dim, cfg.hidden_size, cfg.intermediate_size, cfg.num_layers = 128, 1024, 1536, 3
+    cfg.head_dim, cfg.hidden_size, cfg.intermediate_size, cfg.num_layers = 128, hidden, inter, 3
     llm = LLM(EngineArgs(model_config=cfg, device="cuda", block_size=16, num_blocks=64, max_model_len=256, max_num_seqs=2,
                          max_num_batched_tokens=64, enable_cuda_graphs=False))
     m, seen = llm.runner.model, []
@@ -171,8 +174,9 @@ def test_dense_layer_of_one_and_two_rows():
         self.native_layers = False
         a = orig(self, ctx).clone()
         self.native_layers = True
+        n0 = _lib.LAUNCHES[0]
         b = orig(self, ctx)
-        seen.append((ctx.num_tokens, torch.equal(a, b)))
+        seen.append((ctx.num_tokens, torch.equal(a, b) and (ctx.num_tokens > 2 or _lib.LAUNCHES[0] - n0 < 8 * cfg.num_layers)))
         return b
 
     type(m).forward = both
