@@ -206,3 +206,26 @@ def test_async_chunks_of_a_long_prompt_behind_a_busy_gpu():
         got.append(llm.take_scores()["a"][0][1])
     assert ops.read_status() == 0
     assert torch.equal(got[0], got[1])
+
+
+def test_async_ids_behind_a_busy_copy_stream():
+    """The sampled ids are copied to the host on a stream of their own; their memory must not be reused before that."""
+    cfg = _cfg()
+    prompts = _prompts(cfg, (9, 40, 17))
+    got = []
+    for mode in (False, True):
+        llm = LLM(EngineArgs(model_config=cfg, device="cuda", block_size=16, num_blocks=200, max_model_len=128, max_num_seqs=4,
+                             max_num_batched_tokens=64, async_scheduling=mode, enable_prefix_caching=False))
+        for i, p in enumerate(prompts):
+            llm.add_request(p, SamplingParams(temperature=0.0, max_tokens=12, ignore_eos=True), request_id=str(i))
+        out = {}
+        while llm.has_unfinished_requests():
+            if mode:
+                with torch.cuda.stream(llm.runner.copy_stream):
+                    torch.cuda._sleep(20_000_000)          # about 10 ms ahead of each copy
+            for o in llm.step():
+                if o.finished:
+                    out[o.request_id] = o.outputs[0].token_ids
+        got.append(out)
+    assert got[0] == got[1] and len(got[0]) == 3
+    assert ops.read_status() == 0

@@ -876,6 +876,7 @@ class ModelRunner(E.ModelRunnerBase):
             host.copy_(ids[:n], non_blocking=True)
             status.copy_(self._status_dev, non_blocking=True)
             ev.record(self.copy_stream)
+        ids.record_stream(self.copy_stream)        # its memory is not handed out again before the copy has run
         self.d2h_bytes += n * 8 + 4
 
         def get():
