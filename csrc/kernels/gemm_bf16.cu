@@ -1,14 +1,21 @@
 // bf16 GEMM  C[M,N] = A[M,K] * W[N,K]^T  (+bias[N]) (+residual[M,N]) on tcgen05 / TMEM.
 //
-// Two kernels:
+// Three kernels:
+//   gemm_bf16_pair_kernel a CTA pair on one 256 x 256 tile, persistent, stream-K. For M > 256 (gated: M > 128), and for
+//                         129-256 rows on N >= 16384.
 //   gemm_bf16_tn_kernel   persistent, 128 x BN output tiles (BN = 128 | 256), TMA-fed
 //                         smem ring, accumulators double-buffered in TMEM so the epilogue
-//                         of tile i overlaps the main loop of tile i+1. For M > 256.
-//   gemm_bf16_swap_kernel small-M form of the tensor-parallel and the allocation-free entries:
-//                         the weight tile is the 128-row MMA operand and the activations are the
+//                         of tile i overlaps the main loop of tile i+1. For 33-128 rows on N >= 16384
+//                         (BN = 256; from 17 where gemm_bf16_impl says so), 129-256 rows below, and larger
+//                         batches that 256-row tiles would pad by 8 % more than 128-row ones.
+//   gemm_bf16_swap_kernel the weight tile is the 128-row MMA operand and the activations are the
 //                         N operand (UMMA N = M padded to 16), so the weight stream is read exactly
 //                         once; split-K over blockIdx.y with fp32 partials reduced in fixed order.
-//                         Plain products of up to 128 rows run in gemm_cluster.cu instead.
+//                         For up to 256 rows in the tensor-parallel and the allocation-free entries,
+//                         batched products that the cluster kernel does not take (129-256 rows, N not a
+//                         multiple of 128, results off 16 bytes), and products whose bias or residual
+//                         lies off 16 bytes (above 128 rows or on wide matrices) or off 8 (any).
+// The other products of up to 128 rows run in gemm_cluster.cu, most of one and some of two rows in gemv.cu (gemv_takes).
 //
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
 // warps 2..5 = epilogue (each owns the TMEM lane quarter warp_id % 4).
@@ -549,14 +556,6 @@ __device__ __forceinline__ void epilogue_store_chunk(const GemmParams& p, float 
   }
 }
 
-__device__ __forceinline__ float gated_act(float g, int kind) {
-  if (kind == 0) return g / (1.f + __expf(-g));
-  if (kind == 1) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    return 0.5f * g * (1.f + tanhf(k0 * (g + k1 * g * g * g)));
-  }
-  return 0.5f * g * (1.f + erff(g * 0.7071067811865476f));
-}
 // act(gate) * up on 32 columns; both inputs are rounded to bf16 first so that the result equals
 // a bf16 GEMM followed by the separate activation kernel bit for bit.
 __device__ __forceinline__ void epilogue_store_gated(const GemmParams& p, const float (&g)[32],
@@ -572,7 +571,7 @@ __device__ __forceinline__ void epilogue_store_gated(const GemmParams& p, const 
       for (int j = 0; j < 8; ++j) {
         const float gg = __bfloat162float(__float2bfloat16(g[i + j]));
         const float uu = __bfloat162float(__float2bfloat16(u[i + j]));
-        r[j] = gated_act(gg, kind) * uu;
+        r[j] = act_of(gg, kind) * uu;
       }
       uint4 w;
       w.x = pack_bf16x2(r[0], r[1]);

@@ -71,17 +71,12 @@ struct alignas(8) ClusterBars {
   uint32_t tmem_base;
 };
 
-__device__ __forceinline__ float gate_of(float g, int kind) {
-  if (kind == 0) return g / (1.f + __expf(-g));
-  if (kind == 1) return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
-  return 0.5f * g * (1.f + erff(g * 0.7071067811865476f));
-}
 __device__ __forceinline__ float rounded(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
 // act(gate) * up; both are rounded first, as where the product and the activation are two kernels
 __device__ __forceinline__ float4 gated4(const float4& g, const float4& u, int kind) {
-  return make_float4(gate_of(rounded(g.x), kind) * rounded(u.x), gate_of(rounded(g.y), kind) * rounded(u.y),
-                     gate_of(rounded(g.z), kind) * rounded(u.z), gate_of(rounded(g.w), kind) * rounded(u.w));
+  return make_float4(act_of(rounded(g.x), kind) * rounded(u.x), act_of(rounded(g.y), kind) * rounded(u.y),
+                     act_of(rounded(g.z), kind) * rounded(u.z), act_of(rounded(g.w), kind) * rounded(u.w));
 }
 // col: first of the lane's four columns of the output, m: row of the output
 __device__ __forceinline__ void finish_row(const ClusterParams& p, float4 a, int m, int col) {

@@ -56,11 +56,6 @@ __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
     f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
 }
-__device__ __forceinline__ float gemv_gate(float g, int kind) {
-  if (kind == 0) return g / (1.f + __expf(-g));
-  if (kind == 1) return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
-  return 0.5f * g * (1.f + erff(g * 0.7071067811865476f));
-}
 
 template <int M>
 __global__ void __launch_bounds__(kVThreads, 3) gemv_kernel(GemvParams p) {
@@ -230,7 +225,7 @@ __global__ void __launch_bounds__(kVThreads, 3) gemv_kernel(GemvParams p) {
       if (p.gated) {
         if (i < p.N / 2) {
           const float gg = __bfloat162float(__float2bfloat16(v0)), uu = __bfloat162float(__float2bfloat16(v1));
-          reinterpret_cast<__nv_bfloat16*>(p.out)[lane * p.ldo + i] = __float2bfloat16(gemv_gate(gg, p.gated - 1) * uu);
+          reinterpret_cast<__nv_bfloat16*>(p.out)[lane * p.ldo + i] = __float2bfloat16(act_of(gg, p.gated - 1) * uu);
         }
       } else if (2 * i < p.N) {                           // N is even
         const long long at = lane * p.ldo + 2 * i;

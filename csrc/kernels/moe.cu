@@ -485,11 +485,7 @@ __global__ void __launch_bounds__(192, 2)
             if (m < rows) {
               const float gg = __bfloat162float(__float2bfloat16(__uint_as_float(g[i])));
               const float uu = __bfloat162float(__float2bfloat16(__uint_as_float(u[i])));
-              float a;
-              if (kind == 0) a = gg / (1.f + __expf(-gg));
-              else if (kind == 1) a = 0.5f * gg * (1.f + tanhf(0.7978845608028654f * (gg + 0.044715f * gg * gg * gg)));
-              else a = 0.5f * gg * (1.f + erff(gg * 0.7071067811865476f));
-              p.out[(size_t)(row0 + m) * half_n + n] = __float2bfloat16(a * uu);
+              p.out[(size_t)(row0 + m) * half_n + n] = __float2bfloat16(act_of(gg, kind) * uu);
             }
           }
         }

@@ -104,17 +104,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-enum ActKind : int { kSilu = 0, kGeluTanh = 1, kGeluErf = 2 };
-
-__device__ __forceinline__ float act_fn(float g, int kind) {
-  if (kind == kSilu) return g / (1.f + __expf(-g));
-  if (kind == kGeluTanh) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    return 0.5f * g * (1.f + tanhf(k0 * (g + k1 * g * g * g)));
-  }
-  return 0.5f * g * (1.f + erff(g * 0.7071067811865476f));
-}
-
 // x: [T, 2*I] = [gate | up] (or, with kind | 0x100, blocks of [128 gate | 128 up]);
 // out: [T, I] = act(gate) * up.
 __global__ void __launch_bounds__(256)
@@ -136,10 +125,10 @@ __global__ void __launch_bounds__(256)
     const uint4 u = *reinterpret_cast<const uint4*>(x + (size_t)t * ldx + uoff);
     uint4 o;
     float2 a, b;
-    a = unpack_bf16x2(g.x); b = unpack_bf16x2(u.x); o.x = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
-    a = unpack_bf16x2(g.y); b = unpack_bf16x2(u.y); o.y = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
-    a = unpack_bf16x2(g.z); b = unpack_bf16x2(u.z); o.z = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
-    a = unpack_bf16x2(g.w); b = unpack_bf16x2(u.w); o.w = pack_bf16x2(act_fn(a.x, kind) * b.x, act_fn(a.y, kind) * b.y);
+    a = unpack_bf16x2(g.x); b = unpack_bf16x2(u.x); o.x = pack_bf16x2(act_of(a.x, kind) * b.x, act_of(a.y, kind) * b.y);
+    a = unpack_bf16x2(g.y); b = unpack_bf16x2(u.y); o.y = pack_bf16x2(act_of(a.x, kind) * b.x, act_of(a.y, kind) * b.y);
+    a = unpack_bf16x2(g.z); b = unpack_bf16x2(u.z); o.z = pack_bf16x2(act_of(a.x, kind) * b.x, act_of(a.y, kind) * b.y);
+    a = unpack_bf16x2(g.w); b = unpack_bf16x2(u.w); o.w = pack_bf16x2(act_of(a.x, kind) * b.x, act_of(a.y, kind) * b.y);
     *reinterpret_cast<uint4*>(out + (size_t)t * I + i * 8) = o;
   }
 }
@@ -219,10 +208,10 @@ __global__ void __launch_bounds__(MODE == 1 ? 256 : 1024)
       const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + t * ldx + uoff));
       uint4 o;
       float2 a, b;
-      a = unpack_bf16x2(gt.x); b = unpack_bf16x2(u.x); o.x = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
-      a = unpack_bf16x2(gt.y); b = unpack_bf16x2(u.y); o.y = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
-      a = unpack_bf16x2(gt.z); b = unpack_bf16x2(u.z); o.z = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
-      a = unpack_bf16x2(gt.w); b = unpack_bf16x2(u.w); o.w = pack_bf16x2(act_fn(a.x, KIND) * b.x, act_fn(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.x); b = unpack_bf16x2(u.x); o.x = pack_bf16x2(act_of(a.x, KIND) * b.x, act_of(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.y); b = unpack_bf16x2(u.y); o.y = pack_bf16x2(act_of(a.x, KIND) * b.x, act_of(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.z); b = unpack_bf16x2(u.z); o.z = pack_bf16x2(act_of(a.x, KIND) * b.x, act_of(a.y, KIND) * b.y);
+      a = unpack_bf16x2(gt.w); b = unpack_bf16x2(u.w); o.w = pack_bf16x2(act_of(a.x, KIND) * b.x, act_of(a.y, KIND) * b.y);
       row_cache[i] = o;
       vec_amax(o);
     }
@@ -396,7 +385,7 @@ int b200_quant_fp8_rowwise(const void* x, long ldx, void* residual, const void* 
   const int kind = kind_flags & 0xff;
   auto kernel = mode == 0 ? rowquant_fp8_kernel<0, 0> : mode == 1 ? rowquant_fp8_kernel<1, 0>
               : kind == kSilu ? rowquant_fp8_kernel<2, kSilu> : kind == kGeluTanh ? rowquant_fp8_kernel<2, kGeluTanh>
-                                                                                  : rowquant_fp8_kernel<2, kGeluTanh + 1>;
+                                                                                  : rowquant_fp8_kernel<2, kGeluErf>;
   static PerDeviceOnce attr_once[5];
   if (attr_once[mode < 2 ? mode : kind == kSilu ? 2 : kind == kGeluTanh ? 3 : 4].first())
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 2);

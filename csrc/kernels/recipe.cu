@@ -42,15 +42,6 @@ __device__ __forceinline__ float chain_warp_sum(float v) {
   return v;
 }
 
-__device__ __forceinline__ float chain_act(float g, int kind) {
-  if (kind == 0) return g / (1.f + __expf(-g));
-  if (kind == 1) {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    return 0.5f * g * (1.f + tanhf(k0 * (g + k1 * g * g * g)));
-  }
-  return 0.5f * g * (1.f + erff(g * 0.7071067811865476f));
-}
-
 // Sum of squares of a shared-memory row in the order rmsnorm_kernel uses when it is launched for
 // this width: nt = min(256, H/8 rounded up to a warp) threads, 16-byte vectors strided by nt.
 __device__ float chain_sumsq_block(const bf16* row, int H, float* red) {
@@ -138,7 +129,7 @@ __global__ void __launch_bounds__(256) fused_chain_kernel(const __grid_constant_
           if (st.op == kChAdd) {
             o.x = x.x + y.x; o.y = x.y + y.y;
           } else if (st.op == kChActMul) {
-            o.x = chain_act(x.x, st.flag) * y.x; o.y = chain_act(x.y, st.flag) * y.y;
+            o.x = act_of(x.x, st.flag) * y.x; o.y = act_of(x.y, st.flag) * y.y;
           } else {
             o.x = x.x / (1.f + __expf(-y.x)); o.y = x.y / (1.f + __expf(-y.y));
           }

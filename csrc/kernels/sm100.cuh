@@ -468,6 +468,15 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {
   return __bfloat1622float2(b);
 }
 
+// Activation of a gated block, act(gate) * up. One formula for every kernel that applies it, in an epilogue or on its own: their
+// results are the same bits.
+enum ActKind : int { kSilu = 0, kGeluTanh = 1, kGeluErf = 2 };
+__device__ __forceinline__ float act_of(float g, int kind) {
+  if (kind == kSilu) return g / (1.f + __expf(-g));
+  if (kind == kGeluTanh) return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
+  return 0.5f * g * (1.f + erff(g * 0.7071067811865476f));
+}
+
 }  // namespace b200
 
 // ------------------------------------------------------------------------------------
