@@ -370,9 +370,9 @@ struct alignas(8) GroupedBars {
 
 // grid: (column tiles x parts of a chunk, max_chunks). A CTA whose chunk index is past the device-side count exits. Two CTAs
 // share an SM (96 KB of stages and 256 TMEM columns each), so that one stores its outputs while the other multiplies; a CTA
-// alone, with twice the stages and both halves of the gated accumulators for 256 rows, leaves the tensor pipe idle during
+// alone, with twice the stages and, gated, the accumulators of 256 rows, leaves the tensor pipe idle during
 // its epilogue (us at 8192 tokens, gated / down: 128 experts of 768, top 8, 608 / 525 -> 492 / 349; 64 of 1408, top 6,
-// 799 / 511 -> 637 / 349). The gated product keeps that form where there are too few CTAs to pair up (moe_grouped_gemm_impl).
+// 799 / 511 -> 637 / 349). Where there are too few CTAs to pair up that form stays (moe_grouped_gemm_impl).
 __global__ void __launch_bounds__(192, 2)
     moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW,
                             const __grid_constant__ CUtensorMap tmX, GroupedParams p) {
@@ -737,7 +737,12 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
   p.chunk_expert = (const int32_t*)chunk_expert; p.chunk_row0 = (const int32_t*)chunk_row0;
   p.chunk_n = (const int32_t*)chunk_n; p.meta = (const int32_t*)meta; p.E = E;
   const int stage = kGBM * kGBK * 2 * (act_fuse ? 2 : 1) + sub_rows * kGBK * 2;
-  int stages = (act_fuse && !pairs ? 200 : 96) * 1024 / stage;
+  // Plain product: two stages and a neighbour on the SM, or, where the grid leaves no SM two CTAs, four stages (an expert's last 256
+  // rows are half full on average): 8 experts of 14336, width 1024, us, four / two stages: 66 rows each 123 / 158 (64 CTAs), 400 rows
+  // 130 / 181 (132), 700 rows 256 / 192 (207); 16 of 4096, width 512, 256 rows 47 / 62, 700 rows 89 / 68.
+  const long long most = max_rows / 256 + E / 2, ctas = (long long)tiles * (most > E ? most : E);
+  const bool alone = act_fuse ? !pairs : ctas <= sms;
+  int stages = (alone ? 200 : 96) * 1024 / stage;
   if (stages > kGMaxStages) stages = kGMaxStages;
   const int nkb = (K + kGBK - 1) / kGBK;
   if (stages > nkb) stages = nkb < 2 ? 2 : nkb;

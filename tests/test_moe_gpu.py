@@ -191,3 +191,26 @@ def test_grouped_gemm_gated_of_128_and_256_rows(T, E, k, H, I):
         e = ids[:, j].long()
         got = want[ws.pair_pos.view(T, k)[:, j].long()].float()
         assert _rel(got, torch.nn.functional.silu(g[e, tok]) * u[e, tok]) < 3 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("T,E,I,N", [(300, 2, 1000, 136), (700, 8, 1000, 1024), (1400, 8, 1000, 2048)])
+def test_grouped_gemm_of_few_and_of_many_ctas(T, E, I, N):
+    """Plain products of more than 64 rows an expert with K longer than the ring: grids of fewer CTAs than SMs (four stages) and of
+    more (two stages, two CTAs an SM). fp32 sums, one rounding to bf16."""
+    torch.manual_seed(T)
+    ws = M.MoeWorkspace(torch.device(DEV), T, 2, E, N, I)
+    ids = torch.stack([torch.randperm(E, device=DEV)[:2] for _ in range(T)]).int()
+    M.moe_sort(ids, 0, E, ws)
+    P = 2 * T
+    x = torch.randn(T, I, device=DEV).to(torch.bfloat16)
+    wd = (torch.randn(E, N, I, device=DEV) * I ** -0.5).to(torch.bfloat16)
+    pos = ws.pair_pos.view(T, 2).long()
+    for j in range(2):
+        ws.act[pos[:, j]] = x
+    M.grouped_gemm(ws.act, wd, ws.y, ws, P)
+    assert ops.read_status() == 0
+    tok = torch.arange(T, device=DEV)
+    y = torch.stack([x.double() @ wd[e].double().t() for e in range(E)])
+    for j in range(2):
+        assert _rel(ws.y[pos[:, j]].float(), y[ids[:, j].long(), tok].float()) < 2.0 ** -8
+    assert bool((ws.y[P:] == 0).all())
