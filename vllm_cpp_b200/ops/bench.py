@@ -45,6 +45,17 @@ def small_case(name: str):
         a = torch.randn(64, 4096, device=dev, dtype=torch.bfloat16)
         w = torch.randn(28672, 4096, device=dev, dtype=torch.bfloat16) * 0.05
         fn = lambda: ops.gemm(a, w)
+    elif name in ("gemv_small", "gemm_cluster_small"):          # one row / 32 rows, weights larger than L2
+        a = torch.randn(1 if name == "gemv_small" else 32, 8192, device=dev, dtype=torch.bfloat16)
+        w = torch.randn(14336, 8192, device=dev, dtype=torch.bfloat16) * 0.05
+        fn = lambda: ops.gemm(a, w)
+    elif name == "sample_small":
+        # 40 rows of a vocabulary of 151936: top-k and top-p
+        logits = torch.randn(40, 151936, device=dev) * 2
+        k = torch.full((40,), 50, dtype=torch.int32, device=dev)
+        p = torch.full((40,), 0.95, device=dev)
+        buf = torch.empty_like(logits)
+        fn = lambda: ops.apply_top_k_top_p(buf.copy_(logits), k, p)
     elif name == "prefill_small":
         B, ql = 4, 1024
         nb = ql // bs
@@ -140,16 +151,16 @@ def small_case(name: str):
             fn = lambda: A.prefill(q, pages, out, q_start=qs, num_reqs=B, tile_req=treq, tile_q0=tq0, **kw_)
         else:
             fn = lambda: A.decode(q, pages, out, splits=2, **kw_)
-    elif name == "moe_small":
+    elif name in ("moe_small", "moe_few_small"):                # 128 rows an expert; 4
         from . import moe as M
-        T, E, k, H, I = 2048, 128, 8, 2048, 768
+        T, E, k, H, I = 2048 if name == "moe_small" else 64, 128, 8, 2048, 768
         x = torch.randn(T, H, device=dev).to(torch.bfloat16)
         wgu = (torch.randn(E, 2 * I, H, device=dev) * 0.05).to(torch.bfloat16)
         ids, w = M.router_topk(torch.randn(T, E, device=dev), k)
         ws = M.MoeWorkspace(dev, T, k, E, H, I)
         M.moe_sort(ids, 0, E, ws)
         M.moe_gather(x, ws, E, T * k)
-        fn = lambda: M.grouped_gemm(ws.xs, wgu, ws.gu, ws, T * k)
+        fn = lambda: M.grouped_gemm_gated(ws.xs, wgu, ws.act, ws, T * k, kind=0)
     elif name == "gemm_streamk_small":
         # Llama-8B down projection at a mixed-step batch: 80 pair tiles on 74 CTA pairs, so the six
         # tiles of the ragged wave run as stream-K
@@ -228,8 +239,9 @@ def main():
     ap.add_argument("--quick", action="store_true")
     ap.add_argument("--case", default=None,
                     help="run one small case only (for profiler captures): "
-                         "gemm_small | gemm_decode_small | prefill_small | decode_small | gdn_scan_small | "
-                         "gdn_decode_small | moe_small | gemm_streamk_small | gemm_gated_small | "
+                         "gemm_small | gemm_decode_small | gemv_small | gemm_cluster_small | sample_small | "
+                         "prefill_small | decode_small | gdn_scan_small | "
+                         "gdn_decode_small | moe_small | moe_few_small | gemm_streamk_small | gemm_gated_small | "
                          "gemm_fp8_small | gemm_w4a16_small | gemm_nvfp4_small | gemm_nvfp4_prefill_small | "
                          "decode_d256_small | mla_decode_small | bias_prefill_small | bias_decode_small | delta_small")
     args = ap.parse_args()
