@@ -320,12 +320,15 @@ __global__ void moe_scatter_kernel(const int32_t* __restrict__ topk_ids, int P, 
     pair_pos[i] = -1;
   }
 }
-// xs[pos, :] = x[sorted_token[pos], :] for pos < total (read from meta), rows of H bf16
+// xs[pos, :] = x[sorted_token[pos], :] for pos < total (read from meta), rows of H bf16. PDL: may start while its predecessor runs.
+template <bool PDL>
 __global__ void __launch_bounds__(128)
     moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* sorted_token,
                       const int32_t* meta, int E, __nv_bfloat16* xs, int H) {
-  pdl_wait();
-  pdl_launch_dependents();
+  if constexpr (PDL) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
   const int pos = blockIdx.x;
   if (pos >= meta[2 * E]) return;
   const uint4* s = reinterpret_cast<const uint4*>(x + (size_t)sorted_token[pos] * ldx);
@@ -685,7 +688,15 @@ int b200_moe_sort(const void* topk_ids, int T, int k, int e0, int e1, void* meta
 int b200_moe_gather(const void* x, int ldx, const void* sorted_token, const void* meta, int E,
                     void* xs, int H, int max_rows, cudaStream_t stream) {
   if (max_rows <= 0) return 0;
-  return launch_pdl(moe_gather_kernel, dim3(max_rows), dim3(128), 0, stream, (const bf16*)x, ldx, (const int32_t*)sorted_token,
+  // A CTA is one row, about a microsecond: over several waves of them the two instructions of an early start cost more than the
+  // start gains, also where the launch is an ordinary one (us without / with them, rows of 2048: 3840 rows 4.9 / 4.8, 6400 6.6 / 7.9,
+  // 16384 14.1 / 18.4; with the sort ahead, rows of 1024: 5600 rows 10.4 / 12.3; rows of 4096: 5600 14.8 / 14.6).
+  if (max_rows >= 4096) {
+    moe_gather_kernel<false><<<max_rows, 128, 0, stream>>>((const bf16*)x, ldx, (const int32_t*)sorted_token, (const int32_t*)meta, E,
+                                                           (bf16*)xs, H);
+    RETL;
+  }
+  return launch_pdl(moe_gather_kernel<true>, dim3(max_rows), dim3(128), 0, stream, (const bf16*)x, ldx, (const int32_t*)sorted_token,
                     (const int32_t*)meta, E, (bf16*)xs, H) == cudaSuccess ? 0 : -2;
 }
 

@@ -214,3 +214,16 @@ def test_grouped_gemm_of_few_and_of_many_ctas(T, E, I, N):
     for j in range(2):
         assert _rel(ws.y[pos[:, j]].float(), y[ids[:, j].long(), tok].float()) < 2.0 ** -8
     assert bool((ws.y[P:] == 0).all())
+
+
+@pytest.mark.parametrize("T", [2047, 2048, 3000])
+def test_gather_of_few_and_of_many_rows(T):
+    """With and without an early start (4096 rows): every sorted row is its token's, rows beyond the sorted ones are untouched."""
+    torch.manual_seed(T)
+    ws = M.MoeWorkspace(torch.device(DEV), T, 2, 8, 72, 8)
+    ids = torch.stack([torch.randperm(8, device=DEV)[:2] for _ in range(T)]).int()
+    x = torch.randn(T, 72, device=DEV).to(torch.bfloat16)
+    M.moe_sort(ids, 0, 8, ws)
+    M.moe_gather(x, ws, 8, 2 * T)
+    pos = ws.pair_pos.view(T, 2).long()
+    assert torch.equal(ws.xs[pos[:, 0]], x) and torch.equal(ws.xs[pos[:, 1]], x) and bool((ws.xs[2 * T:] == 0).all())
