@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
   uint8_t* sP = sQ + kQBytes;                        // 2 buffers * (2 halves * 2 KB)
   DecodeTcBars* bars = reinterpret_cast<DecodeTcBars*>(sP + 8192);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int b = blockIdx.x, hkv = blockIdx.y, split = blockIdx.z;
   const int G = p.Hq / p.Hkv;
 
@@ -155,87 +155,92 @@ __global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
   if (ntiles > 0) {
     if (warp == 0) {
       // ------------------------------ TMA producer ------------------------------
-      if (lane == 0) {
+      if (elect_one()) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmKV);
         mbar_expect_tx(&bars->q_full, kQBytes);
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) tma_load_3d(sQ + c * 2048, &tmQ, &bars->q_full, c * 64, hkv * G, b);
-        const int32_t* bt = p.block_table + (size_t)b * p.max_blocks;
-        const int nblk_valid = (seq_len + p.block_size - 1) / p.block_size;
-        const int rows_per_load = min(p.block_size, kTok);
-        const int loads = kTok / rows_per_load;
-        bool ok = true;
-        // Load order K0 K1 V0 K2 V1 K3 ... V(n-1): exactly the order in which the MMA warp
-        // consumes the tiles, with K running one tile further ahead than V (a V slot is held
-        // until the softmax of its tile is done; K slots turn over as soon as QK has run).
-        const int nseq = 2 * ntiles;
-        for (int sq = 0; sq < nseq && ok; ++sq) {
-          int kv, j;
-          if (sq == 0) { kv = 0; j = 0; }
-          else if (sq == nseq - 1) { kv = 1; j = ntiles - 1; }
-          else if (sq & 1) { kv = 0; j = (sq + 1) >> 1; }
-          else { kv = 1; j = (sq - 2) >> 1; }
-          const int tok0 = tok_base + j * kTok;
-          const int sl = sq % kSlots;
-          const uint32_t ph = (sq / kSlots) & 1;
-          if (!mbar_wait(&bars->kv_empty[sl], ph ^ 1, p.status)) { ok = false; break; }
-          uint8_t* dst = sKV + sl * kSlotBytes;
-          mbar_expect_tx(&bars->kv_full[sl], kSlotBytes);
-          for (int l = 0; l < loads; ++l) {
-            const int tk = tok0 + l * rows_per_load;
-            const int bi = tk / p.block_size;
-            const int blk = (bi < nblk_valid) ? bt[bi] : bt[0];
-            const int row = (blk * 2 + kv) * p.block_size + tk % p.block_size;
-#pragma unroll
-            for (int c = 0; c < kChunks; ++c)
-              tma_load_3d(dst + c * kChunkBytes + l * rows_per_load * 128, &tmKV, &bars->kv_full[sl], c * 64, hkv,
-                          row);
-          }
+      }
+      __syncwarp();
+      const int32_t* bt = p.block_table + (size_t)b * p.max_blocks;
+      const int nblk_valid = (seq_len + p.block_size - 1) / p.block_size;
+      const int rows_per_load = min(p.block_size, kTok);
+      const int loads = kTok / rows_per_load;              // pages of a tile (at most 16): a lane each
+      // Load order K0 K1 V0 K2 V1 K3 ... V(n-1): exactly the order in which the MMA warp
+      // consumes the tiles, with K running one tile further ahead than V (a V slot is held
+      // until the softmax of its tile is done; K slots turn over as soon as QK has run).
+      const int nseq = 2 * ntiles;
+      int sl = 0;
+      uint32_t ph = 1;
+      for (int sq = 0; sq < nseq; ++sq) {
+        int kv, j;
+        if (sq == 0) { kv = 0; j = 0; }
+        else if (sq == nseq - 1) { kv = 1; j = ntiles - 1; }
+        else if (sq & 1) { kv = 0; j = (sq + 1) >> 1; }
+        else { kv = 1; j = (sq - 2) >> 1; }
+        int row = 0;
+        if (lane < loads) {
+          const int tk = tok_base + j * kTok + lane * rows_per_load, bi = tk / p.block_size;
+          row = (bt[bi < nblk_valid ? bi : 0] * 2 + kv) * p.block_size + tk % p.block_size;
         }
+        if (!mbar_wait_warp(&bars->kv_empty[sl], ph, p.status)) break;
+        if (lane == 0) mbar_expect_tx(&bars->kv_full[sl], kSlotBytes);
+        __syncwarp();
+        if (lane < loads) {
+          uint8_t* dst = sKV + sl * kSlotBytes + lane * rows_per_load * 128;
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c) tma_load_3d(dst + c * kChunkBytes, &tmKV, &bars->kv_full[sl], c * 64, hkv, row);
+        }
+        __syncwarp();
+        if (++sl == kSlots) { sl = 0; ph ^= 1; }
       }
     } else if (warp == 1) {
-      // ------------------------------ MMA issuer ------------------------------
-      if (lane == 0) {
-        constexpr uint32_t idesc_qk = umma_idesc_bf16(kTok, kNQ, 0, 0);
-        constexpr uint32_t idesc_pv = umma_idesc_bf16(128, kNQ, 1, 0);  // A (V^T) is MN-major
-        bool ok = mbar_wait(&bars->q_full, 0, p.status);
-        const uint32_t q_addr = smem_u32(sQ);
-        for (int j = 0; j <= ntiles && ok; ++j) {
-          if (j < ntiles) {
-            const int it = j == 0 ? 0 : 2 * j - 1, sl = it % kSlots;     // K(j) in load order
-            const uint32_t ph = (it / kSlots) & 1;
-            const int sb = j & 1;
-            if (!mbar_wait(&bars->kv_full[sl], ph, p.status)) { ok = false; break; }
-            if (!mbar_wait(&bars->s_empty[sb], ((j >> 1) & 1) ^ 1, p.status)) { ok = false; break; }
-            tc_fence_after_sync();
-            const uint32_t k_addr = smem_u32(sKV + sl * kSlotBytes);
+      // ------------------------------ MMA issuer (the warp walks the loop, an elected lane issues) ------------------------------
+      constexpr uint32_t idesc_qk = umma_idesc_bf16(kTok, kNQ, 0, 0);
+      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, kNQ, 1, 0);  // A (V^T) is MN-major
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+      bool ok = mbar_wait_warp(&bars->q_full, 0, p.status);
+      const uint32_t q_addr = smem_u32(sQ);
+      for (int j = 0; j <= ntiles && ok; ++j) {
+        if (j < ntiles) {
+          const int it = j == 0 ? 0 : 2 * j - 1, sl = it % kSlots;     // K(j) in load order
+          const uint32_t ph = (it / kSlots) & 1;
+          const int sb = j & 1;
+          if (!(ok = mbar_wait_warp(&bars->kv_full[sl], ph, p.status))) break;
+          if (!(ok = mbar_wait_warp(&bars->s_empty[sb], ((j >> 1) & 1) ^ 1, p.status))) break;
+          tc_fence_after_sync();
+          const uint32_t k_addr = smem_u32(sKV + sl * kSlotBytes);
+          if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t koff = (kk / 4) * kChunkBytes + (kk % 4) * 32;
               const uint32_t qoff = (kk / 4) * 2048 + (kk % 4) * 32;
-              umma_bf16_ss(tmem_s + sb * 16, umma_desc_k_sw128(k_addr + koff, 1024),
+              umma_bf16_ss(tm + sb * 16, umma_desc_k_sw128(k_addr + koff, 1024),
                            umma_desc_k_sw128(q_addr + qoff, 1024), idesc_qk, kk != 0);
             }
             umma_commit(&bars->kv_empty[sl]);
             umma_commit(&bars->s_full[sb]);
           }
-          if (j >= 1) {
-            const int i = j - 1;
-            const int it = i == ntiles - 1 ? 2 * ntiles - 1 : 2 * i + 2, sl = it % kSlots;  // V(i)
-            const uint32_t ph = (it / kSlots) & 1;
-            const int pb = i & 1;
-            if (!mbar_wait(&bars->kv_full[sl], ph, p.status)) { ok = false; break; }
-            if (!mbar_wait(&bars->p_full[pb], (i >> 1) & 1, p.status)) { ok = false; break; }
-            tc_fence_after_sync();
-            const uint32_t v_addr = smem_u32(sKV + sl * kSlotBytes);
-            const uint32_t p_addr = smem_u32(sP + pb * 4096);
+          __syncwarp();
+        }
+        if (j >= 1) {
+          const int i = j - 1;
+          const int it = i == ntiles - 1 ? 2 * ntiles - 1 : 2 * i + 2, sl = it % kSlots;  // V(i)
+          const uint32_t ph = (it / kSlots) & 1;
+          const int pb = i & 1;
+          if (!(ok = mbar_wait_warp(&bars->kv_full[sl], ph, p.status))) break;
+          if (!(ok = mbar_wait_warp(&bars->p_full[pb], (i >> 1) & 1, p.status))) break;
+          tc_fence_after_sync();
+          const uint32_t v_addr = smem_u32(sKV + sl * kSlotBytes);
+          const uint32_t p_addr = smem_u32(sP + pb * 4096);
+          if (elect_one()) {
 #pragma unroll
             for (int dh = 0; dh < D / 128; ++dh) {       // 128 rows of the head dim per instruction
 #pragma unroll
               for (int kk = 0; kk < kTok / 16; ++kk) {
                 const uint32_t poff = (kk / 4) * 2048 + (kk % 4) * 32;
-                umma_bf16_ss(tmem_o + dh * 16,
+                umma_bf16_ss(tm + 32 + dh * 16,
                              umma_desc_mn_sw128(v_addr + dh * 2 * kChunkBytes + kk * 2048, kChunkBytes, 1024),
                              umma_desc_k_sw128(p_addr + poff, 1024), idesc_pv, (i | kk) != 0);
               }
@@ -245,6 +250,7 @@ __global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
             umma_commit(&bars->p_empty[pb]);
             if (i == ntiles - 1) umma_commit(&bars->o_done);
           }
+          __syncwarp();
         }
       }
     } else {

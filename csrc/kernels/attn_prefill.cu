@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
   uint8_t* sP = sKV + kRing * kSlotBytes;
   PrefillBars* bars = reinterpret_cast<PrefillBars*>(sP + kPBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile = blockIdx.x, h = blockIdx.y;
   const int hkv = h / (p.Hq / p.Hkv);
   const int req = p.tile_req[tile];
@@ -135,62 +135,66 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_s0 = tmem_base, tmem_o = tmem_base + 128;
 
+  // The producer and the issuer walk their loops as whole warps and elect the lane that issues (mbar_wait_warp).
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmKV);
       mbar_expect_tx(&bars->q_full, kQBytes);
       for (int dh = 0; dh < kDH; ++dh)
         tma_load_2d(sQ + dh * kQHalf, &tmQ, &bars->q_full, h * D + dh * 64, q_begin + q0);
-      const int32_t* bt = p.block_table + (size_t)req * p.max_blocks;
-      const int nblk_valid = (seq_len + p.block_size - 1) / p.block_size;
-      const int rows_per_load = min(p.block_size, kKT);
-      const int loads = kKT / rows_per_load;
-      bool ok = true;
-      // Load order K0 K1 V0 K2 V1 K3 ... V(n-1): the order in which the MMA warp consumes the
-      // tiles, with K one tile further ahead than V (V slots are held until the softmax of their
-      // tile is done; K slots turn over as soon as QK^T has run).
-      const int nseq = 2 * ntiles;
-      for (int sq = 0; sq < nseq && ok; ++sq) {
-        int kv, j;
-        if (sq == 0) { kv = 0; j = 0; }
-        else if (sq == nseq - 1) { kv = 1; j = ntiles - 1; }
-        else if (sq & 1) { kv = 0; j = (sq + 1) >> 1; }
-        else { kv = 1; j = (sq - 2) >> 1; }
-        const int tok0 = (kt0 + j) * kKT;
-        const int sl = sq % kRing;
-        const uint32_t ph = (sq / kRing) & 1;
-        if (!mbar_wait(&bars->kv_empty[sl], ph ^ 1, p.status)) { ok = false; break; }
-        uint8_t* dst = sKV + sl * kSlotBytes;
-        mbar_expect_tx(&bars->kv_full[sl], kSlotBytes);
-        for (int l = 0; l < loads; ++l) {
-          const int tk = tok0 + l * rows_per_load;
-          const int bi = tk / p.block_size;
-          int blk = (bi < nblk_valid) ? bt[bi] : bt[0];
-          if (blk < 0) blk = 0;
-          const int row = (blk * 2 + kv) * p.block_size + tk % p.block_size;
-          for (int dh = 0; dh < kDH; ++dh)
-            tma_load_3d(dst + dh * kKVHalf + l * rows_per_load * 128, &tmKV, &bars->kv_full[sl],
-                        dh * 64, hkv, row);
-        }
+    }
+    __syncwarp();
+    const int32_t* bt = p.block_table + (size_t)req * p.max_blocks;
+    const int nblk_valid = (seq_len + p.block_size - 1) / p.block_size;
+    const int rows_per_load = min(p.block_size, kKT);
+    const int loads = kKT / rows_per_load;                      // pages of a tile (at most 8): a lane each
+    // Load order K0 K1 V0 K2 V1 K3 ... V(n-1): the order in which the MMA warp consumes the
+    // tiles, with K one tile further ahead than V (V slots are held until the softmax of their
+    // tile is done; K slots turn over as soon as QK^T has run).
+    const int nseq = 2 * ntiles;
+    int sl = 0;
+    uint32_t ph = 1;
+    for (int sq = 0; sq < nseq; ++sq) {
+      int kv, j;
+      if (sq == 0) { kv = 0; j = 0; }
+      else if (sq == nseq - 1) { kv = 1; j = ntiles - 1; }
+      else if (sq & 1) { kv = 0; j = (sq + 1) >> 1; }
+      else { kv = 1; j = (sq - 2) >> 1; }
+      int row = 0;
+      if (lane < loads) {
+        const int tk = (kt0 + j) * kKT + lane * rows_per_load, bi = tk / p.block_size;
+        const int blk = max(0, bt[bi < nblk_valid ? bi : 0]);
+        row = (blk * 2 + kv) * p.block_size + tk % p.block_size;
       }
+      if (!mbar_wait_warp(&bars->kv_empty[sl], ph, p.status)) break;
+      if (lane == 0) mbar_expect_tx(&bars->kv_full[sl], kSlotBytes);
+      __syncwarp();
+      if (lane < loads) {
+        uint8_t* dst = sKV + sl * kSlotBytes + lane * rows_per_load * 128;
+#pragma unroll
+        for (int dh = 0; dh < kDH; ++dh) tma_load_3d(dst + dh * kKVHalf, &tmKV, &bars->kv_full[sl], dh * 64, hkv, row);
+      }
+      __syncwarp();
+      if (++sl == kRing) { sl = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(kQT, kKT, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(kQT, D, 0, 1);  // B (V) is MN-major
-      bool ok = mbar_wait(&bars->q_full, 0, p.status);
-      const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
-      for (int j = 0; j <= ntiles && ok; ++j) {
-        if (j < ntiles) {
-          const int it = j == 0 ? 0 : 2 * j - 1, sl = it % kRing, sb = j & 1;   // K(j) in load order
-          if (!mbar_wait(&bars->kv_full[sl], (it / kRing) & 1, p.status)) { ok = false; break; }
-          if (!mbar_wait(&bars->s_empty[sb], ((j >> 1) & 1) ^ 1, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t k_addr = smem_u32(sKV + sl * kSlotBytes);
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(kQT, kKT, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16(kQT, D, 0, 1);  // B (V) is MN-major
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+    bool ok = mbar_wait_warp(&bars->q_full, 0, p.status);
+    const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
+    for (int j = 0; j <= ntiles && ok; ++j) {
+      if (j < ntiles) {
+        const int it = j == 0 ? 0 : 2 * j - 1, sl = it % kRing, sb = j & 1;   // K(j) in load order
+        if (!(ok = mbar_wait_warp(&bars->kv_full[sl], (it / kRing) & 1, p.status))) break;
+        if (!(ok = mbar_wait_warp(&bars->s_empty[sb], ((j >> 1) & 1) ^ 1, p.status))) break;
+        tc_fence_after_sync();
+        const uint32_t k_addr = smem_u32(sKV + sl * kSlotBytes);
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
-            umma_bf16_ss(tmem_s0 + sb * kKT,
+            umma_bf16_ss(tm + sb * kKT,
                          umma_desc_k_sw128(q_addr + (kk / 4) * kQHalf + (kk % 4) * 32, 1024),
                          umma_desc_k_sw128(k_addr + (kk / 4) * kKVHalf + (kk % 4) * 32, 1024),
                          idesc_qk, kk != 0);
@@ -198,24 +202,28 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
           umma_commit(&bars->kv_empty[sl]);
           umma_commit(&bars->s_full[sb]);
         }
-        if (j >= 1) {
-          const int i = j - 1;
-          const int it = i == ntiles - 1 ? 2 * ntiles - 1 : 2 * i + 2, sl = it % kRing;       // V(i)
-          if (!mbar_wait(&bars->kv_full[sl], (it / kRing) & 1, p.status)) { ok = false; break; }
-          if (!mbar_wait(&bars->p_full, i & 1, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t v_addr = smem_u32(sKV + sl * kSlotBytes);
+        __syncwarp();
+      }
+      if (j >= 1) {
+        const int i = j - 1;
+        const int it = i == ntiles - 1 ? 2 * ntiles - 1 : 2 * i + 2, sl = it % kRing;       // V(i)
+        if (!(ok = mbar_wait_warp(&bars->kv_full[sl], (it / kRing) & 1, p.status))) break;
+        if (!(ok = mbar_wait_warp(&bars->p_full, i & 1, p.status))) break;
+        tc_fence_after_sync();
+        const uint32_t v_addr = smem_u32(sKV + sl * kSlotBytes);
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < kKT / 16; ++kk) {
             // V: MN-major; 64-dim blocks are kKVHalf apart, 8-token groups 1024 B apart,
             // 16 tokens per instruction = 2048 B.
-            umma_bf16_ss(tmem_o, umma_desc_k_sw128(p_addr + kk * 32, 1024),
+            umma_bf16_ss(tm + 128, umma_desc_k_sw128(p_addr + kk * 32, 1024),
                          umma_desc_mn_sw128(v_addr + kk * 2048, kKVHalf, 1024), idesc_pv, (i | kk) != 0);
           }
           umma_commit(&bars->kv_empty[sl]);
           umma_commit(&bars->o_full);     // before p_empty: whoever sees p_empty has this arrival too
           umma_commit(&bars->p_empty);
         }
+        __syncwarp();
       }
     }
   } else {
@@ -411,7 +419,7 @@ __global__ void __launch_bounds__(320, 1)
   __shared__ PairBars bars;
   uint8_t* sQ = smem;
   uint8_t* sKV = sQ + 2 * kPQBytes;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(&bars.q_full, 1);
     for (int i = 0; i < kPRing; ++i) {
@@ -477,55 +485,61 @@ __global__ void __launch_bounds__(320, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(kQT, kPT, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(kQT, 128, 0, 1);      // B (V) is MN-major
-      bool ok = mbar_wait(&bars.q_full, 0, p.status);
-      int j[2] = {-1, -1};          // last product Q K issued
-      bool pv[2] = {false, false};  // P V of that tile issued
-      int left = ok ? 2 : 0;
-      long long t0 = clock64();
-      uint32_t spins = 0;
-      while (left > 0) {
-        bool idle = true;
+    // (the whole warp watches and walks; one elected lane issues)
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(kQT, kPT, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16(kQT, 128, 0, 1);      // B (V) is MN-major
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const auto ready = [](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; };
+    int j[2] = {-1, -1};          // last product Q K issued
+    bool pv[2] = {false, false};  // P V of that tile issued
+    int left = mbar_wait_warp(&bars.q_full, 0, p.status) ? 2 : 0;
+    long long t0 = clock64();
+    uint32_t spins = 0;
+    while (left > 0) {
+      bool idle = true;
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (j[t] >= ntiles) continue;
-          if (j[t] >= 0 && !pv[t]) {
-            const int sq = 2 * j[t] + 1, sl = sq % kPRing;
-            if (!mbar_test_wait(&bars.p_full[t], j[t] & 1) || !mbar_test_wait(&bars.kv_full[sl], (sq / kPRing) & 1)) continue;
-            tc_fence_after_sync();
-            const uint64_t vd = umma_desc_mn_sw128(smem_u32(sKV + sl * kPSlotBytes), 16384, 1024);
+      for (int t = 0; t < 2; ++t) {
+        if (j[t] >= ntiles) continue;
+        if (j[t] >= 0 && !pv[t]) {
+          const int sq = 2 * j[t] + 1, sl = sq % kPRing;
+          if (!ready(&bars.p_full[t], j[t] & 1) || !ready(&bars.kv_full[sl], (sq / kPRing) & 1)) continue;
+          tc_fence_after_sync();
+          const uint64_t vd = umma_desc_mn_sw128(smem_u32(sKV + sl * kPSlotBytes), 16384, 1024);
+          const bool both = j[1 - t] > j[t] || (j[1 - t] == j[t] && pv[1 - t]);                     // the other head had V(j)
+          if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < kPT / 16; ++kk)
-              umma_bf16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (j[t] | kk) != 0);
+              umma_bf16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (j[t] | kk) != 0);
             umma_commit(&bars.pv_done[t]);
-            if (j[1 - t] > j[t] || (j[1 - t] == j[t] && pv[1 - t])) umma_commit(&bars.kv_empty[sl]);   // the other head had V(j)
-            pv[t] = true;
-            if (j[t] == ntiles - 1) { j[t] = ntiles; --left; }
-            idle = false;
-          } else {
-            const int n = j[t] + 1, sq = 2 * n, sl = sq % kPRing;
-            if ((j[t] >= 0 && !mbar_test_wait(&bars.pv_done[t], j[t] & 1)) || !mbar_test_wait(&bars.kv_full[sl], (sq / kPRing) & 1))
-              continue;
-            tc_fence_after_sync();
-            const uint32_t q_addr = smem_u32(sQ + t * kPQBytes), k_addr = smem_u32(sKV + sl * kPSlotBytes);
+            if (both) umma_commit(&bars.kv_empty[sl]);
+          }
+          __syncwarp();
+          pv[t] = true;
+          if (j[t] == ntiles - 1) { j[t] = ntiles; --left; }
+          idle = false;
+        } else {
+          const int n = j[t] + 1, sq = 2 * n, sl = sq % kPRing;
+          if ((j[t] >= 0 && !ready(&bars.pv_done[t], j[t] & 1)) || !ready(&bars.kv_full[sl], (sq / kPRing) & 1)) continue;
+          tc_fence_after_sync();
+          const uint32_t q_addr = smem_u32(sQ + t * kPQBytes), k_addr = smem_u32(sKV + sl * kPSlotBytes);
+          if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-              umma_bf16_ss(tmem + t * 128, umma_desc_k_sw128(q_addr + (kk / 4) * 16384 + (kk % 4) * 32, 1024),
+              umma_bf16_ss(tm + t * 128, umma_desc_k_sw128(q_addr + (kk / 4) * 16384 + (kk % 4) * 32, 1024),
                            umma_desc_k_sw128(k_addr + (kk / 4) * 16384 + (kk % 4) * 32, 1024), idesc_qk, kk != 0);
             umma_commit(&bars.s_full[t]);
-            if (j[1 - t] >= n) umma_commit(&bars.kv_empty[sl]);                                       // the other head had K(n)
-            j[t] = n;
-            pv[t] = false;
-            idle = false;
+            if (j[1 - t] >= n) umma_commit(&bars.kv_empty[sl]);                                     // the other head had K(n)
           }
+          __syncwarp();
+          j[t] = n;
+          pv[t] = false;
+          idle = false;
         }
-        if (!idle) { t0 = clock64(); spins = 0; }
-        else if (((++spins) & 0x3ff) == 0 && clock64() - t0 > kSpinLimitCycles) {
-          if (p.status) atomicExch(p.status, (int)kErrMbarTimeout);
-          break;
-        }
+      }
+      if (!idle) { t0 = clock64(); spins = 0; }
+      else if (((++spins) & 0x3ff) == 0 && __any_sync(0xffffffffu, clock64() - t0 > kSpinLimitCycles)) {
+        if (p.status && lane == 0) atomicExch(p.status, (int)kErrMbarTimeout);
+        break;
       }
     }
   } else {

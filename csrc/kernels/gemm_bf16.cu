@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int stages = p.stages;
   GemmBarriers* bars = reinterpret_cast<GemmBarriers*>(smem + (size_t)stages * kStageBytes);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int kblocks = (p.K + kBK - 1) / kBK;
@@ -233,85 +233,91 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // Weights that nothing in the stream writes: fetch the weight halves of the first ring stages of
   // this CTA's first segment before waiting on the predecessor kernel.
   int npre = 0;
-  if (warp == 0 && lane == 0 && p.w_early && !p.ag_flags) {
+  if (warp == 0 && p.w_early && !p.ag_flags) {
     SegState seg0 = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
     int t0, ka, kz;
     if (seg_next(seg0, num_tiles, kblocks, t0, ka, kz)) {
       int tm0, tn0;
       tile_coords(t0, p.tiles_m, p.tiles_n, tm0, tn0);
-      tma_prefetch_desc(&tmB);
       npre = min(kz - ka, stages);
-      for (int i = 0; i < npre; ++i) {
-        mbar_expect_tx(&bars->full[i], kStageBytes);
-        tma_load_2d(smem + (size_t)i * kStageBytes + kABytes, &tmB, &bars->full[i], (ka + i) * kBK, tn0 * BN);
+      if (elect_one()) {
+        tma_prefetch_desc(&tmB);
+        for (int i = 0; i < npre; ++i) {
+          mbar_expect_tx(&bars->full[i], kStageBytes);
+          tma_load_2d(smem + (size_t)i * kStageBytes + kABytes, &tmB, &bars->full[i], (ka + i) * kBK, tn0 * BN);
+        }
       }
+      __syncwarp();
     }
   }
   pdl_wait();                 // predecessor grid complete, its writes visible
   pdl_launch_dependents();    // the successor may become resident (it waits the same way)
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
+    // ---------------- TMA producer (the warp walks the loop whole, one elected lane issues) ----------------
+    // gather mode: A has one copy per parity of the op counter, pick the one just written
+    const CUtensorMap* ta = (p.ag_flags && ((*p.op_counter - 1) & 1)) ? &tmA_alt : &tmA;
     if (lane == 0) {
-      // gather mode: A has one copy per parity of the op counter, pick the one just written
-      const CUtensorMap* ta = (p.ag_flags && ((*p.op_counter - 1) & 1)) ? &tmA_alt : &tmA;
       tma_prefetch_desc(ta);
       tma_prefetch_desc(&tmB);
-      uint32_t it = 0;
-      bool ok = true;
-      SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
-      int t, kb0, kb1;
-      while (ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1)) {
-        int tm, tn;
-        tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-        if (p.ag_flags) {
+    }
+    uint32_t ph = 1;
+    int s = 0, early = npre;
+    bool ok = true;
+    SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
+    int t, kb0, kb1;
+    while (ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1)) {
+      int tm, tn;
+      tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+      if (p.ag_flags) {
+        if (lane == 0) {
           const uint32_t par = (*p.op_counter - 1) & 1;
           for (int g = tm * 4; g < tm * 4 + 4 && ok; ++g) {
             const int need = min(32, p.M - g * 32);
             if (need > 0)
               ok = wait_counter_ge(p.ag_flags + par * p.ag_flag_parity_stride + g, need, p.status, p.peer_wait);
           }
-          if (!ok) break;
-          fence_proxy_async_global();
         }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          int s = it % stages;
-          uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait(&bars->empty[s], ph ^ 1, p.status)) { ok = false; break; }
-          uint8_t* a_dst = smem + (size_t)s * kStageBytes;
-          uint8_t* b_dst = a_dst + kABytes;
-          if ((int)it >= npre) {  // (the first npre stages already expect their bytes and hold B)
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        fence_proxy_async_global();
+      }
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(&bars->empty[s], ph, p.status))) break;
+        uint8_t* a_dst = smem + (size_t)s * kStageBytes;
+        if (elect_one()) {
+          if (early <= 0) {  // (the first npre stages already expect their bytes and hold B)
             mbar_expect_tx(&bars->full[s], kStageBytes);
-            tma_load_2d(b_dst, &tmB, &bars->full[s], kb * kBK, tn * BN);
+            tma_load_2d(a_dst + kABytes, &tmB, &bars->full[s], kb * kBK, tn * BN);
           }
           tma_load_2d(a_dst, ta, &bars->full[s], kb * kBK, tm * kBM);
         }
+        __syncwarp();
+        --early;
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
-      if (!ok) bars->failed = 1;
     }
+    if (!ok && lane == 0) bars->failed = 1;
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(kBM, BN);
-      uint32_t it = 0, tc = 0;
-      bool ok = true;
-      SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
-      int t, kb0, kb1;
-      for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
-        int buf = tc & 1;
-        uint32_t aph = (tc >> 1) & 1;
-        if (!mbar_wait(&bars->acc_empty[buf], aph ^ 1, p.status)) { ok = false; break; }
+    // ---------------- MMA issuer (likewise) ----------------
+    constexpr uint32_t idesc = umma_idesc_bf16(kBM, BN);
+    const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+    uint32_t tc = 0, ph = 0;
+    int s = 0;
+    bool ok = true;
+    SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
+    int t, kb0, kb1;
+    for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
+      const int buf = tc & 1;
+      const uint32_t aph = (tc >> 1) & 1;
+      if (!(ok = mbar_wait_warp(&bars->acc_empty[buf], aph ^ 1, p.status))) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_u + buf * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(&bars->full[s], ph, p.status))) break;
         tc_fence_after_sync();
-        uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          int s = it % stages;
-          uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait(&bars->full[s], ph, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          uint32_t a_addr = smem_u32(smem + (size_t)s * kStageBytes);
-          uint32_t b_addr = a_addr + kABytes;
-          uint64_t adesc = umma_desc_k_sw128(a_addr, 1024);
-          uint64_t bdesc = umma_desc_k_sw128(b_addr, 1024);
+        const uint32_t a_addr = smem_u32(smem + (size_t)s * kStageBytes);
+        const uint64_t adesc = umma_desc_k_sw128(a_addr, 1024), bdesc = umma_desc_k_sw128(a_addr + kABytes, 1024);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k) {
             // +32 bytes per 16-element K step inside the 128-byte swizzle row.
@@ -319,10 +325,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           umma_commit(&bars->empty[s]);
         }
-        if (ok) umma_commit(&bars->acc_full[buf]);
+        __syncwarp();
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
-      if (!ok) bars->failed = 1;
+      if (ok && elect_one()) umma_commit(&bars->acc_full[buf]);
+      __syncwarp();
     }
+    if (!ok && lane == 0) bars->failed = 1;
   } else {
     // ---------------- Epilogue (warps 2..5) ----------------
     const int quarter = warp & 3;
@@ -502,6 +511,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // Barriers: full[s] lives in the leader and counts the bytes of both CTAs' loads; empty[s],
 // acc_full[b] are signalled in both CTAs by the leader's commits; acc_empty[b] lives in the
 // leader and collects the eight epilogue warps of the pair.
+// The issuing warps walk their loops whole and elect the lane that issues (mbar_wait_warp, sm100.cuh). With loops of one lane
+// an instruction of 256 x 256 x 16 took 190 cycles instead of the pipe's 128: 8192 x 28672 x 4096 1389 -> 1236 us (1133 -> 892
+// on zeros, where power does not bound it: 2.16 PFLOP/s), 3072 x 6144 x 4096 116 -> 100 us, 700 x 4096 x 14336 101 -> 83 us.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void epilogue_store_chunk(const GemmParams& p, float (&v)[32], int row,
                                                      int col0) {
@@ -605,7 +617,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // contiguous 128-byte pieces before they cross NVLink
   uint8_t* stage_smem = reinterpret_cast<uint8_t*>(bars) + ((sizeof(GemmBarriers) + 127) & ~size_t(127));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1;
@@ -639,20 +651,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
+    // gather mode: A has one copy per parity of the op counter, pick the one just written
+    const CUtensorMap* ta = (p.ag_flags && ((*p.op_counter - 1) & 1)) ? &tmA_alt : &tmA;
     if (lane == 0) {
-      // gather mode: A has one copy per parity of the op counter, pick the one just written
-      const CUtensorMap* ta = (p.ag_flags && ((*p.op_counter - 1) & 1)) ? &tmA_alt : &tmA;
       tma_prefetch_desc(ta);
       tma_prefetch_desc(&tmB);
-      uint32_t it = 0;
-      bool ok = true;
-      SegState seg = seg_init_w(p, kblocks, pair, npairs);
-      int t, kb0, kb1;
-      while (ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1)) {
-        int tm, tn;
-        tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-        if (p.ag_flags) {
-          // all-gather + GEMM: this CTA's 128 rows of the tile must have landed (four 32-row groups)
+    }
+    uint32_t ph = 1;
+    int s = 0;
+    bool ok = true;
+    SegState seg = seg_init_w(p, kblocks, pair, npairs);
+    int t, kb0, kb1;
+    while (ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1)) {
+      int tm, tn;
+      tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+      if (p.ag_flags) {
+        // all-gather + GEMM: this CTA's 128 rows of the tile must have landed (four 32-row groups)
+        if (lane == 0) {
           const uint32_t par = (*p.op_counter - 1) & 1;
           const int g0 = (tm * 2 + (int)rank) * 4;
           for (int g = g0; g < g0 + 4 && ok; ++g) {
@@ -660,56 +675,60 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             if (need > 0)
               ok = wait_counter_ge(p.ag_flags + par * p.ag_flag_parity_stride + g, need, p.status, p.peer_wait);
           }
-          if (!ok) break;
-          fence_proxy_async_global();
         }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          int s = it % stages;
-          uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait(&bars->empty[s], ph ^ 1, p.status)) { ok = false; break; }
-          uint8_t* a_dst = smem + (size_t)s * kStageBytes;
-          uint8_t* b_dst = a_dst + kABytes;
-          if (rank == 0) mbar_expect_tx(&bars->full[s], 2 * kStageBytes);
-          const uint32_t leader_bar = mapa_u32(smem_u32(&bars->full[s]), 0);
-          tma_load_2d_pair(a_dst, ta, leader_bar, kb * kBK, tm * 2 * kBM + (int)rank * kBM);
-          tma_load_2d_pair(b_dst, &tmB, leader_bar, kb * kBK, tn * BN + (int)rank * (BN / 2));
-        }
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        fence_proxy_async_global();
       }
-      if (!ok) bars->failed = 1;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(&bars->empty[s], ph, p.status))) break;
+        uint8_t* a_dst = smem + (size_t)s * kStageBytes;
+        const uint32_t leader_bar = mapa_u32(smem_u32(&bars->full[s]), 0);
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(&bars->full[s], 2 * kStageBytes);
+          tma_load_2d_pair(a_dst, ta, leader_bar, kb * kBK, tm * 2 * kBM + (int)rank * kBM);
+          tma_load_2d_pair(a_dst + kABytes, &tmB, leader_bar, kb * kBK, tn * BN + (int)rank * (BN / 2));
+        }
+        __syncwarp();
+        if (++s == stages) { s = 0; ph ^= 1; }
+      }
     }
+    if (!ok && lane == 0) bars->failed = 1;
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = FP8 ? umma_idesc_e4m3(2 * kBM, BN) : umma_idesc_bf16(2 * kBM, BN);
-      uint32_t it = 0, tc = 0;
+      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+      uint32_t tc = 0, ph = 0;
+      int s = 0;
       bool ok = true;
       SegState seg = seg_init_w(p, kblocks, pair, npairs);
       int t, kb0, kb1;
       for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
-        int buf = tc & 1;
-        uint32_t aph = (tc >> 1) & 1;
-        if (!mbar_wait(&bars->acc_empty[buf], aph ^ 1, p.status)) { ok = false; break; }
+        const int buf = tc & 1;
+        const uint32_t aph = (tc >> 1) & 1;
+        if (!(ok = mbar_wait_warp(&bars->acc_empty[buf], aph ^ 1, p.status))) break;
         tc_fence_after_sync();
-        uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          int s = it % stages;
-          uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait(&bars->full[s], ph, p.status)) { ok = false; break; }
+        const uint32_t d_tmem = tmem_u + buf * BN;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!(ok = mbar_wait_warp(&bars->full[s], ph, p.status))) break;
           tc_fence_after_sync();
-          uint32_t a_addr = smem_u32(smem + (size_t)s * kStageBytes);
-          uint32_t b_addr = a_addr + kABytes;
-          uint64_t adesc = umma_desc_k_sw128(a_addr, 1024);
-          uint64_t bdesc = umma_desc_k_sw128(b_addr, 1024);
+          const uint32_t a_addr = smem_u32(smem + (size_t)s * kStageBytes);
+          const uint64_t adesc = umma_desc_k_sw128(a_addr, 1024), bdesc = umma_desc_k_sw128(a_addr + kABytes, 1024);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {     // four 32-byte K steps per 128-byte row
-            if (FP8) umma_f8f6f4_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
-            else umma_bf16_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
+            for (int k = 0; k < 4; ++k) {     // four 32-byte K steps per 128-byte row
+              if (FP8) umma_f8f6f4_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
+              else umma_bf16_ss_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
+            }
+            umma_commit_pair(&bars->empty[s], 3);
           }
-          umma_commit_pair(&bars->empty[s], 3);
+          __syncwarp();
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit_pair(&bars->acc_full[buf], 3);
+        if (ok && elect_one()) umma_commit_pair(&bars->acc_full[buf], 3);
+        __syncwarp();
       }
-      if (!ok) bars->failed = 1;
+      if (!ok && lane == 0) bars->failed = 1;
     }
   } else {
     // ---------------- Epilogue (warps 2..5 of both CTAs) ----------------
@@ -910,7 +929,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int stages = p.stages;
   GemmBarriers* bars = reinterpret_cast<GemmBarriers*>(smem + (size_t)stages * stage_bytes);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int tn = blockIdx.x;
   const int split = blockIdx.y;
@@ -940,64 +959,75 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // Weights that nothing in the stream writes: fill the first ring stages' weight halves while
   // the predecessor kernel is still running; the activation halves follow after the wait.
   int npre = 0;
-  if (warp == 0 && lane == 0 && p.w_early && !p.ag_flags) {
-    tma_prefetch_desc(&tmW);
+  if (warp == 0 && p.w_early && !p.ag_flags) {
     npre = min(nkb, stages);
-    for (int i = 0; i < npre; ++i) {
-      mbar_expect_tx(&bars->full[i], stage_bytes);
-      tma_load_2d(smem + (size_t)i * stage_bytes, &tmW, &bars->full[i], (kb0 + i) * kBK, bz * p.N + tn * kBM);
+    if (elect_one()) {
+      tma_prefetch_desc(&tmW);
+      for (int i = 0; i < npre; ++i) {
+        mbar_expect_tx(&bars->full[i], stage_bytes);
+        tma_load_2d(smem + (size_t)i * stage_bytes, &tmW, &bars->full[i], (kb0 + i) * kBK, bz * p.N + tn * kBM);
+      }
     }
+    __syncwarp();
   }
   pdl_wait();                 // predecessor grid complete, its writes visible
   pdl_launch_dependents();    // the successor may become resident (it waits the same way)
 
   if (warp == 0) {
+    const CUtensorMap* ta = (p.ag_flags && ((*p.op_counter - 1) & 1)) ? &tmA_alt : &tmA;
+    bool ok = true;
     if (lane == 0) {
-      const CUtensorMap* ta = (p.ag_flags && ((*p.op_counter - 1) & 1)) ? &tmA_alt : &tmA;
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(ta);
-      bool ag_ok = true;
       if (p.ag_flags) {
         const uint32_t par = (*p.op_counter - 1) & 1;
-        for (int g = 0; g * 32 < p.M && ag_ok; ++g)
-          ag_ok = wait_counter_ge(p.ag_flags + par * p.ag_flag_parity_stride + g,
-                                  min(32, p.M - g * 32), p.status, p.peer_wait);
-        fence_proxy_async_global();
+        for (int g = 0; g * 32 < p.M && ok; ++g)
+          ok = wait_counter_ge(p.ag_flags + par * p.ag_flag_parity_stride + g,
+                               min(32, p.M - g * 32), p.status, p.peer_wait);
       }
-      for (int i = 0; i < nkb && ag_ok; ++i) {
-        int s = i % stages;
-        uint32_t ph = (i / stages) & 1;
-        if (!mbar_wait(&bars->empty[s], ph ^ 1, p.status)) { bars->failed = 1; break; }
-        uint8_t* w_dst = smem + (size_t)s * stage_bytes;
-        uint8_t* a_dst = w_dst + kWBytes;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (p.ag_flags) fence_proxy_async_global();
+    uint32_t ph = 1;
+    int s = 0;
+    for (int i = 0; i < nkb && ok; ++i) {
+      if (!mbar_wait_warp(&bars->empty[s], ph, p.status)) {
+        if (lane == 0) bars->failed = 1;
+        break;
+      }
+      uint8_t* w_dst = smem + (size_t)s * stage_bytes;
+      if (elect_one()) {
         if (i >= npre) {         // (the first npre stages already expect their bytes and hold W)
           mbar_expect_tx(&bars->full[s], stage_bytes);
           tma_load_2d(w_dst, &tmW, &bars->full[s], (kb0 + i) * kBK, bz * p.N + tn * kBM);
         }
-        tma_load_2d(a_dst, ta, &bars->full[s], bz * p.batch_a_cols + (kb0 + i) * kBK, 0);
+        tma_load_2d(w_dst + kWBytes, ta, &bars->full[s], bz * p.batch_a_cols + (kb0 + i) * kBK, 0);
       }
+      __syncwarp();
+      if (++s == stages) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(kBM, p.mp);
-      bool ok = true;
-      for (int i = 0; i < nkb; ++i) {
-        int s = i % stages;
-        uint32_t ph = (i / stages) & 1;
-        if (!mbar_wait(&bars->full[s], ph, p.status)) { ok = false; break; }
-        tc_fence_after_sync();
-        uint32_t w_addr = smem_u32(smem + (size_t)s * stage_bytes);
-        uint32_t a_addr = w_addr + kWBytes;
-        uint64_t wdesc = umma_desc_k_sw128(w_addr, 1024);
-        uint64_t adesc = umma_desc_k_sw128(a_addr, 1024);
+    const uint32_t idesc = umma_idesc_bf16(kBM, p.mp), acc = __shfl_sync(0xffffffffu, tmem_base, 0);
+    uint32_t ph = 0;
+    int s = 0;
+    bool ok = true;
+    for (int i = 0; i < nkb; ++i) {
+      if (!(ok = mbar_wait_warp(&bars->full[s], ph, p.status))) break;
+      tc_fence_after_sync();
+      const uint32_t w_addr = smem_u32(smem + (size_t)s * stage_bytes);
+      const uint64_t wdesc = umma_desc_k_sw128(w_addr, 1024), adesc = umma_desc_k_sw128(w_addr + kWBytes, 1024);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < kBK / 16; ++k)
-          umma_bf16_ss(tmem_base, wdesc + 2 * k, adesc + 2 * k, idesc, (i | k) != 0);
+          umma_bf16_ss(acc, wdesc + 2 * k, adesc + 2 * k, idesc, (i | k) != 0);
         umma_commit(&bars->empty[s]);
       }
-      if (ok) umma_commit(&bars->acc_full[0]);
-      else bars->failed = 1;
+      __syncwarp();
+      if (++s == stages) { s = 0; ph ^= 1; }
     }
+    if (ok && elect_one()) umma_commit(&bars->acc_full[0]);
+    __syncwarp();
+    if (!ok && lane == 0) bars->failed = 1;
   } else {
     const int quarter = warp & 3;
     bool ok = true;

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   __shared__ ClusterBars bars;
   constexpr int kWBytes = kRows * kRowBytes, kKB = KIND == kFp8 ? 128 : 64;
   constexpr bool EXPERTS = KIND == kExperts;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int ranks = (p.gated ? 2 : 1) * p.splits;
   const int rank = ranks > 1 ? (int)cluster_ctarank() : 0;
   const int split = rank % p.splits, half = rank / p.splits;           // half 1: the up tile
@@ -160,13 +160,16 @@ __global__ void __launch_bounds__(kThreads, 2)
   int stages = min(kRingStages, p.ring_bytes / stage_bytes);
   // weights that nothing in the stream writes are fetched while the predecessor still runs
   int npre = 0;
-  if (!EXPERTS && warp == 0 && lane == 0 && p.w_early) {
-    tma_prefetch_desc(&tmW);
+  if (!EXPERTS && warp == 0 && p.w_early) {
     npre = min(nkb, stages);
-    for (int i = 0; i < npre; ++i) {
-      mbar_expect_tx(&bars.full[i], stage_bytes);
-      tma_load_2d(smem + (size_t)i * stage_bytes, &tmW, &bars.full[i], (kb0 + i) * kKB, w_row);
+    if (elect_one()) {
+      tma_prefetch_desc(&tmW);
+      for (int i = 0; i < npre; ++i) {
+        mbar_expect_tx(&bars.full[i], stage_bytes);
+        tma_load_2d(smem + (size_t)i * stage_bytes, &tmW, &bars.full[i], (kb0 + i) * kKB, w_row);
+      }
     }
+    __syncwarp();
   }
   pdl_wait();
   pdl_launch_dependents();
@@ -184,44 +187,46 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
   }
 
-  uint32_t it = 0;                          // stages used so far, over the passes
-  for (int first = 0, pass = 0; first < total; first += kMostRows, ++pass, it += nkb) {
+  int slot = 0;                             // of the ring, for the warps that load and multiply (over the passes)
+  uint32_t turn = 0;                        // parity of its use
+  for (int first = 0, pass = 0; first < total; first += kMostRows, ++pass) {
     const int rows = min(kMostRows, total - first);
     const int np = EXPERTS ? (rows + 15) & ~15 : p.mp;
     if (warp == 0) {
-      if (lane == 0) {
-        for (int i = 0; i < nkb; ++i) {
-          const uint32_t n = it + i;
-          const int s = n % stages;
-          if (!mbar_wait(&bars.empty[s], ((n / stages) & 1) ^ 1, p.status)) break;
-          uint8_t* w_dst = smem + (size_t)s * stage_bytes;
+      for (int i = 0; i < nkb; ++i) {
+        if (!mbar_wait_warp(&bars.empty[slot], turn ^ 1, p.status)) break;
+        uint8_t* w_dst = smem + (size_t)slot * stage_bytes;
+        if (elect_one()) {
           if (i >= npre) {
-            mbar_expect_tx(&bars.full[s], stage_bytes);
-            if (EXPERTS) tma_load_3d(w_dst, &tmW, &bars.full[s], (kb0 + i) * kKB, w_row, expert);
-            else tma_load_2d(w_dst, &tmW, &bars.full[s], (kb0 + i) * kKB, w_row);
+            mbar_expect_tx(&bars.full[slot], stage_bytes);
+            if (EXPERTS) tma_load_3d(w_dst, &tmW, &bars.full[slot], (kb0 + i) * kKB, w_row, expert);
+            else tma_load_2d(w_dst, &tmW, &bars.full[slot], (kb0 + i) * kKB, w_row);
           }
-          tma_load_2d(w_dst + kWBytes, &tmA.m[map], &bars.full[s], blockIdx.z * p.batch_a_cols + (kb0 + i) * kKB, row_base + first);
+          tma_load_2d(w_dst + kWBytes, &tmA.m[map], &bars.full[slot], blockIdx.z * p.batch_a_cols + (kb0 + i) * kKB, row_base + first);
         }
+        __syncwarp();
+        if (++slot == stages) { slot = 0; turn ^= 1; }
       }
     } else if (warp == 1) {
-      if (lane == 0) {
-        const uint32_t idesc = KIND == kFp8 ? umma_idesc_e4m3(kRows, np) : umma_idesc_bf16(kRows, np);
-        bool ok = true;
-        for (int i = 0; i < nkb; ++i) {
-          const uint32_t n = it + i;
-          const int s = n % stages;
-          if (!mbar_wait(&bars.full[s], (n / stages) & 1, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t w_addr = smem_u32(smem + (size_t)s * stage_bytes);
-          const uint64_t wdesc = umma_desc_k_sw128(w_addr, 1024), adesc = umma_desc_k_sw128(w_addr + kWBytes, 1024);
+      const uint32_t idesc = KIND == kFp8 ? umma_idesc_e4m3(kRows, np) : umma_idesc_bf16(kRows, np);
+      const uint32_t acc = __shfl_sync(0xffffffffu, tmem, 0);
+      bool ok = true;
+      for (int i = 0; i < nkb; ++i) {
+        if (!(ok = mbar_wait_warp(&bars.full[slot], turn, p.status))) break;
+        tc_fence_after_sync();
+        const uint32_t w_addr = smem_u32(smem + (size_t)slot * stage_bytes);
+        const uint64_t wdesc = umma_desc_k_sw128(w_addr, 1024), adesc = umma_desc_k_sw128(w_addr + kWBytes, 1024);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {       // 32 bytes of a row each
-            if (KIND == kFp8) umma_f8f6f4_ss(tmem, wdesc + 2 * k, adesc + 2 * k, idesc, (i | k) != 0);
-            else umma_bf16_ss(tmem, wdesc + 2 * k, adesc + 2 * k, idesc, (i | k) != 0);
+            if (KIND == kFp8) umma_f8f6f4_ss(acc, wdesc + 2 * k, adesc + 2 * k, idesc, (i | k) != 0);
+            else umma_bf16_ss(acc, wdesc + 2 * k, adesc + 2 * k, idesc, (i | k) != 0);
           }
-          umma_commit(&bars.empty[s]);
+          umma_commit(&bars.empty[slot]);
+          if (i == nkb - 1) umma_commit(&bars.acc);
         }
-        if (ok) umma_commit(&bars.acc);
+        __syncwarp();
+        if (++slot == stages) { slot = 0; turn ^= 1; }
       }
     } else {
       // accumulator (lane = weight row, column = batch row) -> this CTA's partial tile [rows][128] over the ring, whose

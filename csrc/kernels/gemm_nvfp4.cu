@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kF4Threads, 1)
   auto sSfa = [&](int s) { return sB(s) + L::b_bytes; };
   auto sSfb = [&](int s) { return sSfa(s) + kF4SfaBytes; };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * 128, n0 = blockIdx.x * NT, split = blockIdx.z;
   const int total_stages = p.K / 256;
   const int st0 = split * p.stages_per_split;
@@ -105,14 +105,16 @@ __global__ void __launch_bounds__(kF4Threads, 1)
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
 
-  if (warp == 0) {
+  if (warp == 0) {          // (these two warps walk their loops whole, one elected lane issues)
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmW);
-      const size_t chunks_per_rowblock = (size_t)(p.K / 64) * 512;
-      for (int i = 0; i < nst; ++i) {
-        const int s = i % kF4Stages, st = st0 + i;
-        if (!mbar_wait_backoff(&bars->empty[s], ((i / kF4Stages) & 1) ^ 1, p.status)) break;
+    }
+    const size_t chunks_per_rowblock = (size_t)(p.K / 64) * 512;
+    for (int i = 0; i < nst; ++i) {
+      const int s = i % kF4Stages, st = st0 + i;
+      if (!__all_sync(0xffffffffu, mbar_wait_backoff(&bars->empty[s], ((i / kF4Stages) & 1) ^ 1, p.status))) break;
+      if (elect_one()) {
         mbar_expect_tx(&bars->full[s], L::stage_bytes);
         tma_load_2d(sA(s), &tmA, &bars->full[s], st * 128, m0);
         tma_load_2d(sB(s), &tmW, &bars->full[s], st * 128, n0);
@@ -124,17 +126,21 @@ __global__ void __launch_bounds__(kF4Threads, 1)
                     p.sfw + (size_t)(n0 / 128 + rb) * chunks_per_rowblock + (size_t)st * kF4SfaBytes, kF4SfaBytes,
                     &bars->full[s]);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_nvfp4(128, NT);
-      bool ok = true;
-      for (int i = 0; i < nst; ++i) {
-        const int s = i % kF4Stages;
-        if (!mbar_wait_backoff(&bars->full[s], (i / kF4Stages) & 1, p.status)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t t_sfa = tmem_base + NT + s * L::sf_cols_per_stage;
-        const uint32_t t_sfb = t_sfa + 16;
+    constexpr uint32_t idesc = umma_idesc_nvfp4(128, NT);
+    const uint32_t acc = __shfl_sync(0xffffffffu, tmem_base, 0);
+    bool ok = true;
+    for (int i = 0; i < nst; ++i) {
+      const int s = i % kF4Stages;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait_backoff(&bars->full[s], (i / kF4Stages) & 1, p.status)))) break;
+      tc_fence_after_sync();
+      const uint32_t t_sfa = acc + NT + s * L::sf_cols_per_stage;
+      const uint32_t t_sfb = t_sfa + 16;
+      const uint64_t adesc = umma_desc_k_sw128(smem_u32(sA(s)), 1024);
+      const uint64_t bdesc = umma_desc_k_sw128(smem_u32(sB(s)), 1024);
+      if (elect_one()) {
         // scale chunks of this stage: A's four K = 64 chunks, then B's per 128-row block
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -144,16 +150,16 @@ __global__ void __launch_bounds__(kF4Threads, 1)
             tmem_cp_32x128b_warpx4(t_sfb + (NT / 32) * j + 4 * rb,
                                    sf_chunk_desc(smem_u32(sSfb(s) + rb * kF4SfaBytes + j * 512)));
         }
-        const uint64_t adesc = umma_desc_k_sw128(smem_u32(sA(s)), 1024);
-        const uint64_t bdesc = umma_desc_k_sw128(smem_u32(sB(s)), 1024);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          umma_nvfp4_ss(tmem_base, adesc + 2 * j, bdesc + 2 * j, idesc, t_sfa + 4 * j, t_sfb + (NT / 32) * j,
+          umma_nvfp4_ss(acc, adesc + 2 * j, bdesc + 2 * j, idesc, t_sfa + 4 * j, t_sfb + (NT / 32) * j,
                         (i | j) != 0);
         umma_commit(&bars->empty[s]);
       }
-      if (ok) umma_commit(&bars->acc_full);
+      __syncwarp();
     }
+    if (ok && elect_one()) umma_commit(&bars->acc_full);
+    __syncwarp();
   } else {
     // ---- epilogue: TMEM lane = row of the tile, column = n
     const int q = warp & 3;                       // lane quarter this warp may read

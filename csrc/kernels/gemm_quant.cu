@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kQThreads, 1)
   constexpr int kABytes = kQM * kQKB, kBBytes = kQN * kQKB, kStage = kABytes + kBBytes;
   const int stages = p.stages;
   QBars* bars = reinterpret_cast<QBars*>(smem + (size_t)stages * kStage);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n * p.splits;     // work items: (tile, K split)
   const int kblocks_total = (p.K + kQKB - 1) / kQKB;
   if (threadIdx.x == 0) {
@@ -79,53 +79,58 @@ __global__ void __launch_bounds__(kQThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
-  if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
-        const int t = w / p.splits, sp = w % p.splits;
-        const int tm = t % p.tiles_m, tn = t / p.tiles_m;
-        const int kb0 = sp * p.kb_per_split, kb1 = min(kblocks_total, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % stages;
-          if (!mbar_wait(&bars->empty[s], ((it / stages) & 1) ^ 1, p.status)) { ok = false; break; }
-          uint8_t* a_dst = smem + (size_t)s * kStage;
+  if (warp == 0) {          // (these two warps walk their loops whole, one elected lane issues)
+    int s = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
+      const int t = w / p.splits, sp = w % p.splits;
+      const int tm = t % p.tiles_m, tn = t / p.tiles_m;
+      const int kb0 = sp * p.kb_per_split, kb1 = min(kblocks_total, kb0 + p.kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(&bars->empty[s], ph, p.status))) break;
+        uint8_t* a_dst = smem + (size_t)s * kStage;
+        if (elect_one()) {
           mbar_expect_tx(&bars->full[s], kStage);
           tma_load_2d(a_dst, &tmA, &bars->full[s], kb * kQKB, tm * kQM);
           tma_load_2d(a_dst + kABytes, &tmB, &bars->full[s], kb * kQKB, tn * kQN);
         }
+        __syncwarp();
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
-      if (!ok) bars->failed = 1;
     }
+    if (!ok && lane == 0) bars->failed = 1;
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_e4m3(kQM, kQN);
-      uint32_t it = 0, tc = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x, ++tc) {
-        const int buf = tc & 1;
-        if (!mbar_wait(&bars->acc_empty[buf], ((tc >> 1) & 1) ^ 1, p.status)) { ok = false; break; }
+    constexpr uint32_t idesc = umma_idesc_e4m3(kQM, kQN);
+    const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+    uint32_t tc = 0, ph = 0;
+    int s = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x, ++tc) {
+      const int buf = tc & 1;
+      if (!(ok = mbar_wait_warp(&bars->acc_empty[buf], ((tc >> 1) & 1) ^ 1, p.status))) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_u + buf * kQN;
+      const int sp = w % p.splits;
+      const int kb0 = sp * p.kb_per_split, kb1 = min(kblocks_total, kb0 + p.kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_warp(&bars->full[s], ph, p.status))) break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + buf * kQN;
-        const int sp = w % p.splits;
-        const int kb0 = sp * p.kb_per_split, kb1 = min(kblocks_total, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % stages;
-          if (!mbar_wait(&bars->full[s], (it / stages) & 1, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem + (size_t)s * kStage);
-          const uint64_t adesc = umma_desc_k_sw128(a_addr, 1024);
-          const uint64_t bdesc = umma_desc_k_sw128(a_addr + kABytes, 1024);
+        const uint32_t a_addr = smem_u32(smem + (size_t)s * kStage);
+        const uint64_t adesc = umma_desc_k_sw128(a_addr, 1024), bdesc = umma_desc_k_sw128(a_addr + kABytes, 1024);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < kQKB / 32; ++k)   // 32 fp8 values = 32 bytes per instruction
             umma_f8f6f4_ss(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, kb != kb0 || k != 0);
           umma_commit(&bars->empty[s]);
         }
-        if (ok) umma_commit(&bars->acc_full[buf]);
+        __syncwarp();
+        if (++s == stages) { s = 0; ph ^= 1; }
       }
-      if (!ok) bars->failed = 1;
+      if (ok && elect_one()) umma_commit(&bars->acc_full[buf]);
+      __syncwarp();
     }
+    if (!ok && lane == 0) bars->failed = 1;
   } else {
     const int quarter = warp & 3;
     uint32_t tc = 0;

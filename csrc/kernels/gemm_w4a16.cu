@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
   uint8_t* sSf = sAct + (size_t)AS * kActBytes;      // RS x 4 KB of block scales
   W4SBars* bars = reinterpret_cast<W4SBars*>(sSf + (size_t)RS * kSfBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tn = blockIdx.x, split = blockIdx.y;
   const int n0 = tn * kWN;
   const int ne_total = (p.K + 63) / 64;
@@ -134,51 +134,54 @@ __global__ void __launch_bounds__(kWThreads, 1)
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
-    // ---------------- packed-weight (and scale) producer ----------------
-    if (lane == 0) {
-      tma_prefetch_desc(&tmW);
-      const int nr = (ne + 3) / 4;
-      for (int i = 0; i < nr; ++i) {
-        const int rs = i % RS;
-        if (!mbar_wait_backoff(&bars->raw_empty[rs], ((i / RS) & 1) ^ 1, p.status)) break;
+    // ---------------- packed-weight (and scale) producer (whole warps walk the loops, an elected lane issues) ----------------
+    if (lane == 0) tma_prefetch_desc(&tmW);
+    const int nr = (ne + 3) / 4;
+    for (int i = 0; i < nr; ++i) {
+      const int rs = i % RS;
+      if (!__all_sync(0xffffffffu, mbar_wait_backoff(&bars->raw_empty[rs], ((i / RS) & 1) ^ 1, p.status))) break;
+      if (elect_one()) {
         mbar_expect_tx(&bars->raw_full[rs], kRawBytes + (p.sf_tma ? kSfBytes : 0));
         tma_load_2d(sRaw + (size_t)rs * kRawBytes, &tmW, &bars->raw_full[rs], k0 / 2 + i * 128, n0);
         if (p.sf_tma) tma_load_2d(sSf + (size_t)rs * kSfBytes, &tmS, &bars->raw_full[rs], k0 / 16 + i * 16, n0);
       }
+      __syncwarp();
     }
   } else if (warp == 2) {
     // ---------------- activation producer ----------------
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      for (int e = 0; e < ne; ++e) {
-        const int as = e % AS;
-        if (!mbar_wait_backoff(&bars->act_empty[as], ((e / AS) & 1) ^ 1, p.status)) break;
+    if (lane == 0) tma_prefetch_desc(&tmA);
+    for (int e = 0; e < ne; ++e) {
+      const int as = e % AS;
+      if (!__all_sync(0xffffffffu, mbar_wait_backoff(&bars->act_empty[as], ((e / AS) & 1) ^ 1, p.status))) break;
+      if (elect_one()) {
         mbar_expect_tx(&bars->act_full[as], kActBytes);
         tma_load_2d(sAct + (size_t)as * kActBytes, &tmA, &bars->act_full[as], k0 + e * 64, 0);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer: D[128 batch rows, 256 weight rows] ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_f16(128, kWN);
-      bool ok = true;
-      for (int e = 0; e < ne; ++e) {
-        const int es = e % ES, as = e % AS;
-        if (!mbar_wait_backoff(&bars->exp_full[es], (e / ES) & 1, p.status) ||
-            !mbar_wait_backoff(&bars->act_full[as], (e / AS) & 1, p.status)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after_sync();
-        const uint64_t adesc = umma_desc_k_sw128(smem_u32(sAct + (size_t)as * kActBytes), 1024);
-        const uint64_t bdesc = umma_desc_k_sw128(smem_u32(sExp + (size_t)es * kExpBytes), 1024);
+    constexpr uint32_t idesc = umma_idesc_f16(128, kWN);
+    const uint32_t acc = __shfl_sync(0xffffffffu, tmem_base, 0);
+    bool ok = true;
+    for (int e = 0; e < ne; ++e) {
+      const int es = e % ES, as = e % AS;
+      ok = __all_sync(0xffffffffu, mbar_wait_backoff(&bars->exp_full[es], (e / ES) & 1, p.status) &&
+                                       mbar_wait_backoff(&bars->act_full[as], (e / AS) & 1, p.status));
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint64_t adesc = umma_desc_k_sw128(smem_u32(sAct + (size_t)as * kActBytes), 1024);
+      const uint64_t bdesc = umma_desc_k_sw128(smem_u32(sExp + (size_t)es * kExpBytes), 1024);
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f16_ss(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, (e | k) != 0);
+        for (int k = 0; k < 4; ++k) umma_f16_ss(acc, adesc + 2 * k, bdesc + 2 * k, idesc, (e | k) != 0);
         umma_commit(&bars->exp_empty[es]);
         umma_commit(&bars->act_empty[as]);
       }
-      if (ok) umma_commit(&bars->acc_full);
+      __syncwarp();
     }
+    if (ok && elect_one()) umma_commit(&bars->acc_full);
+    __syncwarp();
   } else {
     // ---------------- converters (then epilogue) ----------------
     const int cw = warp - 3;                        // 0..15
@@ -336,7 +339,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
   uint8_t* sRaw = sExp + kCES * kCExp;
   uint8_t* sAct = sRaw + kCRS * kCRaw;
   const int act_bytes = p.mp * 128;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, tile = blockIdx.x / p.splits, n0 = tile * kCRows;
   const int blocks = p.K / 256, b0 = blocks * rank / p.splits, nr = blocks * (rank + 1) / p.splits - b0, ne = 4 * nr;
 
@@ -359,42 +362,50 @@ __global__ void __launch_bounds__(kCThreads, 2)
   pdl_launch_dependents();
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmW);
-      for (int i = 0; i < nr; ++i) {
-        const int rs = i % kCRS;
-        if (!mbar_wait(&bars.raw_empty[rs], ((i / kCRS) & 1) ^ 1, p.status)) break;
+    if (lane == 0) tma_prefetch_desc(&tmW);
+    for (int i = 0; i < nr; ++i) {
+      const int rs = i % kCRS;
+      if (!mbar_wait_warp(&bars.raw_empty[rs], ((i / kCRS) & 1) ^ 1, p.status)) break;
+      if (elect_one()) {
         mbar_expect_tx(&bars.raw_full[rs], kCRaw);
         tma_load_2d(sRaw + rs * kCRaw, &tmW, &bars.raw_full[rs], (b0 + i) * 128, n0);
       }
+      __syncwarp();
     }
   } else if (warp == 2 + kCConv) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      for (int e = 0; e < ne; ++e) {
-        const int as = e % p.act_stages;
-        if (!mbar_wait(&bars.act_empty[as], ((e / p.act_stages) & 1) ^ 1, p.status)) break;
+    if (lane == 0) tma_prefetch_desc(&tmA);
+    int as = 0;
+    uint32_t ph = 1;
+    for (int e = 0; e < ne; ++e) {
+      if (!mbar_wait_warp(&bars.act_empty[as], ph, p.status)) break;
+      if (elect_one()) {
         mbar_expect_tx(&bars.act_full[as], act_bytes);
         tma_load_2d(sAct + as * act_bytes, &tmA, &bars.act_full[as], b0 * 256 + e * 64, 0);
       }
+      __syncwarp();
+      if (++as == p.act_stages) { as = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_f16(kCRows, p.mp);
-      bool ok = true;
-      for (int e = 0; e < ne; ++e) {
-        const int es = e % kCES, as = e % p.act_stages;
-        ok = mbar_wait(&bars.act_full[as], (e / p.act_stages) & 1, p.status) && mbar_wait(&bars.exp_full[es], (e / kCES) & 1, p.status);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint64_t wd = umma_desc_k_sw128(smem_u32(sExp + es * kCExp), 1024);
-        const uint64_t ad = umma_desc_k_sw128(smem_u32(sAct + as * act_bytes), 1024);
+    const uint32_t idesc = umma_idesc_f16(kCRows, p.mp), acc = __shfl_sync(0xffffffffu, tmem, 0);
+    int as = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int e = 0; e < ne; ++e) {
+      const int es = e % kCES;
+      ok = mbar_wait_warp(&bars.act_full[as], ph, p.status) && mbar_wait_warp(&bars.exp_full[es], (e / kCES) & 1, p.status);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint64_t wd = umma_desc_k_sw128(smem_u32(sExp + es * kCExp), 1024);
+      const uint64_t ad = umma_desc_k_sw128(smem_u32(sAct + as * act_bytes), 1024);
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f16_ss(tmem, wd + 2 * k, ad + 2 * k, idesc, (e | k) != 0);
+        for (int k = 0; k < 4; ++k) umma_f16_ss(acc, wd + 2 * k, ad + 2 * k, idesc, (e | k) != 0);
         umma_commit(&bars.exp_empty[es]);
         umma_commit(&bars.act_empty[as]);
+        if (e == ne - 1) umma_commit(&bars.acc);
       }
-      if (ok) umma_commit(&bars.acc);
+      __syncwarp();
+      if (++as == p.act_stages) { as = 0; ph ^= 1; }
     }
   } else {
     // A nibble's three magnitude bits in bits 9 to 11 of an f16 are its value times 2^-14 (subnormals included), nibbles k and

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(192, 1)
   uint8_t* sP = sQ + kQBytes;                      // 2 buffers x (2 token halves x 2 KB)
   MlaBars* bars = reinterpret_cast<MlaBars*>(sP + 8192);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int b = blockIdx.x, split = blockIdx.y;
   const int head0 = blockIdx.z * kNQ, G = min(p.Hq - head0, kNQ);
   pdl_wait();
@@ -159,100 +159,112 @@ __global__ void __launch_bounds__(192, 1)
 
   if (ntiles > 0) {
     if (warp == 0) {
-      if (lane == 0) {
+      // (the whole warp walks the loop: a lane per page loads, an elected one issues the products below)
+      if (elect_one()) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmC);
         mbar_expect_tx(&bars->q_full, kQBytes);
         for (int h = 0; h < kQHalves; ++h) tma_load_3d(sQ + h * 2048, &tmQ, &bars->q_full, h * 64, head0, b);
-        const int32_t* bt = p.block_table + (size_t)b * p.max_blocks;
-        const int nblk_valid = (seq_len + p.block_size - 1) / p.block_size;
-        const int rows_per_load = min(p.block_size, kTok);
-        const int loads = kTok / rows_per_load;
-        bool ok = true;
-        int itv = 0, itr = 0;
-        // piece < kVPieces: value columns [128 * piece, +128) into the value ring; piece == kVPieces:
-        // the rotary columns [512, 576) into the rotary ring
-        auto load_piece = [&](int j, int piece) {
-          const bool rope = piece == kVPieces;
-          int& it = rope ? itr : itv;
-          const int n = rope ? kRSlots : kVSlots;
-          const int sl = it % n;
-          const uint32_t ph = (it / n) & 1;
-          ++it;
-          const int bi_ = rope ? kVSlots + sl : sl;                // barrier index
-          if (!mbar_wait(&bars->kv_empty[bi_], ph ^ 1, p.status)) { ok = false; return; }
-          uint8_t* dst = rope ? sRope + sl * kRopeBytes : sKV + sl * kSlotBytes;
-          const int halves = rope ? 1 : 2;
-          mbar_expect_tx(&bars->kv_full[bi_], halves * 16384);
-          const int tok0 = tok_base + j * kTok;
-          for (int l = 0; l < loads; ++l) {
-            const int tk = tok0 + l * rows_per_load;
-            const int bi = tk / p.block_size;
-            const int blk = (bi < nblk_valid) ? bt[bi] : bt[0];
-            const int row = (blk < 0 ? 0 : blk) * p.block_size + tk % p.block_size;
-            for (int hf = 0; hf < halves; ++hf)
-              tma_load_2d(dst + hf * 16384 + l * rows_per_load * 128, &tmC, &bars->kv_full[bi_],
-                          piece * 128 + hf * 64, row);
-          }
-        };
-        // per tile: rotary piece first (its slot turns over early), then the value pieces in the
-        // order both products read them
-        for (int j = 0; j < ntiles && ok; ++j) {
-          load_piece(j, kVPieces);
-          for (int pc = 0; pc < kVPieces && ok; ++pc) load_piece(j, pc);
+      }
+      __syncwarp();
+      const int32_t* bt = p.block_table + (size_t)b * p.max_blocks;
+      const int nblk_valid = (seq_len + p.block_size - 1) / p.block_size;
+      const int rows_per_load = min(p.block_size, kTok);
+      const int loads = kTok / rows_per_load;
+      bool ok = true;
+      int itv = 0, itr = 0;
+      // piece < kVPieces: value columns [128 * piece, +128) into the value ring; piece == kVPieces:
+      // the rotary columns [512, 576) into the rotary ring
+      auto load_piece = [&](int j, int piece) {
+        const bool rope = piece == kVPieces;
+        int& it = rope ? itr : itv;
+        const int n = rope ? kRSlots : kVSlots;
+        const int sl = it % n;
+        const uint32_t ph = (it / n) & 1;
+        ++it;
+        const int bi_ = rope ? kVSlots + sl : sl;                // barrier index
+        if (!(ok = mbar_wait_warp(&bars->kv_empty[bi_], ph ^ 1, p.status))) return;
+        uint8_t* dst = rope ? sRope + sl * kRopeBytes : sKV + sl * kSlotBytes;
+        const int halves = rope ? 1 : 2;
+        if (lane == 0) mbar_expect_tx(&bars->kv_full[bi_], halves * 16384);
+        __syncwarp();
+        for (int l = lane; l < loads; l += 32) {
+          const int tk = tok_base + j * kTok + l * rows_per_load;
+          const int bi = tk / p.block_size;
+          const int blk = (bi < nblk_valid) ? bt[bi] : bt[0];
+          const int row = (blk < 0 ? 0 : blk) * p.block_size + tk % p.block_size;
+          for (int hf = 0; hf < halves; ++hf)
+            tma_load_2d(dst + hf * 16384 + l * rows_per_load * 128, &tmC, &bars->kv_full[bi_],
+                        piece * 128 + hf * 64, row);
         }
+        __syncwarp();
+      };
+      // per tile: rotary piece first (its slot turns over early), then the value pieces in the
+      // order both products read them
+      for (int j = 0; j < ntiles && ok; ++j) {
+        load_piece(j, kVPieces);
+        for (int pc = 0; pc < kVPieces && ok; ++pc) load_piece(j, pc);
       }
     } else if (warp == 1) {
-      if (lane == 0) {
-        constexpr uint32_t idesc_qk = umma_idesc_bf16(kTok, kNQ, 0, 0);
-        constexpr uint32_t idesc_pv = umma_idesc_bf16(128, kNQ, 1, 0);
-        bool ok = mbar_wait(&bars->q_full, 0, p.status);
-        const uint32_t q_addr = smem_u32(sQ);
-        // value piece pc of tile j sits in value slot (4 j + pc) % 5 on that slot's ((4 j + pc) / 5)-th
-        // use; the rotary piece of tile j in rotary slot j % 2
-        auto s_piece = [&](int j, int pc, bool first) -> bool {      // one piece of S(j) = K(j) Q^T
-          const bool rope = pc == kVPieces;
-          const int f = rope ? j : kVPieces * j + pc, n = rope ? kRSlots : kVSlots;
-          const int sl = f % n, bi_ = rope ? kVSlots + sl : sl;
-          if (!mbar_wait(&bars->kv_full[bi_], (f / n) & 1, p.status)) return false;
-          tc_fence_after_sync();
-          const uint32_t k_addr = smem_u32(rope ? sRope + sl * kRopeBytes : sKV + sl * kSlotBytes);
-          const int ksteps = rope ? 4 : 8;
-          for (int kk = 0; kk < ksteps; ++kk) {
+      constexpr uint32_t idesc_qk = umma_idesc_bf16(kTok, kNQ, 0, 0);
+      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, kNQ, 1, 0);
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+      bool ok = mbar_wait_warp(&bars->q_full, 0, p.status);
+      const uint32_t q_addr = smem_u32(sQ);
+      // value piece pc of tile j sits in value slot (4 j + pc) % 5 on that slot's ((4 j + pc) / 5)-th
+      // use; the rotary piece of tile j in rotary slot j % 2
+      auto s_piece = [&](int j, int pc, bool first) -> bool {      // one piece of S(j) = K(j) Q^T
+        const bool rope = pc == kVPieces;
+        const int f = rope ? j : kVPieces * j + pc, n = rope ? kRSlots : kVSlots;
+        const int sl = f % n, bi_ = rope ? kVSlots + sl : sl;
+        if (!mbar_wait_warp(&bars->kv_full[bi_], (f / n) & 1, p.status)) return false;
+        tc_fence_after_sync();
+        const uint32_t k_addr = smem_u32(rope ? sRope + sl * kRopeBytes : sKV + sl * kSlotBytes);
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {
+            if (rope && kk >= 4) break;
             const uint32_t koff = (kk / 4) * 16384 + (kk % 4) * 32;
             const uint32_t qoff = (pc * 2 + kk / 4) * 2048 + (kk % 4) * 32;
-            umma_bf16_ss(tmem_s + (j & 1) * 16, umma_desc_k_sw128(k_addr + koff, 1024),
+            umma_bf16_ss(tm + (j & 1) * 16, umma_desc_k_sw128(k_addr + koff, 1024),
                          umma_desc_k_sw128(q_addr + qoff, 1024), idesc_qk, !(first && kk == 0));
           }
           if (rope) umma_commit(&bars->kv_empty[bi_]);    // the value slots stay until O(j) has read them
-          return true;
-        };
-        // S(0): rotary piece, then the value pieces
-        ok = ok && mbar_wait(&bars->s_empty[0], 1, p.status);
-        ok = ok && s_piece(0, kVPieces, true);
-        for (int pc = 0; pc < kVPieces && ok; ++pc) ok = s_piece(0, pc, false);
-        if (ok) umma_commit(&bars->s_full[0]);
-        for (int j = 0; j < ntiles && ok; ++j) {
-          const bool next = j + 1 < ntiles;
-          if (next) {
-            // what of tile j+1 can be in shared memory already: its rotary piece and one value piece
-            const int sb = (j + 1) & 1;
-            if (!mbar_wait(&bars->s_empty[sb], (((j + 1) >> 1) & 1) ^ 1, p.status)) { ok = false; break; }
-            ok = s_piece(j + 1, kVPieces, true) && s_piece(j + 1, 0, false);
-            if (!ok) break;
-          }
-          // O(j) += V(j)^T P(j)^T, releasing the value slots of tile j one by one
-          const int pb = j & 1;
-          if (!mbar_wait(&bars->p_full[pb], (j >> 1) & 1, p.status)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t p_addr = smem_u32(sP + pb * 4096);
+        }
+        __syncwarp();
+        return true;
+      };
+      const auto commit = [&](uint64_t* bar) {
+        if (elect_one()) umma_commit(bar);
+        __syncwarp();
+      };
+      // S(0): rotary piece, then the value pieces
+      ok = ok && mbar_wait_warp(&bars->s_empty[0], 1, p.status);
+      ok = ok && s_piece(0, kVPieces, true);
+      for (int pc = 0; pc < kVPieces && ok; ++pc) ok = s_piece(0, pc, false);
+      if (ok) commit(&bars->s_full[0]);
+      for (int j = 0; j < ntiles && ok; ++j) {
+        const bool next = j + 1 < ntiles;
+        if (next) {
+          // what of tile j+1 can be in shared memory already: its rotary piece and one value piece
+          const int sb = (j + 1) & 1;
+          if (!(ok = mbar_wait_warp(&bars->s_empty[sb], (((j + 1) >> 1) & 1) ^ 1, p.status))) break;
+          ok = s_piece(j + 1, kVPieces, true) && s_piece(j + 1, 0, false);
+          if (!ok) break;
+        }
+        // O(j) += V(j)^T P(j)^T, releasing the value slots of tile j one by one
+        const int pb = j & 1;
+        if (!(ok = mbar_wait_warp(&bars->p_full[pb], (j >> 1) & 1, p.status))) break;
+        tc_fence_after_sync();
+        const uint32_t p_addr = smem_u32(sP + pb * 4096);
+        if (elect_one()) {
           for (int pc = 0; pc < kVPieces; ++pc) {
             const int f = kVPieces * j + pc, sl = f % kVSlots;
             const uint32_t v_addr = smem_u32(sKV + sl * kSlotBytes);
 #pragma unroll
             for (int kk = 0; kk < kTok / 16; ++kk) {
               const uint32_t poff = (kk / 4) * 2048 + (kk % 4) * 32;
-              umma_bf16_ss(tmem_o + pc * 16, umma_desc_mn_sw128(v_addr + kk * 2048, 16384, 1024),
+              umma_bf16_ss(tm + 32 + pc * 16, umma_desc_mn_sw128(v_addr + kk * 2048, 16384, 1024),
                            umma_desc_k_sw128(p_addr + poff, 1024), idesc_pv, (j | kk) != 0);
             }
             umma_commit(&bars->kv_empty[sl]);
@@ -260,10 +272,11 @@ __global__ void __launch_bounds__(192, 1)
           umma_commit(&bars->pv_done);    // before p_empty: whoever sees p_empty has this arrival too
           umma_commit(&bars->p_empty[pb]);
           if (!next) umma_commit(&bars->o_done);
-          if (next) {
-            for (int pc = 1; pc < kVPieces && ok; ++pc) ok = s_piece(j + 1, pc, false);
-            if (ok) umma_commit(&bars->s_full[(j + 1) & 1]);
-          }
+        }
+        __syncwarp();
+        if (next) {
+          for (int pc = 1; pc < kVPieces && ok; ++pc) ok = s_piece(j + 1, pc, false);
+          if (ok) commit(&bars->s_full[(j + 1) & 1]);
         }
       }
     } else {

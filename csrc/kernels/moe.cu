@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(192, 2)
   const int kStage = kWBytes * (gated ? 2 : 1) + kXBytes;
   const int stages = p.stages;
   GroupedBars* bars = reinterpret_cast<GroupedBars*>(smem + (size_t)stages * kStage);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tn = (int)blockIdx.x % tiles;
   const int nkb = (p.K + kGBK - 1) / kGBK;
   if (threadIdx.x == 0) {
@@ -408,41 +408,50 @@ __global__ void __launch_bounds__(192, 2)
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
   const int x_off = kWBytes * (gated ? 2 : 1);
-  if (warp == 0) {
-    if (lane == 0) {
+  if (warp == 0) {          // (these two warps walk their loops whole, one elected lane issues)
+    if (elect_one()) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % stages;
-        if (!mbar_wait(&bars->empty[s], ((i / stages) & 1) ^ 1, p.status)) break;
-        uint8_t* wd = smem + (size_t)s * kStage;
+    }
+    __syncwarp();
+    int s = 0;
+    uint32_t ph = 1;
+    for (int i = 0; i < nkb; ++i) {
+      if (!mbar_wait_warp(&bars->empty[s], ph, p.status)) break;
+      uint8_t* wd = smem + (size_t)s * kStage;
+      if (elect_one()) {
         mbar_expect_tx(&bars->full[s], kStage);
         tma_load_3d(wd, &tmW, &bars->full[s], i * kGBK, tn * kGBM, e);
         if (gated) tma_load_3d(wd + kWBytes, &tmW, &bars->full[s], i * kGBK, half_n + tn * kGBM, e);
         tma_load_2d(wd + x_off, &tmX, &bars->full[s], i * kGBK, row0);
       }
+      __syncwarp();
+      if (++s == stages) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(kGBM, np);
-      bool ok = true;
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % stages;
-        if (!mbar_wait(&bars->full[s], (i / stages) & 1, p.status)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t wa = smem_u32(smem + (size_t)s * kStage), xa = wa + x_off;
+    const uint32_t idesc = umma_idesc_bf16(kGBM, np), acc = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int i = 0; i < nkb; ++i) {
+      if (!(ok = mbar_wait_warp(&bars->full[s], ph, p.status))) break;
+      tc_fence_after_sync();
+      const uint32_t wa = smem_u32(smem + (size_t)s * kStage);
+      const uint64_t wdesc = umma_desc_k_sw128(wa, 1024), udesc = umma_desc_k_sw128(wa + kWBytes, 1024),
+                     xdesc = umma_desc_k_sw128(wa + x_off, 1024);
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < kGBK / 16; ++kk) {
-          umma_bf16_ss(tmem_base, umma_desc_k_sw128(wa + kk * 32, 1024),
-                       umma_desc_k_sw128(xa + kk * 32, 1024), idesc, (i | kk) != 0);
-          if (gated)
-            umma_bf16_ss(tmem_base + p.sub_rows, umma_desc_k_sw128(wa + kWBytes + kk * 32, 1024),
-                         umma_desc_k_sw128(xa + kk * 32, 1024), idesc, (i | kk) != 0);
+          umma_bf16_ss(acc, wdesc + 2 * kk, xdesc + 2 * kk, idesc, (i | kk) != 0);
+          if (gated) umma_bf16_ss(acc + p.sub_rows, udesc + 2 * kk, xdesc + 2 * kk, idesc, (i | kk) != 0);
         }
         umma_commit(&bars->empty[s]);
       }
-      if (ok) umma_commit(&bars->acc_full);
+      __syncwarp();
+      if (++s == stages) { s = 0; ph ^= 1; }
     }
+    if (ok && elect_one()) umma_commit(&bars->acc_full);
+    __syncwarp();
   } else if (gated) {
     const int quarter = warp & 3;
     if (p.act_fuse == 4) {

@@ -104,6 +104,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return true;
 }
 
+// The whole warp waits, with one answer for all lanes. An issuing warp walks its loop as one and lets elect_one() pick the lane
+// that issues: stage addresses and descriptors then stay in uniform registers, where tcgen05.mma and TMA take them from. In code
+// of one lane each of them is moved there first, which bounded every product whose instructions are short.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status));
+}
+// Index of the calling warp, known to the compiler as the same for all its lanes.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // Same, for single-thread producer / issuer warps that share their SM sub-partition with warps
 // doing real work: sleeps between polls so that the polling does not compete for issue slots.
 __device__ __forceinline__ bool mbar_wait_backoff(uint64_t* bar, uint32_t parity, int* status) {
