@@ -485,61 +485,51 @@ __global__ void __launch_bounds__(320, 1)
       }
     }
   } else if (warp == 1) {
-    // (the whole warp watches and walks; one elected lane issues)
     constexpr uint32_t idesc_qk = umma_idesc_bf16(kQT, kPT, 0, 0);
     constexpr uint32_t idesc_pv = umma_idesc_bf16(kQT, 128, 0, 1);      // B (V) is MN-major
-    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-    const auto ready = [](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; };
-    int j[2] = {-1, -1};          // last product Q K issued
-    bool pv[2] = {false, false};  // P V of that tile issued
-    int left = mbar_wait_warp(&bars.q_full, 0, p.status) ? 2 : 0;
-    long long t0 = clock64();
-    uint32_t spins = 0;
-    while (left > 0) {
-      bool idle = true;
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), q_addr = smem_u32(sQ);
+    const auto qk = [&](int t, int n) {           // S(t) = Q(t) K(n)^T
+      const int sl = (2 * n) % kPRing;
+      const uint32_t k_addr = smem_u32(sKV + sl * kPSlotBytes);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          umma_bf16_ss(tm + t * 128, umma_desc_k_sw128(q_addr + t * kPQBytes + (kk / 4) * 16384 + (kk % 4) * 32, 1024),
+                       umma_desc_k_sw128(k_addr + (kk / 4) * 16384 + (kk % 4) * 32, 1024), idesc_qk, kk != 0);
+        umma_commit(&bars.s_full[t]);
+        if (t == 1) umma_commit(&bars.kv_empty[sl]);
+      }
+      __syncwarp();
+    };
+    bool ok = mbar_wait_warp(&bars.q_full, 0, p.status) && mbar_wait_warp(&bars.kv_full[0], 0, p.status);
+    if (ok && ntiles > 0) {
+      tc_fence_after_sync();
+      qk(0, 0);
+      qk(1, 0);
+    }
+    for (int j = 0; j < ntiles && ok; ++j) {
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
-        if (j[t] >= ntiles) continue;
-        if (j[t] >= 0 && !pv[t]) {
-          const int sq = 2 * j[t] + 1, sl = sq % kPRing;
-          if (!ready(&bars.p_full[t], j[t] & 1) || !ready(&bars.kv_full[sl], (sq / kPRing) & 1)) continue;
-          tc_fence_after_sync();
-          const uint64_t vd = umma_desc_mn_sw128(smem_u32(sKV + sl * kPSlotBytes), 16384, 1024);
-          const bool both = j[1 - t] > j[t] || (j[1 - t] == j[t] && pv[1 - t]);                     // the other head had V(j)
-          if (elect_one()) {
+        const int sv = 2 * j + 1, sk = 2 * j + 2, sl = sv % kPRing;
+        if (t == 0 && !(ok = mbar_wait_warp(&bars.kv_full[sl], (sv / kPRing) & 1, p.status))) break;
+        if (!(ok = mbar_wait_warp(&bars.p_full[t], j & 1, p.status))) break;
+        tc_fence_after_sync();
+        const uint64_t vd = umma_desc_mn_sw128(smem_u32(sKV + sl * kPSlotBytes), 16384, 1024);
+        if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kPT / 16; ++kk)
-              umma_bf16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (j[t] | kk) != 0);
-            umma_commit(&bars.pv_done[t]);
-            if (both) umma_commit(&bars.kv_empty[sl]);
-          }
-          __syncwarp();
-          pv[t] = true;
-          if (j[t] == ntiles - 1) { j[t] = ntiles; --left; }
-          idle = false;
-        } else {
-          const int n = j[t] + 1, sq = 2 * n, sl = sq % kPRing;
-          if ((j[t] >= 0 && !ready(&bars.pv_done[t], j[t] & 1)) || !ready(&bars.kv_full[sl], (sq / kPRing) & 1)) continue;
-          tc_fence_after_sync();
-          const uint32_t q_addr = smem_u32(sQ + t * kPQBytes), k_addr = smem_u32(sKV + sl * kPSlotBytes);
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              umma_bf16_ss(tm + t * 128, umma_desc_k_sw128(q_addr + (kk / 4) * 16384 + (kk % 4) * 32, 1024),
-                           umma_desc_k_sw128(k_addr + (kk / 4) * 16384 + (kk % 4) * 32, 1024), idesc_qk, kk != 0);
-            umma_commit(&bars.s_full[t]);
-            if (j[1 - t] >= n) umma_commit(&bars.kv_empty[sl]);                                     // the other head had K(n)
-          }
-          __syncwarp();
-          j[t] = n;
-          pv[t] = false;
-          idle = false;
+          for (int kk = 0; kk < kPT / 16; ++kk)
+            umma_bf16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (j | kk) != 0);
+          if (t == 1) umma_commit(&bars.kv_empty[sl]);
+          if (j == ntiles - 1) umma_commit(&bars.pv_done[t]);
         }
-      }
-      if (!idle) { t0 = clock64(); spins = 0; }
-      else if (((++spins) & 0x3ff) == 0 && __any_sync(0xffffffffu, clock64() - t0 > kSpinLimitCycles)) {
-        if (p.status && lane == 0) atomicExch(p.status, (int)kErrMbarTimeout);
-        break;
+        __syncwarp();
+        if (j + 1 < ntiles) {
+          if (t == 0) {
+            if (!(ok = mbar_wait_warp(&bars.kv_full[sk % kPRing], (sk / kPRing) & 1, p.status))) break;
+            tc_fence_after_sync();
+          }
+          qk(t, j + 1);
+        }
       }
     }
   } else {
@@ -596,20 +586,26 @@ __global__ void __launch_bounds__(320, 1)
           tmem_st_32x32b_x16(o_addr + c * 16, rr);
         }
       }
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      // (two values an instruction: scale and offset, and the sums)
+      const uint64_t sc2 = pack_f32x2(sc, sc), off2 = pack_f32x2(-m_use, -m_use);
+      uint64_t sum2[2] = {0, 0};
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t pk[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
-          const float a = ex2_fast(fmaf(__uint_as_float(s[c * 64 + 2 * i]), sc, -m_use));
-          const float b = ex2_fast(fmaf(__uint_as_float(s[c * 64 + 2 * i + 1]), sc, -m_use));
-          sum[(2 * i) & 3] += a;
-          sum[(2 * i + 1) & 3] += b;
+          float a, b;
+          unpack_f32x2(fma_f32x2(pack_b32x2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), sc2, off2), a, b);
+          a = ex2_fast(a);
+          b = ex2_fast(b);
+          sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(a, b));
           pk[i] = pack_bf16x2(a, b);
         }
         tmem_st_32x32b_x32(s_addr + c * 32, pk);
       }
+      float sum[4];
+      unpack_f32x2(sum2[0], sum[0], sum[1]);
+      unpack_f32x2(sum2[1], sum[2], sum[3]);
       l = l * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       tmem_st_wait();
       tc_fence_before_sync();
@@ -618,7 +614,7 @@ __global__ void __launch_bounds__(320, 1)
     }
     // every P V before the last is complete (its successor's S has been seen)
     if (ok && ntiles > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars.pv_done[t], (ntiles - 1) & 1, p.status));
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars.pv_done[t], 0, p.status));
       if (ok) tc_fence_after_sync();
     }
     if (ok) {
