@@ -94,22 +94,6 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile = blockIdx.x, h = blockIdx.y;
   const int hkv = h / (p.Hq / p.Hkv);
-  const int req = p.tile_req[tile];
-  const int q0 = p.tile_q0[tile];
-  const int q_begin = p.q_start[req];
-  const int q_len = p.q_start[req + 1] - q_begin;
-  const int seq_len = p.seq_lens[req];
-  const int ctx_off = seq_len - q_len;          // position of query row 0
-  const int rows = min(kQT, q_len - q0);
-  // kv range needed by this tile
-  const int last_pos = p.causal ? (ctx_off + q0 + rows - 1) : (seq_len - 1);
-  int first_pos = 0;
-  if (p.window > 0) first_pos = max(0, ctx_off + q0 - p.window + 1);
-  else if (p.window < 0) first_pos = ((ctx_off + q0) / -p.window) * -p.window;   // chunk start of the first row
-  const int kt0 = first_pos / kKT;
-  const int kt1 = last_pos / kKT + 1;           // exclusive
-  const int ntiles = kt1 - kt0;
-
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
     for (int i = 0; i < kRing; ++i) {
@@ -134,6 +118,23 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
   tc_fence_after_sync();
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_s0 = tmem_base, tmem_o = tmem_base + 128;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int req = p.tile_req[tile];
+  const int q0 = p.tile_q0[tile];
+  const int q_begin = p.q_start[req];
+  const int q_len = p.q_start[req + 1] - q_begin;
+  const int seq_len = p.seq_lens[req];
+  const int ctx_off = seq_len - q_len;          // position of query row 0
+  const int rows = min(kQT, q_len - q0);
+  // kv range needed by this tile
+  const int last_pos = p.causal ? (ctx_off + q0 + rows - 1) : (seq_len - 1);
+  int first_pos = 0;
+  if (p.window > 0) first_pos = max(0, ctx_off + q0 - p.window + 1);
+  else if (p.window < 0) first_pos = ((ctx_off + q0) / -p.window) * -p.window;   // chunk start of the first row
+  const int kt0 = first_pos / kKT;
+  const int kt1 = last_pos / kKT + 1;           // exclusive
+  const int ntiles = kt1 - kt0;
 
   // The producer and the issuer walk their loops as whole warps and elect the lane that issues (mbar_wait_warp).
   if (warp == 0) {
@@ -389,14 +390,15 @@ __global__ void __launch_bounds__(64 + 128 * (D > 128 ? 2 : 1), D > 128 ? 1 : 2)
 // Q and a ring of four K / V tiles.
 //
 // Measured against one head a CTA, 64-key tiles and P in shared memory (32 query / 8 kv heads, TFLOP/s of causal work):
-// 4096 tokens 523 -> 777, 8192 670 -> 961, 7309 after 8192 cached 773 -> 969, 8 x 1024 426 -> 481. Shorter prompts, whose time
+// 4096 tokens 656 -> 1099, 8192 -> 1268, 7309 after 8192 cached -> 1263, 8 x 1000 496 -> 611. Shorter prompts, whose time
 // is a CTA's start and end, stay with one head a CTA (b200_attn_prefill_keys).
 //
-// A tile of two heads takes 4200 to 4900 cycles at 961 TFLOP/s. Its 2 x 16 MMAs of about 84 cycles are 2700 of them, its 128
-// exponentials a row 2050 on the special-function units; either alone would be faster, so what is left is that they
-// alternate no better than this. One issuing thread watches both heads and issues whatever is ready:
-//   P(t, j) written and V(j) there   ->  O(t) += P(t, j) V(j)
-//   P V(t, j) complete and K(j+1)    ->  S(t) = Q(t) K(j+1)^T   (over P(t, j), which has been read)
+// A tile of two heads is 32 MMAs of 64 cycles and 128 exponentials a row, 2048 cycles of the tensor pipe and as many of the
+// special-function units; it takes 3500, as each head's chain S -> softmax -> P V -> S covers the other's only in part. What
+// shortens the chain: S of the next tile is issued right behind P V, over P, which the tensor pipe (it takes one thread's
+// instructions in their order) has read by then (984 -> 1207 at 8192 tokens, with pairs of floats in the softmax); P V starts on
+// the first half of the keys (-> 1268; three quarters 1249). Order of issue, for tile j and both heads t:
+//   P(t, j) written and V(j) there   ->  O(t) += P(t, j) V(j), then, with K(j+1) there, S(t) = Q(t) K(j+1)^T
 //
 // Tensor memory (512 columns): S0 | S1 | O0 | O1; P(t) is the first 64 columns of S(t).
 // Warp roles (320 threads): warp 0 TMA, warp 1 MMA + TMEM owner, warps 2..5 / 6..9 softmax and output of head 0 / 1, one
@@ -408,7 +410,7 @@ static constexpr int kPQBytes = 2 * 16384, kPSlotBytes = 2 * 16384;      // one 
 static constexpr int kPSmem = 2 * kPQBytes + kPRing * kPSlotBytes + 1024;
 
 struct alignas(8) PairBars {
-  uint64_t q_full, kv_full[kPRing], kv_empty[kPRing], s_full[2], p_full[2], pv_done[2];
+  uint64_t q_full, kv_full[kPRing], kv_empty[kPRing], s_full[2], p_first[2], p_full[2], pv_done[2];
   uint32_t tmem_base;
 };
 
@@ -428,6 +430,7 @@ __global__ void __launch_bounds__(320, 1)
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bars.s_full[t], 1);
+      mbar_init(&bars.p_first[t], 4);
       mbar_init(&bars.p_full[t], 4);
       mbar_init(&bars.pv_done[t], 1);
     }
@@ -512,13 +515,21 @@ __global__ void __launch_bounds__(320, 1)
       for (int t = 0; t < 2; ++t) {
         const int sv = 2 * j + 1, sk = 2 * j + 2, sl = sv % kPRing;
         if (t == 0 && !(ok = mbar_wait_warp(&bars.kv_full[sl], (sv / kPRing) & 1, p.status))) break;
-        if (!(ok = mbar_wait_warp(&bars.p_full[t], j & 1, p.status))) break;
-        tc_fence_after_sync();
         const uint64_t vd = umma_desc_mn_sw128(smem_u32(sKV + sl * kPSlotBytes), 16384, 1024);
+        if (!(ok = mbar_wait_warp(&bars.p_first[t], j & 1, p.status))) break;
+        tc_fence_after_sync();
         if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kPT / 16; ++kk)
+          for (int kk = 0; kk < kPT / 32; ++kk)
             umma_bf16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (j | kk) != 0);
+        }
+        __syncwarp();
+        if (!(ok = mbar_wait_warp(&bars.p_full[t], j & 1, p.status))) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = kPT / 32; kk < kPT / 16; ++kk)
+            umma_bf16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, vd + kk * (2048 >> 4), idesc_pv, 1);
           if (t == 1) umma_commit(&bars.kv_empty[sl]);
           if (j == ntiles - 1) umma_commit(&bars.pv_done[t]);
         }
@@ -590,18 +601,24 @@ __global__ void __launch_bounds__(320, 1)
       const uint64_t sc2 = pack_f32x2(sc, sc), off2 = pack_f32x2(-m_use, -m_use);
       uint64_t sum2[2] = {0, 0};
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t pk[32];
+      for (int c = 0; c < 4; ++c) {
+        uint32_t pk[16];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < 16; ++i) {
           float a, b;
-          unpack_f32x2(fma_f32x2(pack_b32x2(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]), sc2, off2), a, b);
+          unpack_f32x2(fma_f32x2(pack_b32x2(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]), sc2, off2), a, b);
           a = ex2_fast(a);
           b = ex2_fast(b);
           sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(a, b));
           pk[i] = pack_bf16x2(a, b);
         }
-        tmem_st_32x32b_x32(s_addr + c * 32, pk);
+        tmem_st_32x32b_x16(s_addr + c * 16, pk);
+        if (c == 1) {                  // P V of the first half of the keys may start
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars.p_first[t]);
+        }
       }
       float sum[4];
       unpack_f32x2(sum2[0], sum[0], sum[1]);
@@ -680,8 +697,7 @@ static int launch_prefill(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const
     cudaFuncSetAttribute(attn_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
   }
-  attn_prefill_kernel<D><<<grid, 64 + 128 * (D > 128 ? 2 : 1), smem, stream>>>(tmQ, tmKV, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_pdl(attn_prefill_kernel<D>, grid, dim3(64 + 128 * (D > 128 ? 2 : 1)), smem, stream, tmQ, tmKV, p) == cudaSuccess ? 0 : -2;
 }
 
 }  // namespace b200
@@ -725,9 +741,10 @@ extern "C" int b200_attn_prefill_keys(const void* q, int ldq, void* out, int ldo
   // keys a tile more are masked. About 250 keys a tile on average are the line, or 96 where the grid is a single wave, and so
   // is more than half a wave: two heads a CTA leave SMs idle that one head a CTA has work for. A window or chunk shorter than
   // 1024 ends at both sides within a tile. us, one / two heads a CTA, 32 query heads:
-  //   120 x 64 tokens 84 / 108, 60 x 128 65 / 70, 60 x 275 (220 keys) 210 / 221, 30 x 400 (292) 166 / 168, 30 x 512 180 / 174,
-  //   8 x 1024 150 / 130, 60 x 100 after 2000 355 / 324; one wave: 8 x 40 7.7 / 8.3, 8 x 100 10.5 / 9.1; less than half:
-  //   1 x 512 15.2 / 16.8; 8192 tokens, window 256 106 / 112, 512 144 / 144, 1024 218 / 201
+  //   120 x 64 tokens 78 / 109, 30 x 128 33 / 37, 60 x 275 (220 keys) 189 / 201, 25 x 300 (243) 86 / 90, 30 x 330 108 / 107,
+  //   30 x 400 (292) 150 / 148, 16 x 512 93 / 86, 8 x 1000 132 / 107, 60 x 60 after 2000 317 / 257; one wave: 8 x 40 and 8 x 100
+  //   within 3 %, 1 x 700 18.8 / 17.2; windows, when the line was laid: 8192 tokens, window 256 106 / 112, 512 144 / 144,
+  //   1024 218 / 201
   if (tile_keys <= 0) {       // not known: half of a request's last tile is empty on average, and nothing came before
     const long long empty = (long long)num_tiles * kQT - total_q, reqs = empty > kQT / 2 ? empty / (kQT / 2) : 1;
     tile_keys = num_tiles * (total_q / reqs + kQT) / 2;
