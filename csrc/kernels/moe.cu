@@ -535,6 +535,181 @@ __global__ void __launch_bounds__(192, 2)
   if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
 }
 
+// Experts of many rows: CTA pairs as in gemm_bf16_pair_kernel, a tile of 256 sorted rows (128 a CTA) x 256 weight rows, gated 128
+// gate rows (staged by the first CTA) and the 128 up rows of the same outputs (by the second). Persistent: a pair takes the tiles
+// pair, pair + pairs, ... of the device-side list of chunks, weight tiles inside a chunk; two accumulators let the epilogue of a tile run
+// under the products of the next, which with a K of 12 k-blocks takes about as long. A chunk's missing rows up to 256
+// are multiplied and not stored.
+static constexpr int kPStages = 6, kPStage = 32 * 1024, kPMostChunks = 1024, kPGroup = 16;
+struct GroupedPairChunk {
+  int expert, row0, rows, first, group;       // first: of the group that the chunk belongs to, group: its chunks
+};
+struct GroupedPairParams {
+  int N, K, E, max_chunks, tiles;       // tiles: of 256 weight rows (gated: 128 outputs)
+  int act_fuse, act;
+  __nv_bfloat16* out;
+  const int32_t *chunk_expert, *chunk_row0, *chunk_n, *meta;
+  int* status;
+};
+struct alignas(8) GroupedPairBars {
+  uint64_t full[kPStages], empty[kPStages], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+};
+
+__global__ void __launch_bounds__(192, 1)
+    moe_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, GroupedPairParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ GroupedPairBars bars;
+  GroupedPairChunk* table = reinterpret_cast<GroupedPairChunk*>(smem + kPStages * kPStage);
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int nkb = (p.K + kGBK - 1) / kGBK, half_n = p.N >> 1;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kPStages; ++s) { mbar_init(&bars.full[s], 1); mbar_init(&bars.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&bars.acc_full[b], 1); mbar_init(&bars.acc_empty[b], 8); }
+    mbar_fence_init();
+  }
+  if (warp == 1) { tmem_alloc_pair(&bars.tmem_base, 512); tmem_relinquish_pair(); }
+  pdl_wait();
+  pdl_launch_dependents();
+  const int chunks = min(p.meta[3 * p.E + 1], p.max_chunks);
+  // Up to kPGroup chunks of an expert take a weight tile one after the other, so that side by side pairs share it in L2 (8 experts
+  // of 14336, width 4096, 4096 tokens: a chunk at a time 1779 us)
+  for (int i = threadIdx.x; i < chunks; i += 192) {
+    const int e = p.chunk_expert[i];
+    int first = i, end = i + 1;
+    while (first > 0 && p.chunk_expert[first - 1] == e) --first;
+    first += (i - first) / kPGroup * kPGroup;
+    while (end < chunks && end < first + kPGroup && p.chunk_expert[end] == e) ++end;
+    table[i] = GroupedPairChunk{e, p.chunk_row0[i], p.chunk_n[i], first, end - first};
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();            // the peer's barriers exist before anything signals them
+  tc_fence_after_sync();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars.tmem_base, 0);
+  const int total = chunks * p.tiles;
+  const auto tile_of = [&](int t, int& tn) {
+    const GroupedPairChunk& g = table[t / p.tiles];
+    const int at = t - g.first * p.tiles;
+    tn = at / g.group;
+    return table[g.first + at - tn * g.group];
+  };
+
+  if (warp == 0) {
+    if (lane == 0) { tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX); }
+    int s = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int t = pair; t < total && ok; t += pairs) {
+      int tn;
+      const GroupedPairChunk c = tile_of(t, tn);
+      const int x_row = c.row0 + rank * 128;
+      const int w_row = p.act_fuse ? rank * half_n + tn * 128 : tn * 256 + rank * 128;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!(ok = mbar_wait_warp(&bars.empty[s], ph, p.status))) break;
+        uint8_t* dst = smem + s * kPStage;
+        const uint32_t leader_bar = mapa_u32(smem_u32(&bars.full[s]), 0);
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(&bars.full[s], 2 * kPStage);
+          tma_load_2d_pair(dst, &tmX, leader_bar, kb * kGBK, x_row);
+          tma_load_3d_pair(dst + kPStage / 2, &tmW, leader_bar, kb * kGBK, w_row, c.expert);
+        }
+        __syncwarp();
+        if (++s == kPStages) { s = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      constexpr uint32_t idesc = umma_idesc_bf16(256, 256);
+      int s = 0;
+      uint32_t ph = 0, n = 0;
+      bool ok = true;
+      for (int t = pair; t < total && ok; t += pairs, ++n) {
+        const int buf = n & 1;
+        if (!(ok = mbar_wait_warp(&bars.acc_empty[buf], ((n >> 1) & 1) ^ 1, p.status))) break;
+        tc_fence_after_sync();
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(ok = mbar_wait_warp(&bars.full[s], ph, p.status))) break;
+          tc_fence_after_sync();
+          const uint32_t a = smem_u32(smem + s * kPStage);
+          const uint64_t adesc = umma_desc_k_sw128(a, 1024), bdesc = umma_desc_k_sw128(a + kPStage / 2, 1024);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16_ss_pair(tmem + buf * 256, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0);
+            umma_commit_pair(&bars.empty[s], 3);
+            if (kb == nkb - 1) umma_commit_pair(&bars.acc_full[buf], 3);
+          }
+          __syncwarp();
+          if (++s == kPStages) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else {
+    const int quarter = warp & 3, r = rank * 128 + quarter * 32 + lane;
+    uint32_t n = 0;
+    for (int t = pair; t < total; t += pairs, ++n) {
+      const int buf = n & 1;
+      int tn;
+      const GroupedPairChunk c = tile_of(t, tn);
+      const bool in = r < c.rows;
+      const size_t row = (size_t)(c.row0 + r);
+      if (!mbar_wait_warp(&bars.acc_full[buf], (n >> 1) & 1, p.status)) break;
+      tc_fence_after_sync();
+      const uint32_t acc = tmem + buf * 256 + ((uint32_t)(quarter * 32) << 16);
+      if (p.act_fuse) {
+        __nv_bfloat16* o = p.out + row * half_n + tn * 128;
+        const int kind = p.act_fuse - 1;
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          uint32_t g[32], u[32];
+          tmem_ld_32x32b_x32(acc + q * 32, g);
+          tmem_ld_32x32b_x32(acc + 128 + q * 32, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            if (!in || tn * 128 + q * 32 + i >= half_n) continue;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float gg = __bfloat162float(__float2bfloat16(__uint_as_float(g[i + j])));
+              v[j] = act_of(gg, kind) * __bfloat162float(__float2bfloat16(__uint_as_float(u[i + j])));
+            }
+            *reinterpret_cast<uint4*>(o + q * 32 + i) =
+                make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+          }
+        }
+      } else {
+        __nv_bfloat16* o = p.out + row * p.N + tn * 256;
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(acc + q * 32, v);
+          tmem_ld_wait();
+          float f[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
+          act_epilogue<true>(f, p.act);
+#pragma unroll
+          for (int i = 0; i < 32; i += 8)
+            if (in && tn * 256 + q * 32 + i < p.N)
+              *reinterpret_cast<uint4*>(o + q * 32 + i) = make_uint4(pack_bf16x2(f[i], f[i + 1]), pack_bf16x2(f[i + 2], f[i + 3]),
+                                                                     pack_bf16x2(f[i + 4], f[i + 5]), pack_bf16x2(f[i + 6], f[i + 7]));
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&bars.acc_empty[buf]), 0));
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();            // neither CTA frees while the other still reads its accumulators
+  tc_fence_after_sync();
+  if (warp == 1) tmem_dealloc_pair(tmem, 512);
+}
+
 // ---------------------------------------------------------------------------------- combine
 // out[t, :] = sum_j w[t, j] * y[pair_pos[t, j], :] (+ shared[t, :] * shared_scale[t]) ;
 // pairs routed to experts of other ranks (pair_pos < 0) are skipped. fp32 accumulation in
@@ -728,6 +903,34 @@ static int moe_grouped_gemm_impl(const void* xs, int max_rows, const void* W, in
     g.chunk_n = (const int32_t*)chunk_n; g.num_chunks = (const int32_t*)meta + 3 * E + 1;
     g.max_rows = max_rows; g.max_chunks = max_chunks; g.E = E; g.N = N; g.K = K; g.gated = act_fuse; g.act = act;
     return launch_experts_cluster(g, stream);
+  }
+  // Experts of many rows go to CTA pairs, which read the weights once for 256 rows and multiply at twice the rate, padded to 256
+  // rows an expert: from 160 rows on average on, plain from 128. us, the kernel below / pairs, gated and plain: 128 experts of
+  // 768, width 2048, 68 rows 152 / 181 and 99 / 94, 128 rows 183 / 186 and 117 / 106, 187 rows 228 / 189 and 131 / 110, 512 rows
+  // 473 / 407 and 292 / 247; 64 of 1408, 768 rows 619 / 487 and 323 / 241; 8 of 1792, width 4096, 150 rows 68 / 72 and 37 / 34,
+  // 1024 rows 268 / 181 and 129 / 96; 8 of 14336, 300 rows 756 / 649 and 363 / 347, 1024 rows 2143 / 1443 and 958 / 766;
+  // 32 of 2880, 75 rows 209 / 248 and 133 / 142.
+  if (act_fuse != 4 && max_rows >= (act_fuse ? 160 : 128) * (long long)E && max_chunks <= kPMostChunks &&
+      !(reinterpret_cast<uintptr_t>(out) & 15)) {
+    GroupedPairParams q{};
+    q.N = N; q.K = K; q.E = E; q.max_chunks = max_chunks; q.tiles = act_fuse ? (N / 2 + 127) / 128 : (N + 255) / 256;
+    q.act_fuse = act_fuse; q.act = act; q.out = (bf16*)out;
+    q.chunk_expert = (const int32_t*)chunk_expert; q.chunk_row0 = (const int32_t*)chunk_row0;
+    q.chunk_n = (const int32_t*)chunk_n; q.meta = (const int32_t*)meta; q.status = device_status_word();
+    CUtensorMap tW, tX;
+    if (!encode_tmap_3d(&tW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)N, (uint64_t)E, (uint64_t)K * 2,
+                        (uint64_t)N * K * 2, kGBK, 128, 1, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_tmap_2d(&tX, xs, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)max_rows + 256, (uint64_t)K, (uint64_t)K, 128, kGBK,
+                        CU_TENSOR_MAP_SWIZZLE_128B))
+      return -3;
+    const size_t bytes = (size_t)kPStages * kPStage + (size_t)max_chunks * sizeof(GroupedPairChunk) + 1024;
+    static PerDeviceOnce once;
+    if (once.first())
+      cudaFuncSetAttribute(moe_grouped_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kPStages * kPStage + kPMostChunks * (int)sizeof(GroupedPairChunk) + 1024);
+    const long long tiles = (long long)max_chunks * q.tiles;
+    const int pairs = (int)(tiles < b200_num_sms() / 2 ? tiles : b200_num_sms() / 2);
+    return launch_cluster_pdl(moe_grouped_pair_kernel, dim3(2 * pairs), 2, 192, bytes, stream, tW, tX, q) == cudaSuccess ? 0 : -2;
   }
   // Gated: 128 rows a CTA and two CTAs an SM, or 256 rows, a CTA with three stages of 64 KB alone on its SM. The smaller CTA
   // hides its epilogue behind its neighbour, but reads the weights once for every 128 rows and has two stages of 48 KB.

@@ -227,3 +227,40 @@ def test_gather_of_few_and_of_many_rows(T):
     M.moe_gather(x, ws, 8, 2 * T)
     pos = ws.pair_pos.view(T, 2).long()
     assert torch.equal(ws.xs[pos[:, 0]], x) and torch.equal(ws.xs[pos[:, 1]], x) and bool((ws.xs[2 * T:] == 0).all())
+
+
+@pytest.mark.parametrize("T,E,H,I,skew", [(700, 8, 72, 136, False), (645, 8, 200, 1000, True), (2600, 4, 64, 128, True),
+                                          (4500, 2, 128, 264, False), (257, 2, 2048, 768, False)])
+def test_grouped_gemm_of_many_rows_an_expert(T, E, H, I, skew):
+    """CTA pairs: ragged weight tiles and k-blocks, chunks of 1 to 256 rows, experts without rows and with more chunks than a group
+    (``skew``: every token's second expert is the last one). Each of the two products rounds its values to bf16 (2^-8), the
+    gated one three times."""
+    torch.manual_seed(T + I)
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    wgu = (torch.randn(E, 2 * I, H, device=DEV) * H ** -0.5).to(torch.bfloat16)
+    wd = (torch.randn(E, H, I, device=DEV) * I ** -0.5).to(torch.bfloat16)
+    first = torch.randint(0, E - 1, (T,), device=DEV)
+    ids = torch.stack([first, torch.full_like(first, E - 1) if skew else (first + 1) % E], 1).int()
+    if skew:
+        ids[:, 0][ids[:, 0] == 1] = 0                           # (an expert without rows)
+    ws = M.MoeWorkspace(torch.device(DEV), T, 2, E, H, I)
+    M.moe_sort(ids, 0, E, ws)
+    P = 2 * T
+    assert P >= 160 * E
+    M.moe_gather(x, ws, E, P)
+    ws.act.fill_(7.0)
+    ws.y.fill_(7.0)
+    M.grouped_gemm_gated(ws.xs, wgu, ws.act, ws, P, kind=0)
+    M.grouped_gemm(ws.act, wd, ws.y, ws, P)
+    assert bool((ws.act[P:] == 7.0).all()) and bool((ws.y[P:] == 7.0).all())        # nothing beyond the sorted rows
+    pos = ws.pair_pos.view(T, 2).long()
+    for e in range(E):
+        at, j = (ids == e).nonzero(as_tuple=True)
+        if not at.numel():
+            continue
+        g, u = (x[at].float() @ wgu[e, h * I:(h + 1) * I].float().t() for h in range(2))
+        act, got = torch.nn.functional.silu(g) * u, ws.act[pos[at, j]].float()
+        assert ((got - act).norm() / act.norm()).item() < 3 * 2.0 ** -8
+        y = got @ wd[e].float().t()
+        assert ((ws.y[pos[at, j]].float() - y).norm() / y.norm()).item() < 2.0 ** -8
+    assert ops.read_status() == 0
