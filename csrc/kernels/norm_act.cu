@@ -30,55 +30,100 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return t;
 }
 
+// A row's norm: V vectors a thread (0: as many as it takes, through shared memory), all of whose loads - the row, the residual, the
+// weights - are on their way before the first is used. Few rows are bound by such round trips to L2, many by memory. us, chained, against a
+// loop over the vectors: 13 rows of 4096 2.4 -> 1.8, of 7168 3.4 -> 2.2; 8192 rows of 2048 23.9 -> 19.0 (7.1 TB/s), of 4096 44.0 -> 40.6.
+__device__ __forceinline__ uint4 add_bf16x8(const uint4& x, const uint4& r) {
+  const uint32_t p[4] = {x.x, x.y, x.z, x.w}, q[4] = {r.x, r.y, r.z, r.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 a = unpack_bf16x2(p[j]), b = unpack_bf16x2(q[j]);
+    o[j] = pack_bf16x2(a.x + b.x, a.y + b.y);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ float add_squares(float ss, const uint4& v) {
+  const uint32_t p[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16x2(p[j]);
+    ss += f.x * f.x + f.y * f.y;
+  }
+  return ss;
+}
+__device__ __forceinline__ uint4 scale_bf16x8(const uint4& v, float inv, const uint4& w, float g) {
+  const uint32_t p[4] = {v.x, v.y, v.z, v.w}, q[4] = {w.x, w.y, w.z, w.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 a = unpack_bf16x2(p[j]), b = unpack_bf16x2(q[j]);
+    o[j] = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+// RMSNorm of row t; every normed vector i of the calling thread goes to put(i, value).
+template <int V, typename Put>
+__device__ __forceinline__ void norm_row(const uint4* __restrict__ xr, uint4* rr, const uint4* __restrict__ wr, uint4* row_cache, float* red,
+                                         int nv, float width, float eps, float g, Put&& put) {
+  float ss = 0.f;
+  if constexpr (V > 0) {
+    uint4 v[V], r[V], w[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      if (i < nv) {
+        v[j] = xr[i];
+        if (rr) r[j] = rr[i];
+        w[j] = wr[i];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      if (i < nv) {
+        if (rr) rr[i] = v[j] = add_bf16x8(v[j], r[j]);
+        ss = add_squares(ss, v[j]);
+      }
+    }
+    const float inv = rsqrtf(block_sum(ss, red) / width + eps);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      if (i < nv) put(i, scale_bf16x8(v[j], inv, w[j], g));
+    }
+  } else {
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+      uint4 v = xr[i];
+      if (rr) rr[i] = v = add_bf16x8(v, rr[i]);
+      row_cache[i] = v;
+      ss = add_squares(ss, v);
+    }
+    const float inv = rsqrtf(block_sum(ss, red) / width + eps);
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) put(i, scale_bf16x8(row_cache[i], inv, wr[i], g));
+  }
+}
+static inline int norm_vectors(int width, int threads) {
+  const int v = (width / 8 + threads - 1) / threads;
+  return v <= 2 ? v : v <= 4 ? 4 : 0;
+}
+
 // x: [T, H] bf16 (row stride ldx). If residual != nullptr: residual += x (bf16-rounded) and
 // the norm is taken over the updated residual. out may alias x.
+template <int V>
 __global__ void __launch_bounds__(256)
-    rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, int ldx, __nv_bfloat16* residual,
+    rmsnorm_kernel(const __nv_bfloat16* x, int ldx, __nv_bfloat16* residual,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* out, int ldo, int H,
                    float eps, int gemma) {
   __shared__ float red[32];
-  extern __shared__ uint4 row_cache[];  // H/8 vectors
+  extern __shared__ uint4 row_cache[];  // (V = 0) H/8 vectors
   pdl_wait();                 // predecessor grid complete, its writes visible
   pdl_launch_dependents();    // the successor may become resident (it waits the same way)
   const int t = blockIdx.x;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)t * ldx);
-  uint4* rr = residual ? reinterpret_cast<uint4*>(residual + (size_t)t * H) : nullptr;
-  const int nv = H >> 3;
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    uint4 v = xr[i];
-    if (rr) {
-      uint4 r = rr[i];
-      float2 a, b;
-      a = unpack_bf16x2(v.x); b = unpack_bf16x2(r.x); v.x = pack_bf16x2(a.x + b.x, a.y + b.y);
-      a = unpack_bf16x2(v.y); b = unpack_bf16x2(r.y); v.y = pack_bf16x2(a.x + b.x, a.y + b.y);
-      a = unpack_bf16x2(v.z); b = unpack_bf16x2(r.z); v.z = pack_bf16x2(a.x + b.x, a.y + b.y);
-      a = unpack_bf16x2(v.w); b = unpack_bf16x2(r.w); v.w = pack_bf16x2(a.x + b.x, a.y + b.y);
-      rr[i] = v;
-    }
-    row_cache[i] = v;
-    float2 f;
-    f = unpack_bf16x2(v.x); ss += f.x * f.x + f.y * f.y;
-    f = unpack_bf16x2(v.y); ss += f.x * f.x + f.y * f.y;
-    f = unpack_bf16x2(v.z); ss += f.x * f.x + f.y * f.y;
-    f = unpack_bf16x2(v.w); ss += f.x * f.x + f.y * f.y;
-  }
-  ss = block_sum(ss, red);
-  const float inv = rsqrtf(ss / (float)H + eps);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
   uint4* orow = reinterpret_cast<uint4*>(out + (size_t)t * ldo);
-  const float g = gemma ? 1.f : 0.f;
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-    uint4 v = row_cache[i];
-    uint4 wv = wr[i];
-    uint4 o;
-    float2 a, b;
-    a = unpack_bf16x2(v.x); b = unpack_bf16x2(wv.x); o.x = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-    a = unpack_bf16x2(v.y); b = unpack_bf16x2(wv.y); o.y = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-    a = unpack_bf16x2(v.z); b = unpack_bf16x2(wv.z); o.z = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-    a = unpack_bf16x2(v.w); b = unpack_bf16x2(wv.w); o.w = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-    orow[i] = o;
-  }
+  norm_row<V>(reinterpret_cast<const uint4*>(x + (size_t)t * ldx),
+              residual ? reinterpret_cast<uint4*>(residual + (size_t)t * H) : nullptr, reinterpret_cast<const uint4*>(w), row_cache, red,
+              H >> 3, (float)H, eps, gemma ? 1.f : 0.f, [&](int i, const uint4& o) { orow[i] = o; });
 }
 
 // LayerNorm with affine weight and optional bias; scalar loop (any H).
@@ -142,7 +187,7 @@ __global__ void __launch_bounds__(256)
 // The row (bf16) stays in shared memory between the producer and the quantisation. One kernel per mode and activation,
 // packed maxima and conversions: bound by instructions, then by memory (8192 rows, us: plain 4096 31.0 -> 21.9, 4.6 TB/s;
 // act 14336 152 -> 146, its exponential and division).
-template <int MODE, int KIND>
+template <int MODE, int KIND, int V = 0>
 __global__ void __launch_bounds__(MODE == 1 ? 256 : 1024)
     rowquant_fp8_kernel(const __nv_bfloat16* __restrict__ x, long ldx, __nv_bfloat16* residual,
                         const __nv_bfloat16* __restrict__ w, float eps, int gemma, int interleaved,
@@ -161,43 +206,11 @@ __global__ void __launch_bounds__(MODE == 1 ? 256 : 1024)
     for (int j = 0; j < 4; ++j) amax2 = __hmax2(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w4[j])));
   };
   if constexpr (MODE == 1) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + t * ldx);
-    uint4* rr = residual ? reinterpret_cast<uint4*>(residual + t * (long)K) : nullptr;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      uint4 v = xr[i];
-      if (rr) {
-        uint4 r = rr[i];
-        float2 a, b;
-        a = unpack_bf16x2(v.x); b = unpack_bf16x2(r.x); v.x = pack_bf16x2(a.x + b.x, a.y + b.y);
-        a = unpack_bf16x2(v.y); b = unpack_bf16x2(r.y); v.y = pack_bf16x2(a.x + b.x, a.y + b.y);
-        a = unpack_bf16x2(v.z); b = unpack_bf16x2(r.z); v.z = pack_bf16x2(a.x + b.x, a.y + b.y);
-        a = unpack_bf16x2(v.w); b = unpack_bf16x2(r.w); v.w = pack_bf16x2(a.x + b.x, a.y + b.y);
-        rr[i] = v;
-      }
-      row_cache[i] = v;
-      float2 f;
-      f = unpack_bf16x2(v.x); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(v.y); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(v.z); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(v.w); ss += f.x * f.x + f.y * f.y;
-    }
-    ss = block_sum(ss, red);
-    const float inv = rsqrtf(ss / (float)K + eps);
-    const uint4* wr = reinterpret_cast<const uint4*>(w);
-    const float g = gemma ? 1.f : 0.f;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      const uint4 v = row_cache[i];
-      const uint4 wv = wr[i];
-      uint4 o;
-      float2 a, b;
-      a = unpack_bf16x2(v.x); b = unpack_bf16x2(wv.x); o.x = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-      a = unpack_bf16x2(v.y); b = unpack_bf16x2(wv.y); o.y = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-      a = unpack_bf16x2(v.z); b = unpack_bf16x2(wv.z); o.z = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-      a = unpack_bf16x2(v.w); b = unpack_bf16x2(wv.w); o.w = pack_bf16x2(a.x * inv * (b.x + g), a.y * inv * (b.y + g));
-      row_cache[i] = o;
-      vec_amax(o);
-    }
+    norm_row<V>(reinterpret_cast<const uint4*>(x + t * ldx), residual ? reinterpret_cast<uint4*>(residual + t * (long)K) : nullptr,
+                reinterpret_cast<const uint4*>(w), row_cache, red, nv, (float)K, eps, gemma ? 1.f : 0.f, [&](int i, const uint4& o) {
+                  row_cache[i] = o;
+                  vec_amax(o);
+                });
   } else if constexpr (MODE == 2) {
     const bool il = interleaved != 0;
 #pragma unroll 2
@@ -363,7 +376,9 @@ int b200_rmsnorm(const void* x, int ldx, void* residual, const void* w, void* ou
   if ((H & 7) || (ldx & 7) || (ldo & 7) || H > 32768) return -1;
   int threads = H / 8 >= 256 ? 256 : ((H / 8 + 31) / 32) * 32;
   if (threads < 32) threads = 32;
-  return launch_pdl(rmsnorm_kernel, dim3(T), dim3(threads), (size_t)H * 2, stream, (const bf16*)x, ldx,
+  const int v = norm_vectors(H, threads);
+  auto kernel = v == 1 ? rmsnorm_kernel<1> : v == 2 ? rmsnorm_kernel<2> : v == 4 ? rmsnorm_kernel<4> : rmsnorm_kernel<0>;
+  return launch_pdl(kernel, dim3(T), dim3(threads), v ? 0 : (size_t)H * 2, stream, (const bf16*)x, ldx,
                     (bf16*)residual, (const bf16*)w, (bf16*)out, ldo, H, eps, gemma) == cudaSuccess ? 0 : -2;
 }
 
@@ -383,11 +398,14 @@ int b200_quant_fp8_rowwise(const void* x, long ldx, void* residual, const void* 
   int threads = K / 8 >= most ? most : ((K / 8 + 31) / 32) * 32;
   if (threads < 32) threads = 32;
   const int kind = kind_flags & 0xff;
-  auto kernel = mode == 0 ? rowquant_fp8_kernel<0, 0> : mode == 1 ? rowquant_fp8_kernel<1, 0>
+  const int v = norm_vectors(K, threads);
+  auto kernel = mode == 0 ? rowquant_fp8_kernel<0, 0>
+              : mode == 1 ? (v == 1 ? rowquant_fp8_kernel<1, 0, 1> : v == 2 ? rowquant_fp8_kernel<1, 0, 2> : v == 4 ? rowquant_fp8_kernel<1, 0, 4>
+                                                                                                         : rowquant_fp8_kernel<1, 0, 0>)
               : kind == kSilu ? rowquant_fp8_kernel<2, kSilu> : kind == kGeluTanh ? rowquant_fp8_kernel<2, kGeluTanh>
                                                                                   : rowquant_fp8_kernel<2, kGeluErf>;
-  static PerDeviceOnce attr_once[5];
-  if (attr_once[mode < 2 ? mode : kind == kSilu ? 2 : kind == kGeluTanh ? 3 : 4].first())
+  static PerDeviceOnce attr_once[9];
+  if (attr_once[mode == 0 ? 0 : mode == 1 ? 1 + v : kind == kSilu ? 6 : kind == kGeluTanh ? 7 : 8].first())
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 2);
   return launch_pdl(kernel, dim3(T), dim3(threads), (size_t)K * 2, stream, (const bf16*)x, ldx, (bf16*)residual,
                     (const bf16*)norm_w, eps, gemma, (kind_flags >> 8) & 1, (uint8_t*)out, ldo, (float*)scales, K) == cudaSuccess
