@@ -24,6 +24,7 @@
 // Replaces the library GEMM calls of the reference (src/vt/cuda/cuda_matmul.cu:284-355 "MatmulBT", :219-274) for
 // decode-sized batches.
 #include "api.h"
+#include "rope.cuh"
 #include "sm100.cuh"
 
 namespace b200 {
@@ -63,6 +64,7 @@ struct ClusterParams {
   // fp8: the sums times a_scale (of the tensor, or per row) and w_scale (of the tensor, or per output column)
   const float *a_scale, *w_scale;
   int a_per_row, w_per_col;
+  RopeOut rope;              // (ROPE) a tile is a head
   int* status;
 };
 
@@ -78,9 +80,8 @@ __device__ __forceinline__ float4 gated4(const float4& g, const float4& u, int k
   return make_float4(act_of(rounded(g.x), kind) * rounded(u.x), act_of(rounded(g.y), kind) * rounded(u.y),
                      act_of(rounded(g.z), kind) * rounded(u.z), act_of(rounded(g.w), kind) * rounded(u.w));
 }
-// col: first of the lane's four columns of the output, m: row of the output
-__device__ __forceinline__ void finish_row(const ClusterParams& p, float4 a, int m, int col) {
-  if (col >= (p.gated ? p.N >> 1 : p.N)) return;                     // (a multiple of 8)
+// The sums' scales, bias, residual and activation. col: first of the lane's four columns of the output, m: row of the output
+__device__ __forceinline__ float4 finished(const ClusterParams& p, float4 a, int m, int col) {
   if (p.a_scale) {
     const float sa = p.a_scale[p.a_per_row ? m : 0];
     const float* sw = p.w_scale + (p.w_per_col ? col : 0);
@@ -101,16 +102,65 @@ __device__ __forceinline__ void finish_row(const ClusterParams& p, float4 a, int
     a.x = act_epilogue<true>(a.x, p.act); a.y = act_epilogue<true>(a.y, p.act);
     a.z = act_epilogue<true>(a.z, p.act); a.w = act_epilogue<true>(a.w, p.act);
   }
+  return a;
+}
+__device__ __forceinline__ void finish_row(const ClusterParams& p, float4 a, int m, int col) {
+  if (col >= (p.gated ? p.N >> 1 : p.N)) return;                     // (a multiple of 8)
+  a = finished(p, a, m, col);
   const size_t at = blockIdx.z * p.batch_out + (size_t)m * p.ldo + col;
   if (p.out_f32)
     *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at) = a;
   else
     *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + at) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
 }
+
+// With a rotation: what a warp needs of its next row, fetched ahead of it.
+struct RopeRow {
+  float4 c, s;
+  int64_t slot;
+};
+__device__ __forceinline__ RopeRow rope_row(const RopeOut& r, int m, int head, int lane) {
+  RopeRow o;
+  o.slot = head >= r.Hq ? r.slot_mapping[m] : -1;
+  if (head < r.Hq + r.Hkv) {
+    const float* cs = r.cos_sin + (size_t)r.positions[m] * 128 + (lane & 15) * 4;
+    o.c = *reinterpret_cast<const float4*>(cs);
+    o.s = *reinterpret_cast<const float4*>(cs + 64);
+  }
+  return o;
+}
+// The row's head as the product would have stored it, rounded, then b200_rope_kv's arithmetic.
+__device__ __forceinline__ void finish_head(const ClusterParams& p, float4 a, int m, int head, const RopeRow& row, int lane) {
+  const RopeOut& r = p.rope;
+  a = finished(p, a, m, head * 128 + lane * 4);
+  uint2 o = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+  const int v0 = r.Hq + r.Hkv;
+  if (head < v0) {
+    const float2 lo = unpack_bf16x2(o.x), hi = unpack_bf16x2(o.y);
+    const float x[4] = {lo.x, lo.y, hi.x, hi.y};
+    o = rope_head(x, row.c, row.s, head < r.Hq ? r.q_norm : r.k_norm, r.eps, r.gemma, lane);
+  }
+  if (head >= r.Hq) {
+    const RopeCacheSlot cache = rope_cache_slot(row.slot, r.kv_cache, r.block_size, r.Hkv);
+    __nv_bfloat16* dst = head < v0 ? cache.k : cache.v;
+    if (dst) *reinterpret_cast<uint2*>(dst + (head < v0 ? head - r.Hq : head - v0) * 128 + lane * 4) = o;
+  }
+  *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldo + head * 128 + lane * 4) = o;
+}
+
 // Batch rows rank, rank + ranks, ... of the pass, dealt to the six warps, four columns a lane.
-template <int S>
+template <int S, bool ROPE>
 __device__ __forceinline__ void reduce_rows(const ClusterParams& p, uint32_t partial, int rank, int ranks, int rows, int row0,
-                                            int col, int warp, int lane) {
+                                            int col, int warp, int lane, RopeRow next) {
+  if constexpr (ROPE) {                    // (one pass, row0 = 0)
+    const int head = col >> 7;
+    for (int m = rank + warp * ranks; m < rows; m += 6 * ranks) {
+      const RopeRow row = next;
+      if (m + 6 * ranks < rows) next = rope_row(p.rope, m + 6 * ranks, head, lane);
+      finish_head(p, sum_of<S>(partial + (uint32_t)m * (kRows * 4) + lane * 16, 0), m, head, row, lane);
+    }
+    return;
+  }
   for (int m = rank + warp * ranks; m < rows; m += 6 * ranks) {
     const uint32_t addr = partial + (uint32_t)m * (kRows * 4) + lane * 16;
     float4 x = sum_of<S>(addr, 0);
@@ -119,7 +169,7 @@ __device__ __forceinline__ void reduce_rows(const ClusterParams& p, uint32_t par
   }
 }
 
-template <ClusterKind KIND>
+template <ClusterKind KIND, bool ROPE = false>
 __global__ void __launch_bounds__(kThreads, 2)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ BatchMaps<KIND> tmA, ClusterParams p,
                         uint32_t tmem_cols) {
@@ -186,6 +236,11 @@ __global__ void __launch_bounds__(kThreads, 2)
       stages = min(kRingStages, p.ring_bytes / stage_bytes);
     }
   }
+
+  // (the warps that load and multiply fetch theirs when they are through: it is a chain of two loads)
+  RopeRow rope{};
+  const bool rotates = ROPE && rank + warp * ranks < total;
+  if (rotates && warp >= 2) rope = rope_row(p.rope, rank + warp * ranks, tile, lane);
 
   int slot = 0;                             // of the ring, for the warps that load and multiply (over the passes)
   uint32_t turn = 0;                        // parity of its use
@@ -254,6 +309,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
       }
     }
+    if (rotates && warp < 2) rope = rope_row(p.rope, rank + warp * ranks, tile, lane);
     tc_fence_before_sync();
     __syncthreads();
     if (ranks > 1) cluster_sync_all();       // every partial tile of the cluster is in place
@@ -261,14 +317,14 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint32_t partial = smem_u32(smem);
     const int col = tile * kRows + lane * 4, row0 = row_base + first;
     switch (p.splits) {
-      case 1: reduce_rows<1>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      case 2: reduce_rows<2>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      case 3: reduce_rows<3>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      case 4: reduce_rows<4>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      case 5: reduce_rows<5>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      case 6: reduce_rows<6>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      case 7: reduce_rows<7>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
-      default: reduce_rows<8>(p, partial, rank, ranks, rows, row0, col, warp, lane); break;
+      case 1: reduce_rows<1, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      case 2: reduce_rows<2, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      case 3: reduce_rows<3, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      case 4: reduce_rows<4, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      case 5: reduce_rows<5, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      case 6: reduce_rows<6, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      case 7: reduce_rows<7, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
+      default: reduce_rows<8, ROPE>(p, partial, rank, ranks, rows, row0, col, warp, lane, rope); break;
     }
     fence_proxy_async_smem();                // (a further pass loads over the partial tile)
     if (ranks > 1) cluster_sync_all();       // nobody reads this CTA's partial any more
@@ -329,18 +385,19 @@ int cluster_splits(int tiles, int most) {
   return s < 1 ? 1 : s;
 }
 
-template <ClusterKind KIND>
+template <ClusterKind KIND, bool ROPE = false>
 static int launch(const CUtensorMap& tmW, const BatchMaps<KIND>& tmA, const ClusterParams& p, dim3 grid, int ranks,
                   uint32_t tmem_cols, cudaStream_t stream) {
   static PerDeviceOnce attr_once;
   if (attr_once.first())
-    cudaFuncSetAttribute(gemm_cluster_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
-  return launch_cluster_pdl(gemm_cluster_kernel<KIND>, grid, ranks, kThreads, p.ring_bytes + 1024, stream, tmW, tmA, p, tmem_cols) ==
+    cudaFuncSetAttribute(gemm_cluster_kernel<KIND, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta);
+  return launch_cluster_pdl(gemm_cluster_kernel<KIND, ROPE>, grid, ranks, kThreads, p.ring_bytes + 1024, stream, tmW, tmA, p, tmem_cols) ==
                  cudaSuccess ? 0 : -2;
 }
 
 int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream) {
   if (g.M < 1 || g.M > kMostRows || (g.gated && (g.N & 255))) return -1;
+  if (g.rope && (g.gated || g.batch > 1 || g.out_f32 || g.N != (g.rope->Hq + 2 * g.rope->Hkv) * kRows)) return -1;
   ClusterParams p{};
   p.M = g.M; p.N = g.N; p.K = g.K;
   p.mp = (g.M + 15) & ~15;
@@ -354,6 +411,7 @@ int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream) {
   p.ldr = g.ldr;
   p.batch_a_cols = g.batch_a_cols;
   p.batch_out = g.batch_out;
+  if (g.rope) p.rope = *g.rope;
   p.status = device_status_word();
   const int tiles = ((g.gated ? g.N / 2 : g.N) + kRows - 1) / kRows;
   p.splits = g.splits > 0 ? g.splits : choose_splits(tiles * g.batch, p.kblocks, g.gated);
@@ -376,12 +434,12 @@ int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream) {
     if (!encode_tmap_2d(&tmW, g.W, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.N, g.K, g.ldw, kRows, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&tm8.m[0], g.A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.M, g.K, g.lda, p.mp, 128, CU_TENSOR_MAP_SWIZZLE_128B))
       return -3;
-    return launch<kFp8>(tmW, tm8, p, grid, ranks, tmem_cols, stream);
+    return (g.rope ? launch<kFp8, true> : launch<kFp8>)(tmW, tm8, p, grid, ranks, tmem_cols, stream);
   }
   BatchMaps<kDense> tmA;
   if (!get_tmap_bf16(&tmW, g.W, (uint64_t)g.batch * g.N, g.K, g.ldw, kRows, 64)) return -3;
   if (!get_tmap_bf16(&tmA.m[0], g.A, g.M, g.batch > 1 ? (uint64_t)g.lda : (uint64_t)g.K, g.lda, p.mp, 64)) return -3;
-  return launch<kDense>(tmW, tmA, p, grid, ranks, tmem_cols, stream);
+  return (g.rope ? launch<kDense, true> : launch<kDense>)(tmW, tmA, p, grid, ranks, tmem_cols, stream);
 }
 
 // out[P, N] = grouped(xs[P, K], W[E, N, K]) for chunks of few rows; gated: W_e = [gate (N / 2) | up (N / 2)], out[P, N / 2].

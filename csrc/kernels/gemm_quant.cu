@@ -541,6 +541,12 @@ static bool fp8_tiles_win(int M, int N, int K) {
   return M > 48 && K <= 64 * (M - 32);
 }
 
+}  // extern "C"
+namespace b200 {
+bool fp8_rows_cluster(int M, int N, int K) { return M <= 128 && !fp8_tiles_win(M, N, K); }
+}  // namespace b200
+extern "C" {
+
 int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo,
                        const float* a_scale, const float* w_scale, int w_scale_per_channel, const void* bias,
                        int M, int N, int K, cudaStream_t stream);
@@ -560,7 +566,7 @@ int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int
                               stream);
   // up to 128 rows: weight-bound, K split over a cluster (gemm_cluster.cu); 32 requests of the fp8 8B shape 166 -> 148 ms
   // against 128 x 128 tiles with split-K partials in memory
-  if (M <= 128 && !(bias_at & 7) && (!fp8_tiles_win(M, N, K) || ((out_at | scale_at) & 15))) {
+  if (M <= 128 && !(bias_at & 7) && (fp8_rows_cluster(M, N, K) || ((out_at | scale_at) & 15))) {
     GemmCluster g{};
     g.A = A; g.lda = lda; g.W = W; g.ldw = ldw; g.out = out; g.ldo = ldo; g.bias = bias;
     g.M = M; g.N = N; g.K = K;

@@ -535,6 +535,20 @@ bool encode_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType dtyp
 // bf16 matrix with 128-byte swizzled boxes; the maps of a process are kept (gemm_bf16.cu).
 bool get_tmap_bf16(CUtensorMap* out, const void* p, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t br, uint32_t bc);
 
+// What a QKV product does with its result before it stores it: per-head RMSNorm of q and k, full NeoX rotation of 128-dim heads, k and v into
+// the paged cache [num_blocks, 2, block_size, Hkv, 128] too (b200_rope_kv, in the epilogue).
+struct RopeOut {
+  int Hq, Hkv;               // columns of the product: q heads | k heads | v heads
+  const int64_t* positions;
+  const float* cos_sin;      // [max_pos, 128]
+  const __nv_bfloat16 *q_norm, *k_norm;
+  float eps;
+  int gemma;
+  const int64_t* slot_mapping;
+  __nv_bfloat16* kv_cache;
+  int block_size;
+};
+
 // Product of at most 128 rows with K split over a cluster (gemm_cluster.cu).
 struct GemmCluster {
   const void *A, *W;
@@ -552,8 +566,10 @@ struct GemmCluster {
   // e4m3 A and W (set a_scale): the sums times a_scale (per tensor or row) and w_scale (per tensor or column)
   const float *a_scale, *w_scale;
   int a_per_row, w_per_col;
+  const RopeOut* rope;       // (not gated, not batched, N = (Hq + 2 Hkv) 128)
 };
 int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream);
+bool fp8_rows_cluster(int M, int N, int K);      // whether an e4m3 product is faster so (gemm_quant.cu)
 
 // One or two rows, on the CUDA cores; optionally with the residual addition and RMSNorm of the rows in front (gemv.cu).
 struct GemvNorm {

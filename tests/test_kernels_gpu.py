@@ -811,3 +811,96 @@ def test_rows_of_one_and_of_eight_ctas(V):
     steps = torch.full((160,), 9, dtype=torch.int64, device=DEV)
     assert torch.equal(ops.random_sample(probs, seeds, steps[:3])[torch.arange(160, device=DEV) % 3], ops.random_sample(*big, steps))
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("H", [8, 264, 2040, 2048, 2056, 4096, 4104, 8192, 8200])
+def test_rmsnorm_of_every_number_of_vectors_a_thread(H):
+    """One, two, four vectors a thread in registers or, beyond 8192, a loop through shared memory; the last one partly
+    empty; results in place of the input."""
+    torch.manual_seed(H)
+    for T in (1, 3):
+        x, w, r = _rand(T, H), _rand(H), _rand(T, H)
+        exp, newr = ref.rmsnorm(x, w, 1e-6, residual=r)
+        r2, x2 = r.clone(), x.clone()
+        ops.rmsnorm(x2, w, 1e-6, residual=r2, out=x2)
+        assert torch.equal(r2, newr)
+        assert _rel_err(x2, exp) < 2.0 ** -8                    # (one rounding to bf16)
+
+
+@pytest.mark.parametrize("Hq,Hkv,T,pad,qk_norm", [(32, 8, 103, 0, False), (5, 3, 600, 0, True), (4, 1, 900, 4, True),
+                                                  (7, 1, 1100, 8, False), (16, 8, 129, 0, True)])
+def test_rope_kv_of_many_tokens(Hq, Hkv, T, pad, qk_norm):
+    """Eight heads a warp: groups that end in k or v heads or in none, rows with a pitch that only 8-byte pieces read, tokens
+    without a slot, q to a tensor of its own."""
+    torch.manual_seed(T)
+    D, bs = 128, 16
+    nb = T // bs + 1
+    ld = (Hq + 2 * Hkv) * D + pad
+    rows = _rand(T, ld)
+    qkv = rows[:, : ld - pad]
+    pos = torch.randint(0, 500, (T,), device=DEV)
+    table = ops.rope_table(ref.rope_inv_freq(D, 1e6).to(DEV), 512)
+    qn, kn = (_rand(D), _rand(D)) if qk_norm else (None, None)
+    slots = torch.randperm(nb * bs, device=DEV)[:T].to(torch.int64)
+    slots[5] = -1
+    eq, ek, ev = ref.rope_kv(qkv.contiguous(), pos, table, Hq, Hkv, D, D, True, qn, kn)
+    exp = torch.zeros(nb, 2, bs, Hkv, D, device=DEV, dtype=torch.bfloat16)
+    ref.write_kv_cache(exp, ek, ev, slots, bs)
+    for own in (False, True):
+        work, cache = rows.clone()[:, : ld - pad], torch.zeros_like(exp)
+        q_out = torch.empty(T, Hq * D, device=DEV, dtype=torch.bfloat16) if own else None
+        ops.rope_kv(work, pos, table, num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, rot_dim=D, q_norm=qn, k_norm=kn,
+                    slot_mapping=slots, kv_cache=cache, block_size=bs, q_out=q_out)
+        got = q_out if own else work[:, : Hq * D]
+        assert _rel_err(got.reshape(T, Hq, D), eq) < 8e-3
+        assert _rel_err(cache[:, 0], exp[:, 0]) < 8e-3
+        assert torch.equal(cache[:, 1], exp[:, 1])
+        if own:
+            assert torch.equal(work[:, : Hq * D], qkv[:, : Hq * D])
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,H,qk_norm,fp8", [(3, 4, 1, 256, True, False), (16, 32, 8, 1024, False, False), (45, 5, 3, 264, True, False),
+                                                    (128, 16, 8, 512, True, False), (1, 6, 2, 256, False, True), (33, 8, 2, 1024, True, True)])
+def test_qkv_product_with_rotation(T, Hq, Hkv, H, qk_norm, fp8):
+    """The attention half of a block does qk-norm, rotation and cache write in the product's epilogue: the bits of the three
+    kernels one after the other."""
+    from vllm_cpp_b200.ops import quant as Q
+    from vllm_cpp_b200.ops.layer import DenseLayerWeights, DenseStep, dense_attn_half
+    torch.manual_seed(T + H)
+    D, bs = 128, 16
+    N, nb = (Hq + 2 * Hkv) * D, T // bs + 2
+    hidden, ln1, wo = _rand(T, H), _rand(H), _rand(H, Hq * D, scale=0.05)
+    wqkv = _rand(N, H, scale=0.05)
+    qn, kn = (_rand(D), _rand(D)) if qk_norm else (None, None)
+    pos = torch.randint(0, 500, (T,), device=DEV)
+    slots = torch.randperm(nb * bs, device=DEV)[:T].to(torch.int64)
+    slots[T // 2] = -1
+    table = ops.rope_table(ref.rope_inv_freq(D, 1e6).to(DEV), 512)
+    cache, exp = (torch.zeros(nb, 2, bs, Hkv, D, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    w, s = DenseLayerWeights(), DenseStep()
+    keep = [torch.empty(T, max(H, Hq * D), device=DEV, dtype=torch.uint8), torch.empty(T, device=DEV)]
+    if fp8:
+        scales = torch.rand(N, device=DEV) * 0.01
+        w8, o8 = wqkv.clamp(-1, 1).to(torch.float8_e4m3fn), wo.to(torch.float8_e4m3fn)
+        so = torch.ones(H, device=DEV)
+        w.fp8, w.qkv, w.o, w.qkv_scale, w.o_scale = 1, w8.data_ptr(), o8.data_ptr(), scales.data_ptr(), so.data_ptr()
+        s.fp8_act, s.fp8_scales = keep[0].data_ptr(), keep[1].data_ptr()
+        a8, sa = Q.quant_fp8_rowwise(hidden, norm_weight=ln1)
+        want = Q.gemm_fp8(a8, w8, sa, scales)
+    else:
+        w.qkv, w.o = wqkv.data_ptr(), wo.data_ptr()
+        want = ops.gemm(ops.rmsnorm(hidden, ln1, 1e-6), wqkv)
+    ops.rope_kv(want, pos, table, num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, rot_dim=D, q_norm=qn, k_norm=kn,
+                slot_mapping=slots, kv_cache=exp, block_size=bs)
+    qkv, attn, resid, normed = (torch.zeros(T, n, device=DEV, dtype=torch.bfloat16) for n in (N, Hq * D, H, H))
+    w.ln1, w.kv_cache = ln1.data_ptr(), cache.data_ptr()
+    w.q_norm, w.k_norm = (t.data_ptr() if t is not None else None for t in (qn, kn))
+    s.T, s.H, s.Hq, s.Hkv, s.D, s.rot, s.block_size, s.neox, s.eps, s.num_blocks = T, H, Hq, Hkv, D, D, bs, 1, 1e-6, nb
+    s.positions, s.cos_sin, s.slot_mapping, s.first_layer = pos.data_ptr(), table.data_ptr(), slots.data_ptr(), 1
+    s.hidden, s.resid, s.normed, s.qkv_buf, s.attn = (t.data_ptr() for t in (hidden, resid, normed, qkv, attn))
+    ws = ops.workspace(torch.device(DEV), ops.GEMM_WS_BYTES)
+    s.gemm_ws, s.gemm_ws_bytes = ws.data_ptr(), ws.numel()
+    dense_attn_half(w, s)
+    assert torch.equal(qkv, want)
+    assert torch.equal(cache, exp)
+    assert ops.read_status() == 0

@@ -264,3 +264,34 @@ def test_grouped_gemm_of_many_rows_an_expert(T, E, H, I, skew):
         y = got @ wd[e].float().t()
         assert ((ws.y[pos[at, j]].float() - y).norm() / y.norm()).item() < 2.0 ** -8
     assert ops.read_status() == 0
+
+
+def test_native_attention_half_same_logits_as_per_op_path():
+    """The attention halves through the native entry (prefill chunks, mixed steps, decodes): the bits of the per-op path."""
+    from vllm_cpp_b200.config import EngineArgs, synthetic_config
+    from vllm_cpp_b200.engine import LLM, SamplingParams
+    cfg = synthetic_config("tiny-moe")
+    cfg.head_dim = 128
+    llm = LLM(EngineArgs(model_config=cfg, device="cuda", block_size=16, num_blocks=200, max_model_len=640, max_num_seqs=4,
+                         max_num_batched_tokens=160, enable_cuda_graphs=False))
+    m, seen = llm.runner.model, []
+    assert m._native_attn_ok()
+    orig = type(m).forward
+
+    def both(self, ctx):
+        self.native_layers = False
+        a = orig(self, ctx).clone()
+        self.native_layers = True
+        seen.append((ctx.num_decodes, ctx.num_prefills, torch.equal(a, orig(self, ctx))))
+        return a
+
+    g = torch.Generator().manual_seed(3)
+    type(m).forward = both
+    try:
+        llm.generate([torch.randint(0, cfg.vocab_size, (n,), generator=g).tolist() for n in (200, 9, 70, 150)],
+                     SamplingParams(temperature=0.0, max_tokens=5, ignore_eos=True))
+    finally:
+        type(m).forward = orig
+    assert any(nd and npf for nd, npf, _ in seen) and any(nd and not npf for nd, npf, _ in seen)
+    assert all(eq for *_, eq in seen), seen
+    assert ops.read_status() == 0

@@ -521,7 +521,7 @@ class DenseModel:
                 w.ln1, w.qkv, w.o, w.ln2 = L["ln1"].data_ptr(), L["qkv"].data_ptr(), L["o"].data_ptr(), L["ln2"].data_ptr()
                 w.q_norm = L["q_norm"].data_ptr() if L.get("q_norm") is not None else None
                 w.k_norm = L["k_norm"].data_ptr() if L.get("k_norm") is not None else None
-                w.gate_up, w.down = L["gate_up"].data_ptr(), L["down"].data_ptr()
+                w.gate_up, w.down = (L[k].data_ptr() if k in L else None for k in ("gate_up", "down"))
                 w.kv_cache = self.kv_caches[l].data_ptr()
                 if hasattr(L["qkv"], "w8"):
                     w.fp8 = 1

@@ -19,6 +19,7 @@ import os
 import torch
 
 from ..config import ModelConfig, ParallelConfig
+from ..utils import nvtx
 from .base import StepContext, shard_cols, shard_rows
 from .dense import ACT_KIND, DenseModel
 
@@ -272,6 +273,16 @@ class MoeModel(DenseModel):
             ids = self.eplb.remap(L["_eplb_idx"], ids)
         return M.ref_moe_block(x, ids, w, L["w_gate_up"], L["w_down"], e0=self.e0)
 
+    def _native_attn_ok(self) -> bool:
+        """The plain attention block on one GPU with bf16 projections, as the native entry takes it."""
+        c = self.cfg
+        if self.device.type != "cuda" or self.tp > 1 or self.ep > 1 or os.environ.get("B200_NATIVE_LAYERS", "1") == "0":
+            return False
+        if (c.post_norm or c.sandwich_norm or c.attention_bias or c.sliding_window or c.attention_chunk_size or c.gemma_norm
+                or c.attn_logit_softcap or c.residual_multiplier != 1.0 or len(set(self.layer_group)) != 1):
+            return False
+        return all(isinstance(L[k], torch.Tensor) and L[k].dtype == torch.bfloat16 for L in self.layers for k in ("qkv", "o"))
+
     # ------------------------------------------------------------------ forward
     def forward(self, ctx: StepContext) -> torch.Tensor:
         if getattr(self, "tpf", None) is not None:
@@ -290,23 +301,34 @@ class MoeModel(DenseModel):
         if self.tp > 1:
             self.comm.all_reduce(hidden)
         pos = ctx.positions[:T]
+        step = None
+        if self.native_layers is None:
+            self.native_layers = type(self).forward is MoeModel.forward and self._native_attn_ok()
+        if self.native_layers and T > 0 and not nvtx.ENABLED:
+            from ..ops.layer import dense_attn_half
+            step = self._native_step(ctx, T, qkv, attn, qkv, qkv, 0, hidden, resid, normed)    # (no MLP: its buffers are not touched)
+            weights = self._native_weights() if step is not None else None
         for l, L in enumerate(self.layers):
             grp = self.layer_group[l]
-            if l == 0:
-                resid.copy_(hidden)
-                x = be.rmsnorm(hidden, L["ln1"], eps, out=normed)
+            if step is not None:
+                step.first_layer = int(l == 0)
+                dense_attn_half(weights[l], step)
             else:
-                x = be.rmsnorm(hidden, L["ln1"], eps, residual=resid, out=normed)
-            be.gemm(x, L["qkv"], out=qkv)
-            be.rope_kv(qkv, pos, self.rope_table, num_q_heads=self.hq, num_kv_heads=self.hkv,
-                       head_dim=self.D, rot_dim=self.rot, neox=c.rope.neox,
-                       q_norm=L.get("q_norm"), k_norm=L.get("k_norm"), eps=eps, gemma=False,
-                       slot_mapping=ctx.slot_mapping[grp][:T], kv_cache=self.kv_caches[l],
-                       block_size=self.block_size)
-            be.attention(qkv[:, : self.hq * self.D], self.kv_caches[l], ctx, grp,
-                         num_q_heads=self.hq, num_kv_heads=self.hkv, head_dim=self.D,
-                         block_size=self.block_size, scale=self.scale, out=attn)
-            be.gemm(attn, L["o"], out=hidden)
+                if l == 0:
+                    resid.copy_(hidden)
+                    x = be.rmsnorm(hidden, L["ln1"], eps, out=normed)
+                else:
+                    x = be.rmsnorm(hidden, L["ln1"], eps, residual=resid, out=normed)
+                be.gemm(x, L["qkv"], out=qkv)
+                be.rope_kv(qkv, pos, self.rope_table, num_q_heads=self.hq, num_kv_heads=self.hkv,
+                           head_dim=self.D, rot_dim=self.rot, neox=c.rope.neox,
+                           q_norm=L.get("q_norm"), k_norm=L.get("k_norm"), eps=eps, gemma=False,
+                           slot_mapping=ctx.slot_mapping[grp][:T], kv_cache=self.kv_caches[l],
+                           block_size=self.block_size)
+                be.attention(qkv[:, : self.hq * self.D], self.kv_caches[l], ctx, grp,
+                             num_q_heads=self.hq, num_kv_heads=self.hkv, head_dim=self.D,
+                             block_size=self.block_size, scale=self.scale, out=attn)
+                be.gemm(attn, L["o"], out=hidden)
             if self.tp > 1:
                 self.comm.all_reduce(hidden)
             x = be.rmsnorm(hidden, L["ln2"], eps, residual=resid, out=normed)

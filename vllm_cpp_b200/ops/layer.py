@@ -33,20 +33,30 @@ class DenseStep(C.Structure):
 _declared = False
 
 
-def dense_layer(weights: DenseLayerWeights, step: DenseStep) -> None:
+def _issue(name: str, weights: DenseLayerWeights, step: DenseStep) -> None:
     global _declared
     L = lib()
     if not _declared:
-        L.b200_dense_layer.argtypes = [C.POINTER(DenseLayerWeights), C.POINTER(DenseStep), P]
-        L.b200_dense_layer.restype = I
+        for f in (L.b200_dense_layer, L.b200_dense_attn_half):
+            f.argtypes = [C.POINTER(DenseLayerWeights), C.POINTER(DenseStep), P]
+            f.restype = I
         _declared = True
-    rc = L.b200_dense_layer(C.byref(weights), C.byref(step), stream_ptr())
+    rc = getattr(L, "b200_" + name)(C.byref(weights), C.byref(step), stream_ptr())
     if rc < 0:
-        raise KernelError(f"dense_layer: kernel launcher returned {rc}")
+        raise KernelError(f"{name}: kernel launcher returned {rc}")
     LAUNCHES[0] += rc
     if _lib_mod.SYNC_CHECK:
-        _lib_mod.sync_check(f"dense_layer T={step.T} decodes={step.num_decodes} prefills={step.num_prefills} "
+        _lib_mod.sync_check(f"{name} T={step.T} decodes={step.num_decodes} prefills={step.num_prefills} "
                             f"splits={step.decode_splits}")
+
+
+def dense_layer(weights: DenseLayerWeights, step: DenseStep) -> None:
+    _issue("dense_layer", weights, step)
+
+
+def dense_attn_half(weights: DenseLayerWeights, step: DenseStep) -> None:
+    """The block up to the output projection (into ``step.hidden``); the MLP's weights are not read."""
+    _issue("dense_attn_half", weights, step)
 
 
 class TpLayers(C.Structure):
