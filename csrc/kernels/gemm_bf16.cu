@@ -22,6 +22,7 @@
 //
 // Replaces the library GEMM calls of the reference (src/vt/cuda/cuda_matmul.cu:284-355
 // "MatmulBT" and :219-274), which hand every projection to cuBLASLt.
+#include <climits>
 #include <mutex>
 #include <unordered_map>
 
@@ -36,6 +37,8 @@ static constexpr int kGemmThreads = 192;
 static constexpr int kMaxStages = 12;
 
 struct GemmParams {
+  int done_offset;           // from a tile's counter of parts that are there to that of parts that are through
+  int parts;                 // > 1: every tile is shared by that many workers, each with its part of K (share_tile)
   int M, N, K;
   void* out;
   int ldo;
@@ -150,10 +153,19 @@ __device__ __forceinline__ int sk_range_start_w(int w, int units, int nworkers) 
   const int q = units / nworkers, r = units % nworkers;
   return w * q + min(w, r);
 }
+template <bool SHARED = false>
 __device__ __forceinline__ SegState seg_init_w(const GemmParams& p, int kblocks, int worker,
                                                int nworkers) {
   SegState s;
   s.sk_tiles = p.sk;
+  if constexpr (SHARED) {                              // one piece each, no whole tiles
+    const int tile = worker / p.parts, part = worker - tile * p.parts;
+    s.t = INT_MAX;
+    s.stride = 0;
+    s.u = tile * kblocks + kblocks * part / p.parts;
+    s.u1 = tile * kblocks + kblocks * (part + 1) / p.parts;
+    return s;
+  }
   s.t = p.sk + worker;
   s.stride = nworkers;
   s.u = sk_range_start_w(worker, p.sk * kblocks, nworkers);
@@ -191,7 +203,68 @@ __device__ __forceinline__ bool wait_flag_set(const uint32_t* f, int* status) {
   }
 }
 
-template <int BN>
+// Tiles shared by equal parts of K. Every part leaves the column chunks that others finish in its slot of the scratch, counts itself in,
+// waits for the rest and finishes its own chunks (c % parts), adding the parts up in their order: the exchange takes about as long for
+// eight parts as for two, where an owner that sums the others' tiles one after the other took 5 us for each. A warp only meets the warps of
+// the same rows. `mine` tells the chunks that this part finishes; false: a wait ran out.
+__device__ __forceinline__ bool wait_count(const uint32_t* f, uint32_t n, int* status) {
+  long long t0 = clock64();
+  uint32_t it = 0;
+  while (true) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+    if (v >= n) return true;
+    if (((++it) & 0xff) == 0 && clock64() - t0 > kPeerWaitCycles) {
+      if (status) atomicExch(status, (int)kErrFlagTimeout);
+      return false;
+    }
+  }
+}
+template <int BN, typename Mine>
+__device__ __forceinline__ bool share_tile(const GemmParams& p, uint32_t t_addr, float* slot, uint32_t* count, int lane, Mine&& mine) {
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    if (mine(c)) continue;
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(t_addr + c * 32, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) __stcg(slot + (size_t)(c * 32 + i) * kBM, __uint_as_float(r[i]));
+  }
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+  return __all_sync(0xffffffffu, wait_count(count, p.parts, p.status));
+}
+// Chunk c of all parts; v: this part's own. first: the slot of part 0, at the thread's row, stride: from a part's slot to the next's.
+__device__ __forceinline__ void add_parts(const GemmParams& p, float (&v)[32], const float* first, size_t stride, int part, int c) {
+  float own[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) own[i] = v[i];
+  for (int x = 0; x < p.parts; ++x) {
+    float f[32];
+    if (x == part) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) f[i] = own[i];
+    } else {
+      const float* src = first + x * stride + (size_t)c * 32 * kBM;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) f[i] = __ldcg(src + (size_t)i * kBM);
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = x == 0 ? f[i] : v[i] + f[i];
+  }
+}
+// The last part to have read the others' clears the tile's counters for the next launch.
+__device__ __forceinline__ void leave_tile(const GemmParams& p, uint32_t* count, int lane) {
+  __syncwarp();
+  if (lane == 0) {
+    uint32_t* done = count + p.done_offset;
+    if (atomicAdd(done, 1u) == (uint32_t)p.parts - 1) { *count = 0; *done = 0; }
+  }
+}
+
+template <int BN, bool SHARED>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmA_alt,
@@ -234,7 +307,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // this CTA's first segment before waiting on the predecessor kernel.
   int npre = 0;
   if (warp == 0 && p.w_early && !p.ag_flags) {
-    SegState seg0 = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
+    SegState seg0 = seg_init_w<SHARED>(p, kblocks, blockIdx.x, gridDim.x);
     int t0, ka, kz;
     if (seg_next(seg0, num_tiles, kblocks, t0, ka, kz)) {
       int tm0, tn0;
@@ -264,7 +337,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     uint32_t ph = 1;
     int s = 0, early = npre;
     bool ok = true;
-    SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
+    SegState seg = seg_init_w<SHARED>(p, kblocks, blockIdx.x, gridDim.x);
     int t, kb0, kb1;
     while (ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1)) {
       int tm, tn;
@@ -304,7 +377,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     uint32_t tc = 0, ph = 0;
     int s = 0;
     bool ok = true;
-    SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
+    SegState seg = seg_init_w<SHARED>(p, kblocks, blockIdx.x, gridDim.x);
     int t, kb0, kb1;
     for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
       const int buf = tc & 1;
@@ -337,7 +410,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int quarter = warp & 3;
     uint32_t tc = 0;
     bool ok = true;
-    SegState seg = seg_init_w(p, kblocks, blockIdx.x, gridDim.x);
+    SegState seg = seg_init_w<SHARED>(p, kblocks, blockIdx.x, gridDim.x);
     int t, kb0, kb1;
     for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
       int tm, tn;
@@ -350,7 +423,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       tc_fence_after_sync();
       const int row = tm * kBM + quarter * 32 + lane;
       const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(quarter * 32) << 16);
-      if (kb0 > 0) {
+      const int part = SHARED ? (int)blockIdx.x % p.parts : 0;
+      uint32_t* count = p.sk_flags + t * 4 + quarter;
+      const auto mine = [&](int c) { return !SHARED || c % p.parts == part; };
+      if constexpr (SHARED) {
+        ok = share_tile<BN>(p, t_addr, p.sk_partials + (size_t)blockIdx.x * kBM * BN + quarter * 32 + lane, count, lane, mine);
+        if (!ok) break;
+      } else if (kb0 > 0) {
         // stream-K partial: raw fp32 accumulators to this CTA's slot, then the flag
         // column-major inside the slot: the 32 lanes of a warp write 32 consecutive floats
         float* dst = p.sk_partials + (size_t)blockIdx.x * kBM * BN + quarter * 32 + lane;
@@ -378,7 +457,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
       // stream-K owner: the CTAs after this one hold the rest of the tile's k-blocks
       int sk_first = 0, sk_last = -1;
-      if (kb1 < kblocks) {
+      if (!SHARED && kb1 < kblocks) {
         const int tile_end = (t + 1) * kblocks;
         sk_first = blockIdx.x + 1;
         sk_last = blockIdx.x;
@@ -392,6 +471,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
+        if (!mine(c)) continue;
         uint32_t r[32];
         tmem_ld_32x32b_x32(t_addr + c * 32, r);
         tmem_ld_wait();
@@ -400,6 +480,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+          if constexpr (SHARED)
+            add_parts(p, v, p.sk_partials + (size_t)(blockIdx.x - part) * kBM * BN + quarter * 32 + lane, (size_t)kBM * BN, part, c);
           for (int x = sk_first; x <= sk_last; ++x) {
             const float* src = p.sk_partials + (size_t)x * kBM * BN + (size_t)c * 32 * kBM + quarter * 32 + lane;
             float f[32];
@@ -487,6 +569,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                          (row0 - owner * p.rows_per_rank) / 32);
         }
       }
+      if constexpr (SHARED) leave_tile(p, count, lane);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
@@ -598,7 +681,7 @@ __device__ __forceinline__ void epilogue_store_gated(const GemmParams& p, const 
 // FP8 = false: bf16 operands, 64 elements per 128-byte smem row. FP8 = true: e4m3 operands
 // (kind::f8f6f4), 128 elements per row; everything else (tiles, rings, stream-K) is shared.
 
-template <int BN, bool FP8 = false>
+template <int BN, bool FP8 = false, bool SHARED = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
                           const __grid_constant__ CUtensorMap tmA_alt,
@@ -660,7 +743,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     uint32_t ph = 1;
     int s = 0;
     bool ok = true;
-    SegState seg = seg_init_w(p, kblocks, pair, npairs);
+    SegState seg = seg_init_w<SHARED>(p, kblocks, pair, npairs);
     int t, kb0, kb1;
     while (ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1)) {
       int tm, tn;
@@ -701,7 +784,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       uint32_t tc = 0, ph = 0;
       int s = 0;
       bool ok = true;
-      SegState seg = seg_init_w(p, kblocks, pair, npairs);
+      SegState seg = seg_init_w<SHARED>(p, kblocks, pair, npairs);
       int t, kb0, kb1;
       for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
         const int buf = tc & 1;
@@ -736,7 +819,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int me = blockIdx.x;                        // partial slot / flag owner
     uint32_t tc = 0;
     bool ok = true;
-    SegState seg = seg_init_w(p, kblocks, pair, npairs);
+    SegState seg = seg_init_w<SHARED>(p, kblocks, pair, npairs);
     int t, kb0, kb1;
     for (; ok && seg_next(seg, num_tiles, kblocks, t, kb0, kb1); ++tc) {
       int tm, tn;
@@ -750,7 +833,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int row = tm * 2 * kBM + (int)rank * kBM + quarter * 32 + lane;
       const uint32_t t_addr = tmem_base + buf * BN + ((uint32_t)(quarter * 32) << 16);
       const uint32_t leader_acc_empty = mapa_u32(smem_u32(&bars->acc_empty[buf]), 0);
-      if (kb0 > 0) {
+      const int part = SHARED ? pair % p.parts : 0;
+      uint32_t* count = p.sk_flags + (t * 2 + (int)rank) * 4 + quarter;
+      const int columns = BN == 256 && p.act_fuse ? 4 : BN / 32;         // (gated: chunk c of the gate and of the up half go together)
+      const auto mine = [&](int c) { return !SHARED || (c & (columns - 1)) % p.parts == part; };
+      if constexpr (SHARED) {
+        ok = share_tile<BN>(p, t_addr, p.sk_partials + (size_t)me * kBM * BN + quarter * 32 + lane, count, lane, mine);
+        if (!ok) break;
+      } else if (kb0 > 0) {
         float* dst = p.sk_partials + (size_t)me * kBM * BN + quarter * 32 + lane;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -772,7 +862,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         continue;
       }
       int sk_first = 0, sk_last = -1;                 // contributing pairs
-      if (kb1 < kblocks) {
+      if (!SHARED && kb1 < kblocks) {
         const int tile_end = (t + 1) * kblocks;
         sk_first = pair + 1;
         sk_last = pair;
@@ -795,6 +885,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+        if constexpr (SHARED)
+          add_parts(p, v, p.sk_partials + (size_t)((pair - part) * 2 + (int)rank) * kBM * BN + quarter * 32 + lane, (size_t)2 * kBM * BN, part, c);
         for (int x = sk_first; x <= sk_last; ++x) {
           const float* src = p.sk_partials + (size_t)(x * 2 + (int)rank) * kBM * BN +
                              (size_t)c * 32 * kBM + quarter * 32 + lane;
@@ -829,6 +921,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       if (BN == 256 && p.act_fuse) {
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
+          if (!mine(c)) continue;
           float g[32], u[32];
           load_chunk(c, g);
           load_chunk(c + 4, u);
@@ -888,12 +981,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       } else {
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
+          if (!mine(c)) continue;
           float v[32];
           load_chunk(c, v);
           const int col0 = tn * BN + c * 32;
           if (row < p.M && col0 < p.N) epilogue_store_chunk(p, v, row, col0);
         }
       }
+      if constexpr (SHARED) leave_tile(p, count, lane);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
@@ -1208,12 +1303,12 @@ static bool streamk_scratch(cudaStream_t stream, float** partials, uint32_t** fl
     float* pp = nullptr;
     uint32_t* ff = nullptr;
     if (cudaMalloc(&pp, n) != cudaSuccess) { cudaGetLastError(); return false; }
-    if (cudaMalloc(&ff, (size_t)b200_num_sms() * 4 * sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaMalloc(&ff, (size_t)b200_num_sms() * 8 * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
       cudaFree(pp);
       return false;
     }
-    cudaMemset(ff, 0, (size_t)b200_num_sms() * 4 * sizeof(uint32_t));
+    cudaMemset(ff, 0, (size_t)b200_num_sms() * 8 * sizeof(uint32_t));
     g_part[dev] = pp;
     g_flags[dev] = ff;
   }
@@ -1225,9 +1320,10 @@ static bool streamk_scratch(cudaStream_t stream, float** partials, uint32_t** fl
 // Stream-K plan for `tiles` tiles of `kblocks` k-blocks on at most `max_workers` workers.
 // Fewer tiles than workers: every tile is cut into the same number of parts (workers that share
 // an operand stay in step). Otherwise only the tiles of the ragged last wave are cut.
-static void plan_streamk(long tiles, int kblocks, int max_workers, int* nworkers, int* sk_tiles) {
+static void plan_streamk(long tiles, int kblocks, int max_workers, int* nworkers, int* sk_tiles, int* shared = nullptr) {
   *nworkers = tiles < max_workers ? (int)tiles : max_workers;
   *sk_tiles = 0;
+  if (shared) *shared = 0;
   if (kblocks < 16 || tiles <= 0) return;
   if (tiles < max_workers) {
     int parts = max_workers / (int)tiles;
@@ -1235,6 +1331,7 @@ static void plan_streamk(long tiles, int kblocks, int max_workers, int* nworkers
     if (parts >= 2) {
       *nworkers = (int)tiles * parts;
       *sk_tiles = (int)tiles;
+      if (shared) *shared = parts;
     }
     // (With 50-88 % of the workers owning a tile, cutting the whole k-range evenly over all workers
     // was measured slower than leaving the rest idle: 71 against 60 us for 32 x 28672 x 4096. The
@@ -1246,6 +1343,46 @@ static void plan_streamk(long tiles, int kblocks, int max_workers, int* nworkers
   // a sliver of a wave would be cut too finely (one owner summing dozens of partials): take a
   // whole wave into the region with it
   *sk_tiles = ((long)r * kblocks < 8l * max_workers) ? r + max_workers : r;
+}
+
+// Which tiles a product of more rows than the cluster kernel takes runs fastest on: an estimate of its time, in us, from the start of a
+// kernel, a k-block of 64 in the first and in further waves, the end of a tile behind which nothing hides, and an exchange of parts
+// (share_tile) or of a stream-K region. Fitted to 3456 timings: 23 matrices from 128 x 2048 to 28672 x 4096, 130 to 2300 rows, and twelve
+// of them up to 8192 rows; 7 % off on average. The choice is 1.0 % from the best of the eight forms on average, up to 2300 rows, and 2.2 %
+// above, where the clocks move as much; the rules that it replaced were 15 and 7 % off and up to 3 times: us, before / after, 1024 x 3072 at
+// 600 rows 31.0 / 12.1, 2048 x 4096 at 300 36.8 / 14.0, 4096 x 1024 at 512 16.8 / 8.0, 4096 x 14336 at 300 59.0 / 46, 28672 x 4096
+// at 300 101 / 83. A tile of 128 x 128 is bound by shared memory, those of a pair by the tensor pipe.
+struct TileForm {
+  int path, rows, cols, streamed;       // path: force_path
+};
+static constexpr TileForm kTileForms[8] = {{3, 128, 128, 0}, {4, 128, 256, 0}, {5, 128, 256, 1}, {6, 128, 128, 1},
+                                           {7, 256, 256, 0}, {8, 256, 128, 0}, {9, 256, 256, 1}, {10, 256, 128, 1}};
+static float tile_form_us(const TileForm& f, long M, long N, long K) {
+  struct Cost { float start, first, share, stream, end, further; };
+  static constexpr Cost kCost[4] = {{4.311f, .209f, 4.078f, 5.302f, .550f, .234f}, {4.829f, .378f, 7.278f, 9.930f, .926f, .405f},
+                                    {5.229f, .171f, 3.763f, 5.497f, 1.018f, .197f}, {6.653f, .331f, 6.465f, 9.562f, .578f, .354f}};
+  const Cost& c = kCost[(f.rows == 256 ? 2 : 0) + (f.cols == 256 ? 1 : 0)];
+  const long tiles = ((M + f.rows - 1) / f.rows) * ((N + f.cols - 1) / f.cols), workers = b200_num_sms() * 128 / f.rows;
+  const int kblocks = (int)((K + kBK - 1) / kBK);
+  if (f.streamed) {
+    int n = 0, sk = 0, parts = 0;
+    plan_streamk(tiles, kblocks, (int)workers, &n, &sk, &parts);
+    if (parts) return c.start + c.first * ((kblocks + parts - 1) / parts) + c.share;
+    const long whole = (tiles - sk) / workers;
+    if (sk) return c.start + c.further * ((sk * (long)kblocks + workers - 1) / workers + whole * kblocks) + c.stream + c.end * whole;
+  }
+  const long waves = (tiles + workers - 1) / workers;
+  return c.start + (waves == 1 ? c.first : c.further) * waves * kblocks + c.end * (waves - 1);
+}
+static int fastest_tiles(long M, long N, long K) {
+  int path = 3;
+  float best = 1e30f;
+  for (const TileForm& f : kTileForms) {
+    if (f.cols > 128 && N <= (f.rows == 256 ? 128 : 255)) continue;
+    const float t = tile_form_us(f, M, N, K);
+    if (t < best) { best = t; path = f.path; }
+  }
+  return path;
 }
 
 template <int BN>
@@ -1261,16 +1398,17 @@ static int launch_tn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUte
   size_t smem = (size_t)stages * stage_bytes + 1024 + sizeof(GemmBarriers);
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
-    cudaFuncSetAttribute(gemm_bf16_tn_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kSmemBudget + 4096);
+    for (auto k : {gemm_bf16_tn_kernel<BN, false>, gemm_bf16_tn_kernel<BN, true>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 4096);
   }
   int tiles = p.tiles_m * p.tiles_n;
   int grid = tiles < b200_num_sms() ? tiles : b200_num_sms();
   if (p.sk) {   // on entry: stream-K wanted; from here on: tiles in the stream-K region
     int sk_tiles = 0;
-    plan_streamk(tiles, kblocks, b200_num_sms(), &grid, &sk_tiles);
+    plan_streamk(tiles, kblocks, b200_num_sms(), &grid, &sk_tiles, p.tp_world > 1 ? nullptr : &p.parts);
+    p.done_offset = b200_num_sms() * 4;
     if (sk_tiles && !streamk_scratch(stream, &p.sk_partials, &p.sk_flags)) {
-      sk_tiles = 0;
+      sk_tiles = p.parts = 0;
       grid = tiles < b200_num_sms() ? tiles : b200_num_sms();
     }
     p.sk = sk_tiles;
@@ -1279,7 +1417,7 @@ static int launch_tn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUte
   // kernel touches nothing a peer can see before its wait on the predecessor, every CTA of a
   // grid is resident before its dependents may start (the grid never exceeds the SM count), and
   // a kernel only ever waits for work that precedes it in its peers' streams.
-  return launch_pdl(gemm_bf16_tn_kernel<BN>, dim3(grid), dim3(kGemmThreads), smem, stream, tmA, tmA2, tmB, p) ==
+  return launch_pdl(p.parts > 1 ? gemm_bf16_tn_kernel<BN, true> : gemm_bf16_tn_kernel<BN, false>, dim3(grid), dim3(kGemmThreads), smem, stream, tmA, tmA2, tmB, p) ==
                  cudaSuccess ? 0 : -2;
 }
 
@@ -1318,8 +1456,8 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (!max_clusters[dev]) {
-    cudaFuncSetAttribute(gemm_bf16_pair_kernel<BN, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kSmemBudget + 4096);
+    for (auto k : {gemm_bf16_pair_kernel<BN, FP8, false>, gemm_bf16_pair_kernel<BN, FP8, true>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 4096);
     cfg.gridDim = dim3(b200_num_sms() & ~1);
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<BN, FP8>, &cfg) != cudaSuccess || n < 1) {
@@ -1334,9 +1472,10 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
   int pairs = tiles < max_pairs ? (int)tiles : max_pairs;
   if (p.sk) {
     int sk_tiles = 0;
-    plan_streamk(tiles, kblocks, max_pairs, &pairs, &sk_tiles);
+    plan_streamk(tiles, kblocks, max_pairs, &pairs, &sk_tiles, p.tp_world > 1 ? nullptr : &p.parts);
+    p.done_offset = b200_num_sms() * 4;
     if (sk_tiles && !streamk_scratch(stream, &p.sk_partials, &p.sk_flags)) {
-      sk_tiles = 0;
+      sk_tiles = p.parts = 0;
       pairs = tiles < max_pairs ? (int)tiles : max_pairs;
     }
     p.sk = sk_tiles;
@@ -1344,7 +1483,8 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CU
   cfg.gridDim = dim3(2 * pairs);
   cfg.dynamicSmemBytes = smem;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_bf16_pair_kernel<BN, FP8>, tmA, tmA2, tmB, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, p.parts > 1 ? gemm_bf16_pair_kernel<BN, FP8, true> : gemm_bf16_pair_kernel<BN, FP8, false>, tmA, tmA2, tmB, p) !=
+      cudaSuccess) {
     cudaGetLastError();
     return -2;
   }
@@ -1486,10 +1626,11 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
     return 0;
   }
   // Up to 128 rows: K split over a cluster, two CTAs per SM. On the widest matrices (no split to gain from) the tiled
-  // kernel, which reads 256 weight rows with one copy of the batch, is the faster one from some rows on
-  // (128256 x 4096: 172.6 against 169.9 us at 40 rows, 178 against 172 at 64; at 32 rows 167 against 170, at 1 158 against 185;
+  // kernels, which read 128 or 256 weight rows with one copy of the batch, are the faster ones from some rows on
+  // (128256 x 4096: 168.2 against 168.4 us at 40 rows, 173.5 against 170.4 at 64; 28672 x 4096 41.2 against 43.3 at 40, 42.6 against 42.5
+  // at 64, 47.5 against 45.0 at 128; 16384 x 2048 14.8 against 14.2, 15.7 against 14.2, 18.2 against 14.7;
   // beyond one wave of CTAs with a short K earlier: 57344 x 512 at 32 rows 16.7 against 15.6, at 16 15.2 against 16.7).
-  const bool tiles_win = N >= 16384 && !(at & 15) && (M > 32 || (M > 16 && K <= 512 && (N + kBM - 1) / kBM > 2 * b200_num_sms()));
+  const bool tiles_win = N >= 16384 && !(at & 15) && (M > 48 || (M > 16 && K <= 512 && (N + kBM - 1) / kBM > 2 * b200_num_sms()));
   const bool cluster = !tp && M <= 128 && !(at & 7) &&
                        (force_path == 0 ? act_fuse || !tiles_win : force_path >= 32 && force_path <= 40);
   if (act_fuse && !cluster && force_path == 0) force_path = 9;      // the gated epilogue lives in the pair kernel
@@ -1540,11 +1681,11 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   const int kblocks = (K + kBK - 1) / kBK;
 
   bool use_swap = (M <= 256);
-  // Batches that the cluster kernel does not take. On wide matrices the batch goes on the (padded) M side
-  // and 256 weight rows share an instruction, with stream-K filling the SMs: 1-CTA 128 x 256 tiles up to 128
-  // rows, CTA pairs above; narrower matrices: 128 x 128 tiles + stream-K.
+  // Batches that the cluster kernel does not take: the tiles that are estimated to be fastest (up to 128 rows those of 128 rows).
   if (at & 15) force_path = 2;
-  if (force_path == 0 && !tp && M <= 256) force_path = N < 16384 ? (M <= 128 ? 2 : 6) : M <= 128 ? 5 : 9;
+  if (force_path == 0 && !tp && !act_fuse)
+    force_path = M > 128 ? fastest_tiles(M, N, K)
+                         : N < 256 || tile_form_us(kTileForms[3], M, N, K) < tile_form_us(kTileForms[2], M, N, K) ? 6 : 5;
   if (force_path == 1 || force_path >= 3) use_swap = false;     // an explicit tiling was asked for
   if (force_path == 2 && M <= 256) use_swap = true;
 
@@ -1634,13 +1775,6 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   // tensor-parallel shards are narrow (N / world or K / world): few tiles or a ragged last wave
   // are the rule, so the tiled path always plans stream-K there
   if (tp && force_path == 1) p.sk = 1;
-  // 256-row pair tiles pad M up to a multiple of 256; where 128-row tiles would do noticeably
-  // fewer rows (e.g. M = 1056: 1280 against 1152) the 1-CTA 128 x 256 tile with stream-K is faster
-  // (measured 907-1253 against 699-1175 TFLOP/s on the four Llama-8B projections at M = 1056).
-  if (force_path == 0 && !tp && !act_fuse && N >= 256) {
-    const long rows256 = (long)((M + 255) / 256) * 256, rows128 = (long)((M + 127) / 128) * 128;
-    if (rows256 * 100 > rows128 * 108) { force_path = 5; use256 = true; p.sk = 1; }
-  }
   // Tensor-parallel GEMMs above the small-M range run on CTA pairs as well (gather prologue,
   // staged scatter epilogue); B200_TP_PAIR=0 keeps them on the 1-CTA tile.
   const bool tp_pair = tp && force_path == 1 && M > 256 && tp_pair_enabled();

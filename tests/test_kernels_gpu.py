@@ -904,3 +904,58 @@ def test_qkv_product_with_rotation(T, Hq, Hkv, H, qk_norm, fp8):
     assert torch.equal(qkv, want)
     assert torch.equal(cache, exp)
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(130, 1024, 1040), (257, 384, 4096), (300, 512, 1288), (129, 128, 8192), (513, 256, 2048)])
+@pytest.mark.parametrize("path", [5, 6, 9, 10])
+def test_gemm_tiles_in_parts(M, N, K, path):
+    """Few tiles: every one is shared by equal parts of K, two to eight of them, also where neither K nor the columns divide;
+    twice on the same counters, with what follows the product. fp32 sums of exact products, rounded to bf16 once (2^-8)."""
+    torch.manual_seed(M + N)
+    a, w, bias, res = _rand(M, K), _rand(N, K, scale=K ** -0.5), _rand(N), _rand(M, N)
+    exp = a.double() @ w.double().t()
+    first = ops.gemm(a, w, force_path=path)
+    assert _rel_err(first.double(), exp) < 2.0 ** -8
+    assert torch.equal(first, ops.gemm(a, w, force_path=path))
+    out = torch.full((M, N), 7.0, device=DEV, dtype=torch.float32)
+    ops.gemm(a, w, bias=bias, residual=res, out=out, force_path=path)
+    assert _rel_err(out.double(), exp + bias.double() + res.double()) < 1e-5
+    if path == 9 and N % 256 == 0:
+        got = ops.gemm_gated(a, ops.interleave_gate_up(w[: N // 2], w[N // 2:]), force_path=9)
+        g, u = exp[:, : N // 2], exp[:, N // 2:]
+        assert _rel_err(got.double(), g * torch.sigmoid(g) * u) < 2.0 ** -6     # (three roundings)
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 8, 64), (200, 136, 328), (260, 128, 72), (300, 200, 1024), (1100, 264, 520), (2000, 3072, 768)])
+def test_gemm_of_the_form_that_is_chosen(M, N, K):
+    """Narrow and ragged matrices through the estimate, against 64 bits."""
+    torch.manual_seed(M)
+    a, w = _rand(M, K), _rand(N, K, scale=K ** -0.5)
+    assert _rel_err(ops.gemm(a, w).double(), a.double() @ w.double().t()) < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("V,n", [(1024, 5), (3000, 5), (151936, 5), (9021, 160)])
+def test_top_k_of_about_what_a_list_holds(V, n):
+    """The search goes on in a list once 1024 values of the row are left: k below, at and above that, ties that do not fit,
+    unaligned rows, one and eight CTAs a row; then top-p among them, with a threshold that the sums' order cannot move."""
+    torch.manual_seed(V + n)
+    x = torch.randn(n, V + 3, device=DEV)[:, :V] * 3
+    x[2] = (x[2] * 2).round()                              # hundreds of ties at every value
+    ks = [min(k, V - 1) for k in (50, 1023, 1024, 1025, 700)]
+    k = torch.tensor([ks[r % 5] for r in range(n)], dtype=torch.int32, device=DEV)
+    got = x.clone()
+    ops.apply_top_k_top_p(got, k, None)
+    for r in range(n):
+        kth = x[r].topk(int(k[r])).values[-1]
+        assert torch.equal(got[r], torch.where(x[r] >= kth, x[r], -float("inf")))
+    # half of the mass: far from a value of the cumulative sum where the values are distinct
+    half = x.clone()
+    ops.apply_top_k_top_p(half, k, torch.full((n,), 0.5, device=DEV))
+    for r in (0, 1, 3, 4):
+        srt = got[r].double().sort(descending=True).values[: int(k[r])]
+        mass = torch.softmax(srt, 0).cumsum(0)
+        least, most = (int((mass < 0.5 + d).sum()) + 1 for d in (-1e-5, 1e-5))
+        assert least <= int(torch.isfinite(half[r]).sum()) <= most
+    assert ops.read_status() == 0
