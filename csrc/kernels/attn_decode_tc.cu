@@ -13,7 +13,7 @@
 // O^T stays in TMEM across tiles (16 fp32 columns); the running max is raised lazily (only
 // when a tile exceeds it by more than 2^8), and raising it rescales those 16 columns in
 // place. K and V tiles share one TMA ring of 128 x D bf16 slots, filled in the order the MMA warp
-// consumes them (K0 K1 V0 K2 V1 ...); two CTAs fit on an SM at head_dim 128. At head_dim 256 the
+// consumes them (K0 K1 V0 K2 V1 ...); two or three CTAs fit on an SM at head_dim 128. At head_dim 256 the
 // P V product runs as two M = 128 instructions (one per half of the head dim), O^T takes two
 // 16-column accumulators and one CTA fits on an SM.
 //
@@ -30,12 +30,12 @@ namespace b200 {
 
 static constexpr int kTok = 128;        // tokens per tile
 static constexpr int kNQ = 16;          // padded query heads (UMMA N)
-static constexpr int kSlots = 3;        // K/V ring slots
+static constexpr int kMostSlots = 3;    // K/V ring slots
 template <int D>
 struct DecodeTcSmem {
   static constexpr int slot_bytes = kTok * D * 2;      // one K or V tile
   static constexpr int q_bytes = (D / 64) * 2048;      // 16 query rows, 64-element chunks of 2 KB
-  static constexpr int p_bytes = 8192;                 // 2 buffers x (2 token halves x 2 KB)
+  static constexpr int p_bytes = 4096;                 // one buffer of P: 2 token halves x 2 KB
 };
 
 struct DecodeTcParams {
@@ -54,7 +54,7 @@ struct DecodeTcParams {
 
 struct alignas(8) DecodeTcBars {
   uint64_t q_full;
-  uint64_t kv_full[kSlots], kv_empty[kSlots];
+  uint64_t kv_full[kMostSlots], kv_empty[kMostSlots];
   uint64_t s_full[2], s_empty[2];
   uint64_t p_full[2], p_empty[2];
   uint64_t pv_done;
@@ -85,21 +85,23 @@ __device__ __forceinline__ float fast_exp2(float x) {
 
 // GP: the GQA group size rounded up to 4 / 8 / 16; the softmax only touches those columns of
 // S^T (the MMA's N stays 16, its minimum at 128 rows).
-template <int GP, int D>
-__global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
+// kSlots: of the ring. Two slots and one buffer of P (three and two otherwise) let three CTAs share an SM at head_dim 128, as many bytes
+// on the way as with two CTAs, and a third chain of loads, products and softmax that hides the others' latencies.
+template <int GP, int D, int kSlots>
+__global__ void __launch_bounds__(192, D == 128 ? (kSlots == 2 ? 3 : 2) : 1)
     attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
                           const __grid_constant__ CUtensorMap tmKV, DecodeTcParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   constexpr int kSlotBytes = DecodeTcSmem<D>::slot_bytes;
-  constexpr int kQBytes = DecodeTcSmem<D>::q_bytes;
+  constexpr int kQBytes = DecodeTcSmem<D>::q_bytes, kPBufs = kSlots - 1;
   constexpr int kChunks = D / 64;                    // 64-element (128-byte) chunks of the head dim
   constexpr int kChunkBytes = kTok * 128;            // one chunk of a K / V tile: 128 tokens x 128 bytes
   uint8_t* sKV = smem;                               // kSlots tiles
   uint8_t* sQ = sKV + kSlots * kSlotBytes;           // kChunks x 2 KB
-  uint8_t* sP = sQ + kQBytes;                        // 2 buffers * (2 halves * 2 KB)
-  DecodeTcBars* bars = reinterpret_cast<DecodeTcBars*>(sP + 8192);
+  uint8_t* sP = sQ + kQBytes;                        // kPBufs x (2 halves x 2 KB)
+  DecodeTcBars* bars = reinterpret_cast<DecodeTcBars*>(sP + kPBufs * 4096);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int b = blockIdx.x, hkv = blockIdx.y, split = blockIdx.z;
@@ -123,7 +125,7 @@ __global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
     mbar_fence_init();
   }
   // zero the P^T buffers once: rows >= G are never written and must stay finite
-  for (int i = threadIdx.x; i < 8192 / 16; i += blockDim.x)
+  for (int i = threadIdx.x; i < kPBufs * 4096 / 16; i += blockDim.x)
     reinterpret_cast<uint4*>(sP)[i] = make_uint4(0, 0, 0, 0);
   fence_proxy_async_smem();
   if (warp == 1) {
@@ -228,9 +230,9 @@ __global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
           const int i = j - 1;
           const int it = i == ntiles - 1 ? 2 * ntiles - 1 : 2 * i + 2, sl = it % kSlots;  // V(i)
           const uint32_t ph = (it / kSlots) & 1;
-          const int pb = i & 1;
+          const int pb = i % kPBufs;
           if (!(ok = mbar_wait_warp(&bars->kv_full[sl], ph, p.status))) break;
-          if (!(ok = mbar_wait_warp(&bars->p_full[pb], (i >> 1) & 1, p.status))) break;
+          if (!(ok = mbar_wait_warp(&bars->p_full[pb], (i / kPBufs) & 1, p.status))) break;
           tc_fence_after_sync();
           const uint32_t v_addr = smem_u32(sKV + sl * kSlotBytes);
           const uint32_t p_addr = smem_u32(sP + pb * 4096);
@@ -311,11 +313,11 @@ __global__ void __launch_bounds__(192, D == 128 ? 2 : 1)
             m[g] = tm;
           }
         }
-        // P^T buffer free? (PV of tile j-2 finished reading it.) This also bounds how far
+        // P^T buffer free? (PV of tile j - kPBufs finished reading it.) This also bounds how far
         // pv_done can lag: it has completed at least j-1 times here, so the parity wait of the
         // rescale below (its j-th completion) cannot be satisfied by an older phase.
-        const int pb = j & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars->p_empty[pb], ((j >> 1) & 1) ^ 1, p.status));
+        const int pb = j % kPBufs;
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->p_empty[pb], ((j / kPBufs) & 1) ^ 1, p.status));
         if (!ok) break;
         if (rescale && j > 0) {
           // all PV products issued so far must have landed before O^T is rescaled in place
@@ -425,21 +427,21 @@ struct DKeyHash {
   }
 };
 
-template <int D>
+template <int D, int kSlots>
 static cudaError_t launch_decode_tc(int G, dim3 grid, cudaStream_t stream, const CUtensorMap& tmQ,
                                     const CUtensorMap& tmKV, const DecodeTcParams& p) {
-  constexpr size_t smem = (size_t)kSlots * DecodeTcSmem<D>::slot_bytes + DecodeTcSmem<D>::q_bytes +
-                          DecodeTcSmem<D>::p_bytes + 1024 + sizeof(DecodeTcBars);
-  static_assert(smem <= 227 * 1024, "shared memory budget");
+  using L = DecodeTcSmem<D>;
+  constexpr size_t smem = (size_t)kSlots * L::slot_bytes + L::q_bytes + (kSlots - 1) * L::p_bytes + 1024 + sizeof(DecodeTcBars);
+  static_assert(smem <= 227 * 1024 && (kSlots != 2 || 3 * (smem + 1024) <= 228 * 1024), "shared memory budget");
   static PerDeviceOnce attr_once;
   if (attr_once.first()) {
-    cudaFuncSetAttribute(attn_decode_tc_kernel<4, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(attn_decode_tc_kernel<8, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(attn_decode_tc_kernel<16, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(attn_decode_tc_kernel<4, D, kSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(attn_decode_tc_kernel<8, D, kSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(attn_decode_tc_kernel<16, D, kSlots>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
-  if (G <= 4) return launch_pdl(attn_decode_tc_kernel<4, D>, grid, dim3(192), smem, stream, tmQ, tmKV, p);
-  if (G <= 8) return launch_pdl(attn_decode_tc_kernel<8, D>, grid, dim3(192), smem, stream, tmQ, tmKV, p);
-  return launch_pdl(attn_decode_tc_kernel<16, D>, grid, dim3(192), smem, stream, tmQ, tmKV, p);
+  const auto kernel = G <= 4 ? attn_decode_tc_kernel<4, D, kSlots> : G <= 8 ? attn_decode_tc_kernel<8, D, kSlots>
+                                                                            : attn_decode_tc_kernel<16, D, kSlots>;
+  return launch_pdl(kernel, grid, dim3(192), smem, stream, tmQ, tmKV, p);
 }
 
 }  // namespace b200
@@ -508,8 +510,12 @@ extern "C" int b200_attn_decode_tc(const void* q, int ldq, void* out, int ldo,
   dim3 grid(B, Hkv, splits);
   const int G = Hq / Hkv;
   cudaError_t le;
-  if (D == 128) le = launch_decode_tc<128>(G, grid, stream, tmQ, tmKV, p);
-  else le = launch_decode_tc<256>(G, grid, stream, tmQ, tmKV, p);
+  // More CTAs than two to an SM: three of them (us, two / three: 40 sequences of about 300 tokens, 8 kv heads, 320 CTAs 16.0 / 12.2;
+  // 120 of 75 20.6 / 16.3, of 340 38.1 / 35.4; 256 of 860 142 / 142). Fewer CTAs keep the deeper ring (13 of 225, 104 CTAs
+  // 6.5 / 7.0; 32 of 450, 256 CTAs 13.2 / 13.7; 30 of 3000, 240 CTAs 62.0 / 64.3).
+  if (D == 256) le = launch_decode_tc<256, 3>(G, grid, stream, tmQ, tmKV, p);
+  else if ((long long)B * Hkv * splits > 2 * b200_num_sms()) le = launch_decode_tc<128, 2>(G, grid, stream, tmQ, tmKV, p);
+  else le = launch_decode_tc<128, 3>(G, grid, stream, tmQ, tmKV, p);
   if (le != cudaSuccess) return -2;
   if (splits > 1)
     return b200_attn_decode_merge(tmp_o, tmp_lse, out, ldo, B, Hq, D, splits, stream);

@@ -959,3 +959,28 @@ def test_top_k_of_about_what_a_list_holds(V, n):
         least, most = (int((mass < 0.5 + d).sum()) + 1 for d in (-1e-5, 1e-5))
         assert least <= int(torch.isfinite(half[r]).sum()) <= most
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("B,Hkv", [(37, 8), (38, 8), (75, 4)])
+def test_attn_decode_of_two_and_of_three_ctas_an_sm(B, Hkv):
+    """Grids of 296 CTAs and of a few more (148 SMs): sequences of none to five tiles, scores that raise the reference maximum late."""
+    torch.manual_seed(B)
+    Hq, D, bs = Hkv * 4, 128, 16
+    lens = [(i * 53) % 600 for i in range(B)]
+    lens[1], lens[2], lens[3] = 1, 128, 129
+    cache, bt = _make_paged([max(n, 1) for n in lens], Hkv, D, bs)
+    cache[:, 0] *= torch.linspace(0.2, 6.0, cache.shape[0], device=DEV)[:, None, None, None].to(torch.bfloat16)
+    q = _rand(B, Hq * D)
+    sl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    out = ops.attn_decode(q, cache, block_table=bt, seq_lens=sl, num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, block_size=bs,
+                          scale=D ** -0.5, splits=1)
+    for b, n in enumerate(lens):
+        if n == 0:
+            assert not out[b].any()
+            continue
+        kv = cache[bt[b, : (n + bs - 1) // bs].long()]                       # [blocks, 2, bs, Hkv, D]
+        k, v = (kv[:, i].reshape(-1, Hkv, D)[:n].float().repeat_interleave(4, 1) for i in range(2))
+        s = torch.einsum("hd,thd->ht", q[b].float().view(Hq, D), k) * D ** -0.5
+        exp = torch.einsum("ht,thd->hd", torch.softmax(s, -1), v)
+        assert _rel_err(out[b].view(Hq, D), exp) < 8e-3                      # P and the result in bf16
+    assert ops.read_status() == 0
