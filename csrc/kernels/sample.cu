@@ -344,10 +344,61 @@ __device__ __forceinline__ float row_max(RowExchange<CTAS, 1>& ex, int turn, flo
   return v;
 }
 
+// Values of the whole row whose key is `least` or more, in the order of their columns, into every CTA's list (`list` has room for
+// them); their number. counts: one word per CTA of the cluster, warp_n: one per warp.
+static constexpr int kMostKept = 1024;
+template <int CTAS, int T>
+__device__ __forceinline__ int gather_kept(const RowSlice& s, uint32_t least, float* list, int* counts, int* warp_n) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = T / 32, rank = row_rank<CTAS>();
+  const int lo = (int)((long long)s.n * warp / warps), hi = (int)((long long)s.n * (warp + 1) / warps);
+  int n = 0;
+  for (int i = lo; i < hi; i += 32) n += __popc(__ballot_sync(0xffffffffu, i + lane < hi && fkey(s.v[i + lane]) >= least));
+  if (lane == 0) warp_n[warp] = n;
+  __syncthreads();
+  int before = 0, mine = 0;
+  for (int w = 0; w < warps; ++w) {
+    if (w < warp) before += warp_n[w];
+    mine += warp_n[w];
+  }
+  if constexpr (CTAS > 1) {
+    if (threadIdx.x < CTAS) {
+      const uint32_t to = mapa_u32(smem_u32(counts + rank), threadIdx.x);
+      asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(to), "r"(mine) : "memory");
+    }
+    cluster_sync_all();
+  } else {
+    if (threadIdx.x == 0) counts[0] = mine;
+    __syncthreads();
+  }
+  int total = 0;
+  for (int r = 0; r < CTAS; ++r) {
+    if (r < rank) before += counts[r];
+    total += counts[r];
+  }
+  for (int i = lo; i < hi; i += 32) {
+    const bool in = i + lane < hi && fkey(s.v[i + lane]) >= least;
+    const uint32_t who = __ballot_sync(0xffffffffu, in);
+    const int at = before + __popc(who & ((1u << lane) - 1));
+    before += __popc(who);
+    if (!in || at >= kMostKept) continue;
+    if constexpr (CTAS > 1) {
+      for (int r = 0; r < CTAS; ++r)
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_u32(smem_u32(list + at), r)), "f"(s.v[i + lane]) : "memory");
+    } else {
+      list[at] = s.v[i + lane];
+    }
+  }
+  if constexpr (CTAS > 1) cluster_sync_all();
+  else __syncthreads();
+  return total;
+}
+
 // top-k: radix select of the k-th largest key, two bits a pass (count based). top-p: the same search
 // for the largest threshold whose kept mass is >= p. Ties at the threshold are all kept (same as the sort-based rule for
-// distinct logits). Bound by the passes' barriers and shared-memory reads, about 2 us a pass, at most 32 passes: 40 rows of
-// 151936 with k = 50, p = 0.95 took 7717 us with a block of 256 threads per row that read the row from L2 for every bit.
+// distinct logits). A pass over the row is bound by its barriers and shared-memory reads, about 2 us, and there are 32 of them; once
+// no more than kMostKept values are at or above the top-k search's prefix, every CTA of the cluster gets them all and goes on
+// by itself, a fraction of a microsecond a pass. 40 rows of 151936 with k = 50, p = 0.95: 107 us, with all passes over the
+// row 264, with a block of 256 threads per row that read the row from L2 for every bit 7717.
 template <int CTAS, int T>
 __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(T)
     top_k_top_p_kernel(float* logits, int ld, int V, const int* __restrict__ top_k,
@@ -355,7 +406,11 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(T)
   extern __shared__ float4 stage_raw[];
   __shared__ RowExchange<CTAS, 1> ex1;
   __shared__ RowExchange<CTAS, 3> ex3;
+  __shared__ RowExchange<1, 1> own1;
+  __shared__ RowExchange<1, 3> own3;
   __shared__ float sh1[T / 32][1], sh3[T / 32][3], shm[32];
+  __shared__ float list[kMostKept];
+  __shared__ int counts[CTAS], warp_n[T / 32];
   const int row = blockIdx.x / CTAS;
   const int k = top_k ? top_k[row] : 0;
   const float pth = top_p ? top_p[row] : 1.f;
@@ -365,59 +420,75 @@ __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(T)
   const RowSlice s = load_row_slice<CTAS, T>(logits + (size_t)row * ld, V, reinterpret_cast<float*>(stage_raw));
   uint32_t thr_key = 0;
   int turn = 0;
+  // what is searched: the CTA's slice, its sums over the cluster, or the row's kept values, its sums within the CTA
+  const float* v = s.v;
+  int n = s.n;
+  constexpr bool kLists = CTAS > 1 || T > 256;         // (the rows that 256 threads pass are as short as a list)
+  bool alone = false;
+  const auto sum3 = [&](float (&c)[3]) {
+    if (kLists && alone) row_sum<1, T, 3>(own3, 0, c, sh3);
+    else row_sum<CTAS, T, 3>(ex3, turn++, c, sh3);
+  };
   if (do_k) {
     // find the largest key T such that count(key >= T) >= k
     uint32_t prefix = 0;
-    for (int bit = 30; bit >= 0; bit -= 2, ++turn) {
+    float kept = (float)V;
+    for (int bit = 30; bit >= 0; bit -= 2) {
+      if (kLists && !alone && kept <= (float)kMostKept && (CTAS > 1 || n > 2 * kMostKept)) {
+        n = gather_kept<CTAS, T>(s, prefix, list, counts, warp_n);
+        v = list;
+        alone = true;
+      }
       const uint32_t c1 = prefix | (1u << bit), c2 = prefix | (2u << bit), c3 = prefix | (3u << bit);
       int n1 = 0, n2 = 0, n3 = 0;
 #pragma unroll 4
-      for (int i = threadIdx.x; i < s.n; i += T) {
-        const uint32_t kk = fkey(s.v[i]);
+      for (int i = threadIdx.x; i < n; i += T) {
+        const uint32_t kk = fkey(v[i]);
         n1 += kk >= c1; n2 += kk >= c2; n3 += kk >= c3;
       }
       float c[3] = {(float)n1, (float)n2, (float)n3};
-      row_sum<CTAS, T, 3>(ex3, turn, c, sh3);
-      if (c[2] >= (float)k) prefix = c3;
-      else if (c[1] >= (float)k) prefix = c2;
-      else if (c[0] >= (float)k) prefix = c1;
+      sum3(c);
+      if (c[2] >= (float)k) { prefix = c3; kept = c[2]; }
+      else if (c[1] >= (float)k) { prefix = c2; kept = c[1]; }
+      else if (c[0] >= (float)k) { prefix = c1; kept = c[0]; }
     }
     thr_key = prefix;
   }
   if (do_p) {
     float mx = -FLT_MAX;
 #pragma unroll 4
-    for (int i = threadIdx.x; i < s.n; i += T) {
-      const float v = s.v[i];
-      if (fkey(v) >= thr_key) mx = fmaxf(mx, v);
+    for (int i = threadIdx.x; i < n; i += T) {
+      const float x = v[i];
+      if (fkey(x) >= thr_key) mx = fmaxf(mx, x);
     }
-    mx = row_max<CTAS>(ex1, 0, mx, shm);
+    mx = alone ? row_max<1>(own1, 0, mx, shm) : row_max<CTAS>(ex1, 0, mx, shm);
     float tot[1] = {0.f};
 #pragma unroll 4
-    for (int i = threadIdx.x; i < s.n; i += T) {
-      const float v = s.v[i];
-      if (fkey(v) >= thr_key) tot[0] += __expf(v - mx);
+    for (int i = threadIdx.x; i < n; i += T) {
+      const float x = v[i];
+      if (fkey(x) >= thr_key) tot[0] += __expf(x - mx);
     }
-    row_sum<CTAS, T, 1>(ex1, 1, tot, sh1);
+    if (alone) row_sum<1, T, 1>(own1, 1, tot, sh1);
+    else row_sum<CTAS, T, 1>(ex1, 1, tot, sh1);
     const float need = pth * tot[0];
     // largest key T (>= thr_key) with mass(key >= T) >= need
     uint32_t prefix = 0;
-    for (int bit = 30; bit >= 0; bit -= 2, ++turn) {
+    for (int bit = 30; bit >= 0; bit -= 2) {
       const uint32_t c1 = prefix | (1u << bit), c2 = prefix | (2u << bit), c3 = prefix | (3u << bit);
       const uint32_t least = c1 > thr_key ? c1 : thr_key;
       float m[3] = {0.f, 0.f, 0.f};
 #pragma unroll 4
-      for (int i = threadIdx.x; i < s.n; i += T) {
-        const float v = s.v[i];
-        const uint32_t kk = fkey(v);
+      for (int i = threadIdx.x; i < n; i += T) {
+        const float x = v[i];
+        const uint32_t kk = fkey(x);
         if (kk >= least) {
-          const float e = __expf(v - mx);
+          const float e = __expf(x - mx);
           m[0] += e;
           m[1] += kk >= c2 ? e : 0.f;
           m[2] += kk >= c3 ? e : 0.f;
         }
       }
-      row_sum<CTAS, T, 3>(ex3, turn, m, sh3);
+      sum3(m);
       if (m[2] >= need) prefix = c3;
       else if (m[1] >= need) prefix = c2;
       else if (m[0] >= need) prefix = c1;
