@@ -23,17 +23,23 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
 // ------------------------------------------------------------------------------------
-// conv1d forward. Grid (C / 128, ceil(T / kConvTokens)); a thread owns one channel and walks
-// the tokens of its block in order, so the three previous inputs stay in registers.
+// conv1d forward. Grid (C / (128 V), ceil(T / kConvTokens)); a thread owns V neighbouring channels and walks
+// the tokens of its block in order, so the three previous inputs stay in registers. Bound by the memory: eight tokens' inputs
+// are on their way at a time, and four channels make 8-byte accesses where strides and addresses allow (7600 x 10240: 193 us token by
+// token and channel by channel, 145 with eight tokens ahead, 104 in this form).
 // ------------------------------------------------------------------------------------
 static constexpr int kConvTokens = 32;
 
+template <int V> struct ConvVec { bf16 v[V]; };
+template <> struct alignas(8) ConvVec<4> { bf16 v[4]; };
+
+template <int V>
 __global__ void __launch_bounds__(128)
     gdn_conv1d_fwd_kernel(const bf16* __restrict__ x, long ldx, const bf16* __restrict__ w,
                           const bf16* __restrict__ state, const int* __restrict__ qsl,
                           const int* __restrict__ slots, const int* __restrict__ has_init,
                           bf16* __restrict__ out, long ldo, int n_seq, int T, int C) {
-  const int c = blockIdx.x * 128 + threadIdx.x;
+  const int c = (blockIdx.x * 128 + threadIdx.x) * V;
   const int t0 = blockIdx.y * kConvTokens;
   if (c >= C || t0 >= T) return;
   const int t1 = min(T, t0 + kConvTokens);
@@ -44,9 +50,14 @@ __global__ void __launch_bounds__(128)
     if (qsl[mid] <= t0) lo = mid; else hi = mid - 1;
   }
   int s = lo;
-  const uint2 wv = *reinterpret_cast<const uint2*>(w + (size_t)c * kConvK);
-  const float2 w01 = unpack_bf16x2(wv.x), w23 = unpack_bf16x2(wv.y);
-  float p1 = 0.f, p2 = 0.f, p3 = 0.f;   // x[t-1], x[t-2], x[t-3]
+  float2 w01[V], w23[V];
+  float p1[V], p2[V], p3[V];            // x[t-1], x[t-2], x[t-3]
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const uint2 wv = *reinterpret_cast<const uint2*>(w + (size_t)(c + e) * kConvK);
+    w01[e] = unpack_bf16x2(wv.x);
+    w23[e] = unpack_bf16x2(wv.y);
+  }
   int seq_begin = qsl[s], seq_end = qsl[s + 1];
   auto load_window = [&](int t) {
     // previous inputs of token t (first token handled by this thread in sequence s)
@@ -54,12 +65,25 @@ __global__ void __launch_bounds__(128)
     const bool init = has_init ? has_init[s] != 0 : true;
     const int slot = slots[s];
     const bf16* st = state + ((size_t)slot * C + c) * (kConvK - 1);   // [oldest, mid, newest]
-    auto prev = [&](int back) -> float {   // input `back` positions before t
-      if (pos - back >= 0) return __bfloat162float(x[(size_t)(t - back) * ldx + c]);
+    auto prev = [&](int back, int e) -> float {   // input `back` positions before t
+      if (pos - back >= 0) return __bfloat162float(x[(size_t)(t - back) * ldx + c + e]);
       if (!init || slot < 0) return 0.f;
-      return __bfloat162float(st[(kConvK - 1) + (pos - back)]);   // pos-back in [-3,-1]
+      return __bfloat162float(st[e * (kConvK - 1) + (kConvK - 1) + (pos - back)]);   // pos-back in [-3,-1]
     };
-    p1 = prev(1); p2 = prev(2); p3 = prev(3);
+#pragma unroll
+    for (int e = 0; e < V; ++e) { p1[e] = prev(1, e); p2[e] = prev(2, e); p3[e] = prev(3, e); }
+  };
+  auto load = [&](int t) { return *reinterpret_cast<const ConvVec<V>*>(x + (size_t)t * ldx + c); };
+  auto token = [&](int t, const ConvVec<V>& in) {
+    ConvVec<V> o;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const float xv = __bfloat162float(in.v[e]);
+      const float acc = w01[e].x * p3[e] + w01[e].y * p2[e] + w23[e].x * p1[e] + w23[e].y * xv;
+      o.v[e] = __float2bfloat16(silu_f(acc));
+      p3[e] = p2[e]; p2[e] = p1[e]; p1[e] = xv;
+    }
+    *reinterpret_cast<ConvVec<V>*>(out + (size_t)t * ldo + c) = o;
   };
   load_window(t0);
   for (int t = t0; t < t1; ++t) {
@@ -70,10 +94,16 @@ __global__ void __launch_bounds__(128)
       if (t < seq_end) load_window(t);
     }
     if (t >= seq_end) break;    // padding rows after the last sequence
-    const float xv = __bfloat162float(x[(size_t)t * ldx + c]);
-    const float acc = w01.x * p3 + w01.y * p2 + w23.x * p1 + w23.y * xv;
-    out[(size_t)t * ldo + c] = __float2bfloat16(silu_f(acc));
-    p3 = p2; p2 = p1; p1 = xv;
+    if (t + 8 <= min(t1, seq_end)) {
+      ConvVec<V> v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = load(t + i);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) token(t + i, v[i]);
+      t += 7;
+    } else {
+      token(t, load(t));
+    }
   }
 }
 
@@ -302,10 +332,12 @@ int b200_gdn_conv1d_fwd(const void* x, long ldx, const void* w, void* conv_state
                         int total_tokens, int C, cudaStream_t stream) {
   if (n_seq <= 0 || total_tokens <= 0) return 0;
   if (x == out || (C & 3)) return -1;
-  dim3 grid((C + 127) / 128, (total_tokens + kConvTokens - 1) / kConvTokens);
-  gdn_conv1d_fwd_kernel<<<grid, 128, 0, stream>>>((const bf16*)x, ldx, (const bf16*)w,
-                                                  (const bf16*)conv_state, qsl, slots, has_init,
-                                                  (bf16*)out, ldo, n_seq, total_tokens, C);
+  const bool four = !((ldx | ldo) & 3) && !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 7);
+  const int per = four ? 512 : 128;
+  dim3 grid((C + per - 1) / per, (total_tokens + kConvTokens - 1) / kConvTokens);
+  auto fwd = four ? gdn_conv1d_fwd_kernel<4> : gdn_conv1d_fwd_kernel<1>;
+  fwd<<<grid, 128, 0, stream>>>((const bf16*)x, ldx, (const bf16*)w, (const bf16*)conv_state, qsl, slots, has_init, (bf16*)out, ldo,
+                                n_seq, total_tokens, C);
   if (cudaGetLastError() != cudaSuccess) return -2;
   dim3 g2((C + 127) / 128, n_seq);
   gdn_conv1d_state_kernel<<<g2, 128, 0, stream>>>((const bf16*)x, ldx, (bf16*)conv_state, qsl, slots,

@@ -28,6 +28,7 @@ typedef __nv_bfloat16 bf16;
 
 static constexpr int kC = 64;      // chunk length
 static constexpr int kD = 128;     // Dk = Dv
+static constexpr int kAPitch = 68;  // of A in shared memory: rows in 16-byte pieces that take turns in the banks
 static constexpr int kScanThreads = 160;   // 4 compute warps + 1 control warp
 
 struct ScanBars {
@@ -58,26 +59,28 @@ struct PrepParams {
   int* status;
 };
 
-__global__ void __launch_bounds__(kScanThreads, 2)
+// Bound by its loads and stores (124 chunks x 48 heads: 0.7 GB, 107 us) and by the chain of the forward substitution, so three CTAs an
+// SM, and everything but the substitution goes to the two warps that it leaves idle. That launch took 735 us with the substitution in
+// shared memory and two lanes a column, 397 with columns in registers, 239 in this form.
+__global__ void __launch_bounds__(kScanThreads, 3)
     gdn_chunk_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                           const __grid_constant__ CUtensorMap tmV, PrepParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sKQ = smem;                    // 2 halves x (64 K rows + 64 Q rows) x 128 B
   uint8_t* sV = sKQ + 32768;              // 2 halves x 64 rows x 128 B
-  uint8_t* sT1 = sV + 16384;              // [i][j] T beta_j            (B operand, K-major)
-  uint8_t* sT2 = sT1 + 8192;              // [i][j] T beta_j e^{G_j}
-  float* sA = reinterpret_cast<float*>(sT2 + 8192);     // [64][65]
-  float* sT = sA + 64 * 65;                              // [64][65]
-  float* sG = sT + 64 * 65;                              // [64]
+  float* sA = reinterpret_cast<float*>(sV + 16384);      // [64][kAPitch], until T is complete
+  uint8_t* sT1 = sV + 16384;              // then [i][j] T beta_j       (B operand, K-major)
+  uint8_t* sT2 = sT1 + 8192;              // and  [i][j] T beta_j e^{G_j}
+  float* sG = sA + 64 * kAPitch;                         // [64]
   float* sBeta = sG + 64;                                // [64]
   ScanBars* bars = reinterpret_cast<ScanBars*>(sBeta + 64);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_index();
   const int n = blockIdx.x, hv = blockIdx.y;
   const int hk = hv / (p.Hv / p.Hk);
   const int tok0 = p.chunk_tok0[n], len = p.chunk_len[n];
-  const bool control = (tid == 128);
+  const bool control = warp == 4;          // (the whole warp; one elected lane issues)
 
   if (tid == 0) {
     mbar_init(&bars->load[0], 1);
@@ -87,16 +90,16 @@ __global__ void __launch_bounds__(kScanThreads, 2)
     mbar_fence_init();
   }
   if (warp == 4) {
-    tmem_alloc(&bars->tmem_base, 256);
+    tmem_alloc(&bars->tmem_base, 128);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = bars->tmem_base;
-  const uint32_t tmem_s = tmem, tmem_u = tmem + 64, tmem_w = tmem + 128;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
+  const uint32_t tmem_s = tmem, tmem_u = tmem, tmem_w = tmem + 64;   // (u over s, which has been read)
 
-  if (control) {
+  if (control && elect_one()) {
     mbar_expect_tx(&bars->load[0], 32768 + 16384);
     for (int h = 0; h < 2; ++h) {
       tma_load_2d(sKQ + h * 16384, &tmK, &bars->load[0], hk * kD + h * 64, tok0);
@@ -104,30 +107,37 @@ __global__ void __launch_bounds__(kScanThreads, 2)
       tma_load_2d(sV + h * 8192, &tmV, &bars->load[0], p.v_col0 + hv * kD + h * 64, tok0);
     }
   }
-  if (tid < 64) {
+  float gsum = 0.f;
+  if (tid < 64) {                          // in-chunk sums of g: of each warp, then the first warp's total on the second's
     const bool valid = tid < len;
-    sG[tid] = valid ? p.g[(size_t)(tok0 + tid) * p.Hv + hv] : 0.f;
+    gsum = valid ? p.g[(size_t)(tok0 + tid) * p.Hv + hv] : 0.f;
     sBeta[tid] = valid ? p.beta[(size_t)(tok0 + tid) * p.Hv + hv] : 0.f;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float before = __shfl_up_sync(0xffffffffu, gsum, o);
+      if ((tid & 31) >= o) gsum += before;
+    }
+    sG[tid] = gsum;
   }
   __syncthreads();
-  if (tid == 0) {
-    float acc = 0.f;
-    for (int i = 0; i < kC; ++i) { acc += sG[i]; sG[i] = acc; }
-  }
+  if (warp == 1) sG[tid] = gsum + sG[31];
   bool ok = true;
   if (control) {
-    ok = mbar_wait(&bars->load[0], 0, p.status);
+    ok = mbar_wait_warp(&bars->load[0], 0, p.status);
     if (ok) {
       tc_fence_after_sync();
       constexpr uint32_t idesc = umma_idesc_bf16(128, 64, 0, 0);
       const uint32_t a0 = smem_u32(sKQ);
+      if (elect_one()) {
 #pragma unroll
-      for (int kk = 0; kk < kD / 16; ++kk) {
-        const uint32_t off = (kk / 4) * 16384 + (kk % 4) * 32;
-        umma_bf16_ss(tmem_s, umma_desc_k_sw128(a0 + off, 1024), umma_desc_k_sw128(a0 + off, 1024), idesc, kk != 0);
+        for (int kk = 0; kk < kD / 16; ++kk) {
+          const uint32_t off = (kk / 4) * 16384 + (kk % 4) * 32;
+          umma_bf16_ss(tmem_s, umma_desc_k_sw128(a0 + off, 1024), umma_desc_k_sw128(a0 + off, 1024), idesc, kk != 0);
+        }
+        umma_commit(&bars->mma[0]);
       }
-      umma_commit(&bars->mma[0]);
-    } else {
+      __syncwarp();
+    } else if (tid == 128) {
       bars->failed = 1;
     }
   }
@@ -150,9 +160,15 @@ __global__ void __launch_bounds__(kScanThreads, 2)
       const int i = tid;
       const float gi = sG[i], bi = sBeta[i];
 #pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        const float kkv = __uint_as_float(j < 32 ? r0[j & 31] : r1[j & 31]);
-        sA[i * 65 + j] = (j < i) ? bi * __expf(gi - sG[j]) * kkv : 0.f;
+      for (int j4 = 0; j4 < 64; j4 += 4) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = j4 + e;
+          const float kkv = __uint_as_float(j < 32 ? r0[j & 31] : r1[j & 31]);
+          v[e] = (j < i) ? bi * __expf(gi - sG[j]) * kkv : 0.f;
+        }
+        *reinterpret_cast<float4*>(sA + i * kAPitch + j4) = make_float4(v[0], v[1], v[2], v[3]);
       }
     } else {
       const int i = tid - 64;
@@ -173,58 +189,52 @@ __global__ void __launch_bounds__(kScanThreads, 2)
         }
         reinterpret_cast<uint4*>(prow)[j8] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
-      // q' = q e^{G_i} Dk^-0.5 into the chunk-indexed buffer
-      const float f = __expf(gi) * scale;
-      const int tq = tok0 + (i < len ? i : 0);
-      const uint4* qrow = reinterpret_cast<const uint4*>(p.q + ((size_t)tq * p.Hk + hk) * kD);
-      uint4* qd = reinterpret_cast<uint4*>(p.qs + (((size_t)n * kC + i) * p.Hv + hv) * kD);
-#pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        uint4 v = qrow[c];
-        float2 a;
-        a = unpack_bf16x2(v.x); v.x = pack_bf16x2(a.x * f, a.y * f);
-        a = unpack_bf16x2(v.y); v.y = pack_bf16x2(a.x * f, a.y * f);
-        a = unpack_bf16x2(v.z); v.z = pack_bf16x2(a.x * f, a.y * f);
-        a = unpack_bf16x2(v.w); v.w = pack_bf16x2(a.x * f, a.y * f);
-        qd[c] = v;
-      }
     }
   }
   __syncthreads();
   const bool failed_a = bars->failed != 0;
 
-  // forward substitution: column c of T = (I + A)^-1 depends only on earlier entries of the
-  // same column, so a pair of lanes owns a column (even / odd j) and never waits on others.
-  if (tid < 128 && !failed_a) {
-    const int c = tid >> 1, half = tid & 1;
+  // Forward substitution: a thread owns a column of T = (I + A)^-1 and keeps it in registers; A's rows are read by all threads alike,
+  // four values a load. The other two warps write q' = q e^{G_i} Dk^-0.5 into the chunk-indexed buffer meanwhile.
+  if (tid < 64 && !failed_a) {
+    float t[kC];
+#pragma unroll
     for (int i = 0; i < kC; ++i) {
-      float acc = 0.f;   // the loop is empty for i <= c; the shuffle stays warp-uniform
-      for (int j = c + half; j < i; j += 2) acc += sA[i * 65 + j] * sT[j * 65 + c];
-      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-      const float v = i < c ? 0.f : (i == c ? 1.f : -acc);
-      if (half == 0) sT[i * 65 + c] = v;
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  if (tid < 128 && !failed_a) {
-    // B operands: row i, 32 columns per thread
-    const int i = tid >> 1, j0 = (tid & 1) * 32;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j8 = 0; j8 < 4; ++j8) {
-      uint32_t a[4], b[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = j0 + j8 * 8 + e * 2;
-        const float t0 = sT[i * 65 + j] * sBeta[j], t1 = sT[i * 65 + j + 1] * sBeta[j + 1];
-        a[e] = pack_bf16x2(t0, t1);
-        b[e] = pack_bf16x2(t0 * __expf(sG[j]), t1 * __expf(sG[j + 1]));
+      for (int j4 = 0; j4 < i; j4 += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(sA + i * kAPitch + j4);
+        acc[0] += a.x * t[j4];
+        if (j4 + 1 < i) acc[1] += a.y * t[j4 + 1];
+        if (j4 + 2 < i) acc[2] += a.z * t[j4 + 2];
+        if (j4 + 3 < i) acc[3] += a.w * t[j4 + 3];
       }
-      const uint32_t off = sw128_off(i, j0 + j8 * 8);
-      *reinterpret_cast<uint4*>(sT1 + off) = make_uint4(a[0], a[1], a[2], a[3]);
-      *reinterpret_cast<uint4*>(sT2 + off) = make_uint4(b[0], b[1], b[2], b[3]);
+      t[i] = (i == tid ? 1.f : 0.f) - ((acc[0] + acc[1]) + (acc[2] + acc[3]));
+    }
+    const float bj = sBeta[tid], ej = __expf(sG[tid]);
+    asm volatile("bar.sync 1, 64;" ::: "memory");        // A has been read
+#pragma unroll
+    for (int i = 0; i < kC; ++i) {
+      const float v = t[i] * bj;
+      const uint32_t off = sw128_off(i, tid);
+      *reinterpret_cast<bf16*>(sT1 + off) = __float2bfloat16(v);
+      *reinterpret_cast<bf16*>(sT2 + off) = __float2bfloat16(v * ej);
     }
     fence_proxy_async_smem();
+  } else if (tid >= 64 && tid < 128 && !failed_a) {
+    const int c = tid & 15;                              // 16 bytes of a row
+    bf16* qd = p.qs + ((size_t)n * kC * p.Hv + hv) * kD + c * 8;
+#pragma unroll 4
+    for (int i = (tid - 64) >> 4; i < kC; i += 4) {
+      const float f = __expf(sG[i]) * 0.08838834764831845f;
+      uint4 v = *reinterpret_cast<const uint4*>(sKQ + (c >> 3) * 16384 + 8192 + sw128_off(i, (c & 7) * 8));
+      float2 a;
+      a = unpack_bf16x2(v.x); v.x = pack_bf16x2(a.x * f, a.y * f);
+      a = unpack_bf16x2(v.y); v.y = pack_bf16x2(a.x * f, a.y * f);
+      a = unpack_bf16x2(v.z); v.z = pack_bf16x2(a.x * f, a.y * f);
+      a = unpack_bf16x2(v.w); v.w = pack_bf16x2(a.x * f, a.y * f);
+      *reinterpret_cast<uint4*>(qd + (size_t)i * p.Hv * kD) = v;
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -232,17 +242,20 @@ __global__ void __launch_bounds__(kScanThreads, 2)
     tc_fence_after_sync();
     constexpr uint32_t idesc = umma_idesc_bf16(128, 64, 1, 0);   // A = V^T / K^T, MN-major
     const uint32_t v0 = smem_u32(sV), k0 = smem_u32(sKQ), t1 = smem_u32(sT1), t2 = smem_u32(sT2);
+    if (elect_one()) {
 #pragma unroll
-    for (int kk = 0; kk < kC / 16; ++kk) {
-      umma_bf16_ss(tmem_u, umma_desc_mn_sw128(v0 + kk * 2048, 8192, 1024),
-                   umma_desc_k_sw128(t1 + kk * 32, 1024), idesc, kk != 0);
-    }
+      for (int kk = 0; kk < kC / 16; ++kk) {
+        umma_bf16_ss(tmem_u, umma_desc_mn_sw128(v0 + kk * 2048, 8192, 1024),
+                     umma_desc_k_sw128(t1 + kk * 32, 1024), idesc, kk != 0);
+      }
 #pragma unroll
-    for (int kk = 0; kk < kC / 16; ++kk) {
-      umma_bf16_ss(tmem_w, umma_desc_mn_sw128(k0 + kk * 2048, 16384, 1024),
-                   umma_desc_k_sw128(t2 + kk * 32, 1024), idesc, kk != 0);
+      for (int kk = 0; kk < kC / 16; ++kk) {
+        umma_bf16_ss(tmem_w, umma_desc_mn_sw128(k0 + kk * 2048, 16384, 1024),
+                     umma_desc_k_sw128(t2 + kk * 32, 1024), idesc, kk != 0);
+      }
+      umma_commit(&bars->mma[1]);
     }
-    umma_commit(&bars->mma[1]);
+    __syncwarp();
   }
   if (tid < 128 && !failed_a) {
     ok = mbar_wait(&bars->mma[1], 0, p.status);
@@ -269,11 +282,11 @@ __global__ void __launch_bounds__(kScanThreads, 2)
   __syncthreads();
   if (warp == 4) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, 256);
+    tmem_dealloc(tmem, 128);
   }
 }
 
-static constexpr size_t kPrepSmem = 32768 + 16384 + 8192 + 8192 + 2 * 64 * 65 * 4 + 2 * 64 * 4 + sizeof(ScanBars) + 1024;
+static constexpr size_t kPrepSmem = 32768 + 16384 + 64 * kAPitch * 4 + 2 * 64 * 4 + sizeof(ScanBars) + 1024;
 
 // ---------------------------------------------------------------------------------------
 // Sequential scan over the chunks of one (sequence, value head).
@@ -307,12 +320,12 @@ __global__ void __launch_bounds__(kScanThreads, 1)
   float* sGc = reinterpret_cast<float*>(sSlot + 2 * kSlotBytes);   // [2][64]
   ScanBars* bars = reinterpret_cast<ScanBars*>(sGc + 128);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_index();
   const int s = blockIdx.x / p.Hv, hv = blockIdx.x % p.Hv;
   const int hk = hv / (p.Hv / p.Hk);
   const int n0 = p.seq_chunk0[s], n1 = p.seq_chunk0[s + 1];
   const int nchunks = n1 - n0;
-  const bool control = (tid == 128);
+  const bool control = warp == 4;
   const int slot = p.slots[s];
   const bool init = slot >= 0 && (p.has_init ? p.has_init[s] != 0 : true);
 
@@ -331,7 +344,7 @@ __global__ void __launch_bounds__(kScanThreads, 1)
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = bars->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
   const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t tmem_h = tmem, tmem_x = tmem + 128, tmem_o = tmem + 192;
 
@@ -339,17 +352,20 @@ __global__ void __launch_bounds__(kScanThreads, 1)
     const int n = n0 + ci;
     uint8_t* base = sSlot + (ci & 1) * kSlotBytes;
     uint64_t* bar = &bars->load[ci & 1];
-    mbar_expect_tx(bar, kSlotBytes);
     const int tok0 = p.chunk_tok0[n];
-    for (int h = 0; h < 2; ++h) {
-      tma_load_2d(base + h * 8192, &tmW, bar, hv * kD + h * 64, n * kC);
-      tma_load_2d(base + 16384 + h * 8192, &tmQs, bar, hv * kD + h * 64, n * kC);
-      tma_load_2d(base + 32768 + h * 8192, &tmK, bar, hk * kD + h * 64, tok0);
+    if (elect_one()) {
+      mbar_expect_tx(bar, kSlotBytes);
+      for (int h = 0; h < 2; ++h) {
+        tma_load_2d(base + h * 8192, &tmW, bar, hv * kD + h * 64, n * kC);
+        tma_load_2d(base + 16384 + h * 8192, &tmQs, bar, hv * kD + h * 64, n * kC);
+        tma_load_2d(base + 32768 + h * 8192, &tmK, bar, hk * kD + h * 64, tok0);
+      }
+      tma_load_2d(base + 49152, &tmP, bar, 0, (n * p.Hv + hv) * kC);
     }
-    tma_load_2d(base + 49152, &tmP, bar, 0, (n * p.Hv + hv) * kC);
+    __syncwarp();
   };
 
-  int loads_issued = 0, loads_consumed = 0;   // control thread only
+  int loads_issued = 0, loads_consumed = 0;   // control warp only
   if (control && nchunks > 0) { issue_loads(0); loads_issued = 1; }
 
   // initial state -> TMEM (row t of h^T = state[slot][hv][t][:])
@@ -413,24 +429,27 @@ __global__ void __launch_bounds__(kScanThreads, 1)
     // ---- phase B: x = w h, o = q' h
     if (control) {
       if (ci + 1 < nchunks) { issue_loads(ci + 1); loads_issued = ci + 2; }   // that slot's MMAs are done
-      const bool got = mbar_wait(&bars->load[ci & 1], ph, p.status);
+      const bool got = mbar_wait_warp(&bars->load[ci & 1], ph, p.status);
       if (got) loads_consumed = ci + 1;
       if (got) {
         tc_fence_after_sync();
         constexpr uint32_t idesc = umma_idesc_bf16(128, 64, 0, 0);
         const uint32_t h0 = smem_u32(sH), w0 = smem_u32(slotp), q0 = smem_u32(slotp + 16384);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t ao = (kk / 4) * 16384 + (kk % 4) * 32, bo = (kk / 4) * 8192 + (kk % 4) * 32;
-          umma_bf16_ss(tmem_x, umma_desc_k_sw128(h0 + ao, 1024), umma_desc_k_sw128(w0 + bo, 1024), idesc, kk != 0);
-        }
+          for (int kk = 0; kk < kD / 16; ++kk) {
+            const uint32_t ao = (kk / 4) * 16384 + (kk % 4) * 32, bo = (kk / 4) * 8192 + (kk % 4) * 32;
+            umma_bf16_ss(tmem_x, umma_desc_k_sw128(h0 + ao, 1024), umma_desc_k_sw128(w0 + bo, 1024), idesc, kk != 0);
+          }
 #pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t ao = (kk / 4) * 16384 + (kk % 4) * 32, bo = (kk / 4) * 8192 + (kk % 4) * 32;
-          umma_bf16_ss(tmem_o, umma_desc_k_sw128(h0 + ao, 1024), umma_desc_k_sw128(q0 + bo, 1024), idesc, kk != 0);
+          for (int kk = 0; kk < kD / 16; ++kk) {
+            const uint32_t ao = (kk / 4) * 16384 + (kk % 4) * 32, bo = (kk / 4) * 8192 + (kk % 4) * 32;
+            umma_bf16_ss(tmem_o, umma_desc_k_sw128(h0 + ao, 1024), umma_desc_k_sw128(q0 + bo, 1024), idesc, kk != 0);
+          }
+          umma_commit(&bars->mma[0]);
         }
-        umma_commit(&bars->mma[0]);
-      } else {
+        __syncwarp();
+      } else if (tid == 128) {
         bars->failed = 1;
       }
     }
@@ -481,15 +500,18 @@ __global__ void __launch_bounds__(kScanThreads, 1)
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, 64, 0, 0);
       const uint32_t vs0 = smem_u32(sVs), vo0 = smem_u32(sVo);
       const uint32_t k0 = smem_u32(slotp + 32768), p0 = smem_u32(slotp + 49152);
+      if (elect_one()) {
 #pragma unroll
-      for (int kk = 0; kk < kC / 16; ++kk)
-        umma_bf16_ss(tmem_h, umma_desc_k_sw128(vs0 + kk * 32, 1024),
-                     umma_desc_mn_sw128(k0 + kk * 2048, 8192, 1024), idesc_h, 1);
+        for (int kk = 0; kk < kC / 16; ++kk)
+          umma_bf16_ss(tmem_h, umma_desc_k_sw128(vs0 + kk * 32, 1024),
+                       umma_desc_mn_sw128(k0 + kk * 2048, 8192, 1024), idesc_h, 1);
 #pragma unroll
-      for (int kk = 0; kk < kC / 16; ++kk)
-        umma_bf16_ss(tmem_o, umma_desc_k_sw128(vo0 + kk * 32, 1024), umma_desc_k_sw128(p0 + kk * 32, 1024),
-                     idesc_o, 1);
-      umma_commit(&bars->mma[1]);
+        for (int kk = 0; kk < kC / 16; ++kk)
+          umma_bf16_ss(tmem_o, umma_desc_k_sw128(vo0 + kk * 32, 1024), umma_desc_k_sw128(p0 + kk * 32, 1024),
+                       idesc_o, 1);
+        umma_commit(&bars->mma[1]);
+      }
+      __syncwarp();
     }
     // ---- phase E: write o
     if (tid < 128) {

@@ -140,3 +140,33 @@ def test_rmsnorm_gated():
     for gate in ("silu", "sigmoid"):
         G.rmsnorm_gated(x, z, w, out, gate=gate, heads=heads)
         assert _rel(out, G.ref_rmsnorm_gated(x, z, w, gate=gate, heads=heads)) < 1e-2
+
+
+@pytest.mark.parametrize("lens", [[1, 63, 64, 65], [7, 8, 9, 25, 31, 32, 33, 127], [3]])
+def test_prefill_at_the_edges_of_tiles(lens):
+    """Sequences around the 64 tokens of a chunk, the 32 of a block of the convolution and the eight that it loads at a time; three
+    padding rows after the last sequence."""
+    Hk, Hv, n, T = 1, 2, len(lens), sum(lens)
+    qsl = [0]
+    for m in lens:
+        qsl.append(qsl[-1] + m)
+    slots, has_init = [n - i for i in range(n)], [i % 2 for i in range(n)]
+    x, a, b, A_log, dt_bias = _gdn_inputs(T + 3, Hk, Hv, seed=7)
+    w = (torch.randn(x.shape[1], 4, device=DEV) * 0.5).to(torch.bfloat16)
+    cstate = torch.randn(n + 2, x.shape[1], 3, device=DEV).to(torch.bfloat16)
+    xc, new = torch.zeros_like(x), cstate.clone()
+    exp, exp_state = G.ref_conv1d(x[:T], w, cstate, qsl, slots, has_init)
+    G.conv1d_fwd(x, w, new, _i32(qsl), _i32(slots), _i32(has_init), xc)
+    assert _rel(xc[:T], exp) < 1e-2 and torch.equal(new, exp_state) and not xc[T:].any()
+    q, k, g, beta = G.ref_post_conv(xc[:T], Hk, Hv, a[:T], b[:T], A_log, dt_bias)
+    g, beta = g.contiguous(), beta.contiguous()
+    v = xc[:T, 2 * Hk * 128:].reshape(T, Hv, 128)
+    state = torch.randn(n + 2, Hv, 128, 128, device=DEV) * 0.1
+    st, out = state.clone(), torch.zeros(T, Hv, 128, dtype=torch.bfloat16, device=DEV)
+    G.chunk_scan(q, k, xc[:T], g, beta, st, qsl, _i32(slots), _i32(has_init), out, G.GdnWorkspace(torch.device(DEV), T, n, Hv),
+                 v_col0=2 * Hk * 128)
+    assert ops.read_status() == 0
+    for s in range(n):
+        at = slice(qsl[s], qsl[s + 1])
+        eo, es = G.ref_recurrent(q[at], k[at], v[at], g[at], beta[at], state[slots[s]] if has_init[s] else torch.zeros_like(state[0]))
+        assert _rel(out[at], eo) < 3e-2 and _rel(st[slots[s]], es) < 3e-2     # W, U and P in bf16, as in the test above
