@@ -1,6 +1,7 @@
 // NVFP4-weight x 16-bit-activation GEMM for decode-sized batches (M <= 128):
 // out[M, N] = A[M, K] * dequant(W)[N, K]^T, W = e2m1 nibbles * e4m3 scale per 16 * fp32 global.
 //
+// Two forms: K in blocks of 256 goes to the cluster kernel further down, the rest (and unaligned scales) to the stream kernel.
 // The packed weights are the only large stream (K / 2 bytes per row), so the kernel is built
 // around keeping them moving: TMA brings 256-row x 256-element packed blocks (32 KB) into a
 // ring; sixteen converter warps expand them to f16 with the hardware conversions
@@ -287,16 +288,21 @@ __global__ void __launch_bounds__(kWThreads, 1)
 }
 
 // ---------------------------------------------------------------------------------------
-// Up to 64 rows: 128 weight rows as the MMA's M, the batch (padded to 16) as its N, K split over a cluster, two CTAs per
+// K in blocks of 256: 128 weight rows as the MMA's M, the batch (padded to 16) as its N, K split over a cluster, two CTAs per
 // SM that fill each other's waits; the parts of K are summed from shared memory to shared memory instead of through a
-// workspace and a second kernel. Bound by the chain expansion - MMA - release of a 64-k tile, about 0.5 us each, of which
-// four MMAs and their barriers are 0.36 (measured with conversions, scale loads and split of the warps varied). us at
-// 9 / 64 rows, the reducing kernel included, against the form above (b200_gemm_w4a16 chooses):
-//   16480 x 5120 33.2 / 43.4 -> 31.8 / 33.9    5120 x 6144 19.9 / 26.5 -> 16.8 / 19.5
-//   34816 x 5120 72.0 / 57.4 -> 55.7 / 58.6    5120 x 17408 34.9 / 42.7 -> 36.6 / 39.5
+// workspace and a second kernel. The expanded weights go from registers to the tensor memory, a lane a weight row, and the MMA
+// reads them there: through shared memory they were written and read once more each, behind a proxy fence, and the expansion
+// by shifts and masks held the ALUs (a tile of 64 k took 380 cycles of an SM more; e2m1 conversions alone 7 % less time). What
+// is left is spread: without the conversions 9 % less, with one MMA of four 6 %, with a third raw stage nothing. Little shared
+// memory (45 KB at 16 rows) lets the next kernel's blocks come in early: a third raw stage costs 0.6 us. us at 9 / 64 / 128
+// rows, the cast of the batch included, for the form above / expanded into shared memory (up to 64 rows) / this one:
+//   16480 x 5120 33.4 41.4 47 / 26.3 29.0 / 18.6 20.7 23.8    5120 x 6144 18.7 25.2 29 / 14.8 17.8 / 11.3 13.9 17.6
+//   34816 x 5120 67.2 55.1 57 / 44.7 48.9 / 29.6 32.0 39.9    5120 x 17408 33.0 40.7 45 / 29.9 33.8 / 20.8 24.3 29.9
+//   4096 x 14336 25.2 29.1 32 / 26.4 29.8 / 18.2 21.4 26.4
 // ---------------------------------------------------------------------------------------
-static constexpr int kCRows = 128, kCRaw = kCRows * 128, kCExp = kCRows * 128;
-static constexpr int kCRS = 2, kCES = 3, kCAS = 12, kCConv = 8, kCThreads = (3 + kCConv) * 32, kCRowsMax = 64;
+static constexpr int kCRows = 128, kCRaw = kCRows * 128, kCExpCols = 32, kCAccCols = 128, kCTmemCols = 256;
+static constexpr int kCRS = 2, kCES = 4, kCAS = 6, kCActBytes = 49152, kCConv = 8, kCThreads = (3 + kCConv) * 32, kCRowsMax = 128;
+static_assert(kCAccCols + kCES * kCExpCols <= kCTmemCols);
 
 struct W4CParams {
   int M, N, K, mp, splits, act_stages;
@@ -314,7 +320,7 @@ struct alignas(8) W4CBars {
 
 template <int S>
 __device__ __forceinline__ void w4_reduce(const W4CParams& p, uint32_t partial, int rank, int tile, int warp, int lane) {
-  const float g = *p.gscale * 128.f;
+  const float g = *p.gscale;
   const int col = tile * kCRows + lane * 4;
   for (int m = rank + warp * S; m < p.M; m += (3 + kCConv) * S) {
     float4 a = sum_of<S>(partial + (uint32_t)m * (kCRows * 4) + lane * 16, 0);
@@ -335,8 +341,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ W4CBars bars;
-  uint8_t* sExp = smem;
-  uint8_t* sRaw = sExp + kCES * kCExp;
+  uint8_t* sRaw = smem;
   uint8_t* sAct = sRaw + kCRS * kCRaw;
   const int act_bytes = p.mp * 128;
   const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -353,11 +358,11 @@ __global__ void __launch_bounds__(kCThreads, 2)
     mbar_init(&bars.acc, 1);
     mbar_fence_init();
   }
-  if (warp == 1) { tmem_alloc(&bars.tmem_base, 64); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(&bars.tmem_base, kCTmemCols); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = bars.tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars.tmem_base, 0);
   pdl_wait();
   pdl_launch_dependents();
 
@@ -386,7 +391,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
       if (++as == p.act_stages) { as = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    const uint32_t idesc = umma_idesc_f16(kCRows, p.mp), acc = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t idesc = umma_idesc_f16(kCRows, p.mp);
     int as = 0;
     uint32_t ph = 0;
     bool ok = true;
@@ -395,11 +400,11 @@ __global__ void __launch_bounds__(kCThreads, 2)
       ok = mbar_wait_warp(&bars.act_full[as], ph, p.status) && mbar_wait_warp(&bars.exp_full[es], (e / kCES) & 1, p.status);
       if (!ok) break;
       tc_fence_after_sync();
-      const uint64_t wd = umma_desc_k_sw128(smem_u32(sExp + es * kCExp), 1024);
+      const uint32_t w = tmem + kCAccCols + es * kCExpCols;
       const uint64_t ad = umma_desc_k_sw128(smem_u32(sAct + as * act_bytes), 1024);
       if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f16_ss(acc, wd + 2 * k, ad + 2 * k, idesc, (e | k) != 0);
+        for (int k = 0; k < 4; ++k) umma_bf16_ts(tmem, w + 8 * k, ad + 2 * k, idesc, (e | k) != 0);
         umma_commit(&bars.exp_empty[es]);
         umma_commit(&bars.act_empty[as]);
         if (e == ne - 1) umma_commit(&bars.acc);
@@ -408,15 +413,12 @@ __global__ void __launch_bounds__(kCThreads, 2)
       if (++as == p.act_stages) { as = 0; ph ^= 1; }
     }
   } else {
-    // A nibble's three magnitude bits in bits 9 to 11 of an f16 are its value times 2^-14 (subnormals included), nibbles k and
-    // k + 4 of a word lie 16 bits apart: four shifts and masks expand two weights (in the order 0 4 1 5 2 6 3 7, which the
-    // cast of the batch follows). Times the block scale x 2^7 they are exact in f16 (6 significant bits, multiples of
-    // 2^-17 up to 21); the 2^7 that is missing joins the global scale.
-    constexpr uint32_t kMag = 0x0e000e00u, kSign = 0x80008000u;
-    // Four warps expand the even tiles of 64 k, four the odd ones, a thread a row: a warp's expansion ends in a fence, and
-    // the other half's work covers it.
+    // A weight (two significant bits) times its block scale (four) is exact in f16: multiples of 2^-10 up to 2688.
+    // Four warps expand the even tiles of 64 k, four the odd ones, a thread a row (its lane of
+    // the tensor memory): a warp's expansion ends in a wait for its stores, and the other half's work covers it.
     // The row's 16 block scales of 256 k come as one load, two blocks ahead.
-    const int ct = threadIdx.x - 64, r = ct & 127, half = ct >> 7;
+    const int r = (warp & 3) * 32 + lane, half = (warp - 2) >> 2;
+    const uint32_t expanded = tmem + ((uint32_t)((warp & 3) * 32) << 16) + kCAccCols;
     const uint4* sf_row = reinterpret_cast<const uint4*>(p.sf + (size_t)min(n0 + r, p.N - 1) * (p.K / 16)) + b0;
     uint4 sf_next = __ldg(sf_row), sf_after = __ldg(sf_row + min(1, nr - 1));
     bool ok = true;
@@ -435,23 +437,26 @@ __global__ void __launch_bounds__(kCThreads, 2)
         const uint4 ra[2] = {*reinterpret_cast<const uint4*>(raw + (((2 * sub) ^ (r & 7)) << 4)),        // (swizzled)
                              *reinterpret_cast<const uint4*>(raw + (((2 * sub + 1) ^ (r & 7)) << 4))};
         const uint32_t sfq = half ? sfw[2 * q + 1] : sfw[2 * q];
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars.exp_empty[es], ((e / kCES) & 1) ^ 1, p.status));
-        if (!ok) break;
-        uint8_t* dst = sExp + es * kCExp + r * 128;
+        uint32_t v[32];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const uint32_t s2 = hmul2_bits(cvt_e4m3x2((uint16_t)(sfq >> (16 * h))), 0x58005800u);             // scales x 2^7
+          const uint32_t s2 = cvt_e4m3x2((uint16_t)(sfq >> (16 * h)));
           const uint32_t sc[2] = {__byte_perm(s2, 0, 0x1010), __byte_perm(s2, 0, 0x3232)};
           const uint32_t words[4] = {ra[h].x, ra[h].y, ra[h].z, ra[h].w};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const uint32_t w = words[c], s = sc[c >> 1];
-            *reinterpret_cast<uint4*>(dst + (((h * 4 + c) ^ (r & 7)) << 4)) =
-                make_uint4(hmul2_bits(((w << 9) & kMag) | ((w << 12) & kSign), s), hmul2_bits(((w << 5) & kMag) | ((w << 8) & kSign), s),
-                           hmul2_bits(((w << 1) & kMag) | ((w << 4) & kSign), s), hmul2_bits(((w >> 3) & kMag) | (w & kSign), s));
+            uint32_t w[4];
+            cvt_e2m1x8(words[c], w);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[(h * 4 + c) * 4 + j] = hmul2_bits(w[j], sc[c >> 1]);
           }
         }
-        fence_proxy_async_smem();
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars.exp_empty[es], ((e / kCES) & 1) ^ 1, p.status));
+        if (!ok) break;
+        tc_fence_after_sync();
+        tmem_st_32x32b_x32(expanded + es * kCExpCols, v);
+        tmem_st_wait();
+        tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars.exp_full[es]);
       }
@@ -492,7 +497,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
   }
   if (p.splits > 1) cluster_sync_all();
   else __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, 64);
+  if (warp == 1) tmem_dealloc(tmem, kCTmemCols);
 }
 
 __global__ void w4s_splitk_reduce_kernel(const float* __restrict__ ws, int splits, int M, int N, bf16* out,
@@ -509,7 +514,7 @@ __global__ void w4s_splitk_reduce_kernel(const float* __restrict__ ws, int split
 
 // bf16 -> f16 with saturation (the MMA runs in f16; activations beyond the f16 range clamp).
 __global__ void __launch_bounds__(256)
-    cast_bf16_f16_kernel(const bf16* __restrict__ a, int lda, __half* __restrict__ out, int M, int K, int nibble_order) {
+    cast_bf16_f16_kernel(const bf16* __restrict__ a, int lda, __half* __restrict__ out, int M, int K) {
   pdl_wait();
   pdl_launch_dependents();
   const size_t total = (size_t)M * (K / 8);
@@ -526,11 +531,7 @@ __global__ void __launch_bounds__(256)
       __half2 h = __floats2half2_rn(f.x, f.y);
       o[j] = *reinterpret_cast<uint32_t*>(&h);
     }
-    if (nibble_order)      // 0 4 1 5 2 6 3 7: as the cluster kernel expands the weights
-      *reinterpret_cast<uint4*>(out + (size_t)m * K + c * 8) = make_uint4(__byte_perm(o[0], o[2], 0x5410), __byte_perm(o[0], o[2], 0x7632),
-                                                                          __byte_perm(o[1], o[3], 0x5410), __byte_perm(o[1], o[3], 0x7632));
-    else
-      *reinterpret_cast<uint4*>(out + (size_t)m * K + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(out + (size_t)m * K + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -577,26 +578,19 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
                  !(reinterpret_cast<uintptr_t>(out) & 7);
   int csplits = 1;
   if (cluster) {
-    // Both forms walk their part of K in steps of 64, in 0.62 (cluster) and 0.64 us a step; start, exchange and end take 6.0 and
-    // 8.9 us, and a row of the batch 0.05 and 0.12 us (the stream form's partials go through memory). So the cluster form
-    // may have a few steps more, but not where a cluster that fits beside its neighbours splits K too coarsely: us, stream /
-    // cluster form, 4096 x 14336 (28 against 40 steps) 26.8 / 31.6 at 9 rows and 30.7 / 34.4 at 64, 12288 x 4096 (24 against
-    // 32) 25.0 / 26.2 and 32.9 / 28.1, 2560 x 9728 (12 against 20) 17.5 / 18.7 and 23.3 / 21.6, 5120 x 6144 (16 and 16)
-    // 19.9 / 16.8 and 26.5 / 19.5. Grids beyond one wave have no partials to save: from 33 rows on the wider tiles win
-    // (34816 x 5120 at 64 rows 57.4 / 58.6).
+    // Always where it can: at 1 to 128 rows from 1024 x 4096 to 57344 x 8192 it is the faster form (figures above it).
     const int tiles = (N + kCRows - 1) / kCRows, blocks = K / 256;
     csplits = cluster_splits(tiles, blocks / 2);
-    const int more = 4 * ((blocks + csplits - 1) / csplits) - ne_per;
-    if (!(reinterpret_cast<uintptr_t>(out) & 15) && (100 * more > 460 + 11 * M || (M > 32 && tiles > sms))) cluster = false;
   }
-  if (!cluster && splits == 1 && (reinterpret_cast<uintptr_t>(out) & 15)) return -1;        // (the stream form's vectors)
+  // (the stream form's vectors; results of 65 and more rows are to be aligned in either form)
+  if ((!cluster || M > 64) && splits == 1 && (reinterpret_cast<uintptr_t>(out) & 15)) return -1;
   __half* a16 = reinterpret_cast<__half*>(workspace);
   {
     const size_t total = (size_t)M * (K / 8);
     int blocks = (int)((total + 255) / 256);
     if (blocks > sms * 4) blocks = sms * 4;
-    if (launch_pdl(cast_bf16_f16_kernel, dim3(blocks), dim3(256), 0, stream, (const bf16*)A, lda, a16, M, K,
-                   cluster ? 1 : 0) != cudaSuccess)
+    if (launch_pdl(cast_bf16_f16_kernel, dim3(blocks), dim3(256), 0, stream, (const bf16*)A, lda, a16, M, K) !=
+        cudaSuccess)
       return -2;
   }
   CUtensorMap tmW, tmA, tmS;
@@ -609,10 +603,10 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
     if (!encode_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, K / 2, kCRows, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&tmA, a16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, M, K, K, c.mp, 64, CU_TENSOR_MAP_SWIZZLE_128B))
       return -3;
-    c.act_stages = 24576 / (c.mp * 128) < kCAS ? 24576 / (c.mp * 128) : kCAS;
-    const size_t smem = (size_t)kCES * kCExp + (size_t)c.act_stages * c.mp * 128 + (size_t)kCRS * kCRaw + 1024;
+    c.act_stages = kCActBytes / (c.mp * 128) < kCAS ? kCActBytes / (c.mp * 128) : kCAS;
+    const size_t smem = (size_t)kCRS * kCRaw + (size_t)c.act_stages * c.mp * 128 + 1024;       // (the partials: 512 bytes a row, over both)
     static PerDeviceOnce once;
-    if (once.first()) cudaFuncSetAttribute(gemm_w4a16_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+    if (once.first()) cudaFuncSetAttribute(gemm_w4a16_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCRS * kCRaw + kCActBytes + 1024);
     return launch_cluster_pdl(gemm_w4a16_cluster_kernel, tiles * c.splits, c.splits, kCThreads, smem, stream, tmW, tmA, c) ==
                    cudaSuccess ? 0 : -2;
   }

@@ -121,6 +121,21 @@ def test_w4a16_stream_and_cluster(M, N, K):
                          out=room[4:].view(M, N))
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 8, 256), (80, 136, 512), (97, 1032, 2304), (112, 264, 14336), (128, 4104, 4096), (128, 38016, 256)])
+def test_w4a16_of_many_rows_over_a_cluster(M, N, K):
+    """65 to 128 rows: paddings to 16 that leave three to six stages of the batch, ragged column tiles, grids beyond one wave."""
+    torch.manual_seed(15)
+    packed = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device=DEV)
+    sf = torch.randint(0x00, 0x7f, (N, K // 16), dtype=torch.uint8, device=DEV)          # every scale, subnormal ones and 448 too
+    g = torch.full((1,), 1e-3, device=DEV)
+    a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
+    bias = torch.randn(N, device=DEV).to(torch.bfloat16)
+    w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
+    out = Q.gemm_w4a16(a, packed, sf, g, bias=bias)
+    assert ops.read_status() == 0
+    assert _within_sum_error(out, a64, w64, a64 @ w64.t() + bias.double(), 2**-25 * w64.abs().sum(1))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 16), (17, 520, 144), (65, 136, 4112), (128, 4104, 8192)])
 @pytest.mark.parametrize("per_token,per_channel", [(False, False), (True, True)])
 def test_gemm_fp8_over_a_cluster(M, N, K, per_token, per_channel):
