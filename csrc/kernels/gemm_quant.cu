@@ -210,25 +210,36 @@ __device__ __forceinline__ float e2m1_value(uint32_t code) {
   const float v = mag < 2 ? 0.5f * (float)mag : (float)(2 + (mag & 1)) * (float)(1 << ((mag >> 1) - 1)) * 0.5f;
   return (code & 8u) ? -v : v;
 }
-// Whole-matrix expansion: packed [N, K/2] + scales [N, K/16] -> bf16 [N, K].
-__global__ void nvfp4_dequant_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict__ sf,
-                                     const float* __restrict__ gscale, bf16* __restrict__ out, long N,
-                                     int K) {
-  const long groups = N * (long)(K / 16);
+// Whole-matrix expansion: packed [N, K/2] + scales [N, K/16] -> bf16 [N, K]. Bound by the memory: a thread takes eight values, so that
+// neighbours write neighbouring 16 bytes, four times at once, and the conversions are the hardware's (34816 x 5120, 0.46 GB: 147 us
+// with values computed from the code's bits, 97 in this form).
+__global__ void __launch_bounds__(256)
+    nvfp4_dequant_kernel(const uint32_t* __restrict__ packed, const uint8_t* __restrict__ sf, const float* __restrict__ gscale,
+                         uint4* __restrict__ out, long words) {
   const float g = *gscale;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < groups; i += (long)gridDim.x * blockDim.x) {
-    const float s = e4m3_to_float(sf[i]) * g;
-    const uint2 raw = reinterpret_cast<const uint2*>(packed)[i];   // 8 bytes = 16 values
-    uint32_t w[8];
-    const uint32_t words[2] = {raw.x, raw.y};
+  const long step = (long)gridDim.x * blockDim.x;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < words; i += 4 * step) {
+    uint32_t w[4];
+    uint8_t code[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t byte = (words[j >> 2] >> ((j & 3) * 8)) & 0xffu;
-      w[j] = pack_bf16x2(e2m1_value(byte & 15u) * s, e2m1_value(byte >> 4) * s);
+    for (int u = 0; u < 4; ++u) {
+      const long at = i + u * step < words ? i + u * step : i;
+      w[u] = packed[at];
+      code[u] = sf[at >> 1];
     }
-    uint4* o = reinterpret_cast<uint4*>(out + i * 16);
-    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i + u * step >= words) break;
+      const float s = e4m3_to_float(code[u]) * g;
+      uint32_t h[4];
+      cvt_e2m1x8(w[u], h);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h[j]));
+        h[j] = pack_bf16x2(v.x * s, v.y * s);
+      }
+      out[i + u * step] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
   }
 }
 
@@ -638,11 +649,10 @@ int b200_nvfp4_dequant(const void* packed, const void* sf, const float* gscale, 
                        cudaStream_t stream) {
   if (N <= 0 || K <= 0) return 0;
   if (K & 15) return -1;
-  const long groups = N * (long)(K / 16);
-  long blocks = (groups + 255) / 256;
+  const long words = N * (long)(K / 8);
+  long blocks = (words + 1023) / 1024;
   if (blocks > (long)b200_num_sms() * 16) blocks = (long)b200_num_sms() * 16;
-  nvfp4_dequant_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const uint8_t*)packed, (const uint8_t*)sf, gscale,
-                                                             (bf16*)out, N, K);
+  nvfp4_dequant_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const uint32_t*)packed, (const uint8_t*)sf, gscale, (uint4*)out, words);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
