@@ -18,7 +18,6 @@ namespace b200 {
 typedef __nv_bfloat16 bf16;
 static constexpr int kConvK = 4;
 
-__device__ __forceinline__ float silu_f(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
@@ -80,7 +79,7 @@ __global__ void __launch_bounds__(128)
     for (int e = 0; e < V; ++e) {
       const float xv = __bfloat162float(in.v[e]);
       const float acc = w01[e].x * p3[e] + w01[e].y * p2[e] + w23[e].x * p1[e] + w23[e].y * xv;
-      o.v[e] = __float2bfloat16(silu_f(acc));
+      o.v[e] = __float2bfloat16(silu_of(acc));
       p3[e] = p2[e]; p2[e] = p1[e]; p1[e] = xv;
     }
     *reinterpret_cast<ConvVec<V>*>(out + (size_t)t * ldo + c) = o;
@@ -155,7 +154,7 @@ __global__ void __launch_bounds__(128)
   const uint2 wv = *reinterpret_cast<const uint2*>(w + (size_t)c * kConvK);
   const float2 w01 = unpack_bf16x2(wv.x), w23 = unpack_bf16x2(wv.y);
   const float acc = w01.x * s0 + w01.y * s1 + w23.x * s2 + w23.y * xv;
-  out[(size_t)b * ldo + c] = __float2bfloat16(silu_f(acc));
+  out[(size_t)b * ldo + c] = __float2bfloat16(silu_of(acc));
   st[0] = st[1];
   st[1] = st[2];
   st[2] = xb;
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(128)
     const float2 f0 = unpack_bf16x2(v.x), f1 = unpack_bf16x2(v.y);
     const float2 z0 = unpack_bf16x2(zv.x), z1 = unpack_bf16x2(zv.y);
     const float2 w0 = unpack_bf16x2(wv.x), w1 = unpack_bf16x2(wv.y);
-    auto gate = [&](float t) { return gate_kind == 0 ? silu_f(t) : sigmoid_f(t); };
+    auto gate = [&](float t) { return gate_kind == 0 ? silu_of(t) : sigmoid_f(t); };
     uint2 o;
     o.x = pack_bf16x2(f0.x * inv * w0.x * gate(z0.x), f0.y * inv * w0.y * gate(z0.y));
     o.y = pack_bf16x2(f1.x * inv * w1.x * gate(z1.x), f1.y * inv * w1.y * gate(z1.y));
