@@ -493,6 +493,7 @@ int b200_delta_chunk(const B200Delta* a, void* tp, void* gc, cudaStream_t stream
 int b200_gemm_gated_apart(int M, int N);
 int b200_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* out, int ldo, int M, int N, int K, int kind, int force_path, cudaStream_t stream);
 int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo, const float* a_scale, const float* w_scale, int w_scale_per_channel, const void* bias, int M, int N, int K, cudaStream_t stream);
+int b200_gemm_fp8_gated(const void* A, int lda, const void* W, int ldw, void* out, int ldo, const float* a_scale, const float* w_scale, int w_scale_per_channel, int M, int N, int K, int act_kind, cudaStream_t stream);
 int b200_gemm_bf16_batched(const void* A, int lda, int a_batch_cols, const void* W, int ldw, void* out, int ldo, long long out_batch_stride, int M, int N, int K, int batch, cudaStream_t stream);
 // ---- gemm_quant.cu
 int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int ldo, const float* a_scale, const float* w_scale, int w_scale_per_channel, const void* bias, int M, int N, int K, cudaStream_t stream);

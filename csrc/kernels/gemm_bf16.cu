@@ -1544,9 +1544,9 @@ extern "C" int b200_gemm_gated_apart(int M, int N) {
 
 // e4m3 x e4m3 -> bf16 on the CTA-pair kernel (M > 256): out = (A W^T) * a_scale * w_scale (+ bias).
 // Reference: MatmulFp8CublasLt / MatmulFp8Cutlass in src/vt/cuda/cuda_matmul.cu.
-extern "C" int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo,
-                                  const float* a_scale, const float* w_scale, int w_scale_per_channel,
-                                  const void* bias, int M, int N, int K, cudaStream_t stream) {
+static int gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo, const float* a_scale,
+                         const float* w_scale, int w_scale_per_channel, const void* bias, int M, int N, int K, int act_fuse,
+                         cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K & 15) || (lda & 15) || (ldw & 15) || (N & 7) || (ldo & 7)) return -1;
   GemmParams p{};
@@ -1563,7 +1563,28 @@ extern "C" int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw
   if (!encode_tmap_2d(&tA, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, lda, kBM, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !encode_tmap_2d(&tB, W, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, ldw, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B))
     return -3;
+  p.act_fuse = act_fuse;
   return launch_pair<256, true>(tA, tA, tB, p, stream);
+}
+
+extern "C" int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo,
+                                  const float* a_scale, const float* w_scale, int w_scale_per_channel,
+                                  const void* bias, int M, int N, int K, cudaStream_t stream) {
+  return gemm_fp8_pair(A, lda, W, ldw, out, ldo, a_scale, w_scale, w_scale_per_channel, bias, M, N, K, 0, stream);
+}
+
+// The same with act(gate) * up in the epilogue: W's rows come in blocks of [128 gate | 128 up], out is [M, N / 2]. Both halves are
+// rounded to bf16 first, so the result has the bytes that the product and the activation kernel after it give. Against those two
+// it saves writing and reading [M, N] (8192 rows, 28672 x 4096, with the row quantisation that
+// follows: 819 -> 744 us; 3792 rows 398 -> 360; 300 rows 66 -> 64).
+extern "C" int b200_gemm_fp8_gated(const void* A, int lda, const void* W, int ldw, void* out, int ldo,
+                                   const float* a_scale, const float* w_scale, int w_scale_per_channel, int M, int N,
+                                   int K, int act_kind, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((N & 255) || act_kind < 0) return -1;
+  const uintptr_t scale_at = w_scale_per_channel & 1 ? reinterpret_cast<uintptr_t>(w_scale) : 0;
+  if ((reinterpret_cast<uintptr_t>(out) | scale_at) & 15) return -1;
+  return gemm_fp8_pair(A, lda, W, ldw, out, ldo, a_scale, w_scale, w_scale_per_channel, nullptr, M, N, K, act_kind + 1, stream);
 }
 
 // Same GEMM with the tensor-parallel prologue / epilogue described by `tp`.

@@ -195,12 +195,20 @@ int b200_dense_layer(const B200DenseLayerWeights* w, const B200DenseStep* s, cud
     if (!w->gate_up_scale || !w->down_scale) return -1;
     B200_TRY(b200_quant_fp8_rowwise(s->hidden, H, s->resid, w->ln2, s->eps, s->gemma, 1, 0, s->fp8_act, H,
                                     s->fp8_scales, T, H, stream));
-    B200_TRY(b200_gemm_fp8(s->fp8_act, H, w->gate_up, H, s->gate_up_buf, 2 * I, (const float*)s->fp8_scales,
-                           w->gate_up_scale, kFp8Scales, nullptr, T, 2 * I, H, stream));
-    // act(gate) * up and its quantisation in one kernel
-    B200_TRY(b200_quant_fp8_rowwise(s->gate_up_buf, 2 * I, nullptr, nullptr, 0.f, 0, 2,
-                                    s->act_kind | (s->gate_up_interleaved ? 0x100 : 0), s->fp8_act, I,
-                                    s->fp8_scales, T, I, stream));
+    // From 257 rows on (the CTA pairs' product) the activation goes into the epilogue, below that into the quantisation: the
+    // cluster's and the 128-row tiles' epilogues hold no gate beside its up half.
+    if (s->gate_up_interleaved && T > 256 && !(I & 127)) {
+      B200_TRY(b200_gemm_fp8_gated(s->fp8_act, H, w->gate_up, H, s->act, I, (const float*)s->fp8_scales, w->gate_up_scale, kFp8Scales,
+                                   T, 2 * I, H, s->act_kind, stream));
+      B200_TRY(b200_quant_fp8_rowwise(s->act, I, nullptr, nullptr, 0.f, 0, 0, 0, s->fp8_act, I, s->fp8_scales, T, I, stream));
+    } else {
+      B200_TRY(b200_gemm_fp8(s->fp8_act, H, w->gate_up, H, s->gate_up_buf, 2 * I, (const float*)s->fp8_scales,
+                             w->gate_up_scale, kFp8Scales, nullptr, T, 2 * I, H, stream));
+      // act(gate) * up and its quantisation in one kernel
+      B200_TRY(b200_quant_fp8_rowwise(s->gate_up_buf, 2 * I, nullptr, nullptr, 0.f, 0, 2,
+                                      s->act_kind | (s->gate_up_interleaved ? 0x100 : 0), s->fp8_act, I,
+                                      s->fp8_scales, T, I, stream));
+    }
     B200_TRY(b200_gemm_fp8(s->fp8_act, I, w->down, I, s->hidden, H, (const float*)s->fp8_scales, w->down_scale, kFp8Scales,
                            nullptr, T, H, I, stream));
     return launches;

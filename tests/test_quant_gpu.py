@@ -333,3 +333,18 @@ def test_nvfp4_plan_cache_and_autotune(monkeypatch):
     b = Q.gemm_nvfp4(ap, sfa, g_a, wp, sfw, g_w, n_tile=384 - Q._NVFP4_PLANS[(64, N, K)])
     assert torch.equal(a, b)                  # the tile width changes the schedule, not the sums
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 256, 16), (300, 1280, 528), (512, 2304, 4096), (4097, 5632, 1024)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_gemm_fp8_with_the_activation_in_its_epilogue(M, N, K, kind):
+    """The bytes of the product followed by the activation: one pair of tiles, ragged rows, tiles shared by parts of K, many waves."""
+    torch.manual_seed(16)
+    a8 = (torch.randn(M, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    w8 = (torch.randn(N, K, device=DEV) * 8).to(torch.float8_e4m3fn)
+    sa, sw = torch.rand(M, device=DEV) * 1e-3, torch.rand(N, device=DEV) * 1e-2
+    two = ops.act_and_mul(Q.gemm_fp8(a8, w8, sa, sw), kind, interleaved=True)
+    out = torch.empty(M, N // 2, dtype=torch.bfloat16, device=DEV)
+    Q.gemm_fp8_gated(a8, w8, sa, sw, kind, out)
+    assert ops.read_status() == 0
+    assert torch.equal(out, two)

@@ -17,6 +17,7 @@ def _declare():
         return
     P, I, L, F, Z = _lib.P, _lib.I, _lib.L, _lib.F, _lib.Z
     _lib.declare("b200_gemm_fp8", [P, I, P, I, P, I, P, P, I, P, I, I, I, P], I)
+    _lib.declare("b200_gemm_fp8_gated", [P, I, P, I, P, I, P, P, I, I, I, I, I, P], I)
     _lib.declare("b200_nvfp4_dequant", [P, P, P, P, L, I, P], I)
     _lib.declare("b200_gemm_w4a16", [P, I, P, P, P, P, I, P, I, I, I, P, Z, P], I)
     _lib.declare("b200_gemm_nvfp4", [P, P, P, P, P, P, P, I, P, I, I, I, I, P, Z, P], I)
@@ -44,6 +45,16 @@ def gemm_fp8(a8, w8, a_scale, w_scale, out=None, bias=None):
     check(lib().b200_gemm_fp8(ptr(a8), a8.stride(0), ptr(w8), w8.stride(0), ptr(out), out.stride(0),
                               ptr(a_scale), ptr(w_scale), flags, ptr(bias), M, N, K,
                               stream_ptr()), "gemm_fp8")
+    return out
+
+
+def gemm_fp8_gated(a8, w8, a_scale, w_scale, kind, out):
+    """``act(gate) * up`` of ``gemm_fp8``'s rows, for weights in blocks of [128 gate | 128 up] rows."""
+    _declare()
+    M, K = a8.shape
+    flags = int(w_scale.numel() > 1) | (2 if a_scale.numel() == M else 0)
+    check(lib().b200_gemm_fp8_gated(ptr(a8), a8.stride(0), ptr(w8), w8.stride(0), ptr(out), out.stride(0), ptr(a_scale), ptr(w_scale),
+                                    flags, M, w8.shape[0], K, kind, stream_ptr()), "gemm_fp8_gated")
     return out
 
 
