@@ -8,8 +8,7 @@
 // (cvt.rn.f16x2.e2m1x2 for two nibbles, cvt.rn.f16x2.e4m3x2 for two scales, one HMUL2 per two
 // elements) straight into 128-byte-swizzled K-major tiles; one thread issues f16 tcgen05 MMAs
 // with the (pre-cast f16, zero-padded) batch as the 128-row operand and 256 weight rows as the N
-// operand - an MMA instruction costs about the same whatever its N, so the wide side is where the
-// weights go. value x block scale is exact in f16 (at most 6 significant bits, magnitude <= 2688);
+// operand. value x block scale is exact in f16 (at most 6 significant bits, magnitude <= 2688);
 // the fp32 global scale is applied to the accumulators in the epilogue. Each converter thread
 // reads its four block scales of a stage as one word, one stage ahead. Split-K over blockIdx.y
 // with fp32 partials.

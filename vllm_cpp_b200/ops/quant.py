@@ -70,7 +70,7 @@ def nvfp4_dequant(packed, sf, gscale, out=None):
 
 def gemm_w4a16(a, packed, sf, gscale, out=None, bias=None, scratch=None):
     """a bf16 [M, K]; packed uint8 [N, K/2]; sf e4m3 bytes [N, K/16]; gscale fp32 [1] (multiplier).
-    M <= 128 runs the fused expand-in-shared-memory kernel; larger M expands the matrix into
+    M <= 128 expands the weights inside the product; larger M expands the matrix into
     ``scratch`` (bf16 [N, K]) once and runs the bf16 GEMM."""
     _declare()
     from . import gemm
