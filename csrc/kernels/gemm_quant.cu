@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(128)
       float a = __bfloat162float(src[e]);
       if (mode == 1) {
         const float u = __bfloat162float(src[K + e]);
-        a = __bfloat162float(__float2bfloat16(a / (1.f + __expf(-a)) * u));
+        a = __bfloat162float(__float2bfloat16(silu_of(a) * u));
       } else if (mode == 2) {
         // attention output gate: x * sigmoid(gate), rounded to bf16 as the separate kernel would
         const float g = __bfloat162float(gate[t * ldg + (long)gidx * 16 + e]);

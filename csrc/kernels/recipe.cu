@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) fused_chain_kernel(const __grid_constant_
         const uint32_t* w = reinterpret_cast<const uint32_t*>((const bf16*)prog.operands[st.operand].ptr);
         uint32_t* d = reinterpret_cast<uint32_t*>(reg(st.dst));
         const int kind = st.flag;
-        auto gate = [&](float t) { return kind == 0 ? t / (1.f + __expf(-t)) : 1.f / (1.f + __expf(-t)); };
+        auto gate = [&](float t) { return kind == 0 ? silu_of(t) : 1.f / (1.f + __expf(-t)); };
         for (int i = threadIdx.x; i < (W >> 1); i += blockDim.x) {
           const float2 x = unpack_bf16x2(a[i]), zz = unpack_bf16x2(z[i]), y = unpack_bf16x2(w[i]);
           d[i] = pack_bf16x2(x.x * inv * y.x * gate(zz.x), x.y * inv * y.y * gate(zz.y));
