@@ -16,6 +16,7 @@ int b200_num_sms();
 // Call once per device before the first stream capture. 0 on success.
 int b200_init_device();
 int b200_read_status();
+size_t b200_tmem_bound_smem(size_t smem, int fit, int cols);
 void* b200_status_ptr();
 const char* b200_kernel_arch();
 
@@ -497,6 +498,7 @@ int b200_gemm_fp8_gated(const void* A, int lda, const void* W, int ldw, void* ou
 int b200_gemm_bf16_batched(const void* A, int lda, int a_batch_cols, const void* W, int ldw, void* out, int ldo, long long out_batch_stride, int M, int N, int K, int batch, cudaStream_t stream);
 // ---- gemm_quant.cu
 int b200_gemm_fp8(const void* A, int lda, const void* W, int ldw, void* out, int ldo, const float* a_scale, const float* w_scale, int w_scale_per_channel, const void* bias, int M, int N, int K, cudaStream_t stream);
+int b200_w4a16_ctas_an_sm(int M);
 int b200_nvfp4_dequant(const void* packed, const void* sf, const float* gscale, void* out, long N, int K, cudaStream_t stream);
 int b200_fp8_init_device();
 int b200_quant_fp8_dynamic(const void* x, long ldx, void* scratch, void* out, long ldo, long T, int H, cudaStream_t stream);

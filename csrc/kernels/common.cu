@@ -93,6 +93,8 @@ int* device_status_word() {
 
 extern "C" {
 
+size_t b200_tmem_bound_smem(size_t smem, int fit, int cols) { return b200::tmem_bound_smem(smem, fit, cols); }
+
 int b200_num_sms() {
   static int cached[64] = {0};
   int dev = 0;

@@ -290,6 +290,13 @@ __global__ void __launch_bounds__(kWThreads, 1)
 static constexpr int kCRows = 128, kCRaw = kCRows * 128, kCExpCols = 32, kCAccCols = 128, kCTmemCols = 256;
 static constexpr int kCRS = 2, kCES = 4, kCAS = 6, kCActBytes = 49152, kCConv = 8, kCThreads = (3 + kCConv) * 32, kCRowsMax = 128;
 static_assert(kCAccCols + kCES * kCExpCols <= kCTmemCols);
+static_assert(2 * kCTmemCols <= 512, "cluster_splits counts on two CTAs an SM");
+static constexpr size_t cluster_form_smem(int mp, int act_stages) {      // (the partials: 512 bytes a row, over both)
+  return (size_t)kCRS * kCRaw + (size_t)act_stages * mp * 128 + 1024;
+}
+static constexpr int cluster_form_stages(int mp) { return kCActBytes / (mp * 128) < kCAS ? kCActBytes / (mp * 128) : kCAS; }
+static constexpr size_t kCMostSmem = (size_t)kCRS * kCRaw + kCActBytes + 1024;
+static_assert(kCMostSmem >= tmem_bound_smem(0, 3, kCTmemCols));
 
 struct W4CParams {
   int M, N, K, mp, splits, act_stages;
@@ -522,11 +529,43 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// What the launch asks for: two CTAs an SM are all that find columns of the tensor memory, and shared memory alone would let in five
+// at 16 rows. Today the registers keep the third out (60 each, 56 would let it in); where they do not, shared memory has to. It is not asked
+// for otherwise: a launch of 45 KB lets the next kernel's CTAs come in early (0.6 us against 77 KB).
+static size_t cluster_form_launch_smem(int mp) {
+  static std::atomic<int> known[64];          // CTAs of the least shared memory that an SM takes
+  const size_t smem = cluster_form_smem(mp, cluster_form_stages(mp));
+  int dev = 0, fit = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCMostSmem;
+  fit = known[dev].load(std::memory_order_relaxed);
+  if (!fit) {
+    if (cudaFuncSetAttribute(gemm_w4a16_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCMostSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_w4a16_cluster_kernel, kCThreads,
+                                                      cluster_form_smem(16, cluster_form_stages(16))) != cudaSuccess || fit < 1) {
+      cudaGetLastError();
+      return kCMostSmem;
+    }
+    known[dev].store(fit, std::memory_order_relaxed);
+  }
+  return tmem_bound_smem(smem, fit, kCTmemCols);
+}
+
 }  // namespace b200
 
 using namespace b200;
 
 extern "C" {
+
+// CTAs of the cluster form that an SM takes as it is launched for M rows (-1: no answer): no more than find columns of its tensor memory.
+int b200_w4a16_ctas_an_sm(int M) {
+  const size_t smem = cluster_form_launch_smem((M + 15) & ~15);
+  int fit = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_w4a16_cluster_kernel, kCThreads, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return fit;
+}
 
 // Small-M fused path (M <= 128, K a multiple of 64). workspace: f16 copy of A (M * K * 2 bytes,
 // rounded up to 256) followed by fp32 [splits, M, N] split-K partials; returns -4 if it is too
@@ -590,12 +629,9 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
     if (!encode_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, K / 2, kCRows, 128, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tmap_2d(&tmA, a16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, M, K, K, c.mp, 64, CU_TENSOR_MAP_SWIZZLE_128B))
       return -3;
-    c.act_stages = kCActBytes / (c.mp * 128) < kCAS ? kCActBytes / (c.mp * 128) : kCAS;
-    const size_t smem = (size_t)kCRS * kCRaw + (size_t)c.act_stages * c.mp * 128 + 1024;       // (the partials: 512 bytes a row, over both)
-    static PerDeviceOnce once;
-    if (once.first()) cudaFuncSetAttribute(gemm_w4a16_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCRS * kCRaw + kCActBytes + 1024);
-    return launch_cluster_pdl(gemm_w4a16_cluster_kernel, tiles * c.splits, c.splits, kCThreads, smem, stream, tmW, tmA, c) ==
-                   cudaSuccess ? 0 : -2;
+    c.act_stages = cluster_form_stages(c.mp);
+    return launch_cluster_pdl(gemm_w4a16_cluster_kernel, tiles * c.splits, c.splits, kCThreads, cluster_form_launch_smem(c.mp), stream, tmW,
+                              tmA, c) == cudaSuccess ? 0 : -2;
   }
   p.sf_tma = ((K & 255) == 0 && (reinterpret_cast<uintptr_t>(sf) & 15) == 0) ? 1 : 0;
   if (!encode_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K / 2, K / 2, kWN, 128,

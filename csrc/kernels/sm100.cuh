@@ -689,6 +689,16 @@ inline cudaError_t launch_cluster_pdl(void (*kernel)(KArgs...), dim3 grid, int r
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(static_cast<Args&&>(args))...);
 }
 #endif
+// Dynamic shared memory for a kernel whose CTAs allocate `cols` of an SM's 512 columns of tensor memory and meet in clusters: `smem`, or,
+// where more of them fit an SM (`fit` CTAs, as far as registers, threads and `smem` bytes each go) than find columns, enough to keep the
+// others out. One CTA too many would wait in tcgen05.alloc, without limit, for columns of CTAs that may themselves be waiting, in a
+// cluster barrier, for a CTA that waits in the same way on another SM.
+constexpr size_t kSmBytes = 228 * 1024;        // shared memory of an SM
+constexpr size_t tmem_bound_smem(size_t smem, int fit, int cols) {
+  const int most = 512 / cols;
+  const size_t least = kSmBytes / (most + 1) + 1;
+  return fit <= most || smem >= least ? smem : least;
+}
 // CTAs of two to an SM that share the K of each of `tiles` row tiles: as many as one wave holds, `most` at most (gemm_cluster.cu).
 int cluster_splits(int tiles, int most);
 // Activations in the epilogue of a product: 0 none, 1 SiLU, 2 GELU-tanh, 3 GELU-erf, 4 squared ReLU. FAST (results that are

@@ -5,6 +5,8 @@ import os
 import re
 import subprocess
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -17,3 +19,21 @@ def test_header_declares_every_exported_launcher():
     declared = set(re.findall(r"\b(b200_[a-z0-9_]+)\(", header))
     assert exported - declared == set(), f"not declared in api.h: {sorted(exported - declared)}"
     assert declared - exported == set(), f"declared but not exported: {sorted(declared - exported)}"
+
+
+@pytest.mark.parametrize("cols", [64, 128, 256, 512])
+def test_shared_memory_keeps_out_ctas_without_tensor_memory(cols):
+    """Of a kernel whose CTAs meet in clusters no more may be resident on an SM than find their columns among its 512, whatever
+    the registers let in; a launch that they bound already asks for no more than it needs."""
+    from vllm_cpp_b200.ops import _lib
+    if not _lib.available():
+        pytest.skip("kernel library not built")
+    bound, sm = _lib.lib().b200_tmem_bound_smem, 228 * 1024
+    for smem in (0, 45 * 1024, 70 * 1024, 81 * 1024, 120 * 1024):
+        for fit in range(1, 11):
+            got = bound(smem, fit, cols)
+            if fit * cols <= 512:
+                assert got == smem
+            else:
+                assert got >= smem and (512 // cols + 1) * got > sm
+                assert got == smem or 512 // cols * (got + 2048) <= sm          # (with a CTA's static part: the others still fit)

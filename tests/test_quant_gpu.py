@@ -121,6 +121,11 @@ def test_w4a16_stream_and_cluster(M, N, K):
                          out=room[4:].view(M, N))
 
 
+def test_w4a16_ctas_find_their_tensor_memory():
+    """As many CTAs an SM as find 256 columns each, and as the split of K over clusters counts on."""
+    assert {ops.lib().b200_w4a16_ctas_an_sm(m) for m in range(1, 129)} == {2}
+
+
 @pytest.mark.parametrize("M,N,K", [(65, 8, 256), (80, 136, 512), (97, 1032, 2304), (112, 264, 14336), (128, 4104, 4096), (128, 38016, 256)])
 def test_w4a16_of_many_rows_over_a_cluster(M, N, K):
     """65 to 128 rows: paddings to 16 that leave three to six stages of the batch, ragged column tiles, grids beyond one wave."""
