@@ -1421,21 +1421,26 @@ static int launch_tn(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUte
                  cudaSuccess ? 0 : -2;
 }
 
+// Stages and shared memory of a pair's CTA. Two stages of a short K leave room for a second CTA on the SM, and the fp8 kernel's registers do
+// too, but not its columns of tensor memory.
+static size_t pair_ring(int BN, int kblocks, int epi_bytes, int* stages) {
+  const int stage_bytes = kBM * 128 + (BN / 2) * 128;
+  int n = (kSmemBudget - 2048 - epi_bytes) / stage_bytes;
+  if (n > kMaxStages) n = kMaxStages;
+  if (n > kblocks + 1) n = kblocks + 1;
+  if (n < 2) n = 2;
+  *stages = n;
+  const int cols = 2 * BN;
+  return tmem_bound_smem((size_t)n * stage_bytes + 1024 + sizeof(GemmBarriers) + epi_bytes, 512 / cols + 1, cols);
+}
+
 // CTA-pair launch: clusters of two, as many as can be resident at once (at most one per SM pair).
 template <int BN, bool FP8 = false>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmA2, const CUtensorMap& tmB, GemmParams& p,
                        cudaStream_t stream) {
-  constexpr int stage_bytes = kBM * 128 + (BN / 2) * 128;
-  constexpr int kbk = FP8 ? 128 : kBK;
+  const int kblocks = (p.K + (FP8 ? 127 : kBK - 1)) / (FP8 ? 128 : kBK);
   // the scatter epilogue stages its stores in 16 KB behind the barriers
-  const int epi_bytes = (p.tp_world > 1 && p.peer_recv[0]) ? 16384 + 128 : 0;
-  int stages = (kSmemBudget - 2048 - epi_bytes) / stage_bytes;
-  if (stages > kMaxStages) stages = kMaxStages;
-  int kblocks = (p.K + kbk - 1) / kbk;
-  if (stages > kblocks + 1) stages = kblocks + 1;
-  if (stages < 2) stages = 2;
-  p.stages = stages;
-  size_t smem = (size_t)stages * stage_bytes + 1024 + sizeof(GemmBarriers) + epi_bytes;
+  const size_t smem = pair_ring(BN, kblocks, (p.tp_world > 1 && p.peer_recv[0]) ? 16384 + 128 : 0, &p.stages);
   static int max_clusters[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1537,6 +1542,11 @@ extern "C" int b200_gemm_bf16_gated(const void* A, int lda, const void* W, int l
 // stream-K, and the merged projection costs less than that. us, two kernels / one: 40960 x 5120 at 33 / 128 rows 83.8 / 92.7,
 // 89.2 / 110.2; 57344 x 8192 157 / 152, 166 / 174; 28672 x 4096 at 64 / 112 / 128 50.6 / 48.1, 51.7 / 52.6, 52.2 / 53.3; 22016 x
 // 4096 at 128 45.4 / 47.0; 37888 x 3584 (a full wave) 56.7 / 56.1; 16384 x 2048 28.8 / 20.4.
+extern "C" size_t b200_gemm_pair_smem(int BN, int kblocks) {
+  int stages = 0;
+  return pair_ring(BN, kblocks, 0, &stages);
+}
+
 extern "C" int b200_gemm_gated_apart(int M, int N) {
   const int tiles = N / 128, sms = b200_num_sms();
   return M <= 128 && ((M > 32 && tiles > 2 * sms) || (M > 96 && tiles > sms && 6 * tiles < 10 * sms));

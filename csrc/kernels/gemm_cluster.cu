@@ -395,6 +395,21 @@ static int launch(const CUtensorMap& tmW, const BatchMaps<KIND>& tmA, const Clus
                  cudaSuccess ? 0 : -2;
 }
 
+// Bytes of a CTA's ring, for `mp` rows (padded to 16) and its `longest` k-blocks, which the partial tile takes afterwards, and its columns of
+// tensor memory. One k-block of 65 to 80 rows would let five CTAs onto an SM that has columns for four.
+static int cluster_ring(int mp, int longest, int ranks, uint32_t* tmem_cols) {
+  const int stage_bytes = (kRows + mp) * kRowBytes;
+  int stages = (kSmemPerCta - 1024) / stage_bytes;
+  if (stages > kRingStages) stages = kRingStages;
+  if (stages > longest) stages = longest;
+  int bytes = stages * stage_bytes;
+  if (bytes < mp * kRows * 4) bytes = mp * kRows * 4;
+  int cols = 32;
+  while (cols < mp) cols <<= 1;
+  *tmem_cols = (uint32_t)cols;
+  return ranks > 1 ? (int)tmem_bound_smem(bytes, 512 / cols + 1, cols) : bytes;
+}
+
 int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream) {
   if (g.M < 1 || g.M > kMostRows || (g.gated && (g.N & 255))) return -1;
   if (g.rope && (g.gated || g.batch > 1 || g.out_f32 || g.N != (g.rope->Hq + 2 * g.rope->Hkv) * kRows)) return -1;
@@ -418,15 +433,8 @@ int launch_gemm_cluster(const GemmCluster& g, cudaStream_t stream) {
   if (p.splits > p.kblocks) p.splits = p.kblocks;
   const int ranks = (g.gated ? 2 : 1) * p.splits;
   if (ranks > 8) return -1;
-  const int stage_bytes = (kRows + p.mp) * kRowBytes;
-  const int longest = (p.kblocks + p.splits - 1) / p.splits;
-  int stages = (kSmemPerCta - 1024) / stage_bytes;
-  if (stages > kRingStages) stages = kRingStages;
-  if (stages > longest) stages = longest;
-  p.ring_bytes = stages * stage_bytes;
-  if (p.ring_bytes < p.mp * kRows * 4) p.ring_bytes = p.mp * kRows * 4;
-  uint32_t tmem_cols = 32;
-  while ((int)tmem_cols < p.mp) tmem_cols <<= 1;
+  uint32_t tmem_cols = 0;
+  p.ring_bytes = cluster_ring(p.mp, (p.kblocks + p.splits - 1) / p.splits, ranks, &tmem_cols);
   CUtensorMap tmW;
   const dim3 grid((unsigned)(tiles * ranks), 1, (unsigned)g.batch);
   if (g.a_scale) {
@@ -468,3 +476,8 @@ int launch_experts_cluster(const ExpertsCluster& g, cudaStream_t stream) {
 }
 
 }  // namespace b200
+
+extern "C" size_t b200_gemm_cluster_smem(int mp, int longest, int ranks) {
+  uint32_t cols = 0;
+  return (size_t)b200::cluster_ring(mp, longest, ranks, &cols) + 1024;
+}

@@ -37,3 +37,18 @@ def test_shared_memory_keeps_out_ctas_without_tensor_memory(cols):
             else:
                 assert got >= smem and (512 // cols + 1) * got > sm
                 assert got == smem or 512 // cols * (got + 2048) <= sm          # (with a CTA's static part: the others still fit)
+
+
+def test_clusters_of_short_products_find_their_tensor_memory():
+    """Of the products whose CTAs meet in clusters, those of one or two k-blocks ask for little shared memory: no more CTAs an SM than
+    have columns, by shared memory alone."""
+    from vllm_cpp_b200.ops import _lib
+    if not _lib.available():
+        pytest.skip("kernel library not built")
+    L, sm = _lib.lib(), 228 * 1024
+    for kblocks in range(1, 20):
+        for bn in (128, 256):
+            assert sm // L.b200_gemm_pair_smem(bn, kblocks) * 2 * bn <= 512
+        for mp in range(16, 129, 16):
+            cols = max(32, 1 << (mp - 1).bit_length())
+            assert sm // L.b200_gemm_cluster_smem(mp, kblocks, 2) * cols <= 512

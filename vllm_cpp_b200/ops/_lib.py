@@ -56,6 +56,8 @@ _SIGS = {
     "b200_init_device": ([], I),
     "b200_read_status": ([], I),
     "b200_tmem_bound_smem": ([Z, I, I], Z),
+    "b200_gemm_pair_smem": ([I, I], Z),
+    "b200_gemm_cluster_smem": ([I, I, I], Z),
     "b200_w4a16_ctas_an_sm": ([I], I),
     "b200_status_ptr": ([], P),
     "b200_set_peer_wait_cycles": ([ctypes.c_longlong], ctypes.c_longlong),
