@@ -493,6 +493,7 @@ int b200_delta_chunk(const B200Delta* a, void* tp, void* gc, cudaStream_t stream
 // ---- gemm_bf16.cu
 int b200_gemm_gated_apart(int M, int N);
 size_t b200_gemm_pair_smem(int BN, int kblocks);
+void* b200_gemm_tile_counters(size_t* words);
 size_t b200_gemm_cluster_smem(int mp, int longest, int ranks);
 int b200_gemm_bf16_gated(const void* A, int lda, const void* W, int ldw, void* out, int ldo, int M, int N, int K, int kind, int force_path, cudaStream_t stream);
 int b200_gemm_fp8_pair(const void* A, int lda, const void* W, int ldw, void* out, int ldo, const float* a_scale, const float* w_scale, int w_scale_per_channel, const void* bias, int M, int N, int K, cudaStream_t stream);

@@ -106,7 +106,8 @@ int b200_num_sms() {
   return n;
 }
 
-// Reads (and clears) the status word of the current device. Synchronises the whole device
+// Reads (and clears) the status word of the current device, and with an error clears what the kernel that gave up has left behind in the
+// products' counters, so that the next launches are right again. Synchronises the whole device
 // first: a pageable cudaMemcpy alone orders only against the legacy default stream, and kernels
 // launched on non-blocking streams could still be running their bounded waits.
 int b200_read_status() {
@@ -115,7 +116,11 @@ int b200_read_status() {
   int v = 0;
   if (cudaDeviceSynchronize() != cudaSuccess) return -2;
   cudaMemcpy(&v, w, sizeof(int), cudaMemcpyDeviceToHost);
-  if (v != 0) cudaMemset(w, 0, sizeof(int));
+  if (v != 0) {
+    b200::clear_tile_counters();
+    cudaMemset(w, 0, sizeof(int));
+    cudaDeviceSynchronize();            // (before launches on streams that do not wait for the default one)
+  }
   return v;
 }
 

@@ -1283,18 +1283,26 @@ bool get_tmap_bf16(CUtensorMap* out, const void* p, uint64_t rows, uint64_t cols
 
 static constexpr int kSmemBudget = 220 * 1024;
 
-// Stream-K scratch of the current device: one 128 x 256 fp32 partial per CTA plus four flags per
+// Stream-K scratch of the current device: one 128 x 256 fp32 partial per CTA plus four flags and four counters per
 // CTA. b200_init_device() allocates it when a device is set up; a first use that finds none
 // allocates it too unless the stream is capturing (a capture that early keeps the plan without
 // stream-K). GEMMs that share it must be ordered on one stream (two streams running stream-K
-// GEMMs at once would mix their partials).
+// GEMMs at once would mix their partials). A kernel leaves its counters and flags at zero, unless a wait in it ran out: then what
+// came late is still there, and b200_read_status(), which reports it, clears them for the next product.
+static std::mutex g_scratch_mu;
+static float* g_part[64] = {};
+static uint32_t* g_flags[64] = {};
+static size_t counter_words() { return (size_t)b200_num_sms() * 8; }
+void clear_tile_counters() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  if (g_flags[dev]) cudaMemset(g_flags[dev], 0, counter_words() * sizeof(uint32_t));
+}
 static bool streamk_scratch(cudaStream_t stream, float** partials, uint32_t** flags) {
-  static std::mutex mu;
-  static float* g_part[64] = {};
-  static uint32_t* g_flags[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  std::lock_guard<std::mutex> lock(mu);
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
   if (!g_part[dev]) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
@@ -1303,12 +1311,12 @@ static bool streamk_scratch(cudaStream_t stream, float** partials, uint32_t** fl
     float* pp = nullptr;
     uint32_t* ff = nullptr;
     if (cudaMalloc(&pp, n) != cudaSuccess) { cudaGetLastError(); return false; }
-    if (cudaMalloc(&ff, (size_t)b200_num_sms() * 8 * sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaMalloc(&ff, counter_words() * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
       cudaFree(pp);
       return false;
     }
-    cudaMemset(ff, 0, (size_t)b200_num_sms() * 8 * sizeof(uint32_t));
+    cudaMemset(ff, 0, counter_words() * sizeof(uint32_t));
     g_part[dev] = pp;
     g_flags[dev] = ff;
   }
@@ -1542,6 +1550,15 @@ extern "C" int b200_gemm_bf16_gated(const void* A, int lda, const void* W, int l
 // stream-K, and the merged projection costs less than that. us, two kernels / one: 40960 x 5120 at 33 / 128 rows 83.8 / 92.7,
 // 89.2 / 110.2; 57344 x 8192 157 / 152, 166 / 174; 28672 x 4096 at 64 / 112 / 128 50.6 / 48.1, 51.7 / 52.6, 52.2 / 53.3; 22016 x
 // 4096 at 128 45.4 / 47.0; 37888 x 3584 (a full wave) 56.7 / 56.1; 16384 x 2048 28.8 / 20.4.
+// The counters and flags of tiles that several CTAs work on (of this device; null before the first such product), and their number.
+extern "C" void* b200_gemm_tile_counters(size_t* words) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  *words = counter_words();
+  return g_flags[dev];
+}
+
 extern "C" size_t b200_gemm_pair_smem(int BN, int kblocks) {
   int stages = 0;
   return pair_ring(BN, kblocks, 0, &stages);

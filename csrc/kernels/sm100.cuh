@@ -618,6 +618,7 @@ int launch_experts_cluster(const ExpertsCluster& g, cudaStream_t stream);
 
 // Process-wide device status word (lazily allocated per device).
 int* device_status_word();
+void clear_tile_counters();      // of the products whose tiles several CTAs share (gemm_bf16.cu), with the device idle
 long long peer_wait_cycles();   // current limit of waits on other GPUs (b200_set_peer_wait_cycles)
 
 // ------------------------------------------------------------------------------------

@@ -53,6 +53,32 @@ def test_peer_wait_runs_out_and_the_context_survives(short_peer_wait):
     tpf.close()
 
 
+def test_products_after_an_error_was_read_are_right():
+    """A product whose tiles several CTAs share leaves its counters above zero when a wait in it runs out. Here they and the status
+    word are set so on the host; the next product would add parts that nobody has written. Reading the status clears them."""
+    import ctypes
+    from vllm_cpp_b200 import ops
+    from vllm_cpp_b200.ops._lib import lib
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(0)
+    a, w = (torch.randn(n, 4096, device=dev).to(torch.bfloat16) for n in (300, 512))
+    want = {path: ops.gemm(a, w, force_path=path) for path in (5, 6, 9, 10)}
+    assert ops.read_status() == 0
+    words = ctypes.c_size_t()
+    counters = lib().b200_gemm_tile_counters(ctypes.byref(words))
+    assert counters and words.value == 8 * ops.num_sms()
+    memset = ctypes.CDLL("libcudart.so.12").cudaMemset
+    memset.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t]
+    for path, exp in want.items():
+        assert torch.equal(ops.gemm(-a, w, force_path=path), -exp)        # (other parts than the next product's)
+        torch.cuda.synchronize()
+        assert memset(counters, 1, 4 * words.value) == 0
+        assert memset(lib().b200_status_ptr(), ERR_FLAG_TIMEOUT, 1) == 0
+        assert ops.read_status() == ERR_FLAG_TIMEOUT
+        assert torch.equal(ops.gemm(a, w, force_path=path), exp)
+        assert ops.read_status() == 0
+
+
 def test_engine_raises_engine_dead_after_a_kernel_gave_up(short_peer_wait):
     from vllm_cpp_b200 import _engine as E
     from vllm_cpp_b200 import ops
