@@ -16,6 +16,7 @@ int b200_num_sms();
 // Call once per device before the first stream capture. 0 on success.
 int b200_init_device();
 int b200_read_status();
+int b200_ctas_by_registers(int regs, int threads);
 size_t b200_tmem_bound_smem(size_t smem, int fit, int cols);
 void* b200_status_ptr();
 const char* b200_kernel_arch();

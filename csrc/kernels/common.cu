@@ -93,6 +93,7 @@ int* device_status_word() {
 
 extern "C" {
 
+int b200_ctas_by_registers(int regs, int threads) { return b200::ctas_by_registers(regs, threads); }
 size_t b200_tmem_bound_smem(size_t smem, int fit, int cols) { return b200::tmem_bound_smem(smem, fit, cols); }
 
 int b200_num_sms() {

@@ -533,18 +533,19 @@ __global__ void __launch_bounds__(256)
 // at 16 rows. Today the registers keep the third out (60 each, 56 would let it in); where they do not, shared memory has to. It is not asked
 // for otherwise: a launch of 45 KB lets the next kernel's CTAs come in early (0.6 us against 77 KB).
 static size_t cluster_form_launch_smem(int mp) {
-  static std::atomic<int> known[64];          // CTAs of the least shared memory that an SM takes
+  static std::atomic<int> known[64];          // CTAs that an SM's registers take (the driver's own count is one for a kernel with tensor memory)
   const size_t smem = cluster_form_smem(mp, cluster_form_stages(mp));
   int dev = 0, fit = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return kCMostSmem;
   fit = known[dev].load(std::memory_order_relaxed);
   if (!fit) {
+    cudaFuncAttributes at{};
     if (cudaFuncSetAttribute(gemm_w4a16_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCMostSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_w4a16_cluster_kernel, kCThreads,
-                                                      cluster_form_smem(16, cluster_form_stages(16))) != cudaSuccess || fit < 1) {
+        cudaFuncGetAttributes(&at, gemm_w4a16_cluster_kernel) != cudaSuccess) {
       cudaGetLastError();
       return kCMostSmem;
     }
+    fit = ctas_by_registers(at.numRegs, kCThreads);
     known[dev].store(fit, std::memory_order_relaxed);
   }
   return tmem_bound_smem(smem, fit, kCTmemCols);
@@ -559,12 +560,13 @@ extern "C" {
 // CTAs of the cluster form that an SM takes as it is launched for M rows (-1: no answer): no more than find columns of its tensor memory.
 int b200_w4a16_ctas_an_sm(int M) {
   const size_t smem = cluster_form_launch_smem((M + 15) & ~15);
-  int fit = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemm_w4a16_cluster_kernel, kCThreads, smem) != cudaSuccess) {
+  cudaFuncAttributes at{};
+  if (cudaFuncGetAttributes(&at, gemm_w4a16_cluster_kernel) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
-  return fit;
+  const int regs = ctas_by_registers(at.numRegs, kCThreads), memory = (int)(kSmBytes / (smem + at.sharedSizeBytes + 1024));
+  return regs < memory ? regs : memory;
 }
 
 // Small-M fused path (M <= 128, K a multiple of 64). workspace: f16 copy of A (M * K * 2 bytes,

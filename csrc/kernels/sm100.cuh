@@ -695,6 +695,11 @@ inline cudaError_t launch_cluster_pdl(void (*kernel)(KArgs...), dim3 grid, int r
 // others out. One CTA too many would wait in tcgen05.alloc, without limit, for columns of CTAs that may themselves be waiting, in a
 // cluster barrier, for a CTA that waits in the same way on another SM.
 constexpr size_t kSmBytes = 228 * 1024;        // shared memory of an SM
+// CTAs that the registers of an SM let in at most: four parts of 16384, of which a warp takes its own from one, in pieces of 256.
+constexpr int ctas_by_registers(int regs, int threads) {
+  const int warp = ((regs < 1 ? 1 : regs) + 7) / 8 * 256;
+  return 4 * (16384 / warp) / ((threads + 31) / 32);
+}
 constexpr size_t tmem_bound_smem(size_t smem, int fit, int cols) {
   const int most = 512 / cols;
   const size_t least = kSmBytes / (most + 1) + 1;

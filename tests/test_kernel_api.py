@@ -29,6 +29,8 @@ def test_shared_memory_keeps_out_ctas_without_tensor_memory(cols):
     if not _lib.available():
         pytest.skip("kernel library not built")
     bound, sm = _lib.lib().b200_tmem_bound_smem, 228 * 1024
+    regs = _lib.lib().b200_ctas_by_registers                 # 352 threads: the third CTA comes in at 56 registers
+    assert [regs(r, 352) for r in (32, 56, 57, 60, 64, 80, 88)] == [5, 3, 2, 2, 2, 2, 1] and regs(168, 192) == 2 and regs(255, 192) == 1
     for smem in (0, 45 * 1024, 70 * 1024, 81 * 1024, 120 * 1024):
         for fit in range(1, 11):
             got = bound(smem, fit, cols)
