@@ -493,6 +493,7 @@ int b200_delta_chunk_fits(const B200Delta* a);
 int b200_delta_chunk(const B200Delta* a, void* tp, void* gc, cudaStream_t stream);
 // ---- gemm_bf16.cu
 int b200_gemm_gated_apart(int M, int N);
+int b200_gemm_form(int M, int N, int K);
 size_t b200_gemm_pair_smem(int BN, int kblocks);
 void* b200_gemm_tile_counters(size_t* words);
 size_t b200_gemm_cluster_smem(int mp, int longest, int ranks);

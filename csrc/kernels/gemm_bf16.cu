@@ -1359,7 +1359,8 @@ static void plan_streamk(long tiles, int kblocks, int max_workers, int* nworkers
 // of them up to 8192 rows; 7 % off on average. The choice is 1.0 % from the best of the eight forms on average, up to 2300 rows, and 2.2 %
 // above, where the clocks move as much; the rules that it replaced were 15 and 7 % off and up to 3 times: us, before / after, 1024 x 3072 at
 // 600 rows 31.0 / 12.1, 2048 x 4096 at 300 36.8 / 14.0, 4096 x 1024 at 512 16.8 / 8.0, 4096 x 14336 at 300 59.0 / 46, 28672 x 4096
-// at 300 101 / 83. A tile of 128 x 128 is bound by shared memory, those of a pair by the tensor pipe.
+// at 300 101 / 83. On wider ones (57344 to 151936, K from 768 to 5120, 130 to 4000 rows, timed in turn) it is 1.6 % from the best of five
+// forms on average, up to 11 % with a K of 768, and 1.027 times as fast as pairs with stream-K throughout. A tile of 128 x 128 is bound by shared memory, those of a pair by the tensor pipe.
 struct TileForm {
   int path, rows, cols, streamed;       // path: force_path
 };
@@ -1391,6 +1392,21 @@ static int fastest_tiles(long M, long N, long K) {
     if (t < best) { best = t; path = f.path; }
   }
   return path;
+}
+
+// Up to 128 rows K is split over a cluster, two CTAs an SM (0). On the widest matrices, which have no split to gain from, tiles that read
+// 128 (6) or 256 (5) weight rows with one copy of the batch are the faster ones from some rows on. Those of 128: from 49 rows where they
+// are one wave, else from 64 where the estimate prefers them (with fewer rows and a K of 1024 they take up to 1.4 times as long as those of
+// 256). Those of 256: from 65 rows, where they are more than two waves from 49, with a K above 1024 from 33. us, cluster / 256 / 128:
+//   16384 x 2048 at 48 rows 15.0 / 20.8 / 14.5, at 64 15.8 / 20.7 / 14.4    28672 x 4096 at 56 41.5 / 43.4 / 41.6, at 96 44.8 / 43.6 / 43.5
+//   57344 x 1024 at 56 28.2 / 35.2 / 29.6, at 64 28.9 / 34.8 / 25.6         128256 x 4096 at 48 177.0 / 175.7 / 174.9, at 96 213 / 200 / 196
+//   151936 x 1024 at 40 63.6 / 74.2 / 106, at 56 62.7 / 61.2 / 81.7, at 64 64.6 / 64.9 / 60.8    151936 x 2048 at 40 112 / 104 / 105
+// Beyond two waves of 128 with a short K earlier: 57344 x 512 at 32 rows 16.7 / 15.6 (256), at 16 15.2 / 16.7.
+static int few_rows_form(int M, int N, int K) {
+  const int sms = b200_num_sms(), wide = (N + 255) / 256, narrow = (N + kBM - 1) / kBM;
+  if (N < 16384) return 0;
+  if (narrow <= sms ? M > 48 : M >= 64 && tile_form_us(kTileForms[3], M, N, K) < tile_form_us(kTileForms[2], M, N, K)) return 6;
+  return M > (wide <= 2 * sms ? 64 : K <= 1024 ? 48 : 32) || (M > 16 && K <= 512 && narrow > 2 * sms) ? 5 : 0;
 }
 
 template <int BN>
@@ -1559,6 +1575,9 @@ extern "C" void* b200_gemm_tile_counters(size_t* words) {
   return g_flags[dev];
 }
 
+// Which form a product runs in: 0 a cluster (up to 128 rows), else the force_path of its tiles.
+extern "C" int b200_gemm_form(int M, int N, int K) { return M <= 128 ? few_rows_form(M, N, K) : fastest_tiles(M, N, K); }
+
 extern "C" size_t b200_gemm_pair_smem(int BN, int kblocks) {
   int stages = 0;
   return pair_ring(BN, kblocks, 0, &stages);
@@ -1673,14 +1692,10 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
     }
     return 0;
   }
-  // Up to 128 rows: K split over a cluster, two CTAs per SM. On the widest matrices (no split to gain from) the tiled
-  // kernels, which read 128 or 256 weight rows with one copy of the batch, are the faster ones from some rows on
-  // (128256 x 4096: 168.2 against 168.4 us at 40 rows, 173.5 against 170.4 at 64; 28672 x 4096 41.2 against 43.3 at 40, 42.6 against 42.5
-  // at 64, 47.5 against 45.0 at 128; 16384 x 2048 14.8 against 14.2, 15.7 against 14.2, 18.2 against 14.7;
-  // beyond one wave of CTAs with a short K earlier: 57344 x 512 at 32 rows 16.7 against 15.6, at 16 15.2 against 16.7).
-  const bool tiles_win = N >= 16384 && !(at & 15) && (M > 48 || (M > 16 && K <= 512 && (N + kBM - 1) / kBM > 2 * b200_num_sms()));
+  // Up to 128 rows: K split over a cluster, or the tiled kernels (few_rows_form).
+  const int few = M <= 128 && !(at & 15) ? few_rows_form(M, N, K) : 0;
   const bool cluster = !tp && M <= 128 && !(at & 7) &&
-                       (force_path == 0 ? act_fuse || !tiles_win : force_path >= 32 && force_path <= 40);
+                       (force_path == 0 ? act_fuse || !few : force_path >= 32 && force_path <= 40);
   if (act_fuse && !cluster && force_path == 0) force_path = 9;      // the gated epilogue lives in the pair kernel
   if ((K & 7) || (lda & 7) || (ldw & 7) || (N & 7) || (ldo & 7) || (residual && (ldr & 7))) return -1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) |
@@ -1729,11 +1744,9 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   const int kblocks = (K + kBK - 1) / kBK;
 
   bool use_swap = (M <= 256);
-  // Batches that the cluster kernel does not take: the tiles that are estimated to be fastest (up to 128 rows those of 128 rows).
+  // Batches that the cluster kernel does not take: the tiles that are estimated to be fastest.
   if (at & 15) force_path = 2;
-  if (force_path == 0 && !tp && !act_fuse)
-    force_path = M > 128 ? fastest_tiles(M, N, K)
-                         : N < 256 || tile_form_us(kTileForms[3], M, N, K) < tile_form_us(kTileForms[2], M, N, K) ? 6 : 5;
+  if (force_path == 0 && !tp && !act_fuse) force_path = M > 128 ? fastest_tiles(M, N, K) : few;
   if (force_path == 1 || force_path >= 3) use_swap = false;     // an explicit tiling was asked for
   if (force_path == 2 && M <= 256) use_swap = true;
 

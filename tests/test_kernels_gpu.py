@@ -936,6 +936,23 @@ def test_gemm_of_the_form_that_is_chosen(M, N, K):
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("N,K,first,form", [(16376, 1024, 129, 0), (16384, 2048, 49, 6), (18432, 1024, 49, 6), (28672, 4096, 65, 5),
+                                            (57344, 1024, 64, 6), (57344, 512, 17, 5), (128256, 4096, 33, 5), (151936, 1024, 49, 5)])
+def test_form_of_few_rows_of_wide_matrices(N, K, first, form):
+    """Where the line between a cluster and the tiles lies (148 SMs), and which tiles follow; both sides give the product."""
+    from vllm_cpp_b200.ops import _lib
+    forms = [_lib.lib().b200_gemm_form(m, N, K) for m in range(1, 129)]
+    assert not any(forms[: first - 1]) and forms[first - 1: first] in ([form], []) and all(forms[first - 1:])
+    if N > 65536:
+        return
+    torch.manual_seed(N)
+    w = _rand(N, K, scale=K ** -0.5)
+    for M in (first - 1, first):
+        a = _rand(M, K)
+        assert _rel_err(ops.gemm(a, w), a.float() @ w.float().t()) < 2.0 ** -8
+    assert ops.read_status() == 0
+
+
 @pytest.mark.parametrize("V,n", [(1024, 5), (3000, 5), (151936, 5), (9021, 160)])
 def test_top_k_of_about_what_a_list_holds(V, n):
     """The search goes on in a list once 1024 values of the row are left: k below, at and above that, ties that do not fit,

@@ -57,6 +57,7 @@ _SIGS = {
     "b200_read_status": ([], I),
     "b200_ctas_by_registers": ([I, I], I),
     "b200_tmem_bound_smem": ([Z, I, I], Z),
+    "b200_gemm_form": ([I, I, I], I),
     "b200_gemm_pair_smem": ([I, I], Z),
     "b200_gemm_tile_counters": ([ctypes.POINTER(Z)], P),
     "b200_gemm_cluster_smem": ([I, I, I], Z),
