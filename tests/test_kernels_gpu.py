@@ -253,6 +253,47 @@ def test_act_and_mul(kind):
     assert _rel_err(ops.act_and_mul(x, kind), ref.act_and_mul(x, kind)) < 5e-3
 
 
+def _all_bf16():
+    return torch.arange(-32768, 32768, device=DEV).to(torch.int16).view(torch.bfloat16)
+
+
+@pytest.mark.parametrize("scale", [0.0, 1.0])
+def test_silu_of_every_gate(scale):
+    """act(gate) * up for all 65536 gates, up 1 and 31 random values: the result lies between the roundings of what the arithmetic may
+    err by, so mostly it is the correctly rounded one. __expf: 2 + 1.173 |x| units of 2^-23, times its share in the result; the
+    quotient and the product with up: 2^-22 and 2^-24, the bounds' own rounding to 32 bits as much. Beyond 32 bits' range: 2e-36."""
+    torch.manual_seed(4)
+    gate = _all_bf16()[None].expand(32, -1)
+    up = torch.exp2(torch.randn(32, 65536, device=DEV) * scale * 3).to(torch.bfloat16)
+    got = ops.act_and_mul(torch.cat([gate, up], 1).contiguous(), 0)
+    g, u = gate.double(), up.double()
+    e = torch.exp(-g.abs())
+    exact = g * u * torch.where(g >= 0, 1.0, e) / (1 + e)
+    part = torch.where(g >= 0, e, torch.ones_like(e)) / (1 + e)
+    err = (2 + 1.173 * g.abs()) * 2.0 ** -23 * part + 2.0 ** -22 + 2 * 2.0 ** -24
+    low, high = ((exact.abs() * (1 + s * err)).to(torch.bfloat16).double() for s in (-1, 1))
+    at, size = torch.isfinite(g) & torch.isfinite(high), got.double().abs()
+    fine = ((size >= low) & (size <= high)) | ((size - exact.abs()).abs() <= 2e-36 * u.clamp_min(1.0))
+    assert bool(fine[at].all())
+    assert torch.equal(torch.signbit(got[at]), torch.signbit(g[at]))                  # (zeros, and what underflows)
+    right = exact.to(torch.bfloat16) == got
+    assert (~right[at & (g.abs() < 20)]).double().mean().item() < 2.0 ** -10            # (the bounds are that much of a step of 2^-8)
+    assert bool((got[gate == float("inf")] == float("inf")).all())
+    assert bool(torch.isnan(got[torch.isnan(gate) | (gate == -float("inf"))]).all())
+
+
+@pytest.mark.parametrize("M", [2, 40, 128, 256])
+def test_silu_of_every_gate_in_a_products_epilogue(M):
+    """The same bits where a product applies it: gates that a unit row picks out of the weights."""
+    gate = _all_bf16().view(256, 256)
+    gate = torch.where(torch.isfinite(gate), gate, torch.zeros_like(gate))
+    up = torch.ones_like(gate)
+    a = torch.eye(256, device=DEV, dtype=torch.bfloat16)[:M]
+    got = ops.gemm_gated(a, ops.interleave_gate_up(gate, up))
+    exp = ops.act_and_mul(torch.cat([gate.t()[:M], up[:M]], 1).contiguous(), 0)
+    assert torch.equal(got, exp) and ops.read_status() == 0
+
+
 def test_embedding_and_gather():
     torch.manual_seed(7)
     table = _rand(1000, 256)
