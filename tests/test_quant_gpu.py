@@ -102,9 +102,9 @@ def test_w4a16_over_a_cluster(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(17, 2560, 9728), (34, 2560, 9728), (64, 4096, 14336), (32, 38016, 256), (33, 38016, 256)])
-def test_w4a16_stream_and_cluster(M, N, K):
-    """Both sides of the lines between the two forms up to 64 rows: parts of K that are too coarse over a cluster, more rows
-    that make up for it, grids beyond one wave."""
+def test_w4a16_results_off_16_bytes(M, N, K):
+    """Coarse parts of K and grids beyond one wave over a cluster, which writes results at multiples of 8 bytes; the stream form, which a K of
+    no 256 goes to, wants 16."""
     torch.manual_seed(14)
     packed = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device=DEV)
     sf = torch.randint(0x20, 0x60, (N, K // 16), dtype=torch.uint8, device=DEV)
@@ -112,13 +112,32 @@ def test_w4a16_stream_and_cluster(M, N, K):
     a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
     w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
     room = torch.empty(M * N + 4, dtype=torch.bfloat16, device=DEV)
-    for out in (Q.gemm_w4a16(a, packed, sf, g), Q.gemm_w4a16(a, packed, sf, g, out=room[4:].view(M, N))):    # 8 bytes off: cluster
+    for out in (Q.gemm_w4a16(a, packed, sf, g), Q.gemm_w4a16(a, packed, sf, g, out=room[4:].view(M, N))):
         assert ops.read_status() == 0
         assert _within_sum_error(out, a64, w64, a64 @ w64.t(), 2**-25 * w64.abs().sum(1))
     if N == 38016:
         with pytest.raises(KernelError):                   # K not a multiple of 256 and no split: no form can write there
             Q.gemm_w4a16(a[:, :K - 64].contiguous(), packed[:, :K // 2 - 32].contiguous(), sf[:, :K // 16 - 4].contiguous(), g,
                          out=room[4:].view(M, N))
+
+
+@pytest.mark.parametrize("M,N,K,off", [(1, 136, 4160, 0), (17, 520, 9664, 0), (64, 2568, 14272, 0), (65, 264, 64, 0), (65, 1032, 9664, 0),
+                                       (128, 136, 14272, 0), (128, 4104, 4160, 0), (2, 38016, 320, 0), (33, 520, 4096, 4), (128, 264, 9728, 8)])
+def test_w4a16_over_stages_in_turn(M, N, K, off):
+    """The stream form: K in blocks of 64 but not of 256, or scales ``off`` 16 bytes. One stage and rings of several turns, one part of K and
+    up to sixteen, ragged column tiles, rows up to all 128."""
+    torch.manual_seed(16)
+    packed = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device=DEV)
+    room = torch.randint(0x00, 0x7f, (N * (K // 16) + 16,), dtype=torch.uint8, device=DEV)
+    sf = room[off:off + N * (K // 16)].view(N, K // 16)
+    g = torch.full((1,), 1e-3, device=DEV)
+    a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
+    bias = torch.randn(N, device=DEV).to(torch.bfloat16)
+    w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
+    for b in (None, bias):
+        out = Q.gemm_w4a16(a, packed, sf, g, bias=b)
+        assert ops.read_status() == 0
+        assert _within_sum_error(out, a64, w64, a64 @ w64.t() + (0 if b is None else b.double()), 2**-25 * w64.abs().sum(1))
 
 
 def test_w4a16_ctas_find_their_tensor_memory():
