@@ -352,6 +352,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
         }
         if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        __syncwarp();          // (a vote orders no memory: what lane 0 has seen, the lane that issues the loads has too)
         fence_proxy_async_global();
       }
       for (int kb = kb0; kb < kb1; ++kb) {
@@ -760,6 +761,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
         }
         if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        __syncwarp();          // (a vote orders no memory: what lane 0 has seen, the lane that issues the loads has too)
         fence_proxy_async_global();
       }
       for (int kb = kb0; kb < kb1; ++kb) {
@@ -1082,6 +1084,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
     }
     ok = __all_sync(0xffffffffu, ok);
+    __syncwarp();              // (as in the tiled kernels)
     if (p.ag_flags) fence_proxy_async_global();
     uint32_t ph = 1;
     int s = 0;
