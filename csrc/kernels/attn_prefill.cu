@@ -586,7 +586,9 @@ __global__ void __launch_bounds__(320, 1)
         m = tile_max;
       }
       const float m_use = (m == -INFINITY) ? 0.f : m;
-      if (__any_sync(0xffffffffu, rescale)) {      // S(j) was issued after P V(j - 1) had completed: O is at rest
+      // O is at rest: S(j) is issued right behind P V(j - 1), by the same elected lane, and a commit covers all that its thread has issued
+      // before. Whoever moves the commit of s_full, or gives the two products to different threads, has to wait for P V(j - 1) here.
+      if (__any_sync(0xffffffffu, rescale)) {
 #pragma unroll 1
         for (int c = 0; c < 8; ++c) {
           uint32_t rr[16];

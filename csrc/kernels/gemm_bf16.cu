@@ -1830,10 +1830,8 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   bool use256 = (N >= 256 && waves256 * 2 * 100 <= waves128 * 135);
   if (force_path == 3) use256 = false;
   if (force_path == 4) use256 = true;
-  // force_path: 0 auto | 1 tiled 1-CTA | 3 / 4 1-CTA with BN 128 / 256 | 5 / 6 1-CTA BN 256 / 128
-  // with stream-K | 7 / 8 CTA pairs with 256 x 256 / 256 x 128 tiles | 9 / 10 pairs with stream-K.
-  // Plain GEMMs above the small-M range run on CTA pairs; the tensor-parallel prologue and
-  // epilogue live in the 1-CTA kernel.
+  // force_path: 0 auto (few_rows_form, fastest_tiles: one of the others by now) | 1 tiled 1-CTA, BN by the waves | 3 / 4 1-CTA with
+  // BN 128 / 256 | 5 / 6 1-CTA BN 256 / 128 with stream-K | 7 / 8 CTA pairs with 256 x 256 / 256 x 128 tiles | 9 / 10 pairs with stream-K.
   if (force_path == 5) { use256 = true; p.sk = !tp; }
   if (force_path == 6) { use256 = false; p.sk = !tp; }
   // tensor-parallel shards are narrow (N / world or K / world): few tiles or a ragged last wave
@@ -1842,12 +1840,12 @@ static int gemm_bf16_impl(const void* A, int lda, const void* W, int ldw, void* 
   // Tensor-parallel GEMMs above the small-M range run on CTA pairs as well (gather prologue,
   // staged scatter epilogue); B200_TP_PAIR=0 keeps them on the 1-CTA tile.
   const bool tp_pair = tp && force_path == 1 && M > 256 && tp_pair_enabled();
-  const bool pair_path = tp_pair || (!tp && (force_path == 0 || (force_path >= 7 && force_path <= 10)));
+  const bool pair_path = tp_pair || (!tp && force_path >= 7 && force_path <= 10);
   if (act_fuse && !pair_path) return -1;
   p.act_fuse = act_fuse;
   if (pair_path) {
-    const bool bn256 = act_fuse || ((force_path == 0 || tp_pair) ? (N > 128) : (force_path == 7 || force_path == 9));
-    p.sk = (force_path == 0 || force_path >= 9 || tp_pair) ? 1 : 0;
+    const bool bn256 = act_fuse || (tp_pair ? N > 128 : force_path == 7 || force_path == 9);
+    p.sk = (force_path >= 9 || tp_pair) ? 1 : 0;
     p.tiles_m = (M + 2 * kBM - 1) / (2 * kBM);
     CUtensorMap tA, tA2, tB;
     if (!get_tmap_bf16(&tA, A, M, K, lda, kBM, kBK)) return -3;

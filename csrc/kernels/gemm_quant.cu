@@ -204,12 +204,6 @@ __global__ void __launch_bounds__(kQThreads, 1)
 // ---------------------------------------------------------------------------------------
 // NVFP4
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ float e2m1_value(uint32_t code) {
-  // sign | 2-bit exponent | 1-bit mantissa: 0, .5, 1, 1.5, 2, 3, 4, 6
-  const uint32_t mag = code & 7u;
-  const float v = mag < 2 ? 0.5f * (float)mag : (float)(2 + (mag & 1)) * (float)(1 << ((mag >> 1) - 1)) * 0.5f;
-  return (code & 8u) ? -v : v;
-}
 // Whole-matrix expansion: packed [N, K/2] + scales [N, K/16] -> bf16 [N, K]. Bound by the memory: a thread takes eight values, so that
 // neighbours write neighbouring 16 bytes, four times at once, and the conversions are the hardware's (34816 x 5120, 0.46 GB: 147 us
 // with values computed from the code's bits, 97 in this form).

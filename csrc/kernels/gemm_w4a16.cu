@@ -610,7 +610,7 @@ int b200_gemm_w4a16(const void* A, int lda, const void* wq, const void* sf, cons
     const int tiles = (N + kCRows - 1) / kCRows, blocks = K / 256;
     csplits = cluster_splits(tiles, blocks / 2);
   }
-  // (the stream form's vectors; results of 65 and more rows are to be aligned in either form)
+  // (the stream form's vectors; from 65 rows on results off 16 bytes are refused in the cluster form too, though it writes 8 at a time)
   if ((!cluster || M > 64) && splits == 1 && (reinterpret_cast<uintptr_t>(out) & 15)) return -1;
   __half* a16 = reinterpret_cast<__half*>(workspace);
   {

@@ -38,6 +38,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// True in one lane of the (whole) calling warp, the same one at every call: elect.sync names the same leader for the same mask. Commits rely
+// on it, as each covers what its own thread has issued.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
