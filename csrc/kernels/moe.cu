@@ -572,7 +572,6 @@ __global__ void __launch_bounds__(192, 1)
   }
   if (warp == 1) { tmem_alloc_pair(&bars.tmem_base, 512); tmem_relinquish_pair(); }
   pdl_wait();
-  pdl_launch_dependents();
   const int chunks = min(p.meta[3 * p.E + 1], p.max_chunks);
   // Up to kPGroup chunks of an expert take a weight tile one after the other, so that side by side pairs share it in L2 (8 experts
   // of 14336, width 4096, 4096 tokens: a chunk at a time 1779 us)
@@ -588,6 +587,7 @@ __global__ void __launch_bounds__(192, 1)
   __syncthreads();
   cluster_sync_all();            // the peer's barriers exist before anything signals them
   tc_fence_after_sync();
+  pdl_launch_dependents();       // (not before the columns are taken: a successor that took some first would wait for this kernel's end)
   const uint32_t tmem = __shfl_sync(0xffffffffu, bars.tmem_base, 0);
   const int total = chunks * p.tiles;
   const auto tile_of = [&](int t, int& tn) {

@@ -54,3 +54,21 @@ def test_clusters_of_short_products_find_their_tensor_memory():
         for mp in range(16, 129, 16):
             cols = max(32, 1 << (mp - 1).bit_length())
             assert sm // L.b200_gemm_cluster_smem(mp, kblocks, 2) * cols <= 512
+
+
+def test_successors_start_once_tensor_memory_is_taken():
+    """A kernel lets its successor in when one thread of every CTA says so. Where the columns of tensor memory are still to be taken then, by
+    another warp, the successor can take them first and wait for the kernel's end, which waits for the columns. So a barrier of
+    the CTA lies between the two."""
+    seen = 0
+    for name in sorted(os.listdir(os.path.join(ROOT, "csrc", "kernels"))):
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "csrc", "kernels", name)).read())
+        for kernel in text.split("__global__")[1:]:
+            taken = re.search(r"\btmem_alloc(_pair)?\(", kernel)
+            let_in = re.search(r"\bpdl_launch_dependents\(", kernel)
+            if taken and let_in:
+                seen += 1
+                assert "__syncthreads();" in kernel[taken.end():let_in.start()], (name, kernel[:100])
+    assert seen >= 8
