@@ -196,8 +196,9 @@ int b200_dense_layer(const B200DenseLayerWeights* w, const B200DenseStep* s, cud
     B200_TRY(b200_quant_fp8_rowwise(s->hidden, H, s->resid, w->ln2, s->eps, s->gemma, 1, 0, s->fp8_act, H,
                                     s->fp8_scales, T, H, stream));
     // From 257 rows on (the CTA pairs' product) the activation goes into the epilogue, below that into the quantisation: the
-    // cluster's and the 128-row tiles' epilogues hold no gate beside its up half.
-    if (s->gate_up_interleaved && T > 256 && !(I & 127)) {
+    // cluster's and the 128-row tiles' epilogues hold no gate beside its up half. It goes to act, which a caller of an fp8 block may leave
+    // out or place off 16 bytes.
+    if (s->gate_up_interleaved && T > 256 && !(I & 127) && s->act && !(reinterpret_cast<uintptr_t>(s->act) & 15)) {
       B200_TRY(b200_gemm_fp8_gated(s->fp8_act, H, w->gate_up, H, s->act, I, (const float*)s->fp8_scales, w->gate_up_scale, kFp8Scales,
                                    T, 2 * I, H, s->act_kind, stream));
       B200_TRY(b200_quant_fp8_rowwise(s->act, I, nullptr, nullptr, 0.f, 0, 0, 0, s->fp8_act, I, s->fp8_scales, T, I, stream));

@@ -947,6 +947,45 @@ def test_qkv_product_with_rotation(T, Hq, Hkv, H, qk_norm, fp8):
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("T,H,I", [(300, 256, 384), (257, 512, 128)])
+def test_fp8_block_with_and_without_a_buffer_for_the_activation(T, H, I):
+    """From 257 rows on act(gate) * up goes to ``act`` where there is one at a multiple of 16 bytes, else through ``gate_up_buf``: the same bits."""
+    from vllm_cpp_b200.ops.layer import DenseLayerWeights, DenseStep, dense_layer
+    torch.manual_seed(T)
+    D, Hq, Hkv, bs = 128, 2, 1, 16
+    N, nb = (Hq + 2 * Hkv) * D, T // bs + 2
+    hidden0, ln1, ln2 = _rand(T, H), _rand(H), _rand(H)
+    w, s = DenseLayerWeights(), DenseStep()
+    mats = {k: _rand(*shape).clamp(-1, 1).to(torch.float8_e4m3fn) for k, shape in
+            (("qkv", (N, H)), ("o", (H, Hq * D)), ("gate_up", (2 * I, H)), ("down", (H, I)))}
+    scales = {k: torch.rand(m.shape[0], device=DEV) * 0.01 for k, m in mats.items()}
+    cache = torch.zeros(nb, 2, bs, Hkv, D, device=DEV, dtype=torch.bfloat16)
+    for k, m in mats.items():
+        setattr(w, k, m.data_ptr())
+        setattr(w, k + "_scale", scales[k].data_ptr())
+    w.fp8, w.ln1, w.ln2, w.kv_cache = 1, ln1.data_ptr(), ln2.data_ptr(), cache.data_ptr()
+    pos, slots = torch.arange(T, device=DEV), torch.arange(T, device=DEV)
+    table = ops.rope_table(ref.rope_inv_freq(D, 1e6).to(DEV), 512)
+    resid, normed, qkv, gate_up = (torch.zeros(T, n, device=DEV, dtype=torch.bfloat16) for n in (H, H, N, 2 * I))
+    room, attn = torch.zeros(T * I + 8, device=DEV, dtype=torch.bfloat16), _rand(T, Hq * D)       # (no request: attn stays as it is)
+    act8, row_scales = torch.empty(T, max(H, Hq * D, I), device=DEV, dtype=torch.uint8), torch.empty(T, device=DEV)
+    ws = ops.workspace(torch.device(DEV), ops.GEMM_WS_BYTES)
+    s.T, s.H, s.Hq, s.Hkv, s.D, s.rot, s.inter, s.block_size, s.neox, s.eps, s.num_blocks = T, H, Hq, Hkv, D, D, I, bs, 1, 1e-6, nb
+    s.gate_up_interleaved, s.first_layer = 1, 1
+    s.positions, s.cos_sin, s.slot_mapping = pos.data_ptr(), table.data_ptr(), slots.data_ptr()
+    s.resid, s.normed, s.qkv_buf, s.attn, s.gate_up_buf = (t.data_ptr() for t in (resid, normed, qkv, attn, gate_up))
+    s.fp8_act, s.fp8_scales, s.gemm_ws, s.gemm_ws_bytes = act8.data_ptr(), row_scales.data_ptr(), ws.data_ptr(), ws.numel()
+    got = []
+    for at in (room.data_ptr(), room.data_ptr() + 8, None):
+        hidden = hidden0.clone()
+        s.hidden, s.act = hidden.data_ptr(), at
+        dense_layer(w, s)
+        got.append(hidden)
+    assert ops.read_status() == 0
+    assert torch.isfinite(got[0]).all() and float(got[0].float().abs().max()) > 0
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("M,N,K", [(130, 1024, 1040), (257, 384, 4096), (300, 512, 1288), (129, 128, 8192), (513, 256, 2048)])
 @pytest.mark.parametrize("path", [5, 6, 9, 10])
 def test_gemm_tiles_in_parts(M, N, K, path):
