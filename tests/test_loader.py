@@ -4,6 +4,7 @@ the format definitions."""
 import json
 import os
 
+import pytest
 import torch
 
 from vllm_cpp_b200 import loader
@@ -124,3 +125,30 @@ def test_fp8_checkpoint_loads_into_w8a8_layers(tmp_path):
     sp = SamplingParams(temperature=0.0, max_tokens=5, ignore_eos=True)
     outs = llm.generate(["The quick brown fox"], sp)
     assert len(outs[0].outputs[0].token_ids) == 5
+
+
+@pytest.mark.parametrize("name,key", [("tiny-moe", "o"), ("tiny-moe", "ln2"), ("tiny-qwen3", "down")])
+def test_native_blocks_follow_weights_that_are_loaded_again(name, key):
+    """The addresses that the native blocks take are those of the tensors that the model holds now, whichever block's was replaced."""
+    cfg = synthetic_config(name)
+    model = LLM(EngineArgs(model_config=cfg, device="cpu", block_size=16, num_blocks=8, max_model_len=64, max_num_seqs=2,
+                           max_num_batched_tokens=32)).runner.model
+    before = model._native_weights()
+    assert model._native_weights() is before
+    last = model.layers[-1]
+    last[key] = last[key].clone()
+    for w, L, cache in zip(model._native_weights(), model.layers, model.kv_caches):
+        for k in ("ln1", "qkv", "o", "ln2", "q_norm", "k_norm", "gate_up", "down"):
+            assert getattr(w, k) == (L[k].data_ptr() if L.get(k) is not None else None), k
+        assert w.kv_cache == cache.data_ptr() and w.fp8 == 0
+
+
+def test_native_blocks_take_fp8_weights_with_their_scales():
+    cfg = synthetic_config("tiny-qwen3")
+    model = LLM(EngineArgs(model_config=cfg, device="cpu", block_size=16, num_blocks=8, max_model_len=64, max_num_seqs=2,
+                           max_num_batched_tokens=32)).runner.model
+    model.quantize_weights("fp8")
+    for w, L in zip(model._native_weights(), model.layers):
+        assert w.fp8 == 1
+        for k in ("qkv", "o", "gate_up", "down"):
+            assert getattr(w, k) == L[k].w8.data_ptr() and getattr(w, k + "_scale") == L[k].w_scale.data_ptr()

@@ -511,25 +511,28 @@ class DenseModel:
         return all(n == 0 for n in n8) or all(n == 4 for n in n8)
 
     def _native_weights(self):
-        ws = getattr(self, "_native_w", None)
-        if ws is None or len(ws) != len(self.layers) or ws[0].kv_cache != self.kv_caches[0].data_ptr() \
-                or ws[0].qkv != self.layers[0]["qkv"].data_ptr():
-            from ..ops.layer import DenseLayerWeights
-            ws = []
-            for l, L in enumerate(self.layers):
+        """The blocks' addresses as the native entries take them, filled in anew whenever one of them has changed: any tensor of any
+        block can have been loaded again since the last forward."""
+        from ..ops.layer import DenseLayerWeights
+        keys = ("ln1", "qkv", "o", "ln2", "q_norm", "k_norm", "gate_up", "down")
+        rows = []
+        for L, cache in zip(self.layers, self.kv_caches):
+            held = [L.get(k) for k in keys]
+            row = [None if t is None else t.data_ptr() for t in held] + [cache.data_ptr()]
+            if hasattr(L["qkv"], "w8"):
+                row += [L[k].w_scale.data_ptr() for k in ("qkv", "o", "gate_up", "down")]
+            rows.append(row)
+        if rows != getattr(self, "_native_at", None):
+            names = (*keys, "kv_cache", "qkv_scale", "o_scale", "gate_up_scale", "down_scale")
+            self._native_w = []
+            for row in rows:
                 w = DenseLayerWeights()
-                w.ln1, w.qkv, w.o, w.ln2 = L["ln1"].data_ptr(), L["qkv"].data_ptr(), L["o"].data_ptr(), L["ln2"].data_ptr()
-                w.q_norm = L["q_norm"].data_ptr() if L.get("q_norm") is not None else None
-                w.k_norm = L["k_norm"].data_ptr() if L.get("k_norm") is not None else None
-                w.gate_up, w.down = (L[k].data_ptr() if k in L else None for k in ("gate_up", "down"))
-                w.kv_cache = self.kv_caches[l].data_ptr()
-                if hasattr(L["qkv"], "w8"):
-                    w.fp8 = 1
-                    w.qkv_scale, w.o_scale = L["qkv"].w_scale.data_ptr(), L["o"].w_scale.data_ptr()
-                    w.gate_up_scale, w.down_scale = L["gate_up"].w_scale.data_ptr(), L["down"].w_scale.data_ptr()
-                ws.append(w)
-            self._native_w = ws
-        return ws
+                for name, at in zip(names, row):
+                    setattr(w, name, at)
+                w.fp8 = int(len(row) == len(names))
+                self._native_w.append(w)
+            self._native_at = rows
+        return self._native_w
 
     def _native_step(self, ctx, T, qkv, attn, gate_up, act, act_kind, hidden=None, resid=None, normed=None):
         """The shapes, step metadata and activation buffers of one forward as the native layer
