@@ -151,9 +151,9 @@ def small_case(name: str):
             fn = lambda: A.prefill(q, pages, out, q_start=qs, num_reqs=B, tile_req=treq, tile_q0=tq0, **kw_)
         else:
             fn = lambda: A.decode(q, pages, out, splits=2, **kw_)
-    elif name in ("moe_small", "moe_few_small"):                # 128 rows an expert; 4
+    elif name in ("moe_small", "moe_few_small", "moe_many_small"):                # 128 rows an expert; 4; 512
         from . import moe as M
-        T, E, k, H, I = 2048 if name == "moe_small" else 64, 128, 8, 2048, 768
+        T, E, k, H, I = {"moe_small": 2048, "moe_few_small": 64, "moe_many_small": 8192}[name], 128, 8, 2048, 768
         x = torch.randn(T, H, device=dev).to(torch.bfloat16)
         wgu = (torch.randn(E, 2 * I, H, device=dev) * 0.05).to(torch.bfloat16)
         ids, w = M.router_topk(torch.randn(T, E, device=dev), k)
@@ -165,6 +165,11 @@ def small_case(name: str):
         # Llama-8B down projection at a mixed-step batch: 80 pair tiles on 74 CTA pairs, so the six
         # tiles of the ragged wave run as stream-K
         a = torch.randn(1280, 14336, device=dev, dtype=torch.bfloat16)
+        w = torch.randn(4096, 14336, device=dev, dtype=torch.bfloat16) * 0.05
+        fn = lambda: ops.gemm(a, w)
+    elif name == "gemm_shared_small":
+        # few tiles and a long K: every tile is shared by parts of K
+        a = torch.randn(300, 14336, device=dev, dtype=torch.bfloat16)
         w = torch.randn(4096, 14336, device=dev, dtype=torch.bfloat16) * 0.05
         fn = lambda: ops.gemm(a, w)
     elif name == "gemm_gated_small":
@@ -241,7 +246,7 @@ def main():
                     help="run one small case only (for profiler captures): "
                          "gemm_small | gemm_decode_small | gemv_small | gemm_cluster_small | sample_small | "
                          "prefill_small | decode_small | gdn_scan_small | "
-                         "gdn_decode_small | moe_small | moe_few_small | gemm_streamk_small | gemm_gated_small | "
+                         "gdn_decode_small | moe_small | moe_few_small | moe_many_small | gemm_streamk_small | gemm_shared_small | gemm_gated_small | "
                          "gemm_fp8_small | gemm_w4a16_small | gemm_nvfp4_small | gemm_nvfp4_prefill_small | "
                          "decode_d256_small | mla_decode_small | bias_prefill_small | bias_decode_small | delta_small")
     args = ap.parse_args()
