@@ -102,9 +102,9 @@ def test_w4a16_over_a_cluster(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(17, 2560, 9728), (34, 2560, 9728), (64, 4096, 14336), (32, 38016, 256), (33, 38016, 256)])
-def test_w4a16_results_off_16_bytes(M, N, K):
-    """Coarse parts of K and grids beyond one wave over a cluster, which writes results at multiples of 8 bytes; the stream form, which a K of
-    no 256 goes to, wants 16."""
+def test_w4a16_stream_and_cluster(M, N, K):
+    """Both sides of the lines between the two forms up to 64 rows: parts of K that are too coarse over a cluster, more rows
+    that make up for it, grids beyond one wave."""
     torch.manual_seed(14)
     packed = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device=DEV)
     sf = torch.randint(0x20, 0x60, (N, K // 16), dtype=torch.uint8, device=DEV)
@@ -112,7 +112,7 @@ def test_w4a16_results_off_16_bytes(M, N, K):
     a = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
     w64, a64 = Q.ref_dequant_nvfp4(packed, sf, g).double(), a.double()
     room = torch.empty(M * N + 4, dtype=torch.bfloat16, device=DEV)
-    for out in (Q.gemm_w4a16(a, packed, sf, g), Q.gemm_w4a16(a, packed, sf, g, out=room[4:].view(M, N))):
+    for out in (Q.gemm_w4a16(a, packed, sf, g), Q.gemm_w4a16(a, packed, sf, g, out=room[4:].view(M, N))):    # 8 bytes off: cluster
         assert ops.read_status() == 0
         assert _within_sum_error(out, a64, w64, a64 @ w64.t(), 2**-25 * w64.abs().sum(1))
     if N == 38016:
